@@ -155,7 +155,9 @@ struct sdlg_ctx {
     cudaEvent_t ev_mat = nullptr, ev_read = nullptr, ev_copy[2] = {nullptr, nullptr};
     bool copy_pending[2] = {false, false}, read_pending = false;
     int next_scratch = 0;
-    int64_t* h_small = nullptr;   // pinned: n_rec[5], status
+    int64_t* h_small = nullptr;   // pinned: the hit count on its way to the device
+    int64_t* h_run = nullptr;     // pinned: what the last run left for the host (RunWord)
+    int64_t h_run_words = 0;
     // the next batch, copied to the device while a run may still be going
     // (sdlg_stage_events) and installed by the next run from the hits: one
     // device allocation of x, y, z, idx, detid (hits each) and the offsets
@@ -180,7 +182,7 @@ struct sdlg_ctx {
     cudaGraphExec_t graph = nullptr;
     int graph_stop = -1, graph_flags = -1;
     // timing
-    cudaEvent_t ev[8];
+    cudaEvent_t ev[2];  // around a run
     Hooks hooks;
     int launches_per_run = 0;
     int last_stop = -1, last_flags = 0;
@@ -373,6 +375,8 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
     return SDLG_OK;
 }
 
+constexpr int64_t kZeroWords = 2 * kNumStages + 11 + 8;
+
 // (re)allocate the batch buffers for the current event sizes and capacities
 int ensure_buffers(sdlg_ctx* ctx) {
     const int n_mod = (int)ctx->detids.size();
@@ -410,10 +414,25 @@ int ensure_buffers(sdlg_ctx* ctx) {
     int rc;
 #define AL(ptr, n) if ((rc = dalloc(ctx, &(ptr), (n))) != SDLG_OK) return rc
     int64_t* small;
-    AL(small, 2 + kNumStages);
+    AL(small, 2 + kNumStamps);
     b.n_hit = small;
     b.n_gm_dev = small + 1;
-    b.n_rec = small + 2;
+    b.stamps = reinterpret_cast<unsigned long long*>(small + 2);
+    // the small counts that every run starts from zero
+    int64_t* zero;
+    AL(zero, kZeroWords);
+    b.n_rec = zero;
+    b.task = reinterpret_cast<unsigned long long*>(zero + kNumStages);
+    unsigned long long* cnt = b.task + kNumStages;
+    b.n_kept_sg = cnt;
+    b.n_pb_sg = cnt + 1;
+    b.n_kept = cnt + 3;
+    b.n_kept2 = cnt + 4;
+    b.n_keptf = cnt + 5;
+    b.n_pb_f = cnt + 6;
+    b.n_pb = cnt + 8;
+    b.status = reinterpret_cast<uint32_t*>(cnt + 10);
+    b.dbg = cnt + 11;
     float* fx; float* fy; float* fz; int32_t* fi; uint32_t* fd; int64_t* eo;
     AL(fx, H); AL(fy, H); AL(fz, H); AL(fi, H); AL(fd, H); AL(eo, ctx->n_ev + 1);
     b.in_x = fx; b.in_y = fy; b.in_z = fz; b.in_idx = fi; b.in_det = fd; b.ev_off = eo;
@@ -442,22 +461,15 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.bucket_cap = (int64_t)1 << 24;  // covers 2^32 candidates of one stage
     AL(b.bucket, b.bucket_cap);
     b.kept_cap = ctx->cap_kept;
-    AL(b.n_kept, 1);
     AL(b.passa, b.kept_cap);
     AL(b.kept, b.kept_cap);
-    AL(b.n_kept2, 1);
     AL(b.passf, b.kept_cap);
-    AL(b.n_keptf, 1);
     AL(b.pb, b.kept_cap);
-    AL(b.n_pb, 2);
     AL(b.sgpack, ctx->cap_obj[kSG] * PK_N);
     AL(b.sgouter, ctx->cap_obj[kSG] * 11);
     AL(b.sgfeat, ctx->cap_obj[kSG] * kFeatN);
     AL(b.mdpack, ctx->cap_obj[kMD] * kMdPack);
     AL(b.counters, ctx->n_ev * 110);
-    AL(b.status, 1);
-    AL(b.task, kNumStages);
-    AL(b.dbg, 8);
     int64_t mx = n_gm;
     for (int s = 0; s < kNumStages; ++s) mx = std::max(mx, ctx->cap_obj[s]);
     b.scan_tmp_cap = mx / 4096 + 16;
@@ -477,93 +489,81 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.olist_cap = 4 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);
     AL(b.olist, b.olist_cap);
 #undef AL
+    if (ctx->h_run_words < run_words(ctx->n_ev)) {
+        if (ctx->h_run) cudaFreeHost(ctx->h_run);
+        ctx->h_run = nullptr;
+        ctx->h_run_words = 0;
+        CK(cudaMallocHost((void**)&ctx->h_run, run_words(ctx->n_ev) * sizeof(int64_t)));
+        ctx->h_run_words = run_words(ctx->n_ev);
+    }
     CK(cudaMemcpyAsync(b.n_gm_dev, &n_gm, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->buffers_ok = true;
     return SDLG_OK;
 }
 
-// events recorded while a stream is captured must become graph nodes
-inline void record(cudaEvent_t e, cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(s, &st);
-    if (st == cudaStreamCaptureStatusActive) cudaEventRecordWithFlags(e, s, cudaEventRecordExternal);
-    else cudaEventRecord(e, s);
+void (*const kLaunch[kNumStages])(const BatchDev&, cudaStream_t, Hooks*) = {launch_md, launch_sg, launch_tl, launch_tp,
+                                                                            launch_tc};
+
+// what stages first..last accumulate into, set to zero
+void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
+    BatchDev& b = ctx->b;
+    ClearJobs j{};
+    const int64_t n_gm = b.n_gm;
+    // (a later stage's own run keeps the pass times of the stages before it)
+    j.stamps = first == 0 ? kNumStamps : kStampEnd + 1;
+    if (first == 0) {
+        j.add(b.n_rec, 2 * kZeroWords);
+        j.add(b.counters, (int64_t)b.n_ev * 110);
+        j.add(b.mod_hit, 2 * (n_gm + 1));
+        for (int st = 0; st < kNumStages; ++st) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
+        j.add(b.mlp_stats, sizeof(MlpStats) / 4);
+    } else {
+        const int ns = last - first + 1;
+        j.add(b.status, 1);
+        j.add(b.dbg, 16);
+        j.add(b.n_rec + first, 2 * ns);
+        j.add(b.task + first, 2 * ns);
+        // the survivor lists' counts: the segment stage's, then the tracklet stage's
+        if (first <= kSG) j.add(b.n_kept_sg, 6);
+        if (first <= kTL && last >= kTL) j.add(b.n_kept, 14);
+        // the counters these stages write (22 per stage in each event's 110:
+        // candidates, then objects): the triplet candidates are counted by the
+        // tracklet stage (Event.cc:547-596 loops over the segment lists)
+        for (int st = first; st <= last; ++st) {
+            const int skip = st == kTP ? 11 : 0;
+            j.add(b.counters + st * 22 + skip, 22 - skip, b.n_ev, 110);
+        }
+        if (first <= kTL && last >= kTL) j.add(b.counters + kTP * 22, 11, b.n_ev, 110);
+        for (int st = first; st <= last; ++st) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
+        if (first <= kTL && last >= kTL) j.add(b.mlp_stats, sizeof(MlpStats) / 4);
+    }
+    if (last >= kTL && first <= kTL) {
+        j.add(b.eoff, 2 * (n_gm + 1));
+        j.add(b.ecur, n_gm);
+    }
+    launch_clear(b, j, ctx->stream, &ctx->hooks);
 }
 
-// the full chain, enqueued on the context stream (also the body of the CUDA graph)
-void enqueue_chain(sdlg_ctx* ctx, int stop_after) {
+// stages first..last (from the hits when first is 0, else on the objects the
+// previous run left for the stages below first), enqueued on the context
+// stream; for first 0 also the body of the CUDA graph
+void enqueue_chain(sdlg_ctx* ctx, int first, int last) {
     BatchDev& b = ctx->b;
     cudaStream_t s = ctx->stream;
-    const int64_t n_gm = b.n_gm;
-    record(ctx->ev[0], s);
-    cudaMemsetAsync(b.status, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(b.dbg, 0, 8 * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.n_rec, 0, kNumStages * sizeof(int64_t), s);
-    cudaMemsetAsync(b.task, 0, kNumStages * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.counters, 0, b.n_ev * 110 * sizeof(uint32_t), s);
-    cudaMemsetAsync(b.mod_hit, 0, (n_gm + 1) * sizeof(int64_t), s);
-    for (int st = 0; st < kNumStages; ++st) cudaMemsetAsync(b.obj[st].mod_cnt, 0, (n_gm + 1) * sizeof(int64_t), s);
-    cudaMemsetAsync(b.mlp_stats, 0, sizeof(MlpStats), s);
     Hooks* h = &ctx->hooks;
-    h->timed = true;
     h->launches = 0;
-    launch_ingest(b, s, h);
-    record(ctx->ev[1], s);
-    if (stop_after >= kMD) launch_md(b, s, h);
-    record(ctx->ev[2], s);
-    if (stop_after >= kSG) launch_sg(b, s, h);
-    record(ctx->ev[3], s);
-    if (stop_after >= kTL) launch_tl(b, s, h);
-    record(ctx->ev[4], s);
-    if (stop_after >= kTP) launch_tp(b, s, h);
-    record(ctx->ev[5], s);
-    if (stop_after >= kTC) launch_tc(b, s, h);
-    record(ctx->ev[6], s);
-    ctx->launches_per_run = h->launches;
-    // status word and attempted appends for the host's overflow check
-    cudaMemcpyAsync(ctx->h_small, b.n_rec, kNumStages * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages, b.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages + 1, b.n_kept, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-}
-
-// stages first..last only (first >= 1), on the objects the previous run left
-// for the stages below first; no graph
-void enqueue_stages(sdlg_ctx* ctx, int first, int last) {
-    BatchDev& b = ctx->b;
-    cudaStream_t s = ctx->stream;
-    const int64_t n_gm = b.n_gm;
-    const int ns = last - first + 1;
-    record(ctx->ev[0], s);
-    cudaMemsetAsync(b.status, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(b.dbg, 0, 8 * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.n_rec + first, 0, ns * sizeof(int64_t), s);
-    cudaMemsetAsync(b.task + first, 0, ns * sizeof(unsigned long long), s);
-    // the counters these stages write (22 per stage in each event's 110:
-    // candidates, then objects): the triplet candidates are counted by the
-    // tracklet stage (Event.cc:547-596 loops over the segment lists)
-    auto zero_counters = [&](int at, int n) {
-        cudaMemset2DAsync(b.counters + at, 110 * sizeof(uint32_t), 0, n * sizeof(uint32_t), b.n_ev, s);
-    };
+    h->ts = stamp_bit(kStampStart);
+    enqueue_clear(ctx, first, last);
+    if (first == 0) launch_ingest(b, s, h);
     for (int st = first; st <= last; ++st) {
-        if (st == kTP) zero_counters(kTP * 22 + 11, 11);
-        else zero_counters(st * 22, 22);
+        h->ts |= stamp_bit(kStampStage + st);
+        kLaunch[st](b, s, h);
     }
-    if (first <= kTL && last >= kTL) zero_counters(kTP * 22, 11);
-    for (int st = first; st <= last; ++st) cudaMemsetAsync(b.obj[st].mod_cnt, 0, (n_gm + 1) * sizeof(int64_t), s);
-    if (first <= kTL && last >= kTL) cudaMemsetAsync(b.mlp_stats, 0, sizeof(MlpStats), s);
-    Hooks* h = &ctx->hooks;
-    h->timed = true;
-    h->launches = 0;
-    record(ctx->ev[1], s);
-    void (*fns[5])(const BatchDev&, cudaStream_t, Hooks*) = {launch_md, launch_sg, launch_tl, launch_tp, launch_tc};
-    for (int st = 0; st < kNumStages; ++st) {
-        if (st >= first && st <= last) fns[st](b, s, h);
-        record(ctx->ev[2 + st], s);
-    }
-    cudaMemcpyAsync(ctx->h_small, b.n_rec, kNumStages * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages, b.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages + 1, b.n_kept, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    // the status word, the attempted appends and the results' offsets for the host
+    h->ts |= stamp_bit(kStampEnd);
+    launch_finish(b, ctx->h_run, s, h);
+    ctx->launches_per_run = h->launches;
 }
 
 #ifdef SDL_DEVICE_CHECKS
@@ -579,36 +579,25 @@ int check_stage(sdlg_ctx* ctx, const char* what) {
     return SDLG_OK;
 }
 
-int launch_checked(sdlg_ctx* ctx, int stop_after) {
+int launch_checked(sdlg_ctx* ctx, int first, int last) {
     BatchDev& b = ctx->b;
     cudaStream_t s = ctx->stream;
-    const int64_t n_gm = b.n_gm;
-    cudaMemsetAsync(b.status, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(b.dbg, 0, 8 * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.n_rec, 0, kNumStages * sizeof(int64_t), s);
-    cudaMemsetAsync(b.task, 0, kNumStages * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.counters, 0, b.n_ev * 110 * sizeof(uint32_t), s);
-    cudaMemsetAsync(b.mod_hit, 0, (n_gm + 1) * sizeof(int64_t), s);
-    for (int st = 0; st < kNumStages; ++st) cudaMemsetAsync(b.obj[st].mod_cnt, 0, (n_gm + 1) * sizeof(int64_t), s);
-    cudaMemsetAsync(b.mlp_stats, 0, sizeof(MlpStats), s);
-    int rc;
-    record(ctx->ev[0], s);
     Hooks* h = &ctx->hooks;
-    h->timed = true;
+    int rc;
     h->launches = 0;
-    launch_ingest(b, s, h);
+    h->ts = stamp_bit(kStampStart);
+    enqueue_clear(ctx, first, last);
+    if (first == 0) launch_ingest(b, s, h);
     if ((rc = check_stage(ctx, "ingest"))) return rc;
-    record(ctx->ev[1], s);
-    void (*fns[5])(const BatchDev&, cudaStream_t, Hooks*) = {launch_md, launch_sg, launch_tl, launch_tp, launch_tc};
     static const char* names[5] = {"MD", "SG", "TL", "TP", "TC"};
-    for (int st = 0; st < 5; ++st) {
-        if (stop_after >= st) fns[st](b, s, h);
+    for (int st = first; st <= last; ++st) {
+        h->ts |= stamp_bit(kStampStage + st);
+        kLaunch[st](b, s, h);
         if ((rc = check_stage(ctx, names[st]))) return rc;
-        record(ctx->ev[2 + st], s);
     }
-    cudaMemcpyAsync(ctx->h_small, b.n_rec, kNumStages * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages, b.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ctx->h_small + kNumStages + 1, b.n_kept, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    h->ts |= stamp_bit(kStampEnd);
+    launch_finish(b, ctx->h_run, s, h);
+    ctx->launches_per_run = h->launches;
     return SDLG_OK;
 }
 #endif
@@ -618,11 +607,13 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
     ctx->ran = true;
     wait_readback(ctx);
 #ifdef SDL_DEVICE_CHECKS
-    return launch_checked(ctx, stop_after);
+    return launch_checked(ctx, 0, stop_after);
 #endif
     const bool use_graph = !(flags & SDLG_FLAG_NO_GRAPH);
     if (!use_graph) {
-        enqueue_chain(ctx, stop_after);
+        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+        enqueue_chain(ctx, 0, stop_after);
+        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         CK(cudaGetLastError());
         return SDLG_OK;
     }
@@ -633,7 +624,7 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
         }
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_chain(ctx, stop_after);
+        enqueue_chain(ctx, 0, stop_after);
         CK(cudaStreamEndCapture(ctx->stream, &g));
         cudaError_t e = cudaGraphInstantiate(&ctx->graph, g, 0);
         cudaGraphDestroy(g);
@@ -641,7 +632,9 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
         ctx->graph_stop = stop_after;
         ctx->graph_flags = flags;
     }
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     CK(cudaGraphLaunch(ctx->graph, ctx->stream));
+    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     return SDLG_OK;
 }
 
@@ -649,7 +642,7 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
 int finish(sdlg_ctx* ctx) {
     for (int attempt = 0; attempt < 16; ++attempt) {  // one overflowing stage per attempt at worst
         CK(cudaStreamSynchronize(ctx->stream));
-        const uint32_t status = (uint32_t)(ctx->h_small[kNumStages] & 0xffffffffu);
+        const uint32_t status = (uint32_t)(ctx->h_run[kRunStatus] & 0xffffffff);
         if (status & kStatusUnknownModule) {
             // new detIds: extend the module table and re-run (modules created on
             // demand, Event.cc:54-78)
@@ -681,12 +674,12 @@ int finish(sdlg_ctx* ctx) {
         bool grew = false;
         for (int s = 0; s < kNumStages; ++s) {
             if (status & (1u << s)) {
-                ctx->cap_obj[s] = std::max<int64_t>(ctx->cap_obj[s] * 2, ctx->h_small[s] + ctx->h_small[s] / 4 + 4096);
+                ctx->cap_obj[s] = std::max<int64_t>(ctx->cap_obj[s] * 2, ctx->h_run[kRunRec + s] + ctx->h_run[kRunRec + s] / 4 + 4096);
                 grew = true;
             }
         }
         if (status & kStatusOverflowKept) {
-            const int64_t need = ctx->h_small[kNumStages + 1];
+            const int64_t need = ctx->h_run[kRunKept];
             ctx->cap_kept = std::max<int64_t>(ctx->cap_kept * 2, need + need / 4 + 4096);
             grew = true;
         }
@@ -814,13 +807,7 @@ int sdlg_create(sdlg_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_mat, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_read, cudaEventDisableTiming);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ctx->ev_copy[k], cudaEventDisableTiming);
-    for (int k = 0; k < 8 && e == cudaSuccess; ++k) e = cudaEventCreate(&ctx->ev[k]);
-    for (int k = 0; k < kNumStages && e == cudaSuccess; ++k) {
-        e = cudaEventCreate(&ctx->hooks.enum_start[k]);
-        if (e == cudaSuccess) e = cudaEventCreate(&ctx->hooks.enum_stop[k]);
-    }
-    for (int k = 0; k < 3; ++k)
-        if (e == cudaSuccess) e = cudaEventCreate(&ctx->hooks.tl_mid[k]);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreate(&ctx->ev[k]);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_small, 16 * sizeof(int64_t));
     // the host libm's float functions for the cut arithmetic (once per process / device)
     const char* lm_err = nullptr;
@@ -880,13 +867,8 @@ int sdlg_destroy(sdlg_ctx* ctx) {
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->gather_stream) cudaStreamDestroy(ctx->gather_stream);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
-    for (int k = 0; k < 8; ++k) if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
-    for (int k = 0; k < kNumStages; ++k) {
-        if (ctx->hooks.enum_start[k]) cudaEventDestroy(ctx->hooks.enum_start[k]);
-        if (ctx->hooks.enum_stop[k]) cudaEventDestroy(ctx->hooks.enum_stop[k]);
-    }
-    for (int k = 0; k < 3; ++k)
-        if (ctx->hooks.tl_mid[k]) cudaEventDestroy(ctx->hooks.tl_mid[k]);
+    for (int k = 0; k < 2; ++k) if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
+    if (ctx->h_run) cudaFreeHost(ctx->h_run);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SDLG_OK;
@@ -1329,10 +1311,12 @@ int sdlg_run_stages(sdlg_ctx* ctx, int first, int last, int flags) {
     ctx->last_flags = flags;
     wait_readback(ctx);
 #ifdef SDL_DEVICE_CHECKS
-    int rc = launch_checked(ctx, last);
+    int rc = launch_checked(ctx, first, last);
     if (rc) return rc;
 #else
-    enqueue_stages(ctx, first, last);
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+    enqueue_chain(ctx, first, last);
+    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     CK(cudaGetLastError());
 #endif
     return finish(ctx);
@@ -1599,12 +1583,24 @@ int sdlg_get_counters(sdlg_ctx* ctx, int64_t event, uint32_t* out110) {
     return SDLG_OK;
 }
 
+// ms between two stamps of the last run; a stamp that the run did not reach
+// (a stage not run) counts as the next one that it did
+static float stamp_ms(const sdlg_ctx* ctx, int from, int to) {
+    const int64_t* t = ctx->h_run + kRunStamps;
+    if (from >= kStampStage && from < kStampEnd)
+        while (from < kStampEnd && !t[from]) ++from;
+    if (to >= kStampStage && to < kStampEnd)
+        while (to < kStampEnd && !t[to]) ++to;
+    return t[from] && t[to] && t[to] > t[from] ? (float)(1e-6 * (double)(t[to] - t[from])) : 0.f;
+}
+
 int sdlg_last_times(sdlg_ctx* ctx, float* out7) {
     if (!ctx || !out7) return SDLG_ERR_ARG;
     cudaSetDevice(ctx->device);
-    CK(cudaEventSynchronize(ctx->ev[6]));
-    for (int k = 0; k < 6; ++k) CK(cudaEventElapsedTime(&out7[k], ctx->ev[k], ctx->ev[k + 1]));
-    CK(cudaEventElapsedTime(&out7[6], ctx->ev[0], ctx->ev[6]));
+    CK(cudaEventSynchronize(ctx->ev[1]));
+    CK(cudaEventElapsedTime(&out7[6], ctx->ev[0], ctx->ev[1]));  // (an error when nothing has run)
+    out7[0] = stamp_ms(ctx, kStampStart, kStampStage);
+    for (int st = 0; st < kNumStages; ++st) out7[1 + st] = stamp_ms(ctx, kStampStage + st, kStampStage + st + 1);
     return SDLG_OK;
 }
 
@@ -1612,11 +1608,11 @@ int sdlg_last_kernel_times(sdlg_ctx* ctx, float* out5) {
     if (!ctx || !out5) return SDLG_ERR_ARG;
     if (!ctx->ran) return fail(ctx, SDLG_ERR_NO_EVENTS, "chain not run");
     cudaSetDevice(ctx->device);
+    CK(cudaStreamSynchronize(ctx->stream));
     for (int k = 0; k < kNumStages; ++k) {
         out5[k] = 0.f;
         if (k > ctx->last_stop) continue;
-        CK(cudaEventSynchronize(ctx->hooks.enum_stop[k]));
-        CK(cudaEventElapsedTime(&out5[k], ctx->hooks.enum_start[k], ctx->hooks.enum_stop[k]));
+        out5[k] = stamp_ms(ctx, kStampEnum + k, kStampEnumEnd + k);
     }
     return SDLG_OK;
 }
@@ -1676,11 +1672,11 @@ int sdlg_last_tl_pass_times4(sdlg_ctx* ctx, float* out4) {
     out4[0] = out4[1] = out4[2] = out4[3] = 0.f;
     if (ctx->last_stop < kTL) return SDLG_OK;
     cudaSetDevice(ctx->device);
-    CK(cudaEventSynchronize(ctx->hooks.enum_stop[kTL]));
-    CK(cudaEventElapsedTime(&out4[0], ctx->hooks.enum_start[kTL], ctx->hooks.tl_mid[0]));
-    CK(cudaEventElapsedTime(&out4[1], ctx->hooks.tl_mid[0], ctx->hooks.tl_mid[1]));
-    CK(cudaEventElapsedTime(&out4[2], ctx->hooks.tl_mid[1], ctx->hooks.tl_mid[2]));
-    CK(cudaEventElapsedTime(&out4[3], ctx->hooks.tl_mid[2], ctx->hooks.enum_stop[kTL]));
+    CK(cudaStreamSynchronize(ctx->stream));
+    out4[0] = stamp_ms(ctx, kStampEnum + kTL, kStampTlMid);
+    out4[1] = stamp_ms(ctx, kStampTlMid, kStampTlMid + 1);
+    out4[2] = stamp_ms(ctx, kStampTlMid + 1, kStampTlMid + 2);
+    out4[3] = stamp_ms(ctx, kStampTlMid + 2, kStampEnumEnd + kTL);
     return SDLG_OK;
 }
 

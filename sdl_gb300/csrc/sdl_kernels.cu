@@ -48,7 +48,20 @@ constexpr int kScanThreads = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanBlock = kScanThreads * kScanItems;
 
-__device__ __forceinline__ bool halted(const BatchDev& b) { return (*b.status & kStatusHalt) != 0; }
+// the launch's device time stamps (none for most launches)
+__device__ __forceinline__ void stamp(const BatchDev& b) {
+    if (b.ts == 0u || (blockIdx.x | blockIdx.y | threadIdx.x) != 0u) return;
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    for (uint32_t m = b.ts; m; m &= m - 1u) b.stamps[__ffs(m) - 1] = t;
+}
+
+// the start of every kernel behind a stage that can overflow: true when the
+// run stops there
+__device__ __forceinline__ bool halted(const BatchDev& b) {
+    stamp(b);
+    return (*b.status & kStatusHalt) != 0;
+}
 
 // add v to *addr with one atomic per group of lanes sharing the address;
 // every lane of the warp must call it
@@ -1887,6 +1900,7 @@ __device__ __forceinline__ uint32_t* counter_at(const BatchDev& b, int ev, int s
 }
 
 __global__ void k_md_count(BatchDev b) {
+    stamp(b);
     const int n_mod = b.geo.n_mod;
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
         const bool in = g < b.n_gm;
@@ -2293,11 +2307,58 @@ unsigned grid_for(int64_t n, int threads, int cap_blocks) {
     return (unsigned)g;
 }
 
-inline void rec_event(cudaEvent_t e, cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(s, &st);
-    if (st == cudaStreamCaptureStatusActive) cudaEventRecordWithFlags(e, s, cudaEventRecordExternal);
-    else cudaEventRecord(e, s);
+// the argument of the next launch: b with the stamps set since the last
+// one, which this launch takes
+BatchDev take(const BatchDev& b, Hooks* h) {
+    BatchDev c = b;
+    c.ts = 0;
+    if (h) {
+        c.ts = h->ts;
+        h->ts = 0;
+        h->launches += 1;
+    }
+    return c;
+}
+inline void mark(Hooks* h, int s) {
+    if (h) h->ts |= stamp_bit(s);
+}
+
+__global__ void __launch_bounds__(256) k_clear(BatchDev b, ClearJobs j) {
+    if (b.ts && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        for (int k = 0; k < j.stamps; ++k) b.stamps[k] = 0ull;
+    stamp(b);
+    const int q = blockIdx.y;
+    const int64_t w = j.words[q], n = w * j.rows[q];
+    uint32_t* p = j.p[q];
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    if (j.rows[q] > 1) {
+        for (int64_t i = t; i < n; i += stride) p[i / w * j.pitch[q] + i % w] = 0u;
+        return;
+    }
+    int64_t done = 0;
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+        for (int64_t i = t; i < n / 4; i += stride) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+        done = n / 4 * 4;
+    }
+    for (int64_t i = done + t; i < n; i += stride) p[i] = 0u;
+}
+
+__global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
+    stamp(b);
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    if (t < kNumStages) host[kRunRec + t] = b.n_rec[t];
+    if (t == kNumStages) host[kRunStatus] = (int64_t)*b.status;
+    if (t == kNumStages + 1) host[kRunKept] = (int64_t)max(*b.n_kept, *b.n_kept_sg);
+    // (this kernel's own stamp is written by the thread that copies it)
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        for (int k = 0; k < kNumStamps; ++k) host[kRunStamps + k] = (int64_t)b.stamps[k];
+    const int64_t per = b.n_ev + 1;
+    for (int64_t i = t; i < kNumStages * per; i += stride) {
+        const int st = (int)(i / per);
+        host[kRunOffsets + i] = b.obj[st].mod_cnt[(i - st * per) * b.geo.n_mod];
+    }
+    uint32_t* c = reinterpret_cast<uint32_t*>(host + kRunOffsets + kNumStages * per);
+    for (int64_t i = t; i < (int64_t)b.n_ev * 110; i += stride) c[i] = b.counters[i];
 }
 
 void scan_h(const BatchDev& b, int64_t* data, const int64_t* n_ptr, int64_t cap, cudaStream_t s, Hooks* h) {
@@ -2319,15 +2380,13 @@ void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h, bool layer_coun
         default: ninner_ptr = ((b.flags & kFlagTCFromTP) ? b.obj[kTP] : b.obj[kTL]).mod_cnt + b.n_gm;
     }
     scan_h(b, b.cand[st], ninner_ptr, b.cand_cap[st], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(b, st);
-    if (h) h->launches += 1;
-    if (h && h->timed) rec_event(h->enum_start[st], s);
-    k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(b);
-    if (h && h->timed) rec_event(h->enum_stop[st], s);
-    if (layer_counters) k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, st);
+    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st);
+    mark(h, kStampEnum + st);
+    k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
+    mark(h, kStampEnumEnd + st);
+    if (layer_counters) k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), st);
     scan_h(b, b.obj[st].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(b, st);
-    if (h) h->launches += layer_counters ? 3 : 2;
+    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st);
 }
 
 // device-to-device copies of 4-byte words (job blockIdx.y), 16 bytes at a
@@ -2355,49 +2414,44 @@ __global__ void __launch_bounds__(256) k_copy_words(CopyJobs j) {
 
 void launch_ingest(const BatchDev& b, cudaStream_t s, Hooks* h) {
     const unsigned g = grid_for(b.n_hit_cap, 256, b.n_sm * 16);
-    k_hit_map<<<g, 256, 0, s>>>(b);
+    k_hit_map<<<g, 256, 0, s>>>(take(b, h));
     scan_h(b, b.mod_hit, b.n_gm_dev, b.n_gm, s, h);
-    k_hit_perm<<<g, 256, 0, s>>>(b);
-    k_hit_scatter<<<g, 256, 0, s>>>(b);
-    if (h) h->launches += 3;
+    k_hit_perm<<<g, 256, 0, s>>>(take(b, h));
+    k_hit_scatter<<<g, 256, 0, s>>>(take(b, h));
 }
 
 void launch_md(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    k_md_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b);
-    if (h) h->launches += 1;
+    k_md_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
     enum_and_group<MDStage>(b, s, h);
 }
 
 void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    k_md_pack<<<b.n_sm * 8, 256, 0, s>>>(b);
-    if (h) h->launches += 1;
+    k_md_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     if (b.flags & kFlagSGLayers) {
         // Event.cc:793-821 increments no per-layer counter
-        k_sg_count_layers<<<b.n_sm * 8, 256, 0, s>>>(b);
-        if (h) h->launches += 1;
+        k_sg_count_layers<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
         enum_and_group<SGLayerStage>(b, s, h, false);
         return;
     }
-    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kMD, kSG);
-    k_sg_count<<<b.n_sm * 8, 256, 0, s>>>(b);
-    k_sg_olist_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b);
+    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kMD, kSG);
+    k_sg_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    k_sg_olist_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
     scan_h(b, b.toff, b.n_gm_dev, b.n_gm, s, h);
-    k_sg_olist_fill<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b);
+    k_sg_olist_fill<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
     scan_h(b, b.cand[kSG], b.obj[kMD].mod_cnt + b.n_gm, b.cand_cap[kSG], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(b, kSG);
-    if (h) h->launches += 5;
+    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kSG);
     // first cuts -> survivor list -> whole algorithm (k_sg_enum_a, k_sg_b)
-    if (h && h->timed) rec_event(h->enum_start[kSG], s);
-    cudaMemsetAsync(b.n_kept, 0, sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.n_pb, 0, 2 * sizeof(unsigned long long), s);
-    k_sg_enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(b);
-    k_sg_b<1><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(b);
-    k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(b);
-    if (h && h->timed) rec_event(h->enum_stop[kSG], s);
-    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kSG);
+    mark(h, kStampEnum + kSG);
+    BatchDev l = b;  // with this list's own counts
+    l.n_kept = b.n_kept_sg;
+    l.n_pb = b.n_pb_sg;
+    k_sg_enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
+    k_sg_b<1><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
+    k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
+    mark(h, kStampEnumEnd + kSG);
+    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG);
     scan_h(b, b.obj[kSG].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(b, kSG);
-    if (h) h->launches += 5;
+    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kSG);
 }
 
 // the join index of stage st's objects (segments or tracklets), keyed by
@@ -2406,48 +2460,41 @@ static void join_index(const BatchDev& b, int st, cudaStream_t s, Hooks* h, bool
     int64_t* off = second ? b.joff2 : b.joff;
     cudaMemsetAsync(off, 0, (b.obj[kMD].cap + 1) * sizeof(int64_t), s);
     cudaMemsetAsync(second ? b.jcur2 : b.jcur, 0, b.obj[kMD].cap * sizeof(int32_t), s);
-    k_join_count<<<b.n_sm * 8, 256, 0, s>>>(b, st, second);
+    k_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
     scan_h(b, off, b.obj[kMD].mod_cnt + b.n_gm, b.obj[kMD].cap, s, h);
-    k_join_scatter<<<b.n_sm * 8, 256, 0, s>>>(b, st, second);
-    if (h) h->launches += 2;
+    k_join_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
 }
 
 void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     // conn sums over segment counts serve the tracklet enumeration and the
     // triplet candidate counters (Event.cc:547-596 loops over the same lists)
-    k_sg_pack<<<b.n_sm * 8, 256, 0, s>>>(b);
-    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kSG, kTP);
+    k_sg_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG, kTP);
     if (b.flags & kFlagTLLayers) {
-        k_tl_count_layers<<<b.n_sm * 8, 256, 0, s>>>(b);
+        k_tl_count_layers<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     } else if (b.flags & kFlagTLNav) {
         join_index(b, kSG, s, h);  // segments by inner MD: the outward lists
-        k_tl_count_nav<<<b.n_sm * 8, 256, 0, s>>>(b);
+        k_tl_count_nav<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     } else {
-        cudaMemsetAsync(b.eoff, 0, (b.n_gm + 1) * sizeof(int64_t), s);
-        cudaMemsetAsync(b.ecur, 0, b.n_gm * sizeof(int32_t), s);
-        k_tl_count<<<b.n_sm * 8, 256, 0, s>>>(b);
+        k_tl_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     }
-    if (h) h->launches += 3;
     scan_h(b, b.cand[kTL], b.obj[kSG].mod_cnt + b.n_gm, b.cand_cap[kTL], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(b, kTL);
-    if (h) h->launches += 1;
+    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kTL);
     // module-map candidates: the module-pair tiles (k_tl_enum_tiles)
     const bool tiles = !(b.flags & (kFlagTLLayers | kFlagTLNav));
     if (tiles) {
-        k_tl_tile_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b);
+        k_tl_tile_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
         scan_h(b, b.eoff, b.n_gm_dev, b.n_gm, s, h);
         scan_h(b, b.toff, b.n_gm_dev, b.n_gm, s, h);
-        k_sg_end_scatter<<<b.n_sm * 8, 256, 0, s>>>(b);
-        k_tile_map<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b);
-        if (h) h->launches += 3;
+        k_sg_end_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+        k_tile_map<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
     }
-    if (h && h->timed) rec_event(h->enum_start[kTL], s);
+    mark(h, kStampEnum + kTL);
     // enumeration + phase A -> survivor list (-> the pre-filter -> kept list)
     // -> phase B1 -> phase B2
-    cudaMemsetAsync(b.n_kept, 0, sizeof(unsigned long long), s);
-    if (tiles) k_tl_enum_tiles<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b);
-    else k_tl_enum_a<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b);
-    if (h && h->timed) rec_event(h->tl_mid[0], s);
+    if (tiles) k_tl_enum_tiles<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
+    else k_tl_enum_a<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
+    mark(h, kStampTlMid + 0);
     // the list phase B1 reads: the enumeration's, the pre-filter's kept
     // entries, then what phase B2's single-precision filter leaves of it (not
     // with DefaultNm1, whose phase B2 keeps what fails the deltaBeta cut)
@@ -2455,40 +2502,35 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     unsigned long long* count = b.n_kept;
     const bool mlp = (b.flags & kFlagMLP) != 0;
     if (mlp) {
-        cudaMemsetAsync(b.n_kept2, 0, sizeof(unsigned long long), s);
-        k_tl_prefilter<<<b.n_sm * kPfCtasPerSm, kMlpTile, 0, s>>>(b);
+        k_tl_prefilter<<<b.n_sm * kPfCtasPerSm, kMlpTile, 0, s>>>(take(b, h));
         list = b.kept;
         count = b.n_kept2;
     }
-    if (h && h->timed) rec_event(h->tl_mid[1], s);
+    mark(h, kStampTlMid + 1);
     const bool filt = !(b.flags & (kFlagTLNm1 | kFlagNoB2Filter));
     if (filt) {
-        cudaMemsetAsync(b.n_keptf, 0, sizeof(unsigned long long), s);
-        cudaMemsetAsync(b.n_pb, 0, 2 * sizeof(unsigned long long), s);
-        k_tl_b2f<0><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b, list, count);
-        k_tl_b2f<1><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b, nullptr, nullptr);
-        k_tl_b2f<2><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b, nullptr, nullptr);
+        BatchDev l = b;  // with the deferred entries' own counts
+        l.n_pb = b.n_pb_f;
+        k_tl_b2f<0><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), list, count);
+        k_tl_b2f<1><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), nullptr, nullptr);
+        k_tl_b2f<2><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), nullptr, nullptr);
         list = b.passf;
         count = b.n_keptf;
     }
-    if (h && h->timed) rec_event(h->tl_mid[2], s);
-    cudaMemsetAsync(b.n_pb, 0, 2 * sizeof(unsigned long long), s);
-    k_tl_b1<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b, list, count);
-    k_tl_b2<kB2BBBB><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b);
-    k_tl_b2<kB2Others><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(b);
-    if (h) h->launches += 3 + (mlp ? 1 : 0) + (filt ? 3 : 0);
-    if (h && h->timed) rec_event(h->enum_stop[kTL], s);
-    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kTL);
+    mark(h, kStampTlMid + 2);
+    k_tl_b1<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h), list, count);
+    k_tl_b2<kB2BBBB><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
+    k_tl_b2<kB2Others><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
+    mark(h, kStampEnumEnd + kTL);
+    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTL);
     scan_h(b, b.obj[kTL].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(b, kTL);
-    if (h) h->launches += 3;
+    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kTL);
 }
 
 
 void launch_tp(const BatchDev& b, cudaStream_t s, Hooks* h) {
     join_index(b, kSG, s, h);
-    k_tp_count<<<b.n_sm * 8, 256, 0, s>>>(b);
-    if (h) h->launches += 1;
+    k_tp_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     enum_and_group<TPStage>(b, s, h);
 }
 
@@ -2499,22 +2541,20 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
             join_index(b, kSG, s, h);        // segments by inner MD
             join_index(b, kTP, s, h, true);  // triplets by innermost MD
         }
-        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kTP, -1);
-        k_tc_count_tp<<<b.n_sm * 8, 256, 0, s>>>(b);
-        if (h) h->launches += 2;
+        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTP, -1);
+        k_tc_count_tp<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
         if (map) enum_and_group<TCTPMapStage>(b, s, h);
         else enum_and_group<TCTPStage>(b, s, h);
         return;
     }
     join_index(b, kTL, s, h);
     if (b.flags & kFlagTCFromTL) {
-        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(b, kTL, -1);
-        k_tc_count_tl<<<b.n_sm * 8, 256, 0, s>>>(b);
+        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTL, -1);
+        k_tc_count_tl<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     } else {
-        k_tc_count<<<b.n_sm * 8, 256, 0, s>>>(b);
-        k_tc_cand_counter<<<grid_for(b.n_ev, 128, 1024), 128, 0, s>>>(b);
+        k_tc_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+        k_tc_cand_counter<<<grid_for(b.n_ev, 128, 1024), 128, 0, s>>>(take(b, h));
     }
-    if (h) h->launches += 2;
     enum_and_group<TCStage>(b, s, h);
 }
 
@@ -2703,6 +2743,16 @@ cudaError_t set_libm_tables(const LibmTab* t) { return cudaMemcpyToSymbol(c_libm
 void launch_libm_eval(int fn, uint32_t start, int64_t n, float* out, int n_sm, cudaStream_t s) {
     if (n <= 0) return;
     k_libm_eval<<<grid_for(n, 256, n_sm * 16), 256, 0, s>>>(fn, start, n, out);
+}
+
+void launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h) {
+    int64_t most = 1;
+    for (int k = 0; k < j.count; ++k) most = most > j.words[k] * j.rows[k] ? most : j.words[k] * j.rows[k];
+    k_clear<<<dim3(grid_for((most + 3) / 4, 256, b.n_sm * 4), (unsigned)j.count), 256, 0, s>>>(take(b, h), j);
+}
+
+void launch_finish(const BatchDev& b, int64_t* host, cudaStream_t s, Hooks* h) {
+    k_finish<<<grid_for((int64_t)b.n_ev * 110, 256, b.n_sm), 256, 0, s>>>(take(b, h), host);
 }
 
 void launch_copy_words(const CopyJobs& j, int n_sm, cudaStream_t s) {

@@ -89,19 +89,74 @@ struct BatchDev {
     int4* pb;                      // candidates through phase B1: (inner, outer, algorithm, muls bits), BBBB
                                    //   from the front, the others from the back
     unsigned long long* n_pb;      // [2]: BBBB entries, other entries (kept_cap in all)
+    // the segment first pass's counts (as n_kept, n_pb) and the B2 filter's
+    // deferred entries (as n_pb): each use has its own, cleared with the rest
+    // of the run's counts (launch_clear)
+    unsigned long long* n_kept_sg;
+    unsigned long long* n_pb_sg;
+    unsigned long long* n_pb_f;
     int n_sm;
     unsigned long long* dbg;       // bounds-check record (debug builds): count, line, index, limit
+    // device clock (%globaltimer, ns) at the start of chosen kernels: a
+    // launch's ts is a mask of the stamps its first thread writes
+    unsigned long long* stamps;    // kNumStamps
+    uint32_t ts;
 };
 
-// Host-side instrumentation of the launches: events around each stage's
-// candidate-evaluation kernel and a count of kernels launched.
-struct Hooks {
-    cudaEvent_t enum_start[kNumStages] = {};
-    cudaEvent_t enum_stop[kNumStages] = {};
-    cudaEvent_t tl_mid[3] = {};  // after phase A, after the pre-filter, after the B2 filter
-    bool timed = false;
-    int launches = 0;
+// Device time stamps of a run.  An event node in a CUDA graph costs about
+// 4.5 us (a kernel node 0.8 us), so the stage and pass boundaries are stamps
+// that the kernels behind them write; only the whole run is between events.
+enum Stamp : int {
+    kStampStart = 0,                                 // the run's first kernel
+    kStampStage = 1,                                 // + st: the first kernel of stage st
+    kStampEnd = kStampStage + kNumStages,            // the run's last kernel
+    kStampEnum = kStampEnd + 1,                      // + st: stage st's candidate evaluation
+    kStampEnumEnd = kStampEnum + kNumStages,         // + st: the kernel after it
+    kStampTlMid = kStampEnumEnd + kNumStages,        // + 0..2: after phase A, after the pre-filter, after the B2 filter
+    kNumStamps = kStampTlMid + 3
 };
+constexpr uint32_t stamp_bit(int s) { return 1u << s; }
+
+// Host-side record of the launches: kernels launched, and the stamps the
+// next one takes.
+struct Hooks {
+    int launches = 0;
+    uint32_t ts = 0;
+};
+
+// Buffers set to zero at the start of a run (4-byte words; rows > 1: a
+// column block of a matrix), all by one kernel: a memset node in a CUDA graph
+// costs 4.6 us.
+constexpr int kClearJobs = 16;
+struct ClearJobs {
+    uint32_t* p[kClearJobs];
+    int64_t words[kClearJobs];
+    int64_t rows[kClearJobs];
+    int64_t pitch[kClearJobs];
+    int count;
+    int stamps;  // the first so many stamps too
+    void add(void* q, int64_t n_words, int64_t n_rows = 1, int64_t n_pitch = 0) {
+        p[count] = static_cast<uint32_t*>(q);
+        words[count] = n_words;
+        rows[count] = n_rows;
+        pitch[count++] = n_pitch;
+    }
+};
+void launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h);
+
+// What the host reads after a run, written by the run's last kernel to
+// pinned memory (8-byte words): the appends attempted per stage, the status
+// word, the longest survivor list, the stamps, the object offsets of every
+// event (n_ev + 1 per stage), the per-layer counters (110 x n_ev 4-byte words).
+enum RunWord : int {
+    kRunRec = 0,
+    kRunStatus = kNumStages,
+    kRunKept = kNumStages + 1,
+    kRunStamps = kNumStages + 2,
+    kRunOffsets = kRunStamps + kNumStamps
+};
+constexpr int64_t run_words(int64_t n_ev) { return kRunOffsets + kNumStages * (n_ev + 1) + 55 * n_ev; }
+void launch_finish(const BatchDev& b, int64_t* host, cudaStream_t s, Hooks* h);
 
 // stage launchers (each enqueues its kernels on stream s)
 void launch_ingest(const BatchDev& b, cudaStream_t s, Hooks* h);

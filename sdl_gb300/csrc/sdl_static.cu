@@ -190,13 +190,14 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.flags = 0;
     // the array keeps the previous call's contents: zero what the kernels
     // accumulate into
-    cudaMemsetAsync(b.status, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(b.n_rec, 0, kNumStages * sizeof(int64_t), s);
-    cudaMemsetAsync(b.task, 0, kNumStages * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.dbg, 0, 8 * sizeof(unsigned long long), s);
-    cudaMemsetAsync(b.counters, 0, 110 * sizeof(uint32_t), s);
-    cudaMemsetAsync(b.mod_hit, 0, (geo.n_mod + 1) * sizeof(int64_t), s);
-    cudaMemsetAsync(O.mod_cnt, 0, (geo.n_mod + 1) * sizeof(int64_t), s);
+    ClearJobs j{};
+    j.add(b.status, 1);
+    j.add(b.n_rec, 2 * kNumStages);
+    j.add(b.task, 2 * (kNumStages + 8));  // and dbg behind it
+    j.add(b.counters, 110);
+    j.add(b.mod_hit, 2 * (geo.n_mod + 1));
+    j.add(O.mod_cnt, 2 * (geo.n_mod + 1));
+    launch_clear(b, j, s, nullptr);
     k_static_init<<<1, 32, 0, s>>>(b, n_hits);
     launch_ingest(b, s, nullptr);
     launch_md(b, s, nullptr);
