@@ -376,7 +376,7 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
     return SDLG_OK;
 }
 
-constexpr int64_t kZeroWords = 2 * kNumStages + 11 + 8;
+constexpr int64_t kZeroWords = 2 * kNumStages + 12 + 8;
 
 // (re)allocate the batch buffers for the current event sizes and capacities
 int ensure_buffers(sdlg_ctx* ctx) {
@@ -415,10 +415,9 @@ int ensure_buffers(sdlg_ctx* ctx) {
     int rc;
 #define AL(ptr, n) if ((rc = dalloc(ctx, &(ptr), (n))) != SDLG_OK) return rc
     int64_t* small;
-    AL(small, 2 + kNumStamps);
+    AL(small, 1 + kNumStamps);
     b.n_hit = small;
-    b.n_gm_dev = small + 1;
-    b.stamps = reinterpret_cast<unsigned long long*>(small + 2);
+    b.stamps = reinterpret_cast<unsigned long long*>(small + 1);
     // the small counts that every run starts from zero
     int64_t* zero;
     AL(zero, kZeroWords);
@@ -432,8 +431,9 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.n_keptf = cnt + 5;
     b.n_pb_f = cnt + 6;
     b.n_pb = cnt + 8;
-    b.status = reinterpret_cast<uint32_t*>(cnt + 10);
-    b.dbg = cnt + 11;
+    b.n_cand_tl = cnt + 10;
+    b.status = reinterpret_cast<uint32_t*>(cnt + 11);
+    b.dbg = cnt + 12;
     float* fx; float* fy; float* fz; int32_t* fi; uint32_t* fd; int64_t* eo;
     AL(fx, H); AL(fy, H); AL(fz, H); AL(fi, H); AL(fd, H); AL(eo, ctx->n_ev + 1);
     b.in_x = fx; b.in_y = fy; b.in_z = fz; b.in_idx = fi; b.in_det = fd; b.ev_off = eo;
@@ -451,7 +451,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
         AL(R.i, C); AL(R.j, C); AL(R.g, C); AL(R.rank, C); AL(R.f, C * std::max(1, nf[s]));
     }
     b.cand_cap[kMD] = n_gm;
-    b.cand_cap[kSG] = ctx->cap_obj[kMD];
+    b.cand_cap[kSG] = std::max(n_gm, ctx->cap_obj[kMD]);  // global modules, or mini-doublets (SDLG_FLAG_SG_LAYERS)
     b.cand_cap[kTL] = ctx->cap_obj[kSG];
     b.cand_cap[kTP] = ctx->cap_obj[kSG];
     b.cand_cap[kTC] = std::max(ctx->cap_obj[kTL], ctx->cap_obj[kTP]);  // tracklets, or triplets (SDLG_FLAG_TC_FROM_TP)
@@ -473,8 +473,8 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.counters, ctx->n_ev * 110);
     int64_t mx = n_gm;
     for (int s = 0; s < kNumStages; ++s) mx = std::max(mx, ctx->cap_obj[s]);
-    b.scan_tmp_cap = mx / 4096 + 16;
-    AL(b.scan_tmp, b.scan_tmp_cap);
+    b.scan_cap = scan_words(n_gm, mx);
+    AL(b.scan_state, kScanSlots * b.scan_cap);
     AL(b.joff, ctx->cap_obj[kMD] + 1);
     AL(b.jcur, ctx->cap_obj[kMD]);
     AL(b.jidx, std::max(ctx->cap_obj[kSG], ctx->cap_obj[kTL]));
@@ -497,8 +497,6 @@ int ensure_buffers(sdlg_ctx* ctx) {
         CK(cudaMallocHost((void**)&ctx->h_run, run_words(ctx->n_ev) * sizeof(int64_t)));
         ctx->h_run_words = run_words(ctx->n_ev);
     }
-    CK(cudaMemcpyAsync(b.n_gm_dev, &n_gm, sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
     ctx->buffers_ok = true;
     return SDLG_OK;
 }
@@ -527,7 +525,7 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
         j.add(b.task + first, 2 * ns);
         // the survivor lists' counts: the segment stage's, then the tracklet stage's
         if (first <= kSG) j.add(b.n_kept_sg, 6);
-        if (first <= kTL && last >= kTL) j.add(b.n_kept, 14);
+        if (first <= kTL && last >= kTL) j.add(b.n_kept, 16);
         // the counters these stages write (22 per stage in each event's 110:
         // candidates, then objects): the triplet candidates are counted by the
         // tracklet stage (Event.cc:547-596 loops over the segment lists)
@@ -539,6 +537,7 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
         for (int st = first; st <= last; ++st) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
         if (first <= kTL && last >= kTL) j.add(b.mlp_stats, sizeof(MlpStats) / 4);
     }
+    j.add(b.scan_state, 2 * kScanSlots * b.scan_cap);
     if (last >= kTL && first <= kTL) {
         j.add(b.eoff, 2 * (n_gm + 1));
         j.add(b.ecur, n_gm);
@@ -667,6 +666,7 @@ int finish(sdlg_ctx* ctx) {
             if (rc) return rc;
             continue;
         }
+        if (status & kStatusScan) return fail(ctx, SDLG_ERR_CUDA, "a prefix sum's wait gave up; results discarded");
         if (status & kStatusMlpTimeout)
             return fail(ctx, SDLG_ERR_CUDA, "tracklet pre-filter: a tensor-core wait gave up; results discarded");
         if (!(status & kStatusHalt)) return SDLG_OK;

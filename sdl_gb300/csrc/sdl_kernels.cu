@@ -44,9 +44,6 @@ __device__ __forceinline__ int64_t checked_idx(int64_t i, int64_t lim, int line,
 constexpr int kWarp = 32;
 constexpr int kEnumThreads = 256;
 constexpr int kTaskDefault = 256;  // candidates per warp task unless tuned
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 8;
-constexpr int kScanBlock = kScanThreads * kScanItems;
 
 // the launch's device time stamps (none for most launches)
 __device__ __forceinline__ void stamp(const BatchDev& b) {
@@ -107,118 +104,6 @@ __device__ __forceinline__ void obj_bounds(const BatchDev& b, int64_t nobj, int6
     }
 }
 
-// ------------------------------------------------------------------ scan
-struct ScanArgs {
-    int64_t* data;      // cap + 1 entries
-    const int64_t* n_ptr;
-    int64_t cap;
-    int64_t* blk;
-    int64_t blk_cap;
-    unsigned long long* dbg;
-};
-
-__global__ void k_scan_reduce(ScanArgs b) {
-    const int64_t n = min(*b.n_ptr, b.cap);
-    const int64_t base = (int64_t)blockIdx.x * kScanBlock;
-    if (base >= n) return;
-    int64_t s = 0;
-    for (int k = 0; k < kScanItems; ++k) {
-        const int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
-        if (i < n) s += AT(b.data, i, b.cap + 1);
-    }
-    for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    __shared__ int64_t ws[32];  // one slot per lane of warp 0
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        int64_t v = threadIdx.x < kScanThreads / 32 ? ws[threadIdx.x] : 0;
-        for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) AT(b.blk, blockIdx.x, b.blk_cap) = v;
-    }
-}
-
-__global__ void k_scan_blocks(ScanArgs b) {
-    const int64_t n = min(*b.n_ptr, b.cap);
-    const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-    __shared__ int64_t carry;
-    __shared__ int64_t ws[32];
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int64_t base = 0; base < nb; base += blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        const int64_t v = i < nb ? AT(b.blk, i, b.blk_cap) : 0;
-        int64_t x = v;
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) ws[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            int64_t t = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t y = __shfl_up_sync(0xffffffffu, t, o);
-                if (lane >= o) t += y;
-            }
-            ws[lane] = t;
-        }
-        __syncthreads();
-        const int64_t incl = x + (w ? ws[w - 1] : 0);
-        if (i < nb) AT(b.blk, i, b.blk_cap) = carry + incl - v;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry += incl;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) AT(b.data, n, b.cap + 1) = carry;
-}
-
-__global__ void k_scan_apply(ScanArgs b) {
-    const int64_t n = min(*b.n_ptr, b.cap);
-    const int64_t base = (int64_t)blockIdx.x * kScanBlock;
-    if (base >= n) return;
-    // each thread owns kScanItems consecutive elements
-    int64_t v[kScanItems];
-    int64_t s = 0;
-    const int64_t my = base + (int64_t)threadIdx.x * kScanItems;
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = (my + k < n) ? AT(b.data, my + k, b.cap + 1) : 0;
-        s += v[k];
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int64_t x = s;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    __shared__ int64_t ws[32];  // one slot per lane of warp 0
-    if (lane == 31) ws[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int64_t t = lane < kScanThreads / 32 ? ws[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        if (lane < kScanThreads / 32) ws[lane] = t;
-    }
-    __syncthreads();
-    int64_t run = AT(b.blk, blockIdx.x, b.blk_cap) + x - s + (w ? ws[w - 1] : 0);
-    for (int k = 0; k < kScanItems; ++k) {
-        if (my + k < n) AT(b.data, my + k, b.cap + 1) = run;
-        run += v[k];
-    }
-}
-
-void scan(const BatchDev& bd, int64_t* data, const int64_t* n_ptr, int64_t cap, cudaStream_t s) {
-    const int64_t nb = (cap + kScanBlock - 1) / kScanBlock;
-    if (nb <= 0) return;
-    ScanArgs a{data, n_ptr, cap, bd.scan_tmp, bd.scan_tmp_cap, bd.dbg};
-    k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(a);
-    k_scan_blocks<<<1, 1024, 0, s>>>(a);
-    k_scan_apply<<<(unsigned)nb, kScanThreads, 0, s>>>(a);
-}
-
 // array sizes
 __device__ __forceinline__ int64_t H(const BatchDev& b) { return b.n_hit_cap; }
 __device__ __forceinline__ int64_t NG1(const BatchDev& b) { return (int64_t)b.n_gm + 1; }
@@ -238,6 +123,150 @@ __device__ __forceinline__ int64_t NCP(const BatchDev& b) {
     return v > 0 ? v : 1;
 }
 __device__ __forceinline__ const ModDev& MOD(const BatchDev& b, int64_t m) { return AT(b.geo.mod, m, NM(b)); }
+
+// ------------------------------------------------------------------ scan
+// Exclusive prefix sums in one pass (decoupled look-back, after Merrill and
+// Garland 2016): each CTA takes the next tile from a counter, so that every
+// tile before its own has been started, publishes the tile's sum, adds up
+// its predecessors' words (a sum, or already a whole prefix) 32 at a time and
+// publishes its prefix.  What is summed is computed where it is loaded (the
+// candidate counts with their layer counters) and what is derived from the
+// prefix is written where it is stored (offsets, bucket and tile tables), so
+// one launch does what took a count kernel, three scan kernels and a table
+// kernel: 17 of a run's launches instead of 85, and of a 2.3k-hit event's
+// 646 us in kernels those took 290.
+//
+// A word holds its kind in the top two bits (0: not there yet, 1: the tile's
+// sum, 2: the prefix through the tile).  The words are cleared with the run's
+// other counts, one slot per scan of a run.  A wait for a predecessor is
+// bounded: past kScanPolls the CTA sets kStatusScan, which halts the run.
+constexpr int kScanThreads = 256;
+constexpr int kScanPolls = 1 << 20;
+constexpr unsigned long long kScanSum = 1ull << 62, kScanPrefix = 2ull << 62, kScanValue = (1ull << 62) - 1;
+
+__device__ __forceinline__ unsigned long long scan_peek(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void scan_post(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// the sum of the tiles before `tile` (value q of kK per tile; whole warp)
+template <int kK>
+__device__ __forceinline__ int64_t scan_lookback(const unsigned long long* words, int64_t tile, int q, bool& ok) {
+    const int lane = threadIdx.x & 31;
+    int64_t sum = 0;
+    for (int64_t t = tile - 1;; t -= kWarp) {
+        const int64_t k = t - lane;
+        unsigned long long w = kScanPrefix;  // before the first tile: a prefix of 0
+        for (int polls = 0;; ++polls) {
+            if (k >= 0) w = scan_peek(words + k * kK + q);
+            if (!__any_sync(0xffffffffu, (w >> 62) == 0ull)) break;
+            if (polls == kScanPolls) {
+                ok = false;
+                return 0;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, (w >> 62) == 2ull);
+        const int last = m ? __ffs(m) - 1 : kWarp;  // the nearest prefix
+        int64_t v = lane <= last ? (int64_t)(w & kScanValue) : 0;
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        sum += v;
+        if (m) return sum;
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
+    constexpr int kK = Op::kVals, kI = Op::kItems, kWarps = kScanThreads / kWarp;
+    constexpr int kTile = kScanThreads * kI;
+    if (halted(b)) return;
+    Op::begin(b);
+    const int64_t n = Op::size(b);
+    const int64_t ntile = n > 0 ? (n + kTile - 1) / kTile : 1;
+    unsigned long long* ticket = b.scan_state + (int64_t)slot * b.scan_cap;
+    unsigned long long* words = ticket + 1;
+    __shared__ int64_t s_tile, s_pre[kK], s_sum[kK][kWarps];
+    __shared__ int s_ok;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            s_tile = (int64_t)atomicAdd(ticket, 1ull);
+            s_ok = 1;
+        }
+        __syncthreads();
+        const int64_t tile = s_tile;
+        if (tile >= ntile) return;
+        const int64_t base = tile * kTile + w * (kWarp * kI) + lane;
+        int64_t v[kI][kK], e[kI][kK], carry[kK];
+#pragma unroll
+        for (int k = 0; k < kI; ++k) Op::load(b, base + k * kWarp, base + k * kWarp < n, v[k]);
+#pragma unroll
+        for (int q = 0; q < kK; ++q) {
+            carry[q] = 0;
+#pragma unroll
+            for (int k = 0; k < kI; ++k) {
+                int64_t x = v[k][q];
+#pragma unroll
+                for (int o = 1; o < kWarp; o <<= 1) {
+                    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                e[k][q] = carry[q] + x - v[k][q];
+                carry[q] += __shfl_sync(0xffffffffu, x, kWarp - 1);
+            }
+            if (lane == 0) s_sum[q][w] = carry[q];
+        }
+        __syncthreads();
+        int64_t total[kK], before[kK];
+#pragma unroll
+        for (int q = 0; q < kK; ++q) {
+            total[q] = before[q] = 0;
+#pragma unroll
+            for (int j = 0; j < kWarps; ++j) {
+                if (j < w) before[q] += s_sum[q][j];
+                total[q] += s_sum[q][j];
+            }
+        }
+        if (w == 0) {
+            bool ok = true;
+#pragma unroll
+            for (int q = 0; q < kK; ++q)
+                if (lane == 0 && tile > 0) scan_post(words + tile * kK + q, kScanSum | (unsigned long long)total[q]);
+#pragma unroll
+            for (int q = 0; q < kK; ++q) {
+                const int64_t pre = tile > 0 && ok ? scan_lookback<kK>(words, tile, q, ok) : 0;
+                if (lane == 0) {
+                    s_pre[q] = pre;
+                    if (ok) scan_post(words + tile * kK + q, kScanPrefix | (unsigned long long)(pre + total[q]));
+                }
+            }
+            if (lane == 0 && !ok) {
+                s_ok = 0;
+                atomicOr(b.status, kStatusScan);
+            }
+        }
+        __syncthreads();
+        if (!s_ok) return;
+#pragma unroll
+        for (int k = 0; k < kI; ++k) {
+            const int64_t i = base + k * kWarp;
+#pragma unroll
+            for (int q = 0; q < kK; ++q) e[k][q] += s_pre[q] + before[q];
+            if (i < n) Op::store(b, i, e[k], v[k]);
+        }
+        if (tile == ntile - 1 && threadIdx.x == 0) {
+#pragma unroll
+            for (int q = 0; q < kK; ++q) total[q] += s_pre[q];
+            Op::total(b, n, total);
+        }
+    }
+}
+struct ScanOp {
+    __device__ static void begin(const BatchDev&) {}
+};
 
 // ------------------------------------------------------------------ ingest
 __global__ void k_hit_map(BatchDev b) {
@@ -269,8 +298,18 @@ __global__ void k_hit_map(BatchDev b) {
     }
 }
 
+// hits per global module -> offsets
+struct ScanHits : ScanOp {
+    static constexpr int kVals = 1, kItems = 4;
+    __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
+    __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) { v[0] = in ? AT(b.mod_hit, i, NG1(b)) : 0; }
+    __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t*) { AT(b.mod_hit, i, NG1(b)) = e[0]; }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(b.mod_hit, n, NG1(b)) = t[0]; }
+};
+
 // sorted position of every input hit in a known module -> hit_perm
 __global__ void k_hit_perm(BatchDev b) {
+    if (halted(b)) return;
     const int64_t n = *b.n_hit;
     for (int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; h < n; h += (int64_t)gridDim.x * blockDim.x) {
         const int gm = AT(b.hit_gm, h, H(b));
@@ -282,6 +321,7 @@ __global__ void k_hit_perm(BatchDev b) {
 // the sorted hit arrays, one thread per sorted position (coalesced writes;
 // the input hit is gathered through hit_perm)
 __global__ void k_hit_scatter(BatchDev b) {
+    if (halted(b)) return;
     const int64_t n = min(AT(b.mod_hit, b.n_gm, NG1(b)), *b.n_hit);  // hits in known modules
     for (int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += (int64_t)gridDim.x * blockDim.x) {
         const int64_t h = AT(b.hit_perm, pos, H(b));
@@ -311,6 +351,10 @@ __global__ void k_hit_scatter(BatchDev b) {
 }
 
 // ------------------------------------------------------------------ helpers
+__device__ __forceinline__ uint32_t* counter_at(const BatchDev& b, int ev, int st, int kind, int slot) {
+    return &AT(b.counters, (int64_t)ev * 110 + st * 22 + kind * 11 + slot, (int64_t)b.n_ev * 110);
+}
+
 __device__ __forceinline__ P3 hit(const BatchDev& b, int64_t k) {
     P3 p;
     p.x = AT(b.hx, k, H(b)); p.y = AT(b.hy, k, H(b)); p.z = AT(b.hz, k, H(b));
@@ -454,12 +498,11 @@ __device__ __forceinline__ bool sg_pair(const BatchDev& b, int a, int bmd, bool 
 }
 
 // segment candidates along the module map (Event.cc:445-522): candidate q of
-// inner MD a is an MD of a connected module, in connection-list order; the
-// outer mini-doublet of candidate q of inner MD a
-__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int a, int64_t q) {
-    const int n_mod = b.geo.n_mod;
-    const int g1 = OG(b, kMD, a);
+// an inner MD of global module g1 is an MD of a connected module, in
+// connection-list order
+__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int g1, int64_t q) {
     if (AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap) return AT(b.olist, AT(b.toff, g1, NG1(b)) + q, b.olist_cap);  // k_sg_olist_fill
+    const int n_mod = b.geo.n_mod;
     const int ev = ev_of(b, g1), m1 = g1 - ev * n_mod;
     int pref;
     const int k = conn_entry(b, ev, m1, q, pref);
@@ -632,37 +675,41 @@ struct TCStage {
     __device__ static int group_of(const BatchDev& b, int t) { return OG(b, kTL, t); }
 };
 
-// inner-object count of a stage (device), clamped to the inner capacity
+// inner-object count of a stage (device), clamped to the inner capacity; the
+// module-map segments' inner objects are the global modules (a module's
+// mini-doublets share one outer list, so the candidates of all of them are
+// consecutive)
+__device__ __forceinline__ int64_t n_objects(const BatchDev& b, int st) { return min(OFF(b, st, b.n_gm), b.obj[st].cap); }
 __device__ __forceinline__ int64_t n_inner(const BatchDev& b, int st) {
     switch (st) {
         case kMD: return b.n_gm;
-        case kSG: return min(OFF(b, kMD, b.n_gm), b.obj[kMD].cap);
+        case kSG: return (b.flags & kFlagSGLayers) ? n_objects(b, kMD) : b.n_gm;
         case kTL:
-        case kTP: return min(OFF(b, kSG, b.n_gm), b.obj[kSG].cap);
+        case kTP: return n_objects(b, kSG);
         default:  // track candidates: tracklets, or triplets (createTrackCandidatesFromTriplets)
-            return (b.flags & kFlagTCFromTP) ? min(OFF(b, kTP, b.n_gm), b.obj[kTP].cap)
-                                             : min(OFF(b, kTL, b.n_gm), b.obj[kTL].cap);
+            return n_objects(b, (b.flags & kFlagTCFromTP) ? kTP : kTL);
     }
 }
 
-// bucket table of stage st's scanned candidate offsets
-__global__ void k_cand_buckets(BatchDev b, int st) {
-    if (halted(b)) return;
-    const int64_t nobj = n_inner(b, st);
-    if (nobj <= 0) return;
-    const int64_t* off = b.cand[st];
-    const int64_t offlim = b.cand_cap[st] + 1;
-    const int64_t total = AT(off, nobj, offlim);
-    if (!buckets_ok(b, total)) return;
-    const int64_t nb = (total + (1ll << kBucketShift) - 1) >> kBucketShift;
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid == 0) AT(b.bucket, nb, b.bucket_cap) = (int)(nobj - 1);
-    for (int64_t s = tid; s < nobj; s += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t lo = AT(off, s, offlim), hi = AT(off, s + 1, offlim);
-        for (int64_t k = (lo + (1ll << kBucketShift) - 1) >> kBucketShift; (k << kBucketShift) < hi; ++k)
-            AT(b.bucket, k, b.bucket_cap) = (int)s;
+// the scan of stage st's candidate counts: offsets per inner object, and the
+// bucket table (an inner object names the buckets that start in it)
+template <int st>
+struct ScanCand : ScanOp {
+    static constexpr int kVals = 1, kItems = 2;
+    __device__ static int64_t size(const BatchDev& b) { return n_inner(b, st); }
+    __device__ static void put(const BatchDev& b, int64_t i, int64_t e, int64_t v) {
+        AT(b.cand[st], i, b.cand_cap[st] + 1) = e;
+        for (int64_t k = (e + (1ll << kBucketShift) - 1) >> kBucketShift; (k << kBucketShift) < e + v; ++k)
+            if (k < b.bucket_cap) AT(b.bucket, k, b.bucket_cap) = (int)i;
     }
-}
+    __device__ static void put_total(const BatchDev& b, int64_t n, int64_t t) {
+        AT(b.cand[st], n, b.cand_cap[st] + 1) = t;
+        const int64_t nb = (t + (1ll << kBucketShift) - 1) >> kBucketShift;
+        if (n > 0 && nb < b.bucket_cap) AT(b.bucket, nb, b.bucket_cap) = (int)(n - 1);
+    }
+    __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t* v) { put(b, i, e[0], v[0]); }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { put_total(b, n, t[0]); }
+};
 
 // A warp's accepted objects, collected in shared memory and appended to the
 // stage's record list in batches of up to kRecBuf: one atomic on the list's
@@ -830,6 +877,8 @@ __global__ void k_sg_pack(BatchDev b) {
             if (k != 6) AT(b.sgouter, k * C + s, 11 * C) = v[fo[k]];
         AT(b.sgouter, 6 * C + s, 11 * C) = 0.1f / v[PK_LRT];  // the PV-offset term of an outer segment
         AT(b.sgouter, 10 * C + s, 11 * C) = v[PK_UY];
+        // segments per module of their outer mini-doublet (ScanTlFront)
+        atomicAdd((unsigned long long*)&AT(b.eoff, __float_as_int(v[PK_G2]), NG1(b)), 1ull);
         float4* dst = reinterpret_cast<float4*>(&AT(b.sgpack, s * PK_N, b.obj[kSG].cap * PK_N));
         for (int k = 0; k < PK_N / 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         // the pre-filter's feature records (inner role, outer role)
@@ -1085,21 +1134,27 @@ __device__ __forceinline__ int64_t tile_count(int64_t na, int64_t nb) {
     return (na > 0 && nb > 0) ? ((na + kTileA - 1) / kTileA) * ((nb + kWarp - 1) / kWarp) : 0;
 }
 
-// tiles per global module (eoff still holds the counts of segments ending there)
-__global__ void k_tl_tile_count(BatchDev b) {
-    if (halted(b)) return;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < b.n_gm; g += (int64_t)gridDim.x * blockDim.x)
-        AT(b.toff, g, NG1(b)) = tile_count(AT(b.eoff, g, NG1(b)), AT(b.conn_sum, g, b.n_gm));
-}
-
-// the segments by the global module of their outer mini-doublet (eoff scanned)
+// the segments by the global module of their outer mini-doublet (eoff
+// scanned), and the reference's tracklet candidate counters (Event.cc:635-663)
 __global__ void k_sg_end_scatter(BatchDev b) {
     if (halted(b)) return;
+    const int n_mod = b.geo.n_mod;
     const int64_t n = n_inner(b, kTL);
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const int g2 = OG(b, kMD, OJ(b, kSG, s));
-        const int64_t pos = AT(b.eoff, g2, NG1(b)) + atomicAdd(&AT(b.ecur, g2, b.n_gm), 1);
-        AT(b.eidx, pos, b.obj[kSG].cap) = (int)s;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s - threadIdx.x < n; s += (int64_t)gridDim.x * blockDim.x) {
+        const bool in = s < n;
+        int64_t c = 0;
+        int ev = 0, slot = 0;
+        if (in) {
+            const int g2 = OG(b, kMD, OJ(b, kSG, s));
+            const int64_t pos = AT(b.eoff, g2, NG1(b)) + atomicAdd(&AT(b.ecur, g2, b.n_gm), 1);
+            AT(b.eidx, pos, b.obj[kSG].cap) = (int)s;
+            c = AT(b.conn_sum, g2, b.n_gm);
+            const int g1 = OG(b, kSG, s);
+            ev = ev_of(b, g1);
+            slot = MOD(b, g1 - ev * n_mod).layer_slot;
+        }
+        const bool act = in && c != 0;
+        warp_add(act ? counter_at(b, ev, kTL, 0, slot) : b.counters, (uint32_t)c, act);
     }
 }
 
@@ -1119,18 +1174,6 @@ __device__ __forceinline__ int tile_module(const BatchDev& b, int64_t t) {
     const int p = lo + lane;
     const unsigned m = __ballot_sync(0xffffffffu, p <= hi && AT(b.toff, p, NG1(b)) <= t);
     return lo + 31 - __clz(m);
-}
-
-// tile -> global module map of the module-pair tiles (toff scanned); not
-// built when the tiles exceed its capacity (the enumeration then searches toff)
-__global__ void k_tile_map(BatchDev b) {
-    if (halted(b)) return;
-    const int64_t ntile = AT(b.toff, b.n_gm, NG1(b));
-    if (ntile > b.tile_cap) return;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t1 = AT(b.toff, g + 1, NG1(b));
-        for (int64_t t = AT(b.toff, g, NG1(b)); t < t1; ++t) AT(b.tile_gm, t, b.tile_cap) = (int)g;
-    }
 }
 
 // The outer object of lane q - q0 of a tile whose outer block starts at entry
@@ -1326,8 +1369,12 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
             int a = 0, bmd = 0;
             bool pass = false, ob = false;
             if (c < end) {
-                a = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
-                bmd = sg_outer_md(b, a, c - AT(off, a, offlim));
+                // candidate c of module g: inner MD (c - off) / sum, entry (c - off) % sum of g's outer list
+                const int g = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
+                const int64_t l = c - AT(off, g, offlim), sum = AT(b.conn_sum, g, b.n_gm);
+                const int64_t k = l <= 0xffffffffll ? (int64_t)((uint32_t)l / (uint32_t)sum) : l / sum;
+                a = (int)(OFF(b, kMD, g) + k);
+                bmd = sg_outer_md(b, g, l - k * sum);
                 (void)IX(bmd, b.obj[kMD].cap);
                 float fv[6];
                 const MDRec orec = md_rec(b, bmd);
@@ -1423,11 +1470,7 @@ __global__ void __launch_bounds__(kMlpTile, kPfCtasPerSm) k_tl_prefilter(BatchDe
     if (halted(b)) return;
     const int64_t n = min((int64_t)*b.n_kept, b.kept_cap);
     const int64_t ntile = (n + kMlpTile - 1) / kMlpTile;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int64_t nobj = n_inner(b, kTL);
-        const int64_t cand = nobj > 0 ? AT(b.cand[kTL], nobj, b.cand_cap[kTL] + 1) : 0;
-        atomicAdd(&b.mlp_stats->candidates, (unsigned long long)cand);
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&b.mlp_stats->candidates, *b.n_cand_tl);
     if ((int64_t)blockIdx.x >= ntile) return;
     const int lane = threadIdx.x & 31;
     mlp_setup(sm, b.mlp_pack);
@@ -1859,23 +1902,27 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
     }
 }
 
-// per-module object counts of a stage -> layer counters (before the scan)
-__global__ void k_obj_counters(BatchDev b, int st) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = g < b.n_gm;
-        uint32_t v = 0;
+// per-module object counts of a stage -> offsets, and the layer counters
+template <int st, bool kCounters>
+struct ScanObj : ScanOp {
+    static constexpr int kVals = 1, kItems = 2;
+    __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
+    __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
+        v[0] = in ? OFF(b, st, g) : 0;
+        if (!kCounters) return;
+        const bool act = v[0] != 0;
         int ev = 0, slot = 0;
-        if (in) {
-            v = (uint32_t)OFF(b, st, g);
+        if (act) {
             ev = ev_of(b, g);
-            slot = MOD(b, g - (int64_t)ev * n_mod).layer_slot;
+            slot = MOD(b, g - (int64_t)ev * b.geo.n_mod).layer_slot;
         }
-        const bool act = in && v != 0;
-        warp_add(act ? &AT(b.counters, (int64_t)ev * 110 + st * 22 + 11 + slot, (int64_t)b.n_ev * 110) : b.counters, v, act);
+        warp_add(act ? counter_at(b, ev, st, 1, slot) : b.counters, (uint32_t)v[0], act);
     }
-}
+    __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t*) {
+        AT(b.obj[st].mod_cnt, g, NG1(b)) = e[0];
+    }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(b.obj[st].mod_cnt, n, NG1(b)) = t[0]; }
+};
 
 __global__ void k_scatter(BatchDev b, int st) {
     if (halted(b)) return;
@@ -1895,163 +1942,210 @@ __global__ void k_scatter(BatchDev b, int st) {
 }
 
 // ------------------------------------------------------------------ counts
-__device__ __forceinline__ uint32_t* counter_at(const BatchDev& b, int ev, int st, int kind, int slot) {
-    return &AT(b.counters, (int64_t)ev * 110 + st * 22 + kind * 11 + slot, (int64_t)b.n_ev * 110);
-}
-
-__global__ void k_md_count(BatchDev b) {
-    stamp(b);
-    const int n_mod = b.geo.n_mod;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = g < b.n_gm;
+// mini-doublet candidates of a module: lower x upper hits (Event.cc:257-301)
+struct ScanMdCand : ScanCand<kMD> {
+    static constexpr int kItems = 1;
+    __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
         int64_t c = 0;
         int ev = 0, slot = 0;
         if (in) {
             ev = ev_of(b, g);
-            const ModDev& m = MOD(b, g - (int64_t)ev * n_mod);
+            const ModDev& m = MOD(b, g - (int64_t)ev * b.geo.n_mod);
             if (m.lower && m.partner >= 0) {
-                const int64_t pg = (int64_t)ev * n_mod + m.partner;
+                const int64_t pg = (int64_t)ev * b.geo.n_mod + m.partner;
                 c = (AT(b.mod_hit, g + 1, NG1(b)) - AT(b.mod_hit, g, NG1(b))) *
                     (AT(b.mod_hit, pg + 1, NG1(b)) - AT(b.mod_hit, pg, NG1(b)));
             }
             slot = m.layer_slot;
-            AT(b.cand[kMD], g, b.cand_cap[kMD] + 1) = c;
         }
-        const bool act = in && c != 0;
+        const bool act = c != 0;
         warp_add(act ? counter_at(b, ev, kMD, 0, slot) : b.counters, (uint32_t)c, act);
+        v[0] = c;
     }
-}
+};
 
-// per lower module: running sums of the object counts of its connected
-// modules (stage src) -> conn_pref per entry and conn_sum per module; the
-// reference's candidate counters of stage cst get n_obj(g) * conn_sum(g).
+// module g's connection entries: running sums of the connected modules'
+// object counts (stage src) -> conn_pref and conn_first per entry, conn_sum
+// per module (returned); the reference's candidate counters of stage cst get
+// n_obj(g) * conn_sum(g).  Every lane of the warp calls it.  Eight entries at
+// a time: their indices, then their offsets, so that a list of a dozen
+// costs two rounds of dependent loads instead of twelve.
+__device__ __forceinline__ int64_t conn_sums(const BatchDev& b, int64_t g, bool in, int src, int cst) {
+    constexpr int kC = 8;
+    const int n_mod = b.geo.n_mod;
+    int64_t sum = 0, cand = 0;
+    int ev = 0, slot = 0;
+    if (in) {
+        ev = ev_of(b, g);
+        const int m = (int)(g - (int64_t)ev * n_mod);
+        const int k0 = AT(b.geo.conn_off, m, NM(b) + 1), k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
+        const int64_t pbase = (int64_t)ev * b.geo.n_conn, ebase = (int64_t)ev * n_mod;
+        for (int k = k0; k < k1; k += kC) {
+            int idx[kC], first[kC], cnt[kC];
+#pragma unroll
+            for (int j = 0; j < kC; ++j) idx[j] = k + j < k1 ? AT(b.geo.conn_idx, k + j, NC(b)) : -1;
+#pragma unroll
+            for (int j = 0; j < kC; ++j) {
+                first[j] = idx[j] >= 0 ? (int)OFF(b, src, ebase + idx[j]) : 0;
+                cnt[j] = idx[j] >= 0 ? (int)OFF(b, src, ebase + idx[j] + 1) - first[j] : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < kC; ++j) {
+                if (idx[j] < 0) break;
+                AT(b.conn_pref, pbase + k + j, NCP(b)) = (int32_t)sum;
+                AT(b.conn_first, pbase + k + j, NCP(b)) = first[j];
+                sum += cnt[j];
+            }
+        }
+        AT(b.conn_sum, g, b.n_gm) = sum;
+        if (cst >= 0) cand = (OFF(b, src, g + 1) - OFF(b, src, g)) * sum;
+        slot = MOD(b, m).layer_slot;
+    }
+    const bool act = cand != 0;
+    warp_add(act ? counter_at(b, ev, cst, 0, slot) : b.counters, (uint32_t)cand, act);
+    return sum;
+}
 __global__ void k_conn_sum(BatchDev b, int src, int cst) {
     if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = g < b.n_gm;
-        int64_t sum = 0, cand = 0;
-        int ev = 0, slot = 0;
-        if (in) {
-            ev = ev_of(b, g);
-            const int m = (int)(g - (int64_t)ev * n_mod);
-            const int k0 = AT(b.geo.conn_off, m, NM(b) + 1), k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
-            const int64_t pbase = (int64_t)ev * b.geo.n_conn;
-            const int64_t ebase = (int64_t)ev * n_mod;
-            for (int k = k0; k < k1; ++k) {
-                AT(b.conn_pref, pbase + k, NCP(b)) = (int32_t)sum;
-                const int64_t g2 = ebase + AT(b.geo.conn_idx, k, NC(b));
-                const int64_t o2 = OFF(b, src, g2);
-                AT(b.conn_first, pbase + k, NCP(b)) = (int32_t)o2;
-                sum += OFF(b, src, g2 + 1) - o2;
-            }
-            AT(b.conn_sum, g, b.n_gm) = sum;
-            cand = (OFF(b, src, g + 1) - OFF(b, src, g)) * sum;
-            slot = MOD(b, m).layer_slot;
-        }
-        const bool act = in && cand != 0 && cst >= 0;
-        warp_add(act ? counter_at(b, ev, cst, 0, slot) : b.counters, (uint32_t)cand, act);
-    }
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x)
+        (void)conn_sums(b, g, g < b.n_gm, src, cst);
 }
 
-// The outer lists of the segment candidates, written out: for every global
-// module g holding mini-doublets, the mini-doublets of g's connected modules
-// in connection-list order (entry q of g's list at olist[toff[g] + q]), so
-// that a candidate finds its outer mini-doublet with one load.  toff holds
-// the list lengths, then (scanned) the offsets; the lists are not written
-// when they exceed olist_cap (the candidates then search the connection list).
-__global__ void k_sg_olist_count(BatchDev b) {
-    if (halted(b)) return;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < b.n_gm; g += (int64_t)gridDim.x * blockDim.x)
-        AT(b.toff, g, NG1(b)) = OFF(b, kMD, g + 1) > OFF(b, kMD, g) ? AT(b.conn_sum, g, b.n_gm) : 0;
-}
+// The front of the module-map segment stage: the connection sums over the
+// mini-doublets, the offsets of the outer lists (toff: for every global
+// module holding mini-doublets, the mini-doublets of its connected modules)
+// and of the candidates (mini-doublets x outer list).
+struct ScanSgFront : ScanCand<kSG> {
+    static constexpr int kVals = 2, kItems = 1;
+    __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
+        const int64_t sum = conn_sums(b, g, in, kMD, kSG);
+        const int64_t n = in ? OFF(b, kMD, g + 1) - OFF(b, kMD, g) : 0;
+        v[0] = n > 0 ? sum : 0;
+        v[1] = n * sum;
+    }
+    __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t* v) {
+        AT(b.toff, g, NG1(b)) = e[0];
+        put(b, g, e[1], v[1]);
+    }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) {
+        AT(b.toff, n, NG1(b)) = t[0];
+        put_total(b, n, t[1]);
+    }
+};
+
+// The outer lists of the segment candidates, written out (entry q of g's list
+// at olist[toff[g] + q]), so that a candidate finds its outer mini-doublet
+// with one load.  A warp looks at 32 modules and writes their lists one after
+// the other, 32 entries at a time.  The lists are not written when they
+// exceed olist_cap (the candidates then search the connection list).
 __global__ void k_sg_olist_fill(BatchDev b) {
     if (halted(b) || AT(b.toff, b.n_gm, NG1(b)) > b.olist_cap) return;
     const int n_mod = b.geo.n_mod;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < b.n_gm; g += (int64_t)gridDim.x * blockDim.x) {
-        int64_t o = AT(b.toff, g, NG1(b));
-        if (AT(b.toff, g + 1, NG1(b)) == o) continue;
-        const int ev = ev_of(b, g), m = (int)(g - (int64_t)ev * n_mod);
-        const int k0 = AT(b.geo.conn_off, m, NM(b) + 1), k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
-        for (int k = k0; k < k1; ++k) {
-            const int64_t g2 = (int64_t)ev * n_mod + AT(b.geo.conn_idx, k, NC(b));
-            const int64_t e = OFF(b, kMD, g2 + 1);
-            for (int64_t md = OFF(b, kMD, g2); md < e; ++md) AT(b.olist, o++, b.olist_cap) = (int)md;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / kWarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x / kWarp) + (threadIdx.x >> 5)) * kWarp; base < b.n_gm;
+         base += warps * kWarp) {
+        const int64_t gl = base + lane;
+        int64_t o = 0;
+        int len = 0;
+        if (gl < b.n_gm) {
+            o = AT(b.toff, gl, NG1(b));
+            len = (int)(AT(b.toff, gl + 1, NG1(b)) - o);
         }
-    }
-}
-
-__global__ void k_sg_count(BatchDev b) {
-    if (halted(b)) return;
-    const int64_t n = n_inner(b, kSG);
-    for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x)
-        AT(b.cand[kSG], a, b.cand_cap[kSG] + 1) = AT(b.conn_sum, OG(b, kMD, a), b.n_gm);
-}
-
-__global__ void k_tl_count(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTL);
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s - threadIdx.x < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = s < n;
-        int64_t c = 0;
-        int ev = 0, slot = 0;
-        if (in) {
-            const int g2 = OG(b, kMD, OJ(b, kSG, s));
-            c = AT(b.conn_sum, g2, b.n_gm);
-            AT(b.cand[kTL], s, b.cand_cap[kTL] + 1) = c;
-            atomicAdd((unsigned long long*)&AT(b.eoff, g2, NG1(b)), 1ull);  // segments ending in g2
-            const int g1 = OG(b, kSG, s);
-            ev = ev_of(b, g1);
-            slot = MOD(b, g1 - ev * n_mod).layer_slot;
+        for (unsigned m = __ballot_sync(0xffffffffu, len > 0); m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const int g = (int)base + j;
+            const int64_t og = __shfl_sync(0xffffffffu, o, j);
+            const int n = __shfl_sync(0xffffffffu, len, j);
+            const int ev = ev_of(b, g), mg = g - ev * n_mod;
+            const int k0 = AT(b.geo.conn_off, mg, NM(b) + 1), k1 = AT(b.geo.conn_off, mg + 1, NM(b) + 1);
+            for (int q0 = 0; q0 < n; q0 += kWarp) {
+                const bool has = q0 + lane < n;
+                const int md = tile_outer(b, ev, mg, k0, k1, q0, has);
+                if (has) AT(b.olist, og + q0 + lane, b.olist_cap) = md;
+            }
         }
-        const bool act = in && c != 0;
-        warp_add(act ? counter_at(b, ev, kTL, 0, slot) : b.counters, (uint32_t)c, act);
     }
 }
 
 // layer-pair segment candidates of every MD (Event.cc:805-818 loops over
 // inner-layer MDs x outer-layer MDs); the reference counts none of them
-__global__ void k_sg_count_layers(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kSG);
-    for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
+struct ScanSgLayers : ScanCand<kSG> {
+    __device__ static void load(const BatchDev& b, int64_t a, bool in, int64_t* v) {
+        v[0] = 0;
+        if (!in) return;
         const int g1 = OG(b, kMD, a);
         const int ev = ev_of(b, g1);
-        const int si = MOD(b, g1 - ev * n_mod).layer_slot;
-        int64_t c = 0;
+        const int si = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
         for (int k = 0; k < 3; ++k) {
             const int so = sg_layer_outer(si, k);
             if (so < 0) break;
-            c += layer_count(b, kMD, ev, so);
+            v[0] += layer_count(b, kMD, ev, so);
         }
-        AT(b.cand[kSG], a, b.cand_cap[kSG] + 1) = c;
     }
-}
+};
 
-// layer-pair tracklet candidates of every segment (Event.cc:762-787), counted
-// per inner layer like the module-map variant
-__global__ void k_tl_count_layers(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTL);
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s - threadIdx.x < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = s < n;
+// The front of the module-map tracklet stage: the connection sums over the
+// segments, the offsets of the segments by the module they end in (eoff, from
+// the counts there), of the module-pair tiles (toff, with the tile -> module
+// map while it fits tile_cap; the enumeration searches toff otherwise) and
+// the candidates' total.
+struct ScanTlFront : ScanOp {
+    static constexpr int kVals = 3, kItems = 1;
+    __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
+    __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
+        const int64_t sum = conn_sums(b, g, in, kSG, kTP);
+        v[0] = in ? AT(b.eoff, g, NG1(b)) : 0;
+        v[1] = tile_count(v[0], sum);
+        v[2] = v[0] * sum;
+    }
+    __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t* v) {
+        AT(b.eoff, g, NG1(b)) = e[0];
+        AT(b.toff, g, NG1(b)) = e[1];
+        for (int64_t t = e[1]; t < e[1] + v[1]; ++t)
+            if (t < b.tile_cap) AT(b.tile_gm, t, b.tile_cap) = (int)g;
+    }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) {
+        AT(b.eoff, n, NG1(b)) = t[0];
+        AT(b.toff, n, NG1(b)) = t[1];
+        *b.n_cand_tl = (unsigned long long)t[2];
+    }
+};
+
+// Tracklet candidates of every segment as a flat space, for the enumeration
+// of the layer pairs (Event.cc:762-787), of navigation (Event.cc:694-751) and
+// for the samples and self-checks of the module map; kCount: with the
+// reference's candidate counters
+template <bool kCount>
+struct ScanTlCand : ScanCand<kTL> {
+    __device__ static void load(const BatchDev& b, int64_t s, bool in, int64_t* v) {
         int64_t c = 0;
         int ev = 0, slot = 0;
         if (in) {
             const int g1 = OG(b, kSG, s);
             ev = ev_of(b, g1);
-            slot = MOD(b, g1 - ev * n_mod).layer_slot;
-            const int so = tl_layer_outer(slot);
-            c = so >= 0 ? layer_count(b, kSG, ev, so) : 0;
-            AT(b.cand[kTL], s, b.cand_cap[kTL] + 1) = c;
+            slot = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
+            const int var = tl_variant(b);
+            if (var == 1) {
+                const int so = tl_layer_outer(slot);
+                c = so >= 0 ? layer_count(b, kSG, ev, so) : 0;
+            } else if (var == 2) {
+                const int m = OJ(b, kSG, s);
+                const int64_t nc = join_n(b, m);
+                for (int64_t k = 0; k < nc; ++k) c += join_n(b, OJ(b, kSG, join_obj(b, m, k)));
+            } else {
+                c = AT(b.conn_sum, OG(b, kMD, OJ(b, kSG, s)), b.n_gm);
+            }
         }
-        const bool act = in && c != 0;
+        const bool act = kCount && c != 0;
         warp_add(act ? counter_at(b, ev, kTL, 0, slot) : b.counters, (uint32_t)c, act);
+        v[0] = c;
     }
-}
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) {
+        put_total(b, n, t[0]);
+        *b.n_cand_tl = (unsigned long long)t[0];
+    }
+};
 
 // objects of stage st per key mini-doublet, then their positions
 __global__ void k_join_count(BatchDev b, int st, bool second) {
@@ -2061,6 +2155,19 @@ __global__ void k_join_count(BatchDev b, int st, bool second) {
     for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x)
         atomicAdd((unsigned long long*)&AT(off, join_key(b, st, o), b.obj[kMD].cap + 1), 1ull);
 }
+template <bool kSecond>
+struct ScanJoin : ScanOp {
+    static constexpr int kVals = 1, kItems = 4;
+    __device__ static int64_t* off(const BatchDev& b) { return kSecond ? b.joff2 : b.joff; }
+    __device__ static int64_t size(const BatchDev& b) { return n_objects(b, kMD); }
+    __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) {
+        v[0] = in ? AT(off(b), i, b.obj[kMD].cap + 1) : 0;
+    }
+    __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t*) {
+        AT(off(b), i, b.obj[kMD].cap + 1) = e[0];
+    }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(off(b), n, b.obj[kMD].cap + 1) = t[0]; }
+};
 __global__ void k_join_scatter(BatchDev b, int st, bool second) {
     if (halted(b)) return;
     const int64_t* off = second ? b.joff2 : b.joff;
@@ -2075,61 +2182,46 @@ __global__ void k_join_scatter(BatchDev b, int st, bool second) {
     }
 }
 
-__global__ void k_tp_count(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTP);
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+// how often module m2 occurs in the connection list of module m1
+__device__ __forceinline__ int conn_mult(const BatchDev& b, int m1, int m2) {
+    int mult = 0;
+    const int k0 = AT(b.geo.conn_off, m1, NM(b) + 1), k1 = AT(b.geo.conn_off, m1 + 1, NM(b) + 1);
+    for (int k = k0; k < k1; ++k) mult += AT(b.geo.conn_idx, k, NC(b)) == m2;
+    return mult;
+}
+
+// triplet candidates of every segment (TPStage)
+struct ScanTpCand : ScanCand<kTP> {
+    __device__ static void load(const BatchDev& b, int64_t s, bool in, int64_t* v) {
+        v[0] = 0;
+        if (!in) return;
+        const int md = OJ(b, kSG, s);
+        const int64_t n = join_n(b, md);
+        if (n == 0) return;
         const int g1 = OG(b, kSG, s);
-        const int ev = ev_of(b, g1), m1 = g1 - ev * n_mod;
-        const int g2 = OG(b, kMD, OJ(b, kSG, s));
-        const int m2 = g2 - ev * n_mod;
-        int mult = 0;
-        const int k0 = AT(b.geo.conn_off, m1, NM(b) + 1), k1 = AT(b.geo.conn_off, m1 + 1, NM(b) + 1);
-        for (int k = k0; k < k1; ++k) mult += AT(b.geo.conn_idx, k, NC(b)) == m2;
-        AT(b.cand[kTP], s, b.cand_cap[kTP] + 1) = (int64_t)mult * join_n(b, OJ(b, kSG, s));
+        const int ev = ev_of(b, g1);
+        v[0] = (int64_t)conn_mult(b, g1 - ev * b.geo.n_mod, OG(b, kMD, md) - ev * b.geo.n_mod) * n;
     }
-}
+};
 
-__global__ void k_tc_count(BatchDev b) {
-    if (halted(b)) return;
-    const int64_t n = n_inner(b, kTC);
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-        int64_t c = 0;
-        const int g1 = OG(b, kTL, t);
-        const ModDev& m1 = MOD(b, mod_of(b, g1));
-        if (m1.subdet == kBarrel && m1.layer == 1) {
-            const int g3 = OG(b, kSG, OJ(b, kTL, t));
-            const ModDev& m3 = MOD(b, mod_of(b, g3));
-            if (m3.subdet == kBarrel && m3.layer == 3) c = join_n(b, OI(b, kSG, OJ(b, kTL, t)));
+// track candidates of every tracklet (TCStage); Event.cc:835: their
+// candidates in the counters are barrel-layer-1 x barrel-layer-3 tracklets
+struct ScanTcCand : ScanCand<kTC> {
+    __device__ static void begin(const BatchDev& b) {
+        for (int ev = blockIdx.x * blockDim.x + threadIdx.x; ev < b.n_ev; ev += gridDim.x * blockDim.x) {
+            const uint32_t n1 = *counter_at(b, ev, kTL, 1, 0), n3 = *counter_at(b, ev, kTL, 1, 2);
+            *counter_at(b, ev, kTC, 0, 0) += n1 * n3;
         }
-        AT(b.cand[kTC], t, b.cand_cap[kTC] + 1) = c;
     }
-}
-
-// navigation tracklet candidates of every segment (Event.cc:694-751) and the
-// reference's candidate counters
-__global__ void k_tl_count_nav(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTL);
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s - threadIdx.x < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = s < n;
-        int64_t c = 0;
-        int ev = 0, slot = 0;
-        if (in) {
-            const int m = OJ(b, kSG, s);
-            const int64_t nc = join_n(b, m);
-            for (int64_t k = 0; k < nc; ++k) c += join_n(b, OJ(b, kSG, join_obj(b, m, k)));
-            AT(b.cand[kTL], s, b.cand_cap[kTL] + 1) = c;
-            const int g1 = OG(b, kSG, s);
-            ev = ev_of(b, g1);
-            slot = MOD(b, g1 - ev * n_mod).layer_slot;
-        }
-        const bool act = in && c != 0;
-        warp_add(act ? counter_at(b, ev, kTL, 0, slot) : b.counters, (uint32_t)c, act);
+    __device__ static void load(const BatchDev& b, int64_t t, bool in, int64_t* v) {
+        v[0] = 0;
+        if (!in) return;
+        const ModDev& m1 = MOD(b, mod_of(b, OG(b, kTL, t)));
+        if (m1.subdet != kBarrel || m1.layer != 1) return;
+        const ModDev& m3 = MOD(b, mod_of(b, OG(b, kSG, OJ(b, kTL, t))));
+        if (m3.subdet == kBarrel && m3.layer == 3) v[0] = join_n(b, OI(b, kSG, OJ(b, kTL, t)));
     }
-}
+};
 
 // createTrackCandidatesFromTracklets (Event.cc:984-1062): the reference's
 // candidates of tracklet t are the tracklets of the modules connected to the
@@ -2139,70 +2231,50 @@ __global__ void k_tl_count_nav(BatchDev b) {
 // once per occurrence of that module in the connection list.  Layer-pair
 // tracklets are listed by no module (Event.cc:785 via
 // addTrackletToLowerLayer), so after them there are no candidates.
-__global__ void k_tc_count_tl(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTC);
-    const bool none = (b.flags & kFlagTLLayers) != 0;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t - threadIdx.x < n; t += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = t < n;
+struct ScanTcFromTl : ScanCand<kTC> {
+    __device__ static void load(const BatchDev& b, int64_t t, bool in, int64_t* v) {
+        const int n_mod = b.geo.n_mod;
         int64_t cref = 0;
         int ev = 0, slot = 0;
-        if (in) {
+        v[0] = 0;
+        if (in && !(b.flags & kFlagTLLayers)) {
             const int gA2 = OG(b, kMD, OJ(b, kSG, OI(b, kTL, t)));
             ev = ev_of(b, gA2);
-            const int mA2 = gA2 - ev * n_mod;
-            cref = none ? 0 : AT(b.conn_sum, gA2, b.n_gm);
+            cref = AT(b.conn_sum, gA2, b.n_gm);
             const int mB = OI(b, kSG, OJ(b, kTL, t));
-            const int mB1 = OG(b, kMD, mB) - ev * n_mod;
-            int mult = 0;
-            const int k0 = AT(b.geo.conn_off, mA2, NM(b) + 1), k1 = AT(b.geo.conn_off, mA2 + 1, NM(b) + 1);
-            for (int k = k0; k < k1; ++k) mult += AT(b.geo.conn_idx, k, NC(b)) == mB1;
-            AT(b.cand[kTC], t, b.cand_cap[kTC] + 1) = none ? 0 : (int64_t)mult * join_n(b, mB);
+            v[0] = (int64_t)conn_mult(b, gA2 - ev * n_mod, OG(b, kMD, mB) - ev * n_mod) * join_n(b, mB);
             slot = MOD(b, OG(b, kTL, t) - ev * n_mod).layer_slot;
         }
-        const bool act = in && cref != 0;
+        const bool act = cref != 0;
         warp_add(act ? counter_at(b, ev, kTC, 0, slot) : b.counters, (uint32_t)cref, act);
     }
-}
+};
 
 // createTrackCandidatesFromTriplets (Event.cc:874-982): candidates of triplet
 // p = the triplets of the modules connected to the module of its outermost MD
 // (conn_sum over triplet counts), with the reference's candidate counters
-__global__ void k_tc_count_tp(BatchDev b) {
-    if (halted(b)) return;
-    const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTC);
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p - threadIdx.x < n; p += (int64_t)gridDim.x * blockDim.x) {
-        const bool in = p < n;
+struct ScanTcFromTp : ScanCand<kTC> {
+    __device__ static void load(const BatchDev& b, int64_t p, bool in, int64_t* v) {
         int64_t c = 0;
         int ev = 0, slot = 0;
+        v[0] = 0;
         if (in) {
             const int mdA = OJ(b, kSG, OJ(b, kTP, p));
             c = AT(b.conn_sum, OG(b, kMD, mdA), b.n_gm);
-            int64_t e = c;  // the trial-segment enumeration: every reference candidate
+            v[0] = c;  // the trial-segment enumeration: every reference candidate
             if (!(b.flags & kFlagSGLayers)) {  // TCTPMapStage: segments leaving mdA x triplets at their outer MD
-                e = 0;
+                v[0] = 0;
                 const int64_t ns = join_n(b, mdA);
-                for (int64_t k = 0; k < ns; ++k) e += join2_n(b, OJ(b, kSG, join_obj(b, mdA, k)));
+                for (int64_t k = 0; k < ns; ++k) v[0] += join2_n(b, OJ(b, kSG, join_obj(b, mdA, k)));
             }
-            AT(b.cand[kTC], p, b.cand_cap[kTC] + 1) = e;
             const int g1 = OG(b, kTP, p);
             ev = ev_of(b, g1);
-            slot = MOD(b, g1 - ev * n_mod).layer_slot;
+            slot = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
         }
-        const bool act = in && c != 0;
+        const bool act = c != 0;
         warp_add(act ? counter_at(b, ev, kTC, 0, slot) : b.counters, (uint32_t)c, act);
     }
-}
-
-// Event.cc:835: track-candidate candidates are barrel-layer-1 x barrel-layer-3 tracklets
-__global__ void k_tc_cand_counter(BatchDev b) {
-    for (int ev = blockIdx.x * blockDim.x + threadIdx.x; ev < b.n_ev; ev += gridDim.x * blockDim.x) {
-        const uint32_t n1 = *counter_at(b, ev, kTL, 1, 0), n3 = *counter_at(b, ev, kTL, 1, 2);
-        *counter_at(b, ev, kTC, 0, 0) += n1 * n3;
-    }
-}
+};
 
 // ------------------------------------------------------------------ output
 __device__ __forceinline__ void put_md(const BatchDev& b, int a, int32_t* o) {
@@ -2361,31 +2433,23 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
     for (int64_t i = t; i < (int64_t)b.n_ev * 110; i += stride) c[i] = b.counters[i];
 }
 
-void scan_h(const BatchDev& b, int64_t* data, const int64_t* n_ptr, int64_t cap, cudaStream_t s, Hooks* h) {
-    scan(b, data, n_ptr, cap, s);
-    if (h) h->launches += 3;
+// cap: an upper bound of the number of elements
+template <class Op>
+void scan(const BatchDev& b, int slot, int64_t cap, cudaStream_t s, Hooks* h) {
+    k_scan<Op><<<grid_for(cap, kScanThreads * Op::kItems, b.n_sm * 8), kScanThreads, 0, s>>>(take(b, h), slot);
 }
 
 int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : 8; }
 
-template <class F>
-void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h, bool layer_counters = true) {
+// stage F's candidates (their offsets scanned by Cand) -> objects
+template <class F, class Cand, bool kCounters = true>
+void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
     constexpr int st = F::kSt;
-    const int64_t* ninner_ptr = nullptr;
-    switch (st) {
-        case kMD: ninner_ptr = b.n_gm_dev; break;
-        case kSG: ninner_ptr = b.obj[kMD].mod_cnt + b.n_gm; break;
-        case kTL:
-        case kTP: ninner_ptr = b.obj[kSG].mod_cnt + b.n_gm; break;
-        default: ninner_ptr = ((b.flags & kFlagTCFromTP) ? b.obj[kTP] : b.obj[kTL]).mod_cnt + b.n_gm;
-    }
-    scan_h(b, b.cand[st], ninner_ptr, b.cand_cap[st], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st);
+    scan<Cand>(b, kScanCand + st, b.cand_cap[st], s, h);
     mark(h, kStampEnum + st);
     k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
-    if (layer_counters) k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), st);
-    scan_h(b, b.obj[st].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
+    scan<ScanObj<st, kCounters>>(b, kScanObj + st, b.n_gm, s, h);
     k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st);
 }
 
@@ -2415,31 +2479,24 @@ __global__ void __launch_bounds__(256) k_copy_words(CopyJobs j) {
 void launch_ingest(const BatchDev& b, cudaStream_t s, Hooks* h) {
     const unsigned g = grid_for(b.n_hit_cap, 256, b.n_sm * 16);
     k_hit_map<<<g, 256, 0, s>>>(take(b, h));
-    scan_h(b, b.mod_hit, b.n_gm_dev, b.n_gm, s, h);
+    scan<ScanHits>(b, kScanHit, b.n_gm, s, h);
     k_hit_perm<<<g, 256, 0, s>>>(take(b, h));
     k_hit_scatter<<<g, 256, 0, s>>>(take(b, h));
 }
 
 void launch_md(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    k_md_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
-    enum_and_group<MDStage>(b, s, h);
+    enum_and_group<MDStage, ScanMdCand>(b, s, h);
 }
 
 void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_md_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     if (b.flags & kFlagSGLayers) {
         // Event.cc:793-821 increments no per-layer counter
-        k_sg_count_layers<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-        enum_and_group<SGLayerStage>(b, s, h, false);
+        enum_and_group<SGLayerStage, ScanSgLayers, false>(b, s, h);
         return;
     }
-    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kMD, kSG);
-    k_sg_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    k_sg_olist_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
-    scan_h(b, b.toff, b.n_gm_dev, b.n_gm, s, h);
+    scan<ScanSgFront>(b, kScanCand + kSG, b.n_gm, s, h);
     k_sg_olist_fill<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
-    scan_h(b, b.cand[kSG], b.obj[kMD].mod_cnt + b.n_gm, b.cand_cap[kSG], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kSG);
     // first cuts -> survivor list -> whole algorithm (k_sg_enum_a, k_sg_b)
     mark(h, kStampEnum + kSG);
     BatchDev l = b;  // with this list's own counts
@@ -2449,19 +2506,19 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_sg_b<1><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     mark(h, kStampEnumEnd + kSG);
-    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG);
-    scan_h(b, b.obj[kSG].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
+    scan<ScanObj<kSG, true>>(b, kScanObj + kSG, b.n_gm, s, h);
     k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kSG);
 }
 
 // the join index of stage st's objects (segments or tracklets), keyed by
 // mini-doublet; second = true builds the second index (triplets)
-static void join_index(const BatchDev& b, int st, cudaStream_t s, Hooks* h, bool second = false) {
+static void join_index(const BatchDev& b, int st, int slot, cudaStream_t s, Hooks* h, bool second = false) {
     int64_t* off = second ? b.joff2 : b.joff;
     cudaMemsetAsync(off, 0, (b.obj[kMD].cap + 1) * sizeof(int64_t), s);
     cudaMemsetAsync(second ? b.jcur2 : b.jcur, 0, b.obj[kMD].cap * sizeof(int32_t), s);
     k_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
-    scan_h(b, off, b.obj[kMD].mod_cnt + b.n_gm, b.obj[kMD].cap, s, h);
+    if (second) scan<ScanJoin<true>>(b, slot, b.obj[kMD].cap, s, h);
+    else scan<ScanJoin<false>>(b, slot, b.obj[kMD].cap, s, h);
     k_join_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
 }
 
@@ -2469,25 +2526,15 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     // conn sums over segment counts serve the tracklet enumeration and the
     // triplet candidate counters (Event.cc:547-596 loops over the same lists)
     k_sg_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG, kTP);
-    if (b.flags & kFlagTLLayers) {
-        k_tl_count_layers<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    } else if (b.flags & kFlagTLNav) {
-        join_index(b, kSG, s, h);  // segments by inner MD: the outward lists
-        k_tl_count_nav<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    } else {
-        k_tl_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    }
-    scan_h(b, b.cand[kTL], b.obj[kSG].mod_cnt + b.n_gm, b.cand_cap[kTL], s, h);
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kTL);
     // module-map candidates: the module-pair tiles (k_tl_enum_tiles)
     const bool tiles = !(b.flags & (kFlagTLLayers | kFlagTLNav));
     if (tiles) {
-        k_tl_tile_count<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
-        scan_h(b, b.eoff, b.n_gm_dev, b.n_gm, s, h);
-        scan_h(b, b.toff, b.n_gm_dev, b.n_gm, s, h);
+        scan<ScanTlFront>(b, kScanTlFront, b.n_gm, s, h);
         k_sg_end_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-        k_tile_map<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
+    } else {
+        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG, kTP);
+        if (b.flags & kFlagTLNav) join_index(b, kSG, kScanJoinNav, s, h);  // segments by inner MD: the outward lists
+        scan<ScanTlCand<true>>(b, kScanCand + kTL, b.cand_cap[kTL], s, h);
     }
     mark(h, kStampEnum + kTL);
     // enumeration + phase A -> survivor list (-> the pre-filter -> kept list)
@@ -2522,40 +2569,35 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_tl_b2<kB2BBBB><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
     k_tl_b2<kB2Others><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + kTL);
-    k_obj_counters<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTL);
-    scan_h(b, b.obj[kTL].mod_cnt, b.n_gm_dev, b.n_gm, s, h);
+    scan<ScanObj<kTL, true>>(b, kScanObj + kTL, b.n_gm, s, h);
     k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kTL);
 }
 
 
 void launch_tp(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    join_index(b, kSG, s, h);
-    k_tp_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    enum_and_group<TPStage>(b, s, h);
+    join_index(b, kSG, kScanJoinTp, s, h);
+    enum_and_group<TPStage, ScanTpCand>(b, s, h);
 }
 
 void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
     if (b.flags & kFlagTCFromTP) {
         const bool map = !(b.flags & kFlagSGLayers);
         if (map) {
-            join_index(b, kSG, s, h);        // segments by inner MD
-            join_index(b, kTP, s, h, true);  // triplets by innermost MD
+            join_index(b, kSG, kScanJoinTc, s, h);           // segments by inner MD
+            join_index(b, kTP, kScanJoinTc2, s, h, true);  // triplets by innermost MD
         }
         k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTP, -1);
-        k_tc_count_tp<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-        if (map) enum_and_group<TCTPMapStage>(b, s, h);
-        else enum_and_group<TCTPStage>(b, s, h);
+        if (map) enum_and_group<TCTPMapStage, ScanTcFromTp>(b, s, h);
+        else enum_and_group<TCTPStage, ScanTcFromTp>(b, s, h);
         return;
     }
-    join_index(b, kTL, s, h);
+    join_index(b, kTL, kScanJoinTc, s, h);
     if (b.flags & kFlagTCFromTL) {
         k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTL, -1);
-        k_tc_count_tl<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+        enum_and_group<TCStage, ScanTcFromTl>(b, s, h);
     } else {
-        k_tc_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-        k_tc_cand_counter<<<grid_for(b.n_ev, 128, 1024), 128, 0, s>>>(take(b, h));
+        enum_and_group<TCStage, ScanTcCand>(b, s, h);
     }
-    enum_and_group<TCStage>(b, s, h);
 }
 
 // ------------------------------------------------------------------ self-check
@@ -2686,9 +2728,17 @@ void launch_math_check(int fn, int exhaustive, unsigned long long start, long lo
     k_math_check<<<n_sm * 16, 256, 0, s>>>(fn, exhaustive, start, n, seed, out);
 }
 
+// the tracklet candidates as a flat space, after a run: the module map's
+// enumeration needs none, and the bucket table holds the last stage's
+static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
+    ClearJobs j{};
+    j.add(b.scan_state + (int64_t)(kScanCand + kTL) * b.scan_cap, 2 * b.scan_cap);
+    launch_clear(b, j, s, nullptr);
+    scan<ScanTlCand<false>>(b, kScanCand + kTL, b.cand_cap[kTL], s, nullptr);
+}
+
 void launch_tl_collect(const BatchDev& b, const MlpCollect& c, cudaStream_t s) {
-    // the bucket table holds the last stage that ran: rebuild the tracklet one
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(b, kTL);
+    tl_cand_space(b, s);
     k_tl_collect<<<b.n_sm * 8, 256, 0, s>>>(b, c);
 }
 
@@ -2697,7 +2747,7 @@ void launch_tl_b2q_check(const BatchDev& b, unsigned long long* out, cudaStream_
 }
 
 void launch_tl_quick_check(const BatchDev& b, unsigned long long* out, cudaStream_t s) {
-    k_cand_buckets<<<b.n_sm * 8, 256, 0, s>>>(b, kTL);
+    tl_cand_space(b, s);
     k_tl_quick_check<<<b.n_sm * 8, 256, 0, s>>>(b, out);
 }
 

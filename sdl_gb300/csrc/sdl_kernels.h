@@ -34,7 +34,6 @@ struct BatchDev {
     int64_t* cand[kNumStages];     // per inner object candidate counts -> offsets (cap_inner + 1)
     int64_t cand_cap[kNumStages];
     int64_t* n_rec;                // kNumStages attempted appends
-    int64_t* n_gm_dev;             // device scalar = n_gm
     // connection-list prefix sums of per-module object counts
     int32_t* conn_pref;            // n_ev * n_conn
     int32_t* conn_first;           // n_ev * n_conn: offset of the entry's module's first object
@@ -48,8 +47,8 @@ struct BatchDev {
     uint32_t* counters;            // n_ev * 110
     uint32_t* status;
     unsigned long long* task;      // kNumStages work counters
-    int64_t* scan_tmp;
-    int64_t scan_tmp_cap;
+    unsigned long long* scan_state;  // kScanSlots x scan_cap: per scan the tile counter and a word per tile and value
+    int64_t scan_cap;
     int32_t* bucket;               // first inner object of every 256 consecutive candidates of the running stage
     int64_t bucket_cap;
     int flags;                     // kFlag* bits
@@ -68,6 +67,7 @@ struct BatchDev {
     int4* passf;                   // what phase B2's single-precision decision (tl_b2_quick) left of
                                    //   the enumeration's or the pre-filter's list, as passa
     unsigned long long* n_keptf;
+    unsigned long long* n_cand_tl;   // tracklet candidates
     // join index (triplets, then track candidates): the segments by their inner
     // mini-doublet, then the tracklets by their inner segment's inner mini-doublet
     int64_t* joff;                 // mini-doublet cap + 1: counts -> offsets
@@ -102,6 +102,24 @@ struct BatchDev {
     unsigned long long* stamps;    // kNumStamps
     uint32_t ts;
 };
+
+// The scans of a run, one slot of scan_state each (k_scan)
+enum ScanSlot : int {
+    kScanHit = 0,
+    kScanCand = 1,                        // + st: candidate offsets (module-map segments: with the outer lists')
+    kScanObj = kScanCand + kNumStages,    // + st: objects per module
+    kScanTlFront = kScanObj + kNumStages,
+    kScanJoinNav,
+    kScanJoinTp,
+    kScanJoinTc,
+    kScanJoinTc2,
+    kScanSlots
+};
+// words of one slot for scans over up to n_gm global modules (tiles of at
+// least 256, up to 3 values each) and objects (tiles of at least 512)
+constexpr int64_t scan_words(int64_t n_gm, int64_t objects) {
+    return 1 + (3 * (n_gm / 256 + 1) > objects / 512 + 1 ? 3 * (n_gm / 256 + 1) : objects / 512 + 1);
+}
 
 // Device time stamps of a run.  An event node in a CUDA graph costs about
 // 4.5 us (a kernel node 0.8 us), so the stage and pass boundaries are stamps

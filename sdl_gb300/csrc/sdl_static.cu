@@ -33,16 +33,15 @@ namespace {
 constexpr int64_t kMaxHits = SDLG_STATIC_MAX_HITS;
 constexpr int64_t kMaxModules = SDLG_STATIC_MAX_MODULES;
 constexpr int64_t kMaxMD = SDLG_STATIC_MAX_MINI_DOUBLETS;
-constexpr int64_t kScanTmp = kMaxModules / 4096 + 16;
 
 // Layout of the array, in 8-byte words.
-constexpr int64_t kSmall = 0;                                   // n_hit, n_gm, n_rec[5]
+constexpr int64_t kSmall = 0;                                   // n_hit, (free), n_rec[5]
 constexpr int64_t kEvOff = 16;                                  // ev_off[2]
 constexpr int64_t kModHit = kEvOff + 2;                         // kMaxModules + 1
 constexpr int64_t kCandMD = kModHit + kMaxModules + 1;          // kMaxModules + 1
 constexpr int64_t kModCnt = kCandMD + kMaxModules + 1;          // kMaxModules + 1
-constexpr int64_t kScan = kModCnt + kMaxModules + 1;            // kScanTmp
-constexpr int64_t kWords64 = (kScan + kScanTmp + 31) / 32 * 32;  // 256-byte multiple: the 4-byte regions start aligned
+constexpr int64_t kSpare = kModCnt + kMaxModules + 1;           // 32 (free)
+constexpr int64_t kWords64 = (kSpare + 32 + 31) / 32 * 32;  // 256-byte multiple: the 4-byte regions start aligned
 // 4-byte regions follow the 8-byte ones
 constexpr int64_t kHitArrays = 18;                              // hit_gm, hit_rank, hit_perm and 15 sorted arrays
 constexpr int64_t kObjWords = 3 + 4;                            // i, j, g, f[4]
@@ -75,7 +74,6 @@ int scratch_address(int device, void** out) {
 __global__ void k_static_init(BatchDev b, int64_t n_hits) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         *const_cast<int64_t*>(b.n_hit) = n_hits;
-        *b.n_gm_dev = b.n_gm;
         int64_t* eo = const_cast<int64_t*>(b.ev_off);
         eo[0] = 0;
         eo[1] = n_hits;
@@ -87,7 +85,7 @@ __global__ void k_static_init(BatchDev b, int64_t n_hits) {
 __global__ void k_static_out(BatchDev b, int32_t* pairs, int64_t cap, int64_t* count, uint32_t* status) {
     const int64_t n = b.obj[kMD].mod_cnt[b.n_gm];
     const uint32_t st = *b.status;
-    const bool ok = (st & 0x1fu) == 0;
+    const bool ok = (st & kStatusHalt) == 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *count = ok ? n : b.n_rec[kMD];
         *status = st;
@@ -150,15 +148,12 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.n_gm = geo.n_mod;
     b.n_hit_cap = H;
     b.n_hit = w64 + kSmall;
-    b.n_gm_dev = w64 + kSmall + 1;
     b.n_rec = w64 + kSmall + 2;
     b.ev_off = w64 + kEvOff;
     b.in_x = d_x; b.in_y = d_y; b.in_z = d_z; b.in_idx = d_idx; b.in_det = d_detid;
     b.mod_hit = w64 + kModHit;
     b.cand[kMD] = w64 + kCandMD;
     b.cand_cap[kMD] = geo.n_mod;
-    b.scan_tmp = w64 + kScan;
-    b.scan_tmp_cap = kScanTmp;
     int64_t o = 0;
     b.hit_gm = w32 + o; o += H;
     b.hit_rank = w32 + o; o += H;
@@ -174,6 +169,11 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     O.g = w32 + o; o += kMaxMD;
     O.f = f32 + o; o += 4 * kMaxMD;
     O.mod_cnt = w64 + kModCnt;
+    // the scans' words lie where the object values go: the last scan is over
+    // when the objects are written
+    b.scan_state = reinterpret_cast<unsigned long long*>(O.f);
+    b.scan_cap = scan_words(geo.n_mod, kMaxMD);
+    static_assert(8 * kScanSlots * scan_words(kMaxModules, kMaxMD) <= 4 * 4 * kMaxMD, "the scans' words fit");
     Recs& R = b.rec[kMD];
     R.nf = 4;
     R.i = w32 + o; o += kMaxMD;
@@ -197,6 +197,7 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     j.add(b.counters, 110);
     j.add(b.mod_hit, 2 * (geo.n_mod + 1));
     j.add(O.mod_cnt, 2 * (geo.n_mod + 1));
+    j.add(b.scan_state, 2 * kScanSlots * b.scan_cap);
     launch_clear(b, j, s, nullptr);
     k_static_init<<<1, 32, 0, s>>>(b, n_hits);
     launch_ingest(b, s, nullptr);
