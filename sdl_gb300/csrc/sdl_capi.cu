@@ -376,7 +376,7 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
     return SDLG_OK;
 }
 
-constexpr int64_t kZeroWords = 2 * kNumStages + 12 + 8;
+constexpr int64_t kZeroWords = (2 * kNumStages + 10) * kLine;
 
 // (re)allocate the batch buffers for the current event sizes and capacities
 int ensure_buffers(sdlg_ctx* ctx) {
@@ -422,18 +422,18 @@ int ensure_buffers(sdlg_ctx* ctx) {
     int64_t* zero;
     AL(zero, kZeroWords);
     b.n_rec = zero;
-    b.task = reinterpret_cast<unsigned long long*>(zero + kNumStages);
-    unsigned long long* cnt = b.task + kNumStages;
+    b.task = reinterpret_cast<unsigned long long*>(zero + kNumStages * kLine);
+    unsigned long long* cnt = b.task + kNumStages * kLine;
     b.n_kept_sg = cnt;
-    b.n_pb_sg = cnt + 1;
-    b.n_kept = cnt + 3;
-    b.n_kept2 = cnt + 4;
-    b.n_keptf = cnt + 5;
-    b.n_pb_f = cnt + 6;
-    b.n_pb = cnt + 8;
-    b.n_cand_tl = cnt + 10;
-    b.status = reinterpret_cast<uint32_t*>(cnt + 11);
-    b.dbg = cnt + 12;
+    b.n_pb_sg = cnt + kLine;
+    b.n_kept = cnt + 2 * kLine;
+    b.n_kept2 = cnt + 3 * kLine;
+    b.n_keptf = cnt + 4 * kLine;
+    b.n_pb_f = cnt + 5 * kLine;
+    b.n_pb = cnt + 6 * kLine;
+    b.n_cand_tl = cnt + 7 * kLine;
+    b.status = reinterpret_cast<uint32_t*>(cnt + 8 * kLine);
+    b.dbg = cnt + 9 * kLine;
     float* fx; float* fy; float* fz; int32_t* fi; uint32_t* fd; int64_t* eo;
     AL(fx, H); AL(fy, H); AL(fz, H); AL(fi, H); AL(fd, H); AL(eo, ctx->n_ev + 1);
     b.in_x = fx; b.in_y = fy; b.in_z = fz; b.in_idx = fi; b.in_det = fd; b.ev_off = eo;
@@ -451,7 +451,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
         AL(R.i, C); AL(R.j, C); AL(R.g, C); AL(R.rank, C); AL(R.f, C * std::max(1, nf[s]));
     }
     b.cand_cap[kMD] = n_gm;
-    b.cand_cap[kSG] = std::max(n_gm, ctx->cap_obj[kMD]);  // global modules, or mini-doublets (SDLG_FLAG_SG_LAYERS)
+    b.cand_cap[kSG] = ctx->cap_obj[kMD];
     b.cand_cap[kTL] = ctx->cap_obj[kSG];
     b.cand_cap[kTP] = ctx->cap_obj[kSG];
     b.cand_cap[kTC] = std::max(ctx->cap_obj[kTL], ctx->cap_obj[kTP]);  // tracklets, or triplets (SDLG_FLAG_TC_FROM_TP)
@@ -485,6 +485,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.ecur, n_gm);
     AL(b.eidx, ctx->cap_obj[kSG]);
     AL(b.toff, n_gm + 1);
+    AL(b.coff, n_gm + 1);
     b.tile_cap = 2 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);
     AL(b.tile_gm, b.tile_cap);
     b.olist_cap = 4 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);
@@ -521,11 +522,11 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
         const int ns = last - first + 1;
         j.add(b.status, 1);
         j.add(b.dbg, 16);
-        j.add(b.n_rec + first, 2 * ns);
-        j.add(b.task + first, 2 * ns);
+        j.add(b.n_rec + first * kLine, 2 * kLine * ns);
+        j.add(b.task + first * kLine, 2 * kLine * ns);
         // the survivor lists' counts: the segment stage's, then the tracklet stage's
-        if (first <= kSG) j.add(b.n_kept_sg, 6);
-        if (first <= kTL && last >= kTL) j.add(b.n_kept, 16);
+        if (first <= kSG) j.add(b.n_kept_sg, 4 * kLine);
+        if (first <= kTL && last >= kTL) j.add(b.n_kept, 12 * kLine);
         // the counters these stages write (22 per stage in each event's 110:
         // candidates, then objects): the triplet candidates are counted by the
         // tracklet stage (Event.cc:547-596 loops over the segment lists)

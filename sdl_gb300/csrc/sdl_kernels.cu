@@ -128,8 +128,10 @@ __device__ __forceinline__ const ModDev& MOD(const BatchDev& b, int64_t m) { ret
 // Exclusive prefix sums in one pass (decoupled look-back, after Merrill and
 // Garland 2016): each CTA takes the next tile from a counter, so that every
 // tile before its own has been started, publishes the tile's sum, adds up
-// its predecessors' words (a sum, or already a whole prefix) 32 at a time and
-// publishes its prefix.  What is summed is computed where it is loaded (the
+// its predecessors' words (a sum, or already a whole prefix), one per thread,
+// and publishes its prefix.  The whole CTA looks back because the tiles in
+// flight publish their sums at about the same time, so that a tile has
+// hundreds of sums to add before it meets a prefix.  What is summed is computed where it is loaded (the
 // candidate counts with their layer counters) and what is derived from the
 // prefix is written where it is stored (offsets, bucket and tile tables), so
 // one launch does what took a count kernel, three scan kernels and a table
@@ -140,7 +142,7 @@ __device__ __forceinline__ const ModDev& MOD(const BatchDev& b, int64_t m) { ret
 // sum, 2: the prefix through the tile).  The words are cleared with the run's
 // other counts, one slot per scan of a run.  A wait for a predecessor is
 // bounded: past kScanPolls the CTA sets kStatusScan, which halts the run.
-constexpr int kScanThreads = 256;
+constexpr int kScanThreads = 512;
 constexpr int kScanPolls = 1 << 20;
 constexpr unsigned long long kScanSum = 1ull << 62, kScanPrefix = 2ull << 62, kScanValue = (1ull << 62) - 1;
 
@@ -153,34 +155,64 @@ __device__ __forceinline__ void scan_post(unsigned long long* p, unsigned long l
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// the sum of the tiles before `tile` (value q of kK per tile; whole warp)
+// the sums of the tiles before `tile` (kK values per tile); the whole CTA
+// calls it, and every thread gets them
 template <int kK>
-__device__ __forceinline__ int64_t scan_lookback(const unsigned long long* words, int64_t tile, int q, bool& ok) {
-    const int lane = threadIdx.x & 31;
-    int64_t sum = 0;
-    for (int64_t t = tile - 1;; t -= kWarp) {
-        const int64_t k = t - lane;
-        unsigned long long w = kScanPrefix;  // before the first tile: a prefix of 0
-        for (int polls = 0;; ++polls) {
-            if (k >= 0) w = scan_peek(words + k * kK + q);
-            if (!__any_sync(0xffffffffu, (w >> 62) == 0ull)) break;
-            if (polls == kScanPolls) {
-                ok = false;
-                return 0;
+struct ScanBack {
+    int64_t sum[kK][kScanThreads / kWarp];
+    bool done[kK][kScanThreads / kWarp];  // a prefix is among the warp's words
+    int ok;
+};
+template <int kK>
+__device__ __forceinline__ bool scan_lookback(const unsigned long long* words, int64_t tile, ScanBack<kK>& sb, int64_t* pre) {
+    constexpr int kWarps = kScanThreads / kWarp;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    bool open[kK];
+#pragma unroll
+    for (int q = 0; q < kK; ++q) {
+        pre[q] = 0;
+        open[q] = true;
+    }
+    for (int64_t t = tile - 1;; t -= kScanThreads) {
+        const int64_t k = t - threadIdx.x;
+#pragma unroll
+        for (int q = 0; q < kK; ++q) {
+            unsigned long long x = kScanPrefix;  // before the first tile: a prefix of 0
+            if (k >= 0) {
+                for (int polls = 0; ((x = scan_peek(words + k * kK + q)) >> 62) == 0ull; ++polls)
+                    if (polls == kScanPolls) {
+                        sb.ok = 0;
+                        break;
+                    }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, (x >> 62) == 2ull);
+            const int last = m ? __ffs(m) - 1 : kWarp;  // the nearest prefix
+            int64_t v = lane <= last ? (int64_t)(x & kScanValue) : 0;
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) {
+                sb.sum[q][w] = v;
+                sb.done[q][w] = m != 0u;
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, (w >> 62) == 2ull);
-        const int last = m ? __ffs(m) - 1 : kWarp;  // the nearest prefix
-        int64_t v = lane <= last ? (int64_t)(w & kScanValue) : 0;
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        sum += v;
-        if (m) return sum;
+        __syncthreads();
+        if (!sb.ok) return false;
+        bool all = true;
+#pragma unroll
+        for (int q = 0; q < kK; ++q) {
+            for (int j = 0; j < kWarps && open[q]; ++j) {
+                pre[q] += sb.sum[q][j];
+                open[q] = !sb.done[q][j];
+            }
+            all = all && !open[q];
+        }
+        if (all) return true;
+        __syncthreads();  // the words' sums have been read
     }
 }
 
-template <class Op>
+template <class Op, int kI>
 __global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
-    constexpr int kK = Op::kVals, kI = Op::kItems, kWarps = kScanThreads / kWarp;
+    constexpr int kK = Op::kVals, kWarps = kScanThreads / kWarp;
     constexpr int kTile = kScanThreads * kI;
     if (halted(b)) return;
     Op::begin(b);
@@ -188,13 +220,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
     const int64_t ntile = n > 0 ? (n + kTile - 1) / kTile : 1;
     unsigned long long* ticket = b.scan_state + (int64_t)slot * b.scan_cap;
     unsigned long long* words = ticket + 1;
-    __shared__ int64_t s_tile, s_pre[kK], s_sum[kK][kWarps];
-    __shared__ int s_ok;
+    __shared__ int64_t s_tile, s_sum[kK][kWarps];
+    __shared__ ScanBack<kK> s_back;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
             s_tile = (int64_t)atomicAdd(ticket, 1ull);
-            s_ok = 1;
+            s_back.ok = 1;
         }
         __syncthreads();
         const int64_t tile = s_tile;
@@ -230,36 +262,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
                 total[q] += s_sum[q][j];
             }
         }
-        if (w == 0) {
-            bool ok = true;
+        int64_t pre[kK];
 #pragma unroll
-            for (int q = 0; q < kK; ++q)
-                if (lane == 0 && tile > 0) scan_post(words + tile * kK + q, kScanSum | (unsigned long long)total[q]);
-#pragma unroll
-            for (int q = 0; q < kK; ++q) {
-                const int64_t pre = tile > 0 && ok ? scan_lookback<kK>(words, tile, q, ok) : 0;
-                if (lane == 0) {
-                    s_pre[q] = pre;
-                    if (ok) scan_post(words + tile * kK + q, kScanPrefix | (unsigned long long)(pre + total[q]));
-                }
-            }
-            if (lane == 0 && !ok) {
-                s_ok = 0;
-                atomicOr(b.status, kStatusScan);
-            }
+        for (int q = 0; q < kK; ++q) {
+            pre[q] = 0;
+            if (threadIdx.x == 0 && tile > 0) scan_post(words + tile * kK + q, kScanSum | (unsigned long long)total[q]);
         }
-        __syncthreads();
-        if (!s_ok) return;
+        if (tile > 0 && !scan_lookback<kK>(words, tile, s_back, pre)) {
+            if (threadIdx.x == 0) atomicOr(b.status, kStatusScan);
+            return;
+        }
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int q = 0; q < kK; ++q) scan_post(words + tile * kK + q, kScanPrefix | (unsigned long long)(pre[q] + total[q]));
+        }
 #pragma unroll
         for (int k = 0; k < kI; ++k) {
             const int64_t i = base + k * kWarp;
 #pragma unroll
-            for (int q = 0; q < kK; ++q) e[k][q] += s_pre[q] + before[q];
+            for (int q = 0; q < kK; ++q) e[k][q] += pre[q] + before[q];
             if (i < n) Op::store(b, i, e[k], v[k]);
         }
         if (tile == ntile - 1 && threadIdx.x == 0) {
 #pragma unroll
-            for (int q = 0; q < kK; ++q) total[q] += s_pre[q];
+            for (int q = 0; q < kK; ++q) total[q] += pre[q];
             Op::total(b, n, total);
         }
     }
@@ -300,7 +326,7 @@ __global__ void k_hit_map(BatchDev b) {
 
 // hits per global module -> offsets
 struct ScanHits : ScanOp {
-    static constexpr int kVals = 1, kItems = 4;
+    static constexpr int kVals = 1, kSmall = 2, kBig = 8;
     __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) { v[0] = in ? AT(b.mod_hit, i, NG1(b)) : 0; }
     __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t*) { AT(b.mod_hit, i, NG1(b)) = e[0]; }
@@ -498,10 +524,10 @@ __device__ __forceinline__ bool sg_pair(const BatchDev& b, int a, int bmd, bool 
 }
 
 // segment candidates along the module map (Event.cc:445-522): candidate q of
-// an inner MD of global module g1 is an MD of a connected module, in
-// connection-list order
-__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int g1, int64_t q) {
-    if (AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap) return AT(b.olist, AT(b.toff, g1, NG1(b)) + q, b.olist_cap);  // k_sg_olist_fill
+// inner MD a is an MD of a connected module, in connection-list order
+__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int a, int64_t q) {
+    const int g1 = OG(b, kMD, a);
+    if (AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap) return AT(b.olist, AT(b.toff, g1, NG1(b)) + q, b.olist_cap);  // k_sg_lists
     const int n_mod = b.geo.n_mod;
     const int ev = ev_of(b, g1), m1 = g1 - ev * n_mod;
     int pref;
@@ -675,15 +701,12 @@ struct TCStage {
     __device__ static int group_of(const BatchDev& b, int t) { return OG(b, kTL, t); }
 };
 
-// inner-object count of a stage (device), clamped to the inner capacity; the
-// module-map segments' inner objects are the global modules (a module's
-// mini-doublets share one outer list, so the candidates of all of them are
-// consecutive)
+// inner-object count of a stage (device), clamped to the inner capacity
 __device__ __forceinline__ int64_t n_objects(const BatchDev& b, int st) { return min(OFF(b, st, b.n_gm), b.obj[st].cap); }
 __device__ __forceinline__ int64_t n_inner(const BatchDev& b, int st) {
     switch (st) {
         case kMD: return b.n_gm;
-        case kSG: return (b.flags & kFlagSGLayers) ? n_objects(b, kMD) : b.n_gm;
+        case kSG: return n_objects(b, kMD);
         case kTL:
         case kTP: return n_objects(b, kSG);
         default:  // track candidates: tracklets, or triplets (createTrackCandidatesFromTriplets)
@@ -695,7 +718,7 @@ __device__ __forceinline__ int64_t n_inner(const BatchDev& b, int st) {
 // bucket table (an inner object names the buckets that start in it)
 template <int st>
 struct ScanCand : ScanOp {
-    static constexpr int kVals = 1, kItems = 2;
+    static constexpr int kVals = 1, kSmall = 1, kBig = 4;
     __device__ static int64_t size(const BatchDev& b) { return n_inner(b, st); }
     __device__ static void put(const BatchDev& b, int64_t i, int64_t e, int64_t v) {
         AT(b.cand[st], i, b.cand_cap[st] + 1) = e;
@@ -730,7 +753,7 @@ __device__ __forceinline__ void rec_flush(const BatchDev& b, int st, RecBuf<kNF>
     const Recs& R = b.rec[st];
     const Objs& O = b.obj[st];
     unsigned long long p0 = 0;
-    if (lane == 0 && rb.n) p0 = atomicAdd((unsigned long long*)(b.n_rec + st), (unsigned long long)rb.n);
+    if (lane == 0 && rb.n) p0 = atomicAdd((unsigned long long*)(b.n_rec + st * kLine), (unsigned long long)rb.n);
     p0 = __shfl_sync(0xffffffffu, p0, 0);
     for (int k = lane; k < rb.n; k += kWarp) {
         const int64_t pos = (int64_t)p0 + k;
@@ -767,7 +790,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_enum(BatchDev b) {
     RecBuf<kNF> rb{rbuf[threadIdx.x >> 5]};
     for (;;) {
         unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(b.task + st, 1ull);
+        if (lane == 0) t = atomicAdd(b.task + st * kLine, 1ull);
         t = __shfl_sync(0xffffffffu, t, 0);
         if ((int64_t)t >= ntask) break;
         const int64_t base = (int64_t)t * task;
@@ -1080,7 +1103,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
     PassBuf pb{pbuf[threadIdx.x >> 5]};
     for (;;) {
         unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(b.task + kTL, 1ull);
+        if (lane == 0) t = atomicAdd(b.task + kTL * kLine, 1ull);
         t = __shfl_sync(0xffffffffu, t, 0);
         if ((int64_t)t >= ntask) break;
         const int64_t base = (int64_t)t * task;
@@ -1236,11 +1259,11 @@ __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_
     const int64_t sgcap = b.obj[kSG].cap;
     PassBuf pb{pbuf[w]};
     unsigned long long next = 0;
-    if (lane == 0) next = atomicAdd(b.task + kTL, 1ull);
+    if (lane == 0) next = atomicAdd(b.task + kTL * kLine, 1ull);
     for (;;) {
         const int64_t t = (int64_t)__shfl_sync(0xffffffffu, next, 0);
         if (t >= ntile) break;
-        if (lane == 0) next = atomicAdd(b.task + kTL, 1ull);
+        if (lane == 0) next = atomicAdd(b.task + kTL * kLine, 1ull);
         const int g = mapped ? AT(b.tile_gm, t, b.tile_cap) : tile_module(b, t);
         const int ev = ev_of(b, g), m2 = g - ev * n_mod;
         const int64_t a0 = AT(b.eoff, g, NG1(b));
@@ -1351,7 +1374,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     int nf = 0, nb = 0;
     for (;;) {
         unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(b.task + kSG, 1ull);
+        if (lane == 0) t = atomicAdd(b.task + kSG * kLine, 1ull);
         t = __shfl_sync(0xffffffffu, t, 0);
         if ((int64_t)t >= ntask) break;
         const int64_t base = (int64_t)t * task;
@@ -1369,12 +1392,8 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
             int a = 0, bmd = 0;
             bool pass = false, ob = false;
             if (c < end) {
-                // candidate c of module g: inner MD (c - off) / sum, entry (c - off) % sum of g's outer list
-                const int g = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
-                const int64_t l = c - AT(off, g, offlim), sum = AT(b.conn_sum, g, b.n_gm);
-                const int64_t k = l <= 0xffffffffll ? (int64_t)((uint32_t)l / (uint32_t)sum) : l / sum;
-                a = (int)(OFF(b, kMD, g) + k);
-                bmd = sg_outer_md(b, g, l - k * sum);
+                a = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
+                bmd = sg_outer_md(b, a, c - AT(off, a, offlim));
                 (void)IX(bmd, b.obj[kMD].cap);
                 float fv[6];
                 const MDRec orec = md_rec(b, bmd);
@@ -1905,7 +1924,7 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
 // per-module object counts of a stage -> offsets, and the layer counters
 template <int st, bool kCounters>
 struct ScanObj : ScanOp {
-    static constexpr int kVals = 1, kItems = 2;
+    static constexpr int kVals = 1, kSmall = 1, kBig = 8;
     __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
         v[0] = in ? OFF(b, st, g) : 0;
@@ -1928,7 +1947,7 @@ __global__ void k_scatter(BatchDev b, int st) {
     if (halted(b)) return;
     const Recs& R = b.rec[st];
     const Objs& O = b.obj[st];
-    const int64_t n = min(b.n_rec[st], O.cap);
+    const int64_t n = min(b.n_rec[st * kLine], O.cap);
     const int64_t flim = O.cap * (O.nf > 0 ? O.nf : 1);
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         const int g = AT(R.g, r, O.cap);
@@ -1944,7 +1963,6 @@ __global__ void k_scatter(BatchDev b, int st) {
 // ------------------------------------------------------------------ counts
 // mini-doublet candidates of a module: lower x upper hits (Event.cc:257-301)
 struct ScanMdCand : ScanCand<kMD> {
-    static constexpr int kItems = 1;
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
         int64_t c = 0;
         int ev = 0, slot = 0;
@@ -1964,106 +1982,146 @@ struct ScanMdCand : ScanCand<kMD> {
     }
 };
 
-// module g's connection entries: running sums of the connected modules'
-// object counts (stage src) -> conn_pref and conn_first per entry, conn_sum
-// per module (returned); the reference's candidate counters of stage cst get
-// n_obj(g) * conn_sum(g).  Every lane of the warp calls it.  Eight entries at
-// a time: their indices, then their offsets, so that a list of a dozen
-// costs two rounds of dependent loads instead of twelve.
-__device__ __forceinline__ int64_t conn_sums(const BatchDev& b, int64_t g, bool in, int src, int cst) {
-    constexpr int kC = 8;
+// The connection entries of 32 consecutive modules (one per lane, g; `need`:
+// the lane's sums are wanted): running sums of the connected modules' object
+// counts (stage src) -> conn_pref and conn_first per entry, conn_sum per
+// module (returned; 0 where not wanted).  Half a warp takes a module, an
+// entry per lane: the lists have 15 entries on average and 33 at most.  Every
+// lane of the warp calls it.
+__device__ __forceinline__ int64_t conn_sums(const BatchDev& b, int64_t g, bool need, int src) {
+    constexpr int kL = 16;
     const int n_mod = b.geo.n_mod;
-    int64_t sum = 0, cand = 0;
-    int ev = 0, slot = 0;
-    if (in) {
+    const int lane = threadIdx.x & 31, half = lane / kL, l = lane % kL;
+    int ev = 0, k0 = 0, k1 = 0;
+    if (need) {
         ev = ev_of(b, g);
         const int m = (int)(g - (int64_t)ev * n_mod);
-        const int k0 = AT(b.geo.conn_off, m, NM(b) + 1), k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
-        const int64_t pbase = (int64_t)ev * b.geo.n_conn, ebase = (int64_t)ev * n_mod;
-        for (int k = k0; k < k1; k += kC) {
-            int idx[kC], first[kC], cnt[kC];
-#pragma unroll
-            for (int j = 0; j < kC; ++j) idx[j] = k + j < k1 ? AT(b.geo.conn_idx, k + j, NC(b)) : -1;
-#pragma unroll
-            for (int j = 0; j < kC; ++j) {
-                first[j] = idx[j] >= 0 ? (int)OFF(b, src, ebase + idx[j]) : 0;
-                cnt[j] = idx[j] >= 0 ? (int)OFF(b, src, ebase + idx[j] + 1) - first[j] : 0;
-            }
-#pragma unroll
-            for (int j = 0; j < kC; ++j) {
-                if (idx[j] < 0) break;
-                AT(b.conn_pref, pbase + k + j, NCP(b)) = (int32_t)sum;
-                AT(b.conn_first, pbase + k + j, NCP(b)) = first[j];
-                sum += cnt[j];
-            }
-        }
-        AT(b.conn_sum, g, b.n_gm) = sum;
-        if (cst >= 0) cand = (OFF(b, src, g + 1) - OFF(b, src, g)) * sum;
-        slot = MOD(b, m).layer_slot;
+        k0 = AT(b.geo.conn_off, m, NM(b) + 1);
+        k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
     }
-    const bool act = cand != 0;
-    warp_add(act ? counter_at(b, ev, cst, 0, slot) : b.counters, (uint32_t)cand, act);
+    int64_t sum = 0;
+    for (unsigned act = __ballot_sync(0xffffffffu, k1 > k0); act;) {
+        const int j0 = __ffs(act) - 1;
+        act &= act - 1u;
+        const int j1 = act ? __ffs(act) - 1 : -1;
+        act &= act - 1u;  // (0 stays 0)
+        const int j = half ? j1 : j0, js = j < 0 ? 0 : j;
+        const int64_t ej = __shfl_sync(0xffffffffu, ev, js);
+        const int e0 = __shfl_sync(0xffffffffu, k0, js);
+        const int e1s = __shfl_sync(0xffffffffu, k1, js), e1 = j < 0 ? e0 : e1s;
+        const int64_t pbase = ej * b.geo.n_conn, ebase = ej * n_mod;
+        int run = 0;
+        for (int k = e0 + l; __any_sync(0xffffffffu, k < e1); k += kL) {
+            int first = 0, x = 0, cnt = 0;
+            if (k < e1) {
+                const int64_t g2 = ebase + AT(b.geo.conn_idx, k, NC(b));
+                first = (int)OFF(b, src, g2);
+                x = cnt = (int)OFF(b, src, g2 + 1) - first;
+            }
+#pragma unroll
+            for (int o = 1; o < kL; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o, kL);
+                if (l >= o) x += y;
+            }
+            if (k < e1) {
+                AT(b.conn_pref, pbase + k, NCP(b)) = run + x - cnt;
+                AT(b.conn_first, pbase + k, NCP(b)) = first;
+            }
+            run += __shfl_sync(0xffffffffu, x, kL - 1, kL);
+        }
+        const int r0 = __shfl_sync(0xffffffffu, run, 0), r1 = __shfl_sync(0xffffffffu, run, kL);
+        if (lane == j0) sum = r0;
+        if (lane == j1) sum = r1;
+    }
     return sum;
 }
-__global__ void k_conn_sum(BatchDev b, int src, int cst) {
+
+// the reference's candidate counters of stage st get c for an object's
+// (module's) candidates, by the layer of module g; every lane calls it
+__device__ __forceinline__ void count_cand(const BatchDev& b, int st, int64_t g, int64_t c) {
+    const bool act = c != 0;
+    int ev = 0, slot = 0;
+    if (act) {
+        ev = ev_of(b, g);
+        slot = MOD(b, g - (int64_t)ev * b.geo.n_mod).layer_slot;
+    }
+    warp_add(act ? counter_at(b, ev, st, 0, slot) : b.counters, (uint32_t)c, act);
+}
+
+// connection sums over the objects of stage src for every module, and the
+// candidate counters of stage cst (none when negative): n_obj(g) * conn_sum(g)
+__device__ __forceinline__ int64_t conn_sum_of(const BatchDev& b, int64_t g, bool in, bool need, int src, int cst) {
+    const int64_t sum = conn_sums(b, g, in && need, src);
+    if (in) AT(b.conn_sum, g, b.n_gm) = sum;
+    if (cst >= 0) count_cand(b, cst, g, in && need ? (OFF(b, src, g + 1) - OFF(b, src, g)) * sum : 0);
+    return sum;
+}
+// kEnds: only for the modules that hold objects or in which segments end
+template <bool kNeeded>
+__device__ __forceinline__ bool conn_needed(const BatchDev& b, int64_t g, bool in, int src, bool ends) {
+    return !kNeeded || (in && (OFF(b, src, g + 1) > OFF(b, src, g) || (ends && AT(b.eoff, g, NG1(b)) > 0)));
+}
+template <bool kNeeded>
+__global__ void k_conn_sum(BatchDev b, int src, int cst, bool ends) {
     if (halted(b)) return;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - threadIdx.x < b.n_gm; g += (int64_t)gridDim.x * blockDim.x)
-        (void)conn_sums(b, g, g < b.n_gm, src, cst);
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - (threadIdx.x & 31) < b.n_gm; g += (int64_t)gridDim.x * blockDim.x)
+        (void)conn_sum_of(b, g, g < b.n_gm, conn_needed<kNeeded>(b, g, g < b.n_gm, src, ends), src, cst);
 }
 
 // The front of the module-map segment stage: the connection sums over the
 // mini-doublets, the offsets of the outer lists (toff: for every global
 // module holding mini-doublets, the mini-doublets of its connected modules)
-// and of the candidates (mini-doublets x outer list).
+// and of the modules' candidates (coff: mini-doublets x outer list).
+// kFused: with the connection sums (for many modules k_conn_sum makes them).
+template <bool kFused>
 struct ScanSgFront : ScanCand<kSG> {
-    static constexpr int kVals = 2, kItems = 1;
+    static constexpr int kVals = 2, kSmall = 1, kBig = 4;
+    __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
-        const int64_t sum = conn_sums(b, g, in, kMD, kSG);
         const int64_t n = in ? OFF(b, kMD, g + 1) - OFF(b, kMD, g) : 0;
+        int64_t sum = 0;
+        if (kFused) sum = conn_sum_of(b, g, in, n > 0, kMD, kSG);
+        else if (n > 0) sum = AT(b.conn_sum, g, b.n_gm);
         v[0] = n > 0 ? sum : 0;
         v[1] = n * sum;
     }
-    __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t* v) {
+    __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t*) {
         AT(b.toff, g, NG1(b)) = e[0];
-        put(b, g, e[1], v[1]);
+        AT(b.coff, g, NG1(b)) = e[1];
     }
     __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) {
         AT(b.toff, n, NG1(b)) = t[0];
-        put_total(b, n, t[1]);
+        put_total(b, n_inner(b, kSG), t[1]);
     }
 };
 
-// The outer lists of the segment candidates, written out (entry q of g's list
-// at olist[toff[g] + q]), so that a candidate finds its outer mini-doublet
-// with one load.  A warp looks at 32 modules and writes their lists one after
-// the other, 32 entries at a time.  The lists are not written when they
-// exceed olist_cap (the candidates then search the connection list).
-__global__ void k_sg_olist_fill(BatchDev b) {
-    if (halted(b) || AT(b.toff, b.n_gm, NG1(b)) > b.olist_cap) return;
+// Eight lanes per module: the candidate offsets and buckets of its
+// mini-doublets (a module's mini-doublets have one outer list, so their
+// offsets are multiples of its length), and the outer list, written out
+// (entry q of g's list at olist[toff[g] + q]) so that a candidate finds its
+// outer mini-doublet with one load: each lane writes the mini-doublets of
+// every eighth connection.  The lists are not written when they exceed
+// olist_cap (the candidates then search the connection list).
+__global__ void k_sg_lists(BatchDev b) {
+    if (halted(b)) return;
+    constexpr int kL = 8;
+    const bool lists = AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap;
     const int n_mod = b.geo.n_mod;
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / kWarp);
-    for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x / kWarp) + (threadIdx.x >> 5)) * kWarp; base < b.n_gm;
-         base += warps * kWarp) {
-        const int64_t gl = base + lane;
-        int64_t o = 0;
-        int len = 0;
-        if (gl < b.n_gm) {
-            o = AT(b.toff, gl, NG1(b));
-            len = (int)(AT(b.toff, gl + 1, NG1(b)) - o);
-        }
-        for (unsigned m = __ballot_sync(0xffffffffu, len > 0); m; m &= m - 1u) {
-            const int j = __ffs(m) - 1;
-            const int g = (int)base + j;
-            const int64_t og = __shfl_sync(0xffffffffu, o, j);
-            const int n = __shfl_sync(0xffffffffu, len, j);
-            const int ev = ev_of(b, g), mg = g - ev * n_mod;
-            const int k0 = AT(b.geo.conn_off, mg, NM(b) + 1), k1 = AT(b.geo.conn_off, mg + 1, NM(b) + 1);
-            for (int q0 = 0; q0 < n; q0 += kWarp) {
-                const bool has = q0 + lane < n;
-                const int md = tile_outer(b, ev, mg, k0, k1, q0, has);
-                if (has) AT(b.olist, og + q0 + lane, b.olist_cap) = md;
-            }
+    const int l = threadIdx.x % kL;
+    for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kL; g < b.n_gm; g += (int64_t)gridDim.x * blockDim.x / kL) {
+        const int64_t a0 = OFF(b, kMD, g), a1 = OFF(b, kMD, g + 1);
+        if (a0 == a1) continue;
+        const int64_t o = AT(b.toff, g, NG1(b)), c0 = AT(b.coff, g, NG1(b)), sum = AT(b.conn_sum, g, b.n_gm);
+        for (int64_t a = a0 + l; a < a1; a += kL) ScanCand<kSG>::put(b, a, c0 + (a - a0) * sum, sum);
+        if (!lists) continue;
+        const int ev = ev_of(b, g), m = (int)(g - (int64_t)ev * n_mod);
+        const int k0 = AT(b.geo.conn_off, m, NM(b) + 1), k1 = AT(b.geo.conn_off, m + 1, NM(b) + 1);
+        const int64_t pbase = (int64_t)ev * b.geo.n_conn;
+        for (int k = k0 + l; k < k1; k += kL) {
+            const int64_t p = AT(b.conn_pref, pbase + k, NCP(b));
+            const int64_t n = (k + 1 < k1 ? (int64_t)AT(b.conn_pref, pbase + k + 1, NCP(b)) : sum) - p;
+            const int first = AT(b.conn_first, pbase + k, NCP(b));
+            for (int64_t i = 0; i < n; ++i) AT(b.olist, o + p + i, b.olist_cap) = first + (int)i;
         }
     }
 }
@@ -2089,13 +2147,16 @@ struct ScanSgLayers : ScanCand<kSG> {
 // segments, the offsets of the segments by the module they end in (eoff, from
 // the counts there), of the module-pair tiles (toff, with the tile -> module
 // map while it fits tile_cap; the enumeration searches toff otherwise) and
-// the candidates' total.
+// the candidates' total.  kFused as above.
+template <bool kFused>
 struct ScanTlFront : ScanOp {
-    static constexpr int kVals = 3, kItems = 1;
+    static constexpr int kVals = 3, kSmall = 1, kBig = 4;
     __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
-        const int64_t sum = conn_sums(b, g, in, kSG, kTP);
         v[0] = in ? AT(b.eoff, g, NG1(b)) : 0;
+        int64_t sum = 0;
+        if (kFused) sum = conn_sum_of(b, g, in, conn_needed<true>(b, g, in, kSG, true), kSG, kTP);
+        else if (v[0] > 0) sum = AT(b.conn_sum, g, b.n_gm);
         v[1] = tile_count(v[0], sum);
         v[2] = v[0] * sum;
     }
@@ -2157,7 +2218,7 @@ __global__ void k_join_count(BatchDev b, int st, bool second) {
 }
 template <bool kSecond>
 struct ScanJoin : ScanOp {
-    static constexpr int kVals = 1, kItems = 4;
+    static constexpr int kVals = 1, kSmall = 2, kBig = 8;
     __device__ static int64_t* off(const BatchDev& b) { return kSecond ? b.joff2 : b.joff; }
     __device__ static int64_t size(const BatchDev& b) { return n_objects(b, kMD); }
     __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) {
@@ -2418,7 +2479,7 @@ __global__ void __launch_bounds__(256) k_clear(BatchDev b, ClearJobs j) {
 __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
     stamp(b);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-    if (t < kNumStages) host[kRunRec + t] = b.n_rec[t];
+    if (t < kNumStages) host[kRunRec + t] = b.n_rec[t * kLine];
     if (t == kNumStages) host[kRunStatus] = (int64_t)*b.status;
     if (t == kNumStages + 1) host[kRunKept] = (int64_t)max(*b.n_kept, *b.n_kept_sg);
     // (this kernel's own stamp is written by the thread that copies it)
@@ -2433,10 +2494,20 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
     for (int64_t i = t; i < (int64_t)b.n_ev * 110; i += stride) c[i] = b.counters[i];
 }
 
-// cap: an upper bound of the number of elements
+// cap: an upper bound of the number of elements.  A round of tiles (about 300
+// CTAs in flight) takes around ten microseconds whatever its size, so the
+// tiles are large where there would be several rounds of small ones (objects
+// per module of 64 events, 2.2M modules: 46 us at 4 per thread, 35 at 8; of
+// one event, 22k modules: 11 us at 4, 8 at 1).  The connection sums of many
+// modules are a kernel of their own for the same reason (64 events: 62 + 43 us
+// against 300 us within the scan; one event: 15 us within it).
+constexpr int64_t kScanSmall = (int64_t)1 << 18;
 template <class Op>
 void scan(const BatchDev& b, int slot, int64_t cap, cudaStream_t s, Hooks* h) {
-    k_scan<Op><<<grid_for(cap, kScanThreads * Op::kItems, b.n_sm * 8), kScanThreads, 0, s>>>(take(b, h), slot);
+    if (cap <= kScanSmall)
+        k_scan<Op, Op::kSmall><<<grid_for(cap, kScanThreads * Op::kSmall, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
+    else
+        k_scan<Op, Op::kBig><<<grid_for(cap, kScanThreads * Op::kBig, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
 }
 
 int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : 8; }
@@ -2495,8 +2566,14 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
         enum_and_group<SGLayerStage, ScanSgLayers, false>(b, s, h);
         return;
     }
-    scan<ScanSgFront>(b, kScanCand + kSG, b.n_gm, s, h);
-    k_sg_olist_fill<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h));
+    const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
+    if (b.n_gm <= kScanSmall) {
+        scan<ScanSgFront<true>>(b, kScanCand + kSG, b.n_gm, s, h);
+    } else {
+        k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kMD, kSG, false);
+        scan<ScanSgFront<false>>(b, kScanCand + kSG, b.n_gm, s, h);
+    }
+    k_sg_lists<<<grid_for(8 * (int64_t)b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h));
     // first cuts -> survivor list -> whole algorithm (k_sg_enum_a, k_sg_b)
     mark(h, kStampEnum + kSG);
     BatchDev l = b;  // with this list's own counts
@@ -2528,11 +2605,17 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_sg_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     // module-map candidates: the module-pair tiles (k_tl_enum_tiles)
     const bool tiles = !(b.flags & (kFlagTLLayers | kFlagTLNav));
+    const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
     if (tiles) {
-        scan<ScanTlFront>(b, kScanTlFront, b.n_gm, s, h);
+        if (b.n_gm <= kScanSmall) {
+            scan<ScanTlFront<true>>(b, kScanTlFront, b.n_gm, s, h);
+        } else {
+            k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kSG, kTP, true);
+            scan<ScanTlFront<false>>(b, kScanTlFront, b.n_gm, s, h);
+        }
         k_sg_end_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     } else {
-        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kSG, kTP);
+        k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kSG, kTP, false);
         if (b.flags & kFlagTLNav) join_index(b, kSG, kScanJoinNav, s, h);  // segments by inner MD: the outward lists
         scan<ScanTlCand<true>>(b, kScanCand + kTL, b.cand_cap[kTL], s, h);
     }
@@ -2586,14 +2669,14 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
             join_index(b, kSG, kScanJoinTc, s, h);           // segments by inner MD
             join_index(b, kTP, kScanJoinTc2, s, h, true);  // triplets by innermost MD
         }
-        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTP, -1);
+        k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTP, -1, false);
         if (map) enum_and_group<TCTPMapStage, ScanTcFromTp>(b, s, h);
         else enum_and_group<TCTPStage, ScanTcFromTp>(b, s, h);
         return;
     }
     join_index(b, kTL, kScanJoinTc, s, h);
     if (b.flags & kFlagTCFromTL) {
-        k_conn_sum<<<grid_for(b.n_gm, 256, b.n_sm * 16), 256, 0, s>>>(take(b, h), kTL, -1);
+        k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTL, -1, false);
         enum_and_group<TCStage, ScanTcFromTl>(b, s, h);
     } else {
         enum_and_group<TCStage, ScanTcCand>(b, s, h);

@@ -8,6 +8,10 @@
 
 namespace sdlg {
 
+// Counters that kernels update atomically at the same time lie 256 bytes
+// apart (8-byte words): atomics on one line take turns at its L2 slice.
+constexpr int64_t kLine = 32;
+
 struct BatchDev {
     Geometry geo;
     int n_ev;
@@ -33,7 +37,7 @@ struct BatchDev {
     Recs rec[kNumStages];
     int64_t* cand[kNumStages];     // per inner object candidate counts -> offsets (cap_inner + 1)
     int64_t cand_cap[kNumStages];
-    int64_t* n_rec;                // kNumStages attempted appends
+    int64_t* n_rec;                // per stage (kLine apart): attempted appends
     // connection-list prefix sums of per-module object counts
     int32_t* conn_pref;            // n_ev * n_conn
     int32_t* conn_first;           // n_ev * n_conn: offset of the entry's module's first object
@@ -46,7 +50,7 @@ struct BatchDev {
     float* mdpack;                 // mini-doublet cap * kMdPack: packed records for the segment stage
     uint32_t* counters;            // n_ev * 110
     uint32_t* status;
-    unsigned long long* task;      // kNumStages work counters
+    unsigned long long* task;      // per stage (kLine apart): work counter
     unsigned long long* scan_state;  // kScanSlots x scan_cap: per scan the tile counter and a word per tile and value
     int64_t scan_cap;
     int32_t* bucket;               // first inner object of every 256 consecutive candidates of the running stage
@@ -84,7 +88,8 @@ struct BatchDev {
     int64_t* toff;                 // n_gm + 1: tile counts -> offsets
     int32_t* tile_gm;              // tile_cap: the global module of each tile (when the tiles fit)
     int64_t tile_cap;
-    int32_t* olist;                // olist_cap: the segment candidates' outer lists (k_sg_olist_fill; offsets in toff)
+    int64_t* coff;                 // n_gm + 1: offsets of the modules' segment candidates
+    int32_t* olist;                // olist_cap: the segment candidates' outer lists (k_sg_lists; offsets in toff)
     int64_t olist_cap;
     int4* pb;                      // candidates through phase B1: (inner, outer, algorithm, muls bits), BBBB
                                    //   from the front, the others from the back
@@ -115,10 +120,10 @@ enum ScanSlot : int {
     kScanJoinTc2,
     kScanSlots
 };
-// words of one slot for scans over up to n_gm global modules (tiles of at
-// least 256, up to 3 values each) and objects (tiles of at least 512)
+// words of one slot for scans over up to n_gm global modules (up to 3 values
+// each) and objects, in tiles of at least 512
 constexpr int64_t scan_words(int64_t n_gm, int64_t objects) {
-    return 1 + (3 * (n_gm / 256 + 1) > objects / 512 + 1 ? 3 * (n_gm / 256 + 1) : objects / 512 + 1);
+    return 1 + (3 * (n_gm / 512 + 1) > objects / 512 + 1 ? 3 * (n_gm / 512 + 1) : objects / 512 + 1);
 }
 
 // Device time stamps of a run.  An event node in a CUDA graph costs about
