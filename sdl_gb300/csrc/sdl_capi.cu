@@ -415,9 +415,10 @@ int ensure_buffers(sdlg_ctx* ctx) {
     int rc;
 #define AL(ptr, n) if ((rc = dalloc(ctx, &(ptr), (n))) != SDLG_OK) return rc
     int64_t* small;
-    AL(small, 1 + kNumStamps);
+    AL(small, 1 + kNumStamps + kNumStages);
     b.n_hit = small;
     b.stamps = reinterpret_cast<unsigned long long*>(small + 1);
+    b.task_size = reinterpret_cast<int*>(small + 1 + kNumStamps);
     // the small counts that every run starts from zero
     int64_t* zero;
     AL(zero, kZeroWords);

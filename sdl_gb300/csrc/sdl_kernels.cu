@@ -44,6 +44,7 @@ __device__ __forceinline__ int64_t checked_idx(int64_t i, int64_t lim, int line,
 constexpr int kWarp = 32;
 constexpr int kEnumThreads = 256;
 constexpr int kTaskDefault = 256;  // candidates per warp task unless tuned
+constexpr int kGridDefault = 8;    // CTAs per SM of an enumeration unless tuned
 
 // the launch's device time stamps (none for most launches)
 __device__ __forceinline__ void stamp(const BatchDev& b) {
@@ -725,8 +726,17 @@ struct ScanCand : ScanOp {
         for (int64_t k = (e + (1ll << kBucketShift) - 1) >> kBucketShift; (k << kBucketShift) < e + v; ++k)
             if (k < b.bucket_cap) AT(b.bucket, k, b.bucket_cap) = (int)i;
     }
+    // and the candidates per warp task of the enumeration: the stage's size
+    // where there are enough candidates, less where that would leave warps
+    // without a task (a 2.3k-hit event's 2,000 mini-doublet candidates were
+    // nine tasks of 256, eight dependent rounds each: 67 us for the stage
+    // against 31 us)
     __device__ static void put_total(const BatchDev& b, int64_t n, int64_t t) {
         AT(b.cand[st], n, b.cand_cap[st] + 1) = t;
+        const int64_t warps = (int64_t)b.n_sm * (b.enum_grid[st] > 0 ? b.enum_grid[st] : kGridDefault) * (kEnumThreads / kWarp);
+        int task = b.enum_task[st] > 0 ? b.enum_task[st] : kTaskDefault;
+        while (task > kWarp && t < warps * task) task = max(kWarp, (task >> 1) / kWarp * kWarp);
+        b.task_size[st] = task;
         const int64_t nb = (t + (1ll << kBucketShift) - 1) >> kBucketShift;
         if (n > 0 && nb < b.bucket_cap) AT(b.bucket, nb, b.bucket_cap) = (int)(n - 1);
     }
@@ -784,7 +794,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_enum(BatchDev b) {
     const int64_t* off = b.cand[st];
     const int64_t offlim = b.cand_cap[st] + 1;
     const int64_t total = AT(off, nobj, offlim);
-    const int task = b.enum_task[st] > 0 ? b.enum_task[st] : kTaskDefault;
+    const int task = b.task_size[st];
     const int64_t ntask = (total + task - 1) / task;
     const int lane = threadIdx.x & 31;
     RecBuf<kNF> rb{rbuf[threadIdx.x >> 5]};
@@ -1096,7 +1106,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
     const int64_t* off = b.cand[kTL];
     const int64_t offlim = b.cand_cap[kTL] + 1;
     const int64_t total = AT(off, nobj, offlim);
-    const int task = b.enum_task[kTL] > 0 ? b.enum_task[kTL] : kTaskDefault;
+    const int task = b.task_size[kTL];
     const int64_t ntask = (total + task - 1) / task;
     const int lane = threadIdx.x & 31;
     const int lay = tl_variant(b);
@@ -1366,7 +1376,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     const int64_t* off = b.cand[kSG];
     const int64_t offlim = b.cand_cap[kSG] + 1;
     const int64_t total = AT(off, nobj, offlim);
-    const int task = b.enum_task[kSG] > 0 ? b.enum_task[kSG] : kTaskDefault;
+    const int task = b.task_size[kSG];
     const int64_t ntask = (total + task - 1) / task;
     const int lane = threadIdx.x & 31;
     int4* fb = sbuf[threadIdx.x >> 5][0];
@@ -2510,7 +2520,7 @@ void scan(const BatchDev& b, int slot, int64_t cap, cudaStream_t s, Hooks* h) {
         k_scan<Op, Op::kBig><<<grid_for(cap, kScanThreads * Op::kBig, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
 }
 
-int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : 8; }
+int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : kGridDefault; }
 
 // stage F's candidates (their offsets scanned by Cand) -> objects
 template <class F, class Cand, bool kCounters = true>

@@ -60,6 +60,7 @@ struct BatchDev {
     // candidates per warp task (a multiple of 32) and CTAs per SM
     int enum_task[kNumStages];
     int enum_grid[kNumStages];
+    int* task_size;                // per stage: candidates per warp task of this run (ScanCand)
     const unsigned char* mlp_pack; // packed pre-filter weights and threshold (kPackBytes)
     MlpStats* mlp_stats;           // pre-filter counts of the last run
     int4* passa;                   // tracklet candidates through phase A: (inner, outer, algorithm, 1 when

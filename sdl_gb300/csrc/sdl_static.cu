@@ -35,7 +35,7 @@ constexpr int64_t kMaxModules = SDLG_STATIC_MAX_MODULES;
 constexpr int64_t kMaxMD = SDLG_STATIC_MAX_MINI_DOUBLETS;
 
 // Layout of the array, in 8-byte words.
-constexpr int64_t kSmall = 0;                                   // n_hit, (free), n_rec[5]
+constexpr int64_t kSmall = 0;                                   // n_hit, (free), n_rec[5], (free), task_size
 constexpr int64_t kEvOff = 16;                                  // ev_off[2]
 constexpr int64_t kModHit = kEvOff + 2;                         // kMaxModules + 1
 constexpr int64_t kCandMD = kModHit + kMaxModules + 1;          // kMaxModules + 1
@@ -148,6 +148,7 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.n_gm = geo.n_mod;
     b.n_hit_cap = H;
     b.n_hit = w64 + kSmall;
+    b.task_size = reinterpret_cast<int*>(w64 + kSmall + 8);
     b.n_rec = w64 + kSmall + 2;
     b.ev_off = w64 + kEvOff;
     b.in_x = d_x; b.in_y = d_y; b.in_z = d_z; b.in_idx = d_idx; b.in_det = d_detid;
