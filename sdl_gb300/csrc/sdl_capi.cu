@@ -101,6 +101,7 @@ struct sdlg_ctx {
     std::vector<uint32_t> detids;  // sorted module table
     std::vector<ModDev> mods;
     std::vector<int32_t> conn_off, conn_idx;
+    bool conn_dup = false;  // some connection list repeats a module
     // device geometry
     uint32_t* d_detid = nullptr;
     ModDev* d_mod = nullptr;
@@ -336,6 +337,7 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
     }
     ctx->conn_off.assign(n + 1, 0);
     ctx->conn_idx.clear();
+    ctx->conn_dup = false;
     for (int i = 0; i < n; ++i) {
         auto it = ctx->hg.conn.find(valid[i]);
         if (it != ctx->hg.conn.end())
@@ -344,6 +346,9 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
                 if (k >= 0) ctx->conn_idx.push_back(k);
             }
         ctx->conn_off[i + 1] = (int32_t)ctx->conn_idx.size();
+        std::vector<int32_t> l(ctx->conn_idx.begin() + ctx->conn_off[i], ctx->conn_idx.end());
+        std::sort(l.begin(), l.end());
+        ctx->conn_dup = ctx->conn_dup || std::adjacent_find(l.begin(), l.end()) != l.end();
     }
     // layers as runs of consecutive module indices (Layer.cc:3-50 pairs layers)
     std::vector<std::vector<int32_t>> runs(kNumSlots);
@@ -400,6 +405,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.geo.mod = ctx->d_mod;
     b.geo.conn_off = ctx->d_conn_off;
     b.geo.conn_idx = ctx->d_conn_idx;
+    b.geo.conn_dup = ctx->conn_dup;
     b.geo.slot_run = ctx->d_slot_run;
     b.geo.n_slot_run = (int)ctx->slot_run.size();
     b.n_ev = (int)ctx->n_ev;
@@ -449,6 +455,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
         Recs& R = b.rec[s];
         O.cap = C; O.nf = nf[s]; R.nf = nf[s];
         AL(O.i, C); AL(O.j, C); AL(O.g, C); AL(O.f, C * std::max(1, nf[s])); AL(O.mod_cnt, n_gm + 1);
+        if (s == kTP) continue;  // triplets are written in place
         AL(R.i, C); AL(R.j, C); AL(R.g, C); AL(R.rank, C); AL(R.f, C * std::max(1, nf[s]));
     }
     b.cand_cap[kMD] = n_gm;
@@ -477,13 +484,17 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.scan_cap = scan_words(n_gm, mx);
     AL(b.scan_state, kScanSlots * b.scan_cap);
     AL(b.joff, ctx->cap_obj[kMD] + 1);
-    AL(b.jcur, ctx->cap_obj[kMD]);
-    AL(b.jidx, std::max(ctx->cap_obj[kSG], ctx->cap_obj[kTL]));
+    AL(b.jrank, ctx->cap_obj[kSG]);
+    AL(b.jidx, ctx->cap_obj[kSG]);
     AL(b.joff2, ctx->cap_obj[kMD] + 1);
     AL(b.jcur2, ctx->cap_obj[kMD]);
     AL(b.jidx2, ctx->cap_obj[kTP]);
+    AL(b.joft, ctx->cap_obj[kSG] + 1);
+    AL(b.trank, ctx->cap_obj[kTL]);
+    AL(b.jidt, ctx->cap_obj[kTL]);
+    AL(b.sgkey, b.geo.conn_dup ? ctx->cap_obj[kSG] : 1);
     AL(b.eoff, n_gm + 1);
-    AL(b.ecur, n_gm);
+    AL(b.erank, ctx->cap_obj[kSG]);
     AL(b.eidx, ctx->cap_obj[kSG]);
     AL(b.toff, n_gm + 1);
     AL(b.coff, n_gm + 1);
@@ -511,13 +522,16 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
     BatchDev& b = ctx->b;
     ClearJobs j{};
     const int64_t n_gm = b.n_gm;
+    // objects counted per module as they are made (the joins write their offsets)
+    auto counted = [&](int st) { return st <= kTL || (st == kTC && (b.flags & kFlagTCFromTP)); };
     // (a later stage's own run keeps the pass times of the stages before it)
     j.stamps = first == 0 ? kNumStamps : kStampEnd + 1;
     if (first == 0) {
         j.add(b.n_rec, 2 * kZeroWords);
         j.add(b.counters, (int64_t)b.n_ev * 110);
         j.add(b.mod_hit, 2 * (n_gm + 1));
-        for (int st = 0; st < kNumStages; ++st) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
+        for (int st = 0; st < kNumStages; ++st)
+            if (counted(st)) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
         j.add(b.mlp_stats, sizeof(MlpStats) / 4);
     } else {
         const int ns = last - first + 1;
@@ -536,14 +550,12 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
             j.add(b.counters + st * 22 + skip, 22 - skip, b.n_ev, 110);
         }
         if (first <= kTL && last >= kTL) j.add(b.counters + kTP * 22, 11, b.n_ev, 110);
-        for (int st = first; st <= last; ++st) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
+        for (int st = first; st <= last; ++st)
+            if (counted(st)) j.add(b.obj[st].mod_cnt, 2 * (n_gm + 1));
         if (first <= kTL && last >= kTL) j.add(b.mlp_stats, sizeof(MlpStats) / 4);
     }
     j.add(b.scan_state, 2 * kScanSlots * b.scan_cap);
-    if (last >= kTL && first <= kTL) {
-        j.add(b.eoff, 2 * (n_gm + 1));
-        j.add(b.ecur, n_gm);
-    }
+    if (last >= kTL && first <= kTL) j.add(b.eoff, 2 * (n_gm + 1));
     launch_clear(b, j, ctx->stream, &ctx->hooks);
 }
 
@@ -556,6 +568,8 @@ void enqueue_chain(sdlg_ctx* ctx, int first, int last) {
     Hooks* h = &ctx->hooks;
     h->launches = 0;
     h->ts = stamp_bit(kStampStart);
+    b.first = first;
+    b.last = last;
     enqueue_clear(ctx, first, last);
     if (first == 0) launch_ingest(b, s, h);
     for (int st = first; st <= last; ++st) {
@@ -588,6 +602,8 @@ int launch_checked(sdlg_ctx* ctx, int first, int last) {
     int rc;
     h->launches = 0;
     h->ts = stamp_bit(kStampStart);
+    b.first = first;
+    b.last = last;
     enqueue_clear(ctx, first, last);
     if (first == 0) launch_ingest(b, s, h);
     if ((rc = check_stage(ctx, "ingest"))) return rc;
@@ -2001,6 +2017,7 @@ bool ctx_geometry(const sdlg_ctx* ctx, Geometry* g, int* device, int* n_sm) {
     g->mod = ctx->d_mod;
     g->conn_off = ctx->d_conn_off;
     g->conn_idx = ctx->d_conn_idx;
+    g->conn_dup = ctx->conn_dup;
     g->slot_run = ctx->d_slot_run;
     g->n_slot_run = (int)ctx->slot_run.size();
     *device = ctx->device;

@@ -402,6 +402,7 @@ __device__ __forceinline__ float OF(const BatchDev& b, int st, int f, int64_t k)
     return AT(O.f, (int64_t)f * O.cap + k, O.cap * (O.nf > 0 ? O.nf : 1));
 }
 __device__ __forceinline__ int64_t OFF(const BatchDev& b, int st, int64_t g) { return AT(b.obj[st].mod_cnt, g, NG1(b)); }
+__device__ __forceinline__ int64_t n_objects(const BatchDev& b, int st) { return min(OFF(b, st, b.n_gm), b.obj[st].cap); }
 
 
 // ------------------------------------------------------------------ stage functors
@@ -474,23 +475,24 @@ __device__ __forceinline__ MDRec md_rec(const BatchDev& b, int64_t a) {
 
 __global__ void k_md_pack(BatchDev b) {
     if (halted(b)) return;
-    const int64_t n = min(OFF(b, kMD, b.n_gm), b.obj[kMD].cap);  // mini-doublets
+    const int64_t n = n_objects(b, kMD);
     for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
         const int lm = mod_of(b, OG(b, kMD, a));
-        const int anc = md_anchor(MOD(b, lm), OI(b, kMD, a), OJ(b, kMD, a));
+        const ModDev& M = MOD(b, lm);
+        const int anc = md_anchor(M, OI(b, kMD, a), OJ(b, kMD, a));
         const P3 p = hit(b, anc);
+        const float a1 = AT(b.ha1, anc, H(b));
         float4* q = reinterpret_cast<float4*>(&AT(b.mdpack, a * kMdPack, b.obj[kMD].cap * kMdPack));
         q[0] = make_float4(p.x, p.y, p.z, p.rt);
-        q[1] = make_float4(p.phi, p.r3, AT(b.ha1, anc, H(b)), AT(b.htf, anc, H(b)));
+        q[1] = make_float4(p.phi, p.r3, a1, AT(b.htf, anc, H(b)));
         q[2] = make_float4(OF(b, kMD, 0, a), OF(b, kMD, 1, a), OF(b, kMD, 2, a), OF(b, kMD, 3, a));
         // what the segment algorithms compute from this mini-doublet alone as
         // the outer one: the barrel cut for the layer below, the endcap strip
         // edges' phi
-        const ModDev& M = MOD(b, lm);
         const int am = mod_of(b, AT(b.hgm, anc, H(b)));
         float c0 = 0.f, c1 = 0.f;
         if (M.subdet == kBarrel) {
-            if (M.layer >= 2) c0 = sg_barrel_cut(M.layer - 1, p.rt, AT(b.ha1, anc, H(b)));
+            if (M.layer >= 2) c0 = sg_barrel_cut(M.layer - 1, p.rt, a1);
         } else if (M.type == kTwoS) {
             c0 = strip_edge(p, MOD(b, am), true).phi;
             c1 = strip_edge(p, MOD(b, am), false).phi;
@@ -637,13 +639,18 @@ __device__ __forceinline__ int tl_outer_layer(const BatchDev& b, int s, int64_t 
     return layer_object(b, kSG, ev, tl_layer_outer(MOD(b, g1 - ev * n_mod).layer_slot), q);
 }
 
-// The triplets and track candidates are equi-joins on a mini-doublet: the
-// join index lists the objects of stage st (segments, or tracklets) by their
-// key mini-doublet (a segment's inner one; a tracklet's inner segment's inner
-// one), so that each join visits only matching objects (joff: offsets per
-// mini-doublet, jidx: the objects).
+// The triplets and track candidates are equi-joins.  A triplet's segments
+// share a mini-doublet: the join index lists the segments by their inner one
+// (joff: offsets per mini-doublet, jidx: the segments), so that each join
+// visits only matching objects.  A track candidate's tracklets share a segment
+// (the same two mini-doublets): the tracklets by their inner segment (joft,
+// jidt).  A connection list that repeats a module makes its segments several
+// times; all of them go by the first of the same mini-doublets (sgkey).
 __device__ __forceinline__ int join_key(const BatchDev& b, int st, int64_t o) {
-    return st == kSG ? OI(b, kSG, o) : OI(b, kSG, OI(b, st, o));  // tracklets, triplets: inner segment's inner MD
+    return st == kSG ? OI(b, kSG, o) : OI(b, kSG, OI(b, st, o));  // triplets: inner segment's inner MD
+}
+__device__ __forceinline__ int sg_key(const BatchDev& b, int s) {
+    return b.geo.conn_dup ? AT(b.sgkey, s, b.obj[kSG].cap) : s;
 }
 // the second index (the triplets by their innermost MD)
 __device__ __forceinline__ int64_t join2_n(const BatchDev& b, int md) {
@@ -656,54 +663,10 @@ __device__ __forceinline__ int64_t join_n(const BatchDev& b, int md) {
     return AT(b.joff, md + 1, b.obj[kMD].cap + 1) - AT(b.joff, md, b.obj[kMD].cap + 1);
 }
 __device__ __forceinline__ int join_obj(const BatchDev& b, int md, int64_t k) {
-    return AT(b.jidx, AT(b.joff, md, b.obj[kMD].cap + 1) + k, max(b.obj[kSG].cap, b.obj[kTL].cap));
+    return AT(b.jidx, AT(b.joff, md, b.obj[kMD].cap + 1) + k, b.obj[kSG].cap);
 }
 
-// triplet candidates (Event.cc:524-597 via Triplet.cc:55): candidate q of
-// inner segment s1 is the (q mod n)-th segment starting at its outer
-// mini-doublet; the multiplicity of the outer module in the connection list
-// repeats each, as the reference's nested loops do (k_tp_count)
-struct TPStage {
-    static constexpr int kSt = kTP;
-    __device__ static bool eval(const BatchDev& b, int s1, int64_t q, int& oi, int& oj, float* fv) {
-        const int omd = OJ(b, kSG, s1);
-        const int64_t n2 = join_n(b, omd);
-        if (n2 <= 0) {
-#ifdef SDL_DEVICE_CHECKS
-            IX(-2, 0);
-#endif
-            return false;
-        }
-        oi = s1;
-        oj = join_obj(b, omd, q % n2);
-        (void)fv;
-        return true;
-    }
-    __device__ static int group_of(const BatchDev& b, int s) { return OG(b, kSG, s); }
-};
-
-// track candidates (Event.cc:823-872, and 984-1062 for
-// createTrackCandidatesFromTracklets, via TrackCandidate.cc:161): candidate q
-// of inner tracklet t1 is the (q mod n)-th of the n tracklets whose inner
-// segment starts at the inner mini-doublet of t1's outer segment (repeated
-// connections repeat them, k_tc_count_tl); it matches when that segment's
-// outer mini-doublet is the same too
-struct TCStage {
-    static constexpr int kSt = kTC;
-    __device__ static bool eval(const BatchDev& b, int t1, int64_t q, int& oi, int& oj, float* fv) {
-        const int sB = OJ(b, kTL, t1);
-        const int mB = OI(b, kSG, sB);
-        const int t2 = join_obj(b, mB, q % join_n(b, mB));  // n > 0 when t1 has candidates
-        const int sC = OI(b, kTL, t2);
-        oi = t1; oj = t2;
-        (void)fv;
-        return OI(b, kSG, sC) == OI(b, kSG, sB) && OJ(b, kSG, sC) == OJ(b, kSG, sB);  // TrackCandidate.cc:161
-    }
-    __device__ static int group_of(const BatchDev& b, int t) { return OG(b, kTL, t); }
-};
-
 // inner-object count of a stage (device), clamped to the inner capacity
-__device__ __forceinline__ int64_t n_objects(const BatchDev& b, int st) { return min(OFF(b, st, b.n_gm), b.obj[st].cap); }
 __device__ __forceinline__ int64_t n_inner(const BatchDev& b, int st) {
     switch (st) {
         case kMD: return b.n_gm;
@@ -893,38 +856,46 @@ __device__ __forceinline__ void sg_pack_record(const BatchDev& b, int im, int om
     }
 }
 
+// what the tracklet and triplet stages read of segment s (mini-doublets im
+// and om, f6 as kept): the packed record, the outer-role fields, the
+// pre-filter's features; and its place among the segments that end in its
+// outer module (eoff counts, erank) and that start at its inner mini-doublet
+// (joff counts, jrank)
+__device__ __forceinline__ void sg_pack_write(const BatchDev& b, int64_t s, int im, int om, const float* f6) {
+    float v[PK_N];
+    sg_pack_record(b, im, om, f6, v);
+    const uint32_t fl = __float_as_uint(v[PK_FLAGS]);
+    const int64_t C = b.obj[kSG].cap;
+    AT(b.erank, s, C) = (int)atomicAdd((unsigned long long*)&AT(b.eoff, __float_as_int(v[PK_G2]), NG1(b)), 1ull);
+    AT(b.jrank, s, C) = (int)atomicAdd((unsigned long long*)&AT(b.joff, im, b.obj[kMD].cap + 1), 1ull);
+    const int fo[10] = {PK_LRT, PK_LZ, PK_LTD, PK_LA1, PK_UPHI, PK_FLAGS, -1, PK_LX, PK_LY, PK_UX};
+#pragma unroll
+    for (int k = 0; k < 10; ++k)
+        if (k != 6) AT(b.sgouter, k * C + s, 11 * C) = v[fo[k]];
+    AT(b.sgouter, 6 * C + s, 11 * C) = 0.1f / v[PK_LRT];  // the PV-offset term of an outer segment
+    AT(b.sgouter, 10 * C + s, 11 * C) = v[PK_UY];
+    float4* dst = reinterpret_cast<float4*>(&AT(b.sgpack, s * PK_N, C * PK_N));
+    for (int k = 0; k < PK_N / 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    // the pre-filter's feature records (inner role, outer role)
+    const float lz = v[PK_LZ], lrt = v[PK_LRT], uz = v[PK_UZ], urt = v[PK_URT];
+    const float drIn = urt - lrt;
+    const float slope = (uz - lz) / (fabsf(drIn) > 1e-3f ? drIn : copysignf(1e-3f, drIn));
+    const float scode = ((fl & F_LO_E) ? 1.f : 0.f) + ((fl & F_LO_PS) ? 0.25f : 0.f);
+    const float tcode = ((fl & F_UP_E) ? 0.5f : 0.f) + ((fl & F_UP_2S) ? 0.125f : 0.f);
+    float4* fd = reinterpret_cast<float4*>(&AT(b.sgfeat, s * kFeatN, C * kFeatN));
+    fd[0] = make_float4(v[PK_LX], v[PK_LY], lz, lrt);
+    fd[1] = make_float4(v[PK_LPHI], v[PK_DPC], slope, scode);
+    fd[2] = make_float4(v[PK_UX], v[PK_UY], uz, urt);
+    fd[3] = make_float4(v[PK_UPHI], v[PK_ALPHAUP], tcode, 0.f);
+}
 __global__ void k_sg_pack(BatchDev b) {
     if (halted(b)) return;
-    const int64_t n = n_inner(b, kTL);
+    const int64_t n = n_objects(b, kSG);
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
         float f6[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k) f6[k] = OF(b, kSG, k, s);
-        float v[PK_N];
-        sg_pack_record(b, OI(b, kSG, s), OJ(b, kSG, s), f6, v);
-        const uint32_t fl = __float_as_uint(v[PK_FLAGS]);
-        const int64_t C = b.obj[kSG].cap;
-        const int fo[10] = {PK_LRT, PK_LZ, PK_LTD, PK_LA1, PK_UPHI, PK_FLAGS, -1, PK_LX, PK_LY, PK_UX};
-#pragma unroll
-        for (int k = 0; k < 10; ++k)
-            if (k != 6) AT(b.sgouter, k * C + s, 11 * C) = v[fo[k]];
-        AT(b.sgouter, 6 * C + s, 11 * C) = 0.1f / v[PK_LRT];  // the PV-offset term of an outer segment
-        AT(b.sgouter, 10 * C + s, 11 * C) = v[PK_UY];
-        // segments per module of their outer mini-doublet (ScanTlFront)
-        atomicAdd((unsigned long long*)&AT(b.eoff, __float_as_int(v[PK_G2]), NG1(b)), 1ull);
-        float4* dst = reinterpret_cast<float4*>(&AT(b.sgpack, s * PK_N, b.obj[kSG].cap * PK_N));
-        for (int k = 0; k < PK_N / 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-        // the pre-filter's feature records (inner role, outer role)
-        const float lz = v[PK_LZ], lrt = v[PK_LRT], uz = v[PK_UZ], urt = v[PK_URT];
-        const float drIn = urt - lrt;
-        const float slope = (uz - lz) / (fabsf(drIn) > 1e-3f ? drIn : copysignf(1e-3f, drIn));
-        const float scode = ((fl & F_LO_E) ? 1.f : 0.f) + ((fl & F_LO_PS) ? 0.25f : 0.f);
-        const float tcode = ((fl & F_UP_E) ? 0.5f : 0.f) + ((fl & F_UP_2S) ? 0.125f : 0.f);
-        float4* fd = reinterpret_cast<float4*>(&AT(b.sgfeat, s * kFeatN, b.obj[kSG].cap * kFeatN));
-        fd[0] = make_float4(v[PK_LX], v[PK_LY], lz, lrt);
-        fd[1] = make_float4(v[PK_LPHI], v[PK_DPC], slope, scode);
-        fd[2] = make_float4(v[PK_UX], v[PK_UY], uz, urt);
-        fd[3] = make_float4(v[PK_UPHI], v[PK_ALPHAUP], tcode, 0.f);
+        sg_pack_write(b, s, OI(b, kSG, s), OJ(b, kSG, s), f6);
     }
 }
 
@@ -1167,20 +1138,23 @@ __device__ __forceinline__ int64_t tile_count(int64_t na, int64_t nb) {
     return (na > 0 && nb > 0) ? ((na + kTileA - 1) / kTileA) * ((nb + kWarp - 1) / kWarp) : 0;
 }
 
-// the segments by the global module of their outer mini-doublet (eoff
-// scanned), and the reference's tracklet candidate counters (Event.cc:635-663)
-__global__ void k_sg_end_scatter(BatchDev b) {
+// the segments by their inner mini-doublet (joff scanned) and, for the
+// module-map tracklets, by the global module of their outer one (eoff
+// scanned) with the reference's candidate counters (Event.cc:635-663)
+__global__ void k_sg_index(BatchDev b) {
     if (halted(b)) return;
     const int n_mod = b.geo.n_mod;
-    const int64_t n = n_inner(b, kTL);
+    const int64_t n = n_objects(b, kSG), C = b.obj[kSG].cap;
+    const bool map = tl_variant(b) == 0;
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s - threadIdx.x < n; s += (int64_t)gridDim.x * blockDim.x) {
         const bool in = s < n;
         int64_t c = 0;
         int ev = 0, slot = 0;
+        if (in) AT(b.jidx, AT(b.joff, OI(b, kSG, s), b.obj[kMD].cap + 1) + AT(b.jrank, s, C), C) = (int)s;
+        if (!map) continue;
         if (in) {
             const int g2 = OG(b, kMD, OJ(b, kSG, s));
-            const int64_t pos = AT(b.eoff, g2, NG1(b)) + atomicAdd(&AT(b.ecur, g2, b.n_gm), 1);
-            AT(b.eidx, pos, b.obj[kSG].cap) = (int)s;
+            AT(b.eidx, AT(b.eoff, g2, NG1(b)) + AT(b.erank, s, C), C) = (int)s;
             c = AT(b.conn_sum, g2, b.n_gm);
             const int g1 = OG(b, kSG, s);
             ev = ev_of(b, g1);
@@ -1188,6 +1162,22 @@ __global__ void k_sg_end_scatter(BatchDev b) {
         }
         const bool act = in && c != 0;
         warp_add(act ? counter_at(b, ev, kTL, 0, slot) : b.counters, (uint32_t)c, act);
+    }
+}
+// the first segment of every segment's two mini-doublets (geometries whose
+// connection lists repeat a module)
+__global__ void k_sg_keys(BatchDev b) {
+    if (halted(b)) return;
+    const int64_t n = n_objects(b, kSG);
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
+        const int md = OI(b, kSG, s), om = OJ(b, kSG, s);
+        int key = (int)s;
+        const int64_t m = join_n(b, md);
+        for (int64_t k = 0; k < m; ++k) {
+            const int t = join_obj(b, md, k);
+            if (t < key && OJ(b, kSG, t) == om) key = t;
+        }
+        AT(b.sgkey, s, b.obj[kSG].cap) = key;
     }
 }
 
@@ -1953,21 +1943,50 @@ struct ScanObj : ScanOp {
     __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(b.obj[st].mod_cnt, n, NG1(b)) = t[0]; }
 };
 
-__global__ void k_scatter(BatchDev b, int st) {
+// a tracklet's place among those of its inner segment s
+__device__ __forceinline__ int tl_join_add(const BatchDev& b, int s) {
+    return (int)atomicAdd((unsigned long long*)&AT(b.joft, sg_key(b, s), b.obj[kSG].cap + 1), 1ull);
+}
+__global__ void k_tl_join_count(BatchDev b) {
+    if (halted(b)) return;
+    const int64_t n = n_objects(b, kTL);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+        AT(b.trank, t, b.obj[kTL].cap) = tl_join_add(b, OI(b, kTL, t));
+}
+
+// The stage's records into the dense arrays grouped by inner module.  kJoin
+// (tracklets): with each one's place among those of its inner segment, for the
+// track candidates (when that stage is part of the run; otherwise it does that
+// itself).  The counts that later stages accumulate per mini-doublet and per
+// segment start at zero here, where their number is known.  (The packed
+// records of mini-doublets and segments are not written here: in the records'
+// order their writes and the hits' reads scatter, segment stage of 128 dense
+// events 7.1 -> 11.9 ms, and one PU 200 event gained nothing either.)
+template <int st, bool kJoin>
+__global__ void __launch_bounds__(256) k_scatter(BatchDev b) {
     if (halted(b)) return;
     const Recs& R = b.rec[st];
     const Objs& O = b.obj[st];
     const int64_t n = min(b.n_rec[st * kLine], O.cap);
-    const int64_t flim = O.cap * (O.nf > 0 ? O.nf : 1);
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    constexpr int kNF = st == kMD ? 4 : (st == kSG ? 6 : 0);
+    for (int64_t r = tid; r < n; r += stride) {
         const int g = AT(R.g, r, O.cap);
         const int64_t pos = OFF(b, st, g) + AT(R.rank, r, O.cap);
         if (pos >= O.cap) continue;
-        AT(O.i, pos, O.cap) = AT(R.i, r, O.cap);
+        const int i = AT(R.i, r, O.cap);
+        AT(O.i, pos, O.cap) = i;
         AT(O.j, pos, O.cap) = AT(R.j, r, O.cap);
         AT(O.g, pos, O.cap) = g;
-        for (int k = 0; k < O.nf; ++k) AT(O.f, (int64_t)k * O.cap + pos, flim) = AT(R.f, (int64_t)k * O.cap + r, flim);
+#pragma unroll
+        for (int k = 0; k < kNF; ++k)
+            AT(O.f, (int64_t)k * O.cap + pos, O.cap * kNF) = AT(R.f, (int64_t)k * O.cap + r, O.cap * kNF);
+        if (kJoin) AT(b.trank, pos, O.cap) = tl_join_add(b, i);
     }
+    if (st == kMD && b.joff)
+        for (int64_t k = tid; k <= n; k += stride) AT(b.joff, k, O.cap + 1) = 0;
+    if (st == kSG)
+        for (int64_t k = tid; k <= n; k += stride) AT(b.joft, k, O.cap + 1) = 0;
 }
 
 // ------------------------------------------------------------------ counts
@@ -2085,7 +2104,7 @@ __global__ void k_conn_sum(BatchDev b, int src, int cst, bool ends) {
 // kFused: with the connection sums (for many modules k_conn_sum makes them).
 template <bool kFused>
 struct ScanSgFront : ScanCand<kSG> {
-    static constexpr int kVals = 2, kSmall = 1, kBig = 4;
+    static constexpr int kVals = 2, kSmall = kFused ? 1 : 4, kBig = kSmall;  // (kFused: few modules)
     __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
         const int64_t n = in ? OFF(b, kMD, g + 1) - OFF(b, kMD, g) : 0;
@@ -2160,7 +2179,7 @@ struct ScanSgLayers : ScanCand<kSG> {
 // the candidates' total.  kFused as above.
 template <bool kFused>
 struct ScanTlFront : ScanOp {
-    static constexpr int kVals = 3, kSmall = 1, kBig = 4;
+    static constexpr int kVals = 3, kSmall = kFused ? 1 : 4, kBig = kSmall;
     __device__ static int64_t size(const BatchDev& b) { return b.n_gm; }
     __device__ static void load(const BatchDev& b, int64_t g, bool in, int64_t* v) {
         v[0] = in ? AT(b.eoff, g, NG1(b)) : 0;
@@ -2218,40 +2237,37 @@ struct ScanTlCand : ScanCand<kTL> {
     }
 };
 
-// objects of stage st per key mini-doublet, then their positions
-__global__ void k_join_count(BatchDev b, int st, bool second) {
+// the triplets by their innermost mini-doublet (createTrackCandidatesFromTriplets)
+__global__ void k_join2_count(BatchDev b) {
     if (halted(b)) return;
-    int64_t* off = second ? b.joff2 : b.joff;
-    const int64_t n = min(OFF(b, st, b.n_gm), b.obj[st].cap);
+    const int64_t n = n_objects(b, kTP);
     for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd((unsigned long long*)&AT(off, join_key(b, st, o), b.obj[kMD].cap + 1), 1ull);
+        atomicAdd((unsigned long long*)&AT(b.joff2, join_key(b, kTP, o), b.obj[kMD].cap + 1), 1ull);
 }
-template <bool kSecond>
+__global__ void k_join2_scatter(BatchDev b) {
+    if (halted(b)) return;
+    const int64_t n = n_objects(b, kTP);
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
+        const int k = join_key(b, kTP, o);
+        const int64_t pos = AT(b.joff2, k, b.obj[kMD].cap + 1) + atomicAdd(&AT(b.jcur2, k, b.obj[kMD].cap), 1);
+        AT(b.jidx2, pos, b.obj[kTP].cap) = (int)o;
+    }
+}
+// counts of a join index (0: segments by mini-doublet, 1: triplets by
+// mini-doublet, 2: tracklets by segment) -> offsets
+template <int kIndex>
 struct ScanJoin : ScanOp {
-    static constexpr int kVals = 1, kSmall = 2, kBig = 8;
-    __device__ static int64_t* off(const BatchDev& b) { return kSecond ? b.joff2 : b.joff; }
-    __device__ static int64_t size(const BatchDev& b) { return n_objects(b, kMD); }
+    static constexpr int kVals = 1, kSmall = 2, kBig = 8, kKey = kIndex == 2 ? kSG : kMD;
+    __device__ static int64_t* off(const BatchDev& b) { return kIndex == 0 ? b.joff : (kIndex == 1 ? b.joff2 : b.joft); }
+    __device__ static int64_t size(const BatchDev& b) { return n_objects(b, kKey); }
     __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) {
-        v[0] = in ? AT(off(b), i, b.obj[kMD].cap + 1) : 0;
+        v[0] = in ? AT(off(b), i, b.obj[kKey].cap + 1) : 0;
     }
     __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t*) {
-        AT(off(b), i, b.obj[kMD].cap + 1) = e[0];
+        AT(off(b), i, b.obj[kKey].cap + 1) = e[0];
     }
-    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(off(b), n, b.obj[kMD].cap + 1) = t[0]; }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(off(b), n, b.obj[kKey].cap + 1) = t[0]; }
 };
-__global__ void k_join_scatter(BatchDev b, int st, bool second) {
-    if (halted(b)) return;
-    const int64_t* off = second ? b.joff2 : b.joff;
-    int32_t* cur = second ? b.jcur2 : b.jcur;
-    int32_t* idx = second ? b.jidx2 : b.jidx;
-    const int64_t cap = second ? b.obj[kTP].cap : max(b.obj[kSG].cap, b.obj[kTL].cap);
-    const int64_t n = min(OFF(b, st, b.n_gm), b.obj[st].cap);
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
-        const int k = join_key(b, st, o);
-        const int64_t pos = AT(off, k, b.obj[kMD].cap + 1) + atomicAdd(&AT(cur, k, b.obj[kMD].cap), 1);
-        AT(idx, pos, cap) = (int)o;
-    }
-}
 
 // how often module m2 occurs in the connection list of module m1
 __device__ __forceinline__ int conn_mult(const BatchDev& b, int m1, int m2) {
@@ -2261,8 +2277,25 @@ __device__ __forceinline__ int conn_mult(const BatchDev& b, int m1, int m2) {
     return mult;
 }
 
-// triplet candidates of every segment (TPStage)
-struct ScanTpCand : ScanCand<kTP> {
+// The triplets and track candidates of every inner object, each of which is
+// made (k_expand): their offsets are the objects' places, and the total is
+// known before any is written.
+template <int st>
+struct ScanJoined : ScanCand<st> {
+    __device__ static void store(const BatchDev& b, int64_t i, const int64_t* e, const int64_t*) {
+        AT(b.cand[st], i, b.cand_cap[st] + 1) = e[0];
+    }
+    __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) {
+        AT(b.cand[st], n, b.cand_cap[st] + 1) = t[0];
+        b.n_rec[st * kLine] = t[0];
+        if (t[0] > b.obj[st].cap) atomicOr(b.status, 1u << st);
+    }
+};
+
+// triplets of segment s (Event.cc:524-597 via Triplet.cc:55): the segments
+// starting at its outer mini-doublet; the multiplicity of the outer module in
+// the connection list repeats each, as the reference's nested loops do
+struct ScanTp : ScanJoined<kTP> {
     __device__ static void load(const BatchDev& b, int64_t s, bool in, int64_t* v) {
         v[0] = 0;
         if (!in) return;
@@ -2275,9 +2308,21 @@ struct ScanTpCand : ScanCand<kTP> {
     }
 };
 
-// track candidates of every tracklet (TCStage); Event.cc:835: their
+// tracklets whose inner segment has the mini-doublets of segment s
+__device__ __forceinline__ int64_t tl_join_n(const BatchDev& b, int s) {
+    const int k = sg_key(b, s);
+    return AT(b.joft, k + 1, b.obj[kSG].cap + 1) - AT(b.joft, k, b.obj[kSG].cap + 1);
+}
+// tracklet t into the index of tracklets by inner segment (joft scanned)
+__device__ __forceinline__ void tl_join_place(const BatchDev& b, int64_t t) {
+    const int64_t at = AT(b.joft, sg_key(b, OI(b, kTL, t)), b.obj[kSG].cap + 1);
+    AT(b.jidt, at + AT(b.trank, t, b.obj[kTL].cap), b.obj[kTL].cap) = (int)t;
+}
+
+// track candidates of tracklet t (Event.cc:823-872 via TrackCandidate.cc:161):
+// the tracklets whose inner segment matches its outer one; Event.cc:835: the
 // candidates in the counters are barrel-layer-1 x barrel-layer-3 tracklets
-struct ScanTcCand : ScanCand<kTC> {
+struct ScanTc : ScanJoined<kTC> {
     __device__ static void begin(const BatchDev& b) {
         for (int ev = blockIdx.x * blockDim.x + threadIdx.x; ev < b.n_ev; ev += gridDim.x * blockDim.x) {
             const uint32_t n1 = *counter_at(b, ev, kTL, 1, 0), n3 = *counter_at(b, ev, kTL, 1, 2);
@@ -2287,10 +2332,12 @@ struct ScanTcCand : ScanCand<kTC> {
     __device__ static void load(const BatchDev& b, int64_t t, bool in, int64_t* v) {
         v[0] = 0;
         if (!in) return;
+        tl_join_place(b, t);
         const ModDev& m1 = MOD(b, mod_of(b, OG(b, kTL, t)));
         if (m1.subdet != kBarrel || m1.layer != 1) return;
-        const ModDev& m3 = MOD(b, mod_of(b, OG(b, kSG, OJ(b, kTL, t))));
-        if (m3.subdet == kBarrel && m3.layer == 3) v[0] = join_n(b, OI(b, kSG, OJ(b, kTL, t)));
+        const int sB = OJ(b, kTL, t);
+        const ModDev& m3 = MOD(b, mod_of(b, OG(b, kSG, sB)));
+        if (m3.subdet == kBarrel && m3.layer == 3) v[0] = tl_join_n(b, sB);
     }
 };
 
@@ -2302,18 +2349,19 @@ struct ScanTcCand : ScanCand<kTC> {
 // once per occurrence of that module in the connection list.  Layer-pair
 // tracklets are listed by no module (Event.cc:785 via
 // addTrackletToLowerLayer), so after them there are no candidates.
-struct ScanTcFromTl : ScanCand<kTC> {
+struct ScanTcFromTl : ScanJoined<kTC> {
     __device__ static void load(const BatchDev& b, int64_t t, bool in, int64_t* v) {
         const int n_mod = b.geo.n_mod;
         int64_t cref = 0;
         int ev = 0, slot = 0;
         v[0] = 0;
+        if (in) tl_join_place(b, t);
         if (in && !(b.flags & kFlagTLLayers)) {
             const int gA2 = OG(b, kMD, OJ(b, kSG, OI(b, kTL, t)));
             ev = ev_of(b, gA2);
             cref = AT(b.conn_sum, gA2, b.n_gm);
-            const int mB = OI(b, kSG, OJ(b, kTL, t));
-            v[0] = (int64_t)conn_mult(b, gA2 - ev * n_mod, OG(b, kMD, mB) - ev * n_mod) * join_n(b, mB);
+            const int sB = OJ(b, kTL, t);
+            v[0] = (int64_t)conn_mult(b, gA2 - ev * n_mod, OG(b, kMD, OI(b, kSG, sB)) - ev * n_mod) * tl_join_n(b, sB);
             slot = MOD(b, OG(b, kTL, t) - ev * n_mod).layer_slot;
         }
         const bool act = cref != 0;
@@ -2346,6 +2394,86 @@ struct ScanTcFromTp : ScanCand<kTC> {
         warp_add(act ? counter_at(b, ev, kTC, 0, slot) : b.counters, (uint32_t)c, act);
     }
 };
+
+// The triplets (st kTP) and track candidates (kTC) from their scanned counts:
+// every candidate is an object and its offset its place, so there is nothing
+// to evaluate, rank or regroup.  A warp takes 32 consecutive inner objects and
+// writes their objects 32 at a time, coalesced; each lane finds the inner
+// object of its output among the lanes' offsets.  blockIdx.y 1: the objects'
+// offsets per module and the layer counters.  (64 events: the triplet stage 480 -> 142 us,
+// the track-candidate stage 354 -> 166 us against enumerating, ranking and
+// scattering.)
+template <int st>
+__global__ void __launch_bounds__(256) k_expand(BatchDev b) {
+    if (halted(b)) return;
+    constexpr int ist = st == kTP ? kSG : kTL;
+    const int64_t* off = b.cand[st];
+    const int64_t offlim = b.cand_cap[st] + 1;
+    const int64_t n = n_inner(b, st);
+    if (blockIdx.y == 1) {
+        for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g - (threadIdx.x & 31) <= b.n_gm;
+             g += (int64_t)gridDim.x * blockDim.x) {
+            int64_t c = 0;
+            if (g <= b.n_gm) {
+                const int64_t o = AT(off, min(OFF(b, ist, g), n), offlim);
+                AT(b.obj[st].mod_cnt, g, NG1(b)) = o;
+                if (g < b.n_gm) c = AT(off, min(OFF(b, ist, g + 1), n), offlim) - o;
+            }
+            const bool act = c != 0;
+            int ev = 0, slot = 0;
+            if (act) {
+                ev = ev_of(b, g);
+                slot = MOD(b, g - (int64_t)ev * b.geo.n_mod).layer_slot;
+            }
+            warp_add(act ? counter_at(b, ev, st, 1, slot) : b.counters, (uint32_t)c, act);
+        }
+        return;
+    }
+    const Objs& O = b.obj[st];
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / kWarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x / kWarp) + (threadIdx.x >> 5)) * kWarp; base < n; base += warps * kWarp) {
+        const int64_t i = base + lane;
+        const int64_t e0 = AT(off, base, offlim);
+        const int64_t mine = AT(off, min(i, n), offlim);
+        const int total = (int)(AT(off, min(base + kWarp, n), offlim) - e0);  // (below the capacity, an int's range)
+        const int lo = (int)(mine - e0);
+        int64_t list = 0;
+        int len = 0, g = 0;
+        if (i < n && AT(off, i + 1, offlim) > mine) {
+            g = OG(b, ist, i);
+            if (st == kTP) {
+                const int md = OJ(b, kSG, i);
+                list = AT(b.joff, md, b.obj[kMD].cap + 1);
+                len = (int)(AT(b.joff, md + 1, b.obj[kMD].cap + 1) - list);
+            } else {
+                const int k = sg_key(b, OJ(b, kTL, i));
+                list = AT(b.joft, k, b.obj[kSG].cap + 1);
+                len = (int)(AT(b.joft, k + 1, b.obj[kSG].cap + 1) - list);
+            }
+        }
+        for (int t0 = 0; t0 < total; t0 += kWarp) {
+            const int t = t0 + lane;
+            int src = 0;  // the last lane with lo <= t
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                const int x = __shfl_sync(0xffffffffu, lo, src + o);
+                if (x <= t) src += o;
+            }
+            const int q = t - __shfl_sync(0xffffffffu, lo, src);
+            const int64_t l = __shfl_sync(0xffffffffu, list, src);
+            const int m = __shfl_sync(0xffffffffu, len, src);
+            const int gs = __shfl_sync(0xffffffffu, g, src);
+            if (t < total) {
+                const int64_t pos = e0 + t;
+                const int64_t k = l + (q < m ? q : q % m);
+                AT(O.i, pos, O.cap) = (int)base + src;
+                AT(O.j, pos, O.cap) = st == kTP ? AT(b.jidx, k, b.obj[kSG].cap) : AT(b.jidt, k, b.obj[kTL].cap);
+                AT(O.g, pos, O.cap) = gs;
+            }
+        }
+    }
+}
 
 // ------------------------------------------------------------------ output
 __device__ __forceinline__ void put_md(const BatchDev& b, int a, int32_t* o) {
@@ -2514,13 +2642,27 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
 constexpr int64_t kScanSmall = (int64_t)1 << 18;
 template <class Op>
 void scan(const BatchDev& b, int slot, int64_t cap, cudaStream_t s, Hooks* h) {
-    if (cap <= kScanSmall)
-        k_scan<Op, Op::kSmall><<<grid_for(cap, kScanThreads * Op::kSmall, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
-    else
-        k_scan<Op, Op::kBig><<<grid_for(cap, kScanThreads * Op::kBig, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
+    const int items = cap <= kScanSmall ? Op::kSmall : Op::kBig;
+    auto* k = cap <= kScanSmall ? k_scan<Op, Op::kSmall> : k_scan<Op, Op::kBig>;
+    k<<<grid_for(cap, kScanThreads * items, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
 }
 
 int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : kGridDefault; }
+
+template <int st>
+void scatter(const BatchDev& b, cudaStream_t s, Hooks* h) {
+    if (st == kTL && b.last >= kTC) k_scatter<st, st == kTL><<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    else k_scatter<st, false><<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+}
+
+// triplets or track candidates: counts scanned by Count -> objects
+template <int st, class Count>
+void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
+    scan<Count>(b, kScanCand + st, b.cand_cap[st], s, h);
+    mark(h, kStampEnum + st);
+    k_expand<st><<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
+    mark(h, kStampEnumEnd + st);
+}
 
 // stage F's candidates (their offsets scanned by Cand) -> objects
 template <class F, class Cand, bool kCounters = true>
@@ -2531,7 +2673,7 @@ void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
     scan<ScanObj<st, kCounters>>(b, kScanObj + st, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st);
+    scatter<st>(b, s, h);
 }
 
 // device-to-device copies of 4-byte words (job blockIdx.y), 16 bytes at a
@@ -2594,19 +2736,7 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     mark(h, kStampEnumEnd + kSG);
     scan<ScanObj<kSG, true>>(b, kScanObj + kSG, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kSG);
-}
-
-// the join index of stage st's objects (segments or tracklets), keyed by
-// mini-doublet; second = true builds the second index (triplets)
-static void join_index(const BatchDev& b, int st, int slot, cudaStream_t s, Hooks* h, bool second = false) {
-    int64_t* off = second ? b.joff2 : b.joff;
-    cudaMemsetAsync(off, 0, (b.obj[kMD].cap + 1) * sizeof(int64_t), s);
-    cudaMemsetAsync(second ? b.jcur2 : b.jcur, 0, b.obj[kMD].cap * sizeof(int32_t), s);
-    k_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
-    if (second) scan<ScanJoin<true>>(b, slot, b.obj[kMD].cap, s, h);
-    else scan<ScanJoin<false>>(b, slot, b.obj[kMD].cap, s, h);
-    k_join_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), st, second);
+    scatter<kSG>(b, s, h);
 }
 
 void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
@@ -2616,19 +2746,19 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     // module-map candidates: the module-pair tiles (k_tl_enum_tiles)
     const bool tiles = !(b.flags & (kFlagTLLayers | kFlagTLNav));
     const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
-    if (tiles) {
-        if (b.n_gm <= kScanSmall) {
-            scan<ScanTlFront<true>>(b, kScanTlFront, b.n_gm, s, h);
-        } else {
-            k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kSG, kTP, true);
-            scan<ScanTlFront<false>>(b, kScanTlFront, b.n_gm, s, h);
-        }
-        k_sg_end_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    } else {
+    if (!tiles) {
         k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kSG, kTP, false);
-        if (b.flags & kFlagTLNav) join_index(b, kSG, kScanJoinNav, s, h);  // segments by inner MD: the outward lists
-        scan<ScanTlCand<true>>(b, kScanCand + kTL, b.cand_cap[kTL], s, h);
+    } else if (b.n_gm <= kScanSmall) {
+        scan<ScanTlFront<true>>(b, kScanTlFront, b.n_gm, s, h);
+    } else {
+        k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kSG, kTP, true);
+        scan<ScanTlFront<false>>(b, kScanTlFront, b.n_gm, s, h);
     }
+    // the segments by inner mini-doublet, for navigation and the triplets
+    scan<ScanJoin<0>>(b, kScanJoinSg, b.obj[kMD].cap, s, h);
+    k_sg_index<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    if (b.geo.conn_dup) k_sg_keys<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    if (!tiles) scan<ScanTlCand<true>>(b, kScanCand + kTL, b.cand_cap[kTL], s, h);
     mark(h, kStampEnum + kTL);
     // enumeration + phase A -> survivor list (-> the pre-filter -> kept list)
     // -> phase B1 -> phase B2
@@ -2663,33 +2793,37 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_tl_b2<kB2Others><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + kTL);
     scan<ScanObj<kTL, true>>(b, kScanObj + kTL, b.n_gm, s, h);
-    k_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h), kTL);
+    scatter<kTL>(b, s, h);
 }
 
 
-void launch_tp(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    join_index(b, kSG, kScanJoinTp, s, h);
-    enum_and_group<TPStage, ScanTpCand>(b, s, h);
-}
+void launch_tp(const BatchDev& b, cudaStream_t s, Hooks* h) { expand<kTP, ScanTp>(b, s, h); }
 
 void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
     if (b.flags & kFlagTCFromTP) {
         const bool map = !(b.flags & kFlagSGLayers);
         if (map) {
-            join_index(b, kSG, kScanJoinTc, s, h);           // segments by inner MD
-            join_index(b, kTP, kScanJoinTc2, s, h, true);  // triplets by innermost MD
+            ClearJobs j{};
+            j.add(b.joff2, 2 * (b.obj[kMD].cap + 1));
+            j.add(b.jcur2, b.obj[kMD].cap);
+            launch_clear(b, j, s, h);
+            k_join2_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+            scan<ScanJoin<1>>(b, kScanJoinTc, b.obj[kMD].cap, s, h);
+            k_join2_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
         }
         k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTP, -1, false);
         if (map) enum_and_group<TCTPMapStage, ScanTcFromTp>(b, s, h);
         else enum_and_group<TCTPStage, ScanTcFromTp>(b, s, h);
         return;
     }
-    join_index(b, kTL, kScanJoinTc, s, h);
+    // the tracklets by inner segment
+    if (b.first > kTL) k_tl_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));  // (else in k_scatter)
+    scan<ScanJoin<2>>(b, kScanJoinTc, b.obj[kSG].cap, s, h);
     if (b.flags & kFlagTCFromTL) {
         k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTL, -1, false);
-        enum_and_group<TCStage, ScanTcFromTl>(b, s, h);
+        expand<kTC, ScanTcFromTl>(b, s, h);
     } else {
-        enum_and_group<TCStage, ScanTcCand>(b, s, h);
+        expand<kTC, ScanTc>(b, s, h);
     }
 }
 

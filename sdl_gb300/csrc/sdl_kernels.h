@@ -56,6 +56,7 @@ struct BatchDev {
     int32_t* bucket;               // first inner object of every 256 consecutive candidates of the running stage
     int64_t bucket_cap;
     int flags;                     // kFlag* bits
+    int first, last;               // the stages being enqueued
     // launch shape of each stage's candidate-evaluation kernel (autotuned):
     // candidates per warp task (a multiple of 32) and CTAs per SM
     int enum_task[kNumStages];
@@ -73,18 +74,23 @@ struct BatchDev {
                                    //   the enumeration's or the pre-filter's list, as passa
     unsigned long long* n_keptf;
     unsigned long long* n_cand_tl;   // tracklet candidates
-    // join index (triplets, then track candidates): the segments by their inner
-    // mini-doublet, then the tracklets by their inner segment's inner mini-doublet
+    // join indices: the segments by their inner mini-doublet (navigation,
+    // triplets), the triplets by theirs (createTrackCandidatesFromTriplets), the
+    // tracklets by their inner segment (track candidates)
     int64_t* joff;                 // mini-doublet cap + 1: counts -> offsets
-    int32_t* jcur;                 // mini-doublet cap: fill cursors
-    int32_t* jidx;                 // max(segment cap, tracklet cap): object indices
-    int64_t* joff2;                // a second index (createTrackCandidatesFromTriplets: the triplets by their
-    int32_t* jcur2;                //   innermost mini-doublet, beside the segments by inner mini-doublet)
+    int32_t* jrank;                // segment cap: place among its mini-doublet's
+    int32_t* jidx;                 // segment cap: segment indices
+    int64_t* joff2;                // mini-doublet cap + 1
+    int32_t* jcur2;                // mini-doublet cap: fill cursors
     int32_t* jidx2;                // triplet cap
+    int64_t* joft;                 // segment cap + 1
+    int32_t* trank;                // tracklet cap: place among its inner segment's
+    int32_t* jidt;                 // tracklet cap: tracklet indices
+    int32_t* sgkey;                // segment cap: first segment of the same mini-doublets (when geo.conn_dup)
     // module-pair tiles of the module-map tracklet candidates: the segments by
     // the global module of their outer mini-doublet, and the tiles per module
     int64_t* eoff;                 // n_gm + 1: counts -> offsets
-    int32_t* ecur;                 // n_gm: fill cursors
+    int32_t* erank;                // segment cap: place among its module's
     int32_t* eidx;                 // segment cap: segment indices
     int64_t* toff;                 // n_gm + 1: tile counts -> offsets
     int32_t* tile_gm;              // tile_cap: the global module of each tile (when the tiles fit)
@@ -115,10 +121,8 @@ enum ScanSlot : int {
     kScanCand = 1,                        // + st: candidate offsets (module-map segments: with the outer lists')
     kScanObj = kScanCand + kNumStages,    // + st: objects per module
     kScanTlFront = kScanObj + kNumStages,
-    kScanJoinNav,
-    kScanJoinTp,
+    kScanJoinSg,
     kScanJoinTc,
-    kScanJoinTc2,
     kScanSlots
 };
 // words of one slot for scans over up to n_gm global modules (up to 3 values
@@ -151,7 +155,7 @@ struct Hooks {
 // Buffers set to zero at the start of a run (4-byte words; rows > 1: a
 // column block of a matrix), all by one kernel: a memset node in a CUDA graph
 // costs 4.6 us.
-constexpr int kClearJobs = 16;
+constexpr int kClearJobs = 24;  // (a run takes 17 at most)
 struct ClearJobs {
     uint32_t* p[kClearJobs];
     int64_t words[kClearJobs];
@@ -160,6 +164,7 @@ struct ClearJobs {
     int count;
     int stamps;  // the first so many stamps too
     void add(void* q, int64_t n_words, int64_t n_rows = 1, int64_t n_pitch = 0) {
+        if (count == kClearJobs) return;
         p[count] = static_cast<uint32_t*>(q);
         words[count] = n_words;
         rows[count] = n_rows;
@@ -232,6 +237,7 @@ struct CopyJobs {
     int64_t n[kCopyJobs];  // words
     int count;
     void add(const void* from, void* to, int64_t words) {
+        if (count == kCopyJobs) return;
         src[count] = static_cast<const uint32_t*>(from);
         dst[count] = static_cast<uint32_t*>(to);
         n[count++] = words;

@@ -189,6 +189,7 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.dbg = tail + 5;
     b.n_sm = n_sm;
     b.flags = 0;
+    b.first = b.last = kMD;
     // the array keeps the previous call's contents: zero what the kernels
     // accumulate into
     ClearJobs j{};

@@ -42,6 +42,7 @@ struct Geometry {
     const ModDev* mod;
     const int32_t* conn_off; // n_mod + 1
     const int32_t* conn_idx;
+    bool conn_dup;           // some connection list repeats a module
     // Layers as module-index runs, for the layer-pair variants (Layer.cc:3-50):
     // slot_run[s] .. slot_run[s + 1] are the runs of layer slot s (0-5 barrel
     // layers 1-6, 6-10 endcap layers 1-5); run r spans module indices
