@@ -256,6 +256,15 @@ int ensure_scratch(sdlg_ctx* ctx, int k, size_t bytes, void** p) {
     return SDLG_OK;
 }
 
+// the first scratch buffer for a synchronous call on the context stream
+// (behind a readback that still copies from it)
+int scratch_for(sdlg_ctx* ctx, size_t bytes, void** p) {
+    const int rc = ensure_scratch(ctx, 0, bytes, p);
+    if (rc) return rc;
+    if (ctx->copy_pending[0]) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copy[0], 0));
+    return SDLG_OK;
+}
+
 template <class T>
 int dalloc(sdlg_ctx* ctx, T** p, int64_t n) {
     void* q = nullptr;
@@ -791,15 +800,6 @@ int mlp_reserve(sdlg_ctx* ctx, int64_t need) {
     M.x = x;
     M.y = y;
     M.cap = cap;
-    return SDLG_OK;
-}
-
-// device copy of a host array (caller frees)
-template <class T>
-int to_device(sdlg_ctx* ctx, const T* h, int64_t n, T** d) {
-    *d = nullptr;
-    CK(cudaMalloc(d, std::max<int64_t>(n, 1) * sizeof(T)));
-    if (n) CK(cudaMemcpy(*d, h, n * sizeof(T), cudaMemcpyHostToDevice));
     return SDLG_OK;
 }
 
@@ -1399,9 +1399,8 @@ int sdlg_get_objects(sdlg_ctx* ctx, int stage, int64_t event, int32_t* out, int6
     // 128-event batch's track candidates: 9 ms, against 26 ms for the kernel
     // writing pinned host memory itself)
     void* tmp = nullptr;
-    rc = ensure_scratch(ctx, 0, bytes, &tmp);
+    rc = scratch_for(ctx, bytes, &tmp);
     if (rc) return rc;
-    if (ctx->copy_pending[0]) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copy[0], 0));
     launch_materialize(ctx->b, stage, first, n, static_cast<int32_t*>(tmp), ctx->stream);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, tmp, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1481,10 +1480,9 @@ int sdlg_get_object_links(sdlg_ctx* ctx, int stage, int64_t event, int32_t* link
     const size_t b_links = (size_t)n * 2 * sizeof(int32_t), b_mod = (size_t)n * sizeof(int32_t);
     const size_t b_vals = (size_t)n * nf * sizeof(float);
     void* vtmp = nullptr;
-    rc = ensure_scratch(ctx, 0, b_links + b_mod + b_vals + 16, &vtmp);
+    rc = scratch_for(ctx, b_links + b_mod + b_vals + 16, &vtmp);
     if (rc) return rc;
     char* tmp = static_cast<char*>(vtmp);
-    if (ctx->copy_pending[0]) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copy[0], 0));
     int32_t* d_links = links ? reinterpret_cast<int32_t*>(tmp) : nullptr;
     int32_t* d_mod = module ? reinterpret_cast<int32_t*>(tmp + b_links) : nullptr;
     float* d_vals = (vals && nf) ? reinterpret_cast<float*>(tmp + b_links + b_mod) : nullptr;
@@ -1921,7 +1919,7 @@ int sdlg_mlp_train(sdlg_ctx* ctx, int epochs, int batch, float lr, float pos_wei
         for (int64_t start = 0; start < M.n; start += batch) {
             const int64_t count = std::min<int64_t>(batch, M.n - start);
             cudaError_t e = launch_mlp_fwd_bwd(M.x, M.y, nullptr, M.order, start, count, pos_weight, 1.f / (float)count,
-                                               M.params, M.grad, M.loss, s);
+                                               M.params, M.grad, M.loss, ctx->n_sm, s);
             if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "training step: %s", cudaGetErrorString(e));
             ++M.adam_t;
             const float c1 = (float)(1.0 - std::pow(0.9, (double)M.adam_t));
@@ -1942,26 +1940,26 @@ int sdlg_mlp_gradient(sdlg_ctx* ctx, int64_t n, const float* x, const float* y, 
     if (!ctx->mlp.have) return fail(ctx, SDLG_ERR_ARG, "no pre-filter parameters");
     cudaSetDevice(ctx->device);
     auto& M = ctx->mlp;
-    float *dx = nullptr, *dy = nullptr, *dw = nullptr;
-    int rc = to_device(ctx, x, n * kMlpIn, &dx);
-    if (!rc) rc = to_device(ctx, y, n, &dy);
-    if (!rc) rc = to_device(ctx, w, n, &dw);
-    cudaError_t e = cudaSuccess;
-    double l = 0.0;
-    if (!rc) {
-        cudaMemsetAsync(M.grad, 0, kMlpParams * sizeof(float), ctx->stream);
-        cudaMemsetAsync(M.loss, 0, sizeof(double), ctx->stream);
-        e = launch_mlp_fwd_bwd(dx, dy, dw, nullptr, 0, n, 1.f, 1.f / (float)n, M.params, M.grad, M.loss, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(grad, M.grad, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&l, M.loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(M.grad, 0, kMlpParams * sizeof(float), ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    }
-    cudaFree(dx);
-    cudaFree(dy);
-    cudaFree(dw);
+    // the inputs in the readbacks' device scratch (three allocations and their
+    // frees took 0.2 ms a call)
+    void* tmp = nullptr;
+    int rc = scratch_for(ctx, (size_t)n * (kMlpIn + 2) * sizeof(float), &tmp);
     if (rc) return rc;
-    if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "gradient: %s", cudaGetErrorString(e));
+    float* dx = static_cast<float*>(tmp);
+    float* dw = dx + n * kMlpIn;
+    float* dy = dw + n;
+    double l = 0.0;
+    cudaStream_t s = ctx->stream;
+    CK(cudaMemcpyAsync(dx, x, n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(dw, w, n * sizeof(float), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(dy, y, n * sizeof(float), cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(M.grad, 0, kMlpParams * sizeof(float), s));
+    CK(cudaMemsetAsync(M.loss, 0, sizeof(double), s));
+    CK(launch_mlp_fwd_bwd(dx, dy, dw, nullptr, 0, n, 1.f, 1.f / (float)n, M.params, M.grad, M.loss, ctx->n_sm, s));
+    CK(cudaMemcpyAsync(grad, M.grad, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&l, M.loss, sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemsetAsync(M.grad, 0, kMlpParams * sizeof(float), s));
+    CK(cudaStreamSynchronize(s));
     if (loss) *loss = l / (double)n;
     return SDLG_OK;
 }
@@ -1971,23 +1969,20 @@ int sdlg_mlp_score(sdlg_ctx* ctx, int64_t n, const float* x, float* logits) {
     if (!ctx->mlp.have) return fail(ctx, SDLG_ERR_ARG, "no pre-filter parameters");
     if (!n) return SDLG_OK;
     cudaSetDevice(ctx->device);
-    float *dx = nullptr, *dz = nullptr;
-    int rc = to_device(ctx, x, n * kMlpIn, &dx);
-    if (!rc && cudaMalloc(&dz, n * sizeof(float)) != cudaSuccess) rc = fail(ctx, SDLG_ERR_CUDA, "cudaMalloc");
-    cudaError_t e = cudaSuccess;
-    unsigned int st = 0;
-    if (!rc) {
-        cudaMemsetAsync(ctx->mlp.status, 0, sizeof(unsigned int), ctx->stream);
-        launch_mlp_score(dx, n, ctx->mlp.pack, dz, ctx->mlp.status, ctx->n_sm, ctx->stream);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(logits, dz, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&st, ctx->mlp.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    }
-    cudaFree(dx);
-    cudaFree(dz);
+    void* tmp = nullptr;
+    int rc = scratch_for(ctx, (size_t)n * (kMlpIn + 1) * sizeof(float), &tmp);
     if (rc) return rc;
-    if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "score: %s", cudaGetErrorString(e));
+    float* dx = static_cast<float*>(tmp);
+    float* dz = dx + n * kMlpIn;
+    unsigned int st = 0;
+    cudaStream_t s = ctx->stream;
+    CK(cudaMemcpyAsync(dx, x, n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(ctx->mlp.status, 0, sizeof(unsigned int), s));
+    launch_mlp_score(dx, n, ctx->mlp.pack, dz, ctx->mlp.status, ctx->n_sm, s);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(logits, dz, n * sizeof(float), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&st, ctx->mlp.status, sizeof(st), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
     if (st) return fail(ctx, SDLG_ERR_CUDA, "score: a tensor-core wait gave up");
     return SDLG_OK;
 }
