@@ -390,7 +390,7 @@ int build_module_table(sdlg_ctx* ctx, const std::vector<uint32_t>& extra) {
     return SDLG_OK;
 }
 
-constexpr int64_t kZeroWords = (2 * kNumStages + 10) * kLine;
+constexpr int64_t kZeroWords = (2 * kNumStages + 13) * kLine;
 
 // (re)allocate the batch buffers for the current event sizes and capacities
 int ensure_buffers(sdlg_ctx* ctx) {
@@ -450,6 +450,9 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.n_cand_tl = cnt + 7 * kLine;
     b.status = reinterpret_cast<uint32_t*>(cnt + 8 * kLine);
     b.dbg = cnt + 9 * kLine;
+    b.n_tc_list = cnt + 10 * kLine;
+    b.n_tc_open = cnt + 11 * kLine;
+    b.n_tc_pass = cnt + 12 * kLine;
     float* fx; float* fy; float* fz; int32_t* fi; uint32_t* fd; int64_t* eo;
     AL(fx, H); AL(fy, H); AL(fz, H); AL(fi, H); AL(fd, H); AL(eo, ctx->n_ev + 1);
     b.in_x = fx; b.in_y = fy; b.in_z = fz; b.in_idx = fi; b.in_det = fd; b.ev_off = eo;
@@ -483,6 +486,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.kept, b.kept_cap);
     AL(b.passf, b.kept_cap);
     AL(b.pb, b.kept_cap);
+    b.jidx3 = reinterpret_cast<int32_t*>(b.pb);  // (k_tctp_b has read its list when k_tctp_place writes)
     AL(b.sgpack, ctx->cap_obj[kSG] * PK_N);
     AL(b.sgouter, ctx->cap_obj[kSG] * 11);
     AL(b.sgfeat, ctx->cap_obj[kSG] * kFeatN);
@@ -498,6 +502,8 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.joff2, ctx->cap_obj[kMD] + 1);
     AL(b.jcur2, ctx->cap_obj[kMD]);
     AL(b.jidx2, ctx->cap_obj[kTP]);
+    AL(b.tpend, ctx->cap_obj[kMD]);
+    AL(b.joff3, ctx->cap_obj[kMD] + 1);
     AL(b.joft, ctx->cap_obj[kSG] + 1);
     AL(b.trank, ctx->cap_obj[kTL]);
     AL(b.jidt, ctx->cap_obj[kTL]);
@@ -532,7 +538,7 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
     ClearJobs j{};
     const int64_t n_gm = b.n_gm;
     // objects counted per module as they are made (the joins write their offsets)
-    auto counted = [&](int st) { return st <= kTL || (st == kTC && (b.flags & kFlagTCFromTP)); };
+    auto counted = [&](int st) { return st <= kTL || (st == kTC && (b.flags & kFlagTCFromTP) && (b.flags & kFlagSGLayers)); };
     // (a later stage's own run keeps the pass times of the stages before it)
     j.stamps = first == 0 ? kNumStamps : kStampEnd + 1;
     if (first == 0) {
@@ -546,6 +552,7 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
         const int ns = last - first + 1;
         j.add(b.status, 1);
         j.add(b.dbg, 16);
+        j.add(b.n_tc_list, 6 * kLine);
         j.add(b.n_rec + first * kLine, 2 * kLine * ns);
         j.add(b.task + first * kLine, 2 * kLine * ns);
         // the survivor lists' counts: the segment stage's, then the tracklet stage's

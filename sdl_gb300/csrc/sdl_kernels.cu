@@ -935,43 +935,6 @@ struct TCTPStage {
     __device__ static int group_of(const BatchDev& b, int p) { return OG(b, kTP, p); }
 };
 
-// createTrackCandidatesFromTriplets after module-map segments: the trial
-// segment (mdA, mdB) passes the segment algorithm exactly when the segment
-// stage made it, and it made it once per occurrence of mdB's module in the
-// connection list of mdA's module, which is also how often the reference's
-// loop (over that list) reaches each outer triplet starting at mdB.  So the
-// candidates are: the segments leaving p1's outermost MD mdA (the join index)
-// x the triplets starting at each one's outer MD (the second index); the
-// tracklet algorithm then runs on that segment's packed record and p2's outer
-// segment.  Same track candidates as TCTPStage, without the trial segments.
-struct TCTPMapStage {
-    static constexpr int kSt = kTC;
-    __device__ static bool eval(const BatchDev& b, int p1, int64_t q, int& oi, int& oj, float* fv) {
-        const int mdA = OJ(b, kSG, OJ(b, kTP, p1));
-        const int64_t ns = join_n(b, mdA);
-        int sx = 0, p2 = -1;
-        for (int64_t k = 0; k < ns; ++k) {
-            sx = join_obj(b, mdA, k);
-            const int64_t n = join2_n(b, OJ(b, kSG, sx));
-            if (q < n) {
-                p2 = join2_obj(b, OJ(b, kSG, sx), q);
-                break;
-            }
-            q -= n;
-        }
-        oi = p1;
-        oj = p2;
-        (void)fv;
-        if (p2 < 0) return false;  // not reached: q is below the count (k_tc_count_tp)
-        const int so = OJ(b, kTP, p2);
-        float cut, muls;
-        const int algo = tl_phaseA(load_sgv(b.sgpack, sx), load_sgv(b.sgpack, so), cut, muls);
-        if (algo == kAlgoNone || !tl_phaseB1(algo, b.sgpack, sx, so, cut)) return false;
-        return tl_phaseB2<kB2All>(algo, b.sgpack, sx, so, muls, false);
-    }
-    __device__ static int group_of(const BatchDev& b, int p) { return OG(b, kTP, p); }
-};
-
 // outer segment of flat tracklet candidate c of inner segment s
 // tracklet candidate q of inner segment s by navigation (Event.cc:694-751):
 // over the segments leaving s's outer MD, the segments leaving their outer MD
@@ -1049,15 +1012,17 @@ __device__ __forceinline__ void passbuf_flush(const BatchDev& b, PassBuf& pb) {
     __syncwarp();
     pb.n = 0;
 }
-__device__ __forceinline__ void passbuf_add(const BatchDev& b, PassBuf& pb, int algo, int s, int tt, int b1) {
+__device__ __forceinline__ void passbuf_put(const BatchDev& b, PassBuf& pb, bool pass, int4 e) {
     const int lane = threadIdx.x & 31;
-    const bool pass = algo != kAlgoNone;
     const unsigned m = __ballot_sync(0xffffffffu, pass);
     if (!m) return;
     const int c = __popc(m);
     if (pb.n + c > kPassBuf) passbuf_flush(b, pb);
-    if (pass) pb.e[pb.n + __popc(m & ((1u << lane) - 1u))] = make_int4(s, tt, algo, b1);
+    if (pass) pb.e[pb.n + __popc(m & ((1u << lane) - 1u))] = e;
     pb.n += c;
+}
+__device__ __forceinline__ void passbuf_add(const BatchDev& b, PassBuf& pb, int algo, int s, int tt, int b1) {
+    passbuf_put(b, pb, algo != kAlgoNone, make_int4(s, tt, algo, b1));
 }
 
 // Tracklet candidates (Event.cc:611-693 with Tracklet.cc:144-2665) in three
@@ -2241,8 +2206,10 @@ struct ScanTlCand : ScanCand<kTL> {
 __global__ void k_join2_count(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = n_objects(b, kTP);
-    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x)
+    for (int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         atomicAdd((unsigned long long*)&AT(b.joff2, join_key(b, kTP, o), b.obj[kMD].cap + 1), 1ull);
+        AT(b.tpend, OJ(b, kSG, OJ(b, kTP, o)), b.obj[kMD].cap) = 1;
+    }
 }
 __global__ void k_join2_scatter(BatchDev b) {
     if (halted(b)) return;
@@ -2254,11 +2221,12 @@ __global__ void k_join2_scatter(BatchDev b) {
     }
 }
 // counts of a join index (0: segments by mini-doublet, 1: triplets by
-// mini-doublet, 2: tracklets by segment) -> offsets
+// mini-doublet, 2: tracklets by segment, 3: k_tctp_b's pairs by mini-doublet)
+// -> offsets
 template <int kIndex>
 struct ScanJoin : ScanOp {
     static constexpr int kVals = 1, kSmall = 2, kBig = 8, kKey = kIndex == 2 ? kSG : kMD;
-    __device__ static int64_t* off(const BatchDev& b) { return kIndex == 0 ? b.joff : (kIndex == 1 ? b.joff2 : b.joft); }
+    __device__ static int64_t* off(const BatchDev& b) { return kIndex == 0 ? b.joff : (kIndex == 1 ? b.joff2 : (kIndex == 2 ? b.joft : b.joff3)); }
     __device__ static int64_t size(const BatchDev& b) { return n_objects(b, kKey); }
     __device__ static void load(const BatchDev& b, int64_t i, bool in, int64_t* v) {
         v[0] = in ? AT(off(b), i, b.obj[kKey].cap + 1) : 0;
@@ -2369,29 +2337,155 @@ struct ScanTcFromTl : ScanJoined<kTC> {
     }
 };
 
-// createTrackCandidatesFromTriplets (Event.cc:874-982): candidates of triplet
-// p = the triplets of the modules connected to the module of its outermost MD
-// (conn_sum over triplet counts), with the reference's candidate counters
-struct ScanTcFromTp : ScanCand<kTC> {
-    __device__ static void load(const BatchDev& b, int64_t p, bool in, int64_t* v) {
-        int64_t c = 0;
-        int ev = 0, slot = 0;
-        v[0] = 0;
-        if (in) {
-            const int mdA = OJ(b, kSG, OJ(b, kTP, p));
-            c = AT(b.conn_sum, OG(b, kMD, mdA), b.n_gm);
-            v[0] = c;  // the trial-segment enumeration: every reference candidate
-            if (!(b.flags & kFlagSGLayers)) {  // TCTPMapStage: segments leaving mdA x triplets at their outer MD
-                v[0] = 0;
-                const int64_t ns = join_n(b, mdA);
-                for (int64_t k = 0; k < ns; ++k) v[0] += join2_n(b, OJ(b, kSG, join_obj(b, mdA, k)));
-            }
-            const int g1 = OG(b, kTP, p);
-            ev = ev_of(b, g1);
-            slot = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
+// createTrackCandidatesFromTriplets (Event.cc:874-982): the reference's
+// candidates of triplet p are the triplets of the modules connected to the
+// module of its outermost MD (conn_sum over triplet counts)
+__device__ __forceinline__ int64_t tctp_cand(const BatchDev& b, int64_t p, bool in) {
+    int64_t c = 0;
+    if (in) c = AT(b.conn_sum, OG(b, kMD, OJ(b, kSG, OJ(b, kTP, p))), b.n_gm);
+    count_cand(b, kTC, c ? OG(b, kTP, p) : 0, c);
+    return c;
+}
+// each evaluated with its trial segment (TCTPStage, after layer-pair segments)
+struct ScanTcTrial : ScanCand<kTC> {
+    __device__ static void load(const BatchDev& b, int64_t p, bool in, int64_t* v) { v[0] = tctp_cand(b, p, in); }
+};
+
+// After module-map segments: the trial segment from p1's outermost MD mdA to
+// p2's innermost MD passes the segment algorithm exactly when the segment
+// stage made it, and it made it once per occurrence of p2's module in the
+// connection list of mdA's module, which is also how often the reference's
+// loop (over that list) reaches p2.  So p1's track candidates are the pairs of
+// a segment sx leaving mdA and a triplet p2 starting at sx's outer MD whose
+// tracklet (sx, p2's outer segment) passes the default tracklet algorithm --
+// the same pairs for every triplet that ends in mdA.  Each pair is judged
+// once (six or seven triplets end in a mini-doublet at PU 200), in the tracklet
+// stage's steps: ScanTctp counts the pairs of every segment that leaves a
+// triplet's end, k_tctp_a lists those through the single-precision phases A and
+// B1, k_tctp_b decides phase B2 where its bounds allow and k_tctp_c evaluates
+// the rest exactly; the pairs that pass are indexed by mdA and expanded.  (Three
+// events of PU 100-200: the stage took 1.72 ms with the exact phases on every
+// triplet's every pair, 0.15 ms now.)
+struct ScanTctp : ScanCand<kTL> {
+    __device__ static void load(const BatchDev& b, int64_t s, bool in, int64_t* v) {
+        v[0] = in && AT(b.tpend, OI(b, kSG, s), b.obj[kMD].cap) ? join2_n(b, OJ(b, kSG, s)) : 0;
+    }
+};
+__global__ void __launch_bounds__(kEnumThreads) k_tctp_a(BatchDev b) {
+    __shared__ int4 pbuf[kEnumThreads / kWarp][kPassBuf];
+    if (halted(b)) return;
+    const int64_t nobj = n_objects(b, kSG);
+    if (nobj <= 0) return;
+    const int64_t* off = b.cand[kTL];
+    const int64_t offlim = b.cand_cap[kTL] + 1, C = b.obj[kSG].cap;
+    const int64_t total = AT(off, nobj, offlim);
+    const int task = b.task_size[kTL];
+    const int64_t ntask = (total + task - 1) / task;
+    const int lane = threadIdx.x & 31;
+    PassBuf pb{pbuf[threadIdx.x >> 5]};
+    for (;;) {
+        unsigned long long t = 0;
+        if (lane == 0) t = atomicAdd(b.task + kTC * kLine, 1ull);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if ((int64_t)t >= ntask) break;
+        const int64_t base = (int64_t)t * task;
+        const int64_t end = min(base + task, total);
+        int ilo = 0;
+        if (lane < 2) {
+            int lo, hi;
+            obj_bounds(b, nobj, total, base, end - 1, lo, hi);
+            ilo = find_obj(b, off, offlim, lo, hi, lane == 0 ? base : end - 1);
         }
-        const bool act = c != 0;
-        warp_add(act ? counter_at(b, ev, kTC, 0, slot) : b.counters, (uint32_t)c, act);
+        const int i0 = __shfl_sync(0xffffffffu, ilo, 0);
+        const int i1 = __shfl_sync(0xffffffffu, ilo, 1);
+        for (int64_t cb = base; cb < end; cb += kWarp) {
+            const int64_t c = cb + lane;
+            int algo = kAlgoNone, s = 0, tt = 0, b1 = 0, p2 = 0;
+            if (c < end) {
+                s = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
+                p2 = join2_obj(b, OJ(b, kSG, s), c - AT(off, s, offlim));
+                tt = OJ(b, kTP, p2);
+                bool exact;
+                algo = tl_ab1_decide(load_sgv(b.sgpack, s), load_sgo(b.sgouter, C, tt), load_sgo_xy(b.sgouter, C, tt), b1, exact);
+            }
+            passbuf_put(b, pb, algo != kAlgoNone, make_int4(s, tt, algo | (b1 << 8), p2));
+        }
+    }
+    passbuf_flush(b, pb);
+}
+// pairs through all phases: (p2, sx's inner MD, place among that MD's pairs)
+// to the kept list, a warp at a time
+__device__ __forceinline__ void tctp_pass(const BatchDev& b, bool pass, int s, int p2) {
+    const unsigned m = __ballot_sync(0xffffffffu, pass);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    unsigned long long p0 = 0;
+    if (lane == leader) p0 = atomicAdd(b.n_tc_pass, (unsigned long long)__popc(m));
+    p0 = __shfl_sync(0xffffffffu, p0, leader);
+    if (!pass) return;
+    const int64_t pos = (int64_t)p0 + __popc(m & ((1u << lane) - 1u));  // below the list's length <= kept_cap
+    const int md = OI(b, kSG, s);
+    const int rank = (int)atomicAdd((unsigned long long*)&AT(b.joff3, md, b.obj[kMD].cap + 1), 1ull);
+    AT(b.kept, pos, b.kept_cap) = make_int4(p2, md, rank, 0);
+}
+__global__ void __launch_bounds__(kEnumThreads) k_tctp_b(BatchDev b) {
+    __shared__ int4 pbuf[kEnumThreads / kWarp][kPassBuf];
+    if (halted(b)) return;
+    const int64_t n = min((int64_t)*b.n_tc_list, b.kept_cap);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // the undecided pairs go to the filtered list
+    BatchDev u = b;
+    u.passa = b.passf;
+    u.n_kept = b.n_tc_open;
+    PassBuf pb{pbuf[w]};
+    const int64_t warps = (int64_t)gridDim.x * (kEnumThreads / kWarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * kWarp; base < n; base += warps * kWarp) {
+        int r = 0;
+        int4 e = make_int4(0, 0, 0, 0);
+        if (base + lane < n) {
+            e = AT(b.pb, base + lane, b.kept_cap);
+            r = tl_b2_quick<false>(e.z & 0xff, load_sgv(b.sgpack, e.x), load_sgv(b.sgpack, e.y));
+            if (r == 3 && !(e.z >> 8)) r = 1;  // phase B1 undecided
+        }
+        tctp_pass(b, r == 3, e.x, e.w);
+        passbuf_put(u, pb, r == 1, e);
+    }
+    passbuf_flush(u, pb);
+}
+__global__ void __launch_bounds__(kEnumThreads) k_tctp_c(BatchDev b) {
+    if (halted(b)) return;
+    const int64_t n = min((int64_t)*b.n_tc_open, b.kept_cap);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t warps = (int64_t)gridDim.x * (kEnumThreads / kWarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * kWarp; base < n; base += warps * kWarp) {
+        bool pass = false;
+        int4 e = make_int4(0, 0, 0, 0);
+        if (base + lane < n) {
+            e = AT(b.passf, base + lane, b.kept_cap);
+            float cut, muls;
+            const int algo = tl_phaseA(load_sgv(b.sgpack, e.x), load_sgv(b.sgpack, e.y), cut, muls);
+            pass = algo != kAlgoNone && tl_phaseB1(algo, b.sgpack, e.x, e.y, cut) &&
+                   tl_phaseB2<kB2All>(algo, b.sgpack, e.x, e.y, muls, false);
+        }
+        tctp_pass(b, pass, e.x, e.w);
+    }
+}
+__global__ void k_tctp_place(BatchDev b) {
+    if (halted(b)) return;
+    const int64_t n = min((int64_t)*b.n_tc_pass, b.kept_cap);
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        const int4 e = AT(b.kept, k, b.kept_cap);
+        AT(b.jidx3, AT(b.joff3, e.y, b.obj[kMD].cap + 1) + e.z, b.kept_cap) = e.x;
+    }
+}
+// track candidates of triplet p: the passing pairs of its outermost MD
+struct ScanTcFromTp : ScanJoined<kTC> {
+    __device__ static void load(const BatchDev& b, int64_t p, bool in, int64_t* v) {
+        (void)tctp_cand(b, p, in);
+        v[0] = 0;
+        if (!in) return;
+        const int md = OJ(b, kSG, OJ(b, kTP, p));
+        v[0] = AT(b.joff3, md + 1, b.obj[kMD].cap + 1) - AT(b.joff3, md, b.obj[kMD].cap + 1);
     }
 };
 
@@ -2403,10 +2497,10 @@ struct ScanTcFromTp : ScanCand<kTC> {
 // offsets per module and the layer counters.  (64 events: the triplet stage 480 -> 142 us,
 // the track-candidate stage 354 -> 166 us against enumerating, ranking and
 // scattering.)
-template <int st>
+template <int st, bool kFromTp>
 __global__ void __launch_bounds__(256) k_expand(BatchDev b) {
     if (halted(b)) return;
-    constexpr int ist = st == kTP ? kSG : kTL;
+    constexpr int ist = st == kTP ? kSG : (kFromTp ? kTP : kTL);
     const int64_t* off = b.cand[st];
     const int64_t offlim = b.cand_cap[st] + 1;
     const int64_t n = n_inner(b, st);
@@ -2446,6 +2540,10 @@ __global__ void __launch_bounds__(256) k_expand(BatchDev b) {
                 const int md = OJ(b, kSG, i);
                 list = AT(b.joff, md, b.obj[kMD].cap + 1);
                 len = (int)(AT(b.joff, md + 1, b.obj[kMD].cap + 1) - list);
+            } else if (kFromTp) {
+                const int md = OJ(b, kSG, OJ(b, kTP, i));
+                list = AT(b.joff3, md, b.obj[kMD].cap + 1);
+                len = (int)(AT(b.joff3, md + 1, b.obj[kMD].cap + 1) - list);
             } else {
                 const int k = sg_key(b, OJ(b, kTL, i));
                 list = AT(b.joft, k, b.obj[kSG].cap + 1);
@@ -2468,7 +2566,8 @@ __global__ void __launch_bounds__(256) k_expand(BatchDev b) {
                 const int64_t pos = e0 + t;
                 const int64_t k = l + (q < m ? q : q % m);
                 AT(O.i, pos, O.cap) = (int)base + src;
-                AT(O.j, pos, O.cap) = st == kTP ? AT(b.jidx, k, b.obj[kSG].cap) : AT(b.jidt, k, b.obj[kTL].cap);
+                AT(O.j, pos, O.cap) = st == kTP ? AT(b.jidx, k, b.obj[kSG].cap)
+                                                : (kFromTp ? AT(b.jidx3, k, b.kept_cap) : AT(b.jidt, k, b.obj[kTL].cap));
                 AT(O.g, pos, O.cap) = gs;
             }
         }
@@ -2619,7 +2718,7 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     if (t < kNumStages) host[kRunRec + t] = b.n_rec[t * kLine];
     if (t == kNumStages) host[kRunStatus] = (int64_t)*b.status;
-    if (t == kNumStages + 1) host[kRunKept] = (int64_t)max(*b.n_kept, *b.n_kept_sg);
+    if (t == kNumStages + 1) host[kRunKept] = (int64_t)max(max(*b.n_kept, *b.n_kept_sg), *b.n_tc_list);
     // (this kernel's own stamp is written by the thread that copies it)
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (int k = 0; k < kNumStamps; ++k) host[kRunStamps + k] = (int64_t)b.stamps[k];
@@ -2656,11 +2755,11 @@ void scatter(const BatchDev& b, cudaStream_t s, Hooks* h) {
 }
 
 // triplets or track candidates: counts scanned by Count -> objects
-template <int st, class Count>
+template <int st, class Count, bool kFromTp = false>
 void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
     scan<Count>(b, kScanCand + st, b.cand_cap[st], s, h);
-    mark(h, kStampEnum + st);
-    k_expand<st><<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
+    if (!kFromTp) mark(h, kStampEnum + st);
+    k_expand<st, kFromTp><<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
 }
 
@@ -2801,19 +2900,33 @@ void launch_tp(const BatchDev& b, cudaStream_t s, Hooks* h) { expand<kTP, ScanTp
 
 void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
     if (b.flags & kFlagTCFromTP) {
-        const bool map = !(b.flags & kFlagSGLayers);
-        if (map) {
-            ClearJobs j{};
-            j.add(b.joff2, 2 * (b.obj[kMD].cap + 1));
-            j.add(b.jcur2, b.obj[kMD].cap);
-            launch_clear(b, j, s, h);
-            k_join2_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-            scan<ScanJoin<1>>(b, kScanJoinTc, b.obj[kMD].cap, s, h);
-            k_join2_scatter<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+        const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
+        k_conn_sum<false><<<gconn, 256, 0, s>>>(take(b, h), kTP, -1, false);
+        if (b.flags & kFlagSGLayers) {
+            enum_and_group<TCTPStage, ScanTcTrial>(b, s, h);
+            return;
         }
-        k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTP, -1, false);
-        if (map) enum_and_group<TCTPMapStage, ScanTcFromTp>(b, s, h);
-        else enum_and_group<TCTPStage, ScanTcFromTp>(b, s, h);
+        ClearJobs j{};
+        j.add(b.joff2, 2 * (b.obj[kMD].cap + 1));
+        j.add(b.jcur2, b.obj[kMD].cap);
+        j.add(b.tpend, b.obj[kMD].cap);
+        j.add(b.joff3, 2 * (b.obj[kMD].cap + 1));
+        launch_clear(b, j, s, h);
+        const unsigned g = b.n_sm * 8, ge = b.n_sm * enum_grid(b, kTL);
+        k_join2_count<<<g, 256, 0, s>>>(take(b, h));
+        scan<ScanJoin<1>>(b, kScanJoinTc, b.obj[kMD].cap, s, h);
+        k_join2_scatter<<<g, 256, 0, s>>>(take(b, h));
+        scan<ScanTctp>(b, kScanTctp, b.cand_cap[kTL], s, h);
+        mark(h, kStampEnum + kTC);
+        BatchDev l = b;  // the pairs' list is the tracklets' spare one, with a count of its own
+        l.passa = b.pb;
+        l.n_kept = b.n_tc_list;
+        k_tctp_a<<<ge, kEnumThreads, 0, s>>>(take(l, h));
+        k_tctp_b<<<ge, kEnumThreads, 0, s>>>(take(b, h));
+        k_tctp_c<<<ge, kEnumThreads, 0, s>>>(take(b, h));
+        scan<ScanJoin<3>>(b, kScanTctpJoin, b.obj[kMD].cap, s, h);
+        k_tctp_place<<<g, 256, 0, s>>>(take(b, h));
+        expand<kTC, ScanTcFromTp, true>(b, s, h);
         return;
     }
     // the tracklets by inner segment

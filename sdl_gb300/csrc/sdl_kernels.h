@@ -83,6 +83,14 @@ struct BatchDev {
     int64_t* joff2;                // mini-doublet cap + 1
     int32_t* jcur2;                // mini-doublet cap: fill cursors
     int32_t* jidx2;                // triplet cap
+    // createTrackCandidatesFromTriplets: mini-doublets in which a triplet ends,
+    // and the passing pairs by the segment's inner mini-doublet
+    uint32_t* tpend;               // mini-doublet cap
+    int64_t* joff3;                // mini-doublet cap + 1
+    int32_t* jidx3;                // kept_cap: triplet indices
+    unsigned long long* n_tc_list; // pairs through phases A and B1 (in pb; can exceed kept_cap: overflow)
+    unsigned long long* n_tc_open; // of those, undecided in phase B2 (in passf)
+    unsigned long long* n_tc_pass; // pairs through all phases (in kept)
     int64_t* joft;                 // segment cap + 1
     int32_t* trank;                // tracklet cap: place among its inner segment's
     int32_t* jidt;                 // tracklet cap: tracklet indices
@@ -123,6 +131,8 @@ enum ScanSlot : int {
     kScanTlFront = kScanObj + kNumStages,
     kScanJoinSg,
     kScanJoinTc,
+    kScanTctp,
+    kScanTctpJoin,
     kScanSlots
 };
 // words of one slot for scans over up to n_gm global modules (up to 3 values
@@ -155,7 +165,7 @@ struct Hooks {
 // Buffers set to zero at the start of a run (4-byte words; rows > 1: a
 // column block of a matrix), all by one kernel: a memset node in a CUDA graph
 // costs 4.6 us.
-constexpr int kClearJobs = 24;  // (a run takes 17 at most)
+constexpr int kClearJobs = 24;  // (a run takes 18 at most)
 struct ClearJobs {
     uint32_t* p[kClearJobs];
     int64_t words[kClearJobs];

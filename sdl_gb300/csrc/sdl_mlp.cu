@@ -67,9 +67,8 @@ __global__ void __launch_bounds__(kMlpTile) k_mlp_score(const float* __restrict_
 // stay in registers over all of a CTA's tiles and reach memory by one atomic
 // per CTA and parameter.  111 KB of shared memory: two CTAs per SM, so that one
 // computes while the other waits.  Bound by the FP32 pipes: 98 us of
-// multiply-adds for 262,144 samples.  (A thread per sample with its units in
-// shared memory took 1,023 us, and gradient and scores of these samples with
-// their copies 1,684 us; 463 us now.)
+// multiply-adds for 262,144 samples, which take 190 us.  (A thread per sample
+// with its units in shared memory took 1,023 us.)
 constexpr int kTrainRows = 128;     // samples per tile
 constexpr int kTrainThreads = 256;
 constexpr int kLdM = kTrainRows + 4;
