@@ -513,6 +513,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.eidx, ctx->cap_obj[kSG]);
     AL(b.toff, n_gm + 1);
     AL(b.coff, n_gm + 1);
+    AL(b.layer_runs, ctx->n_ev * kNumSlots * 24);
     b.tile_cap = 2 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);
     AL(b.tile_gm, b.tile_cap);
     b.olist_cap = 4 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);

@@ -580,43 +580,59 @@ __device__ __forceinline__ int layer_object(const BatchDev& b, int st, int ev, i
     return 0;
 }
 
-// segment candidates by layer pairs (Event.cc:432-443, 793-821): candidate q
-// of inner MD a runs over the MDs of the paired outer layers, in table order
-struct SGLayerStage {
-    static constexpr int kSt = kSG;
-    __device__ static bool eval(const BatchDev& b, int a, int64_t q, int& oi, int& oj, float* fv) {
-        const int n_mod = b.geo.n_mod;
-        const int g1 = OG(b, kMD, a);
-        const int ev = ev_of(b, g1), m1 = g1 - ev * n_mod;
-        const int si = MOD(b, m1).layer_slot;
-        int bmd = -1;
+// Segment candidates by layer pairs (Event.cc:432-443, 793-821): candidate q
+// of an inner MD runs over the MDs of the paired outer layers, in table order.
+// Those are up to kLayerRuns runs of consecutive MDs, the same for all MDs of
+// an event's layer slot: one table row per event and slot (k_layer_runs) holds
+// the runs' first MDs, then their cumulative counts.
+constexpr int kLayerRuns = 12;  // three endcap layers of four sides (the detId's two bits)
+constexpr int kLayerRow = 2 * kLayerRuns;
+__device__ __forceinline__ const int* layer_row(const BatchDev& b, int a) {
+    const int g1 = OG(b, kMD, a);
+    const int ev = ev_of(b, g1);
+    const int slot = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
+    return &AT(b.layer_runs, (ev * kNumSlots + slot) * kLayerRow, (int64_t)b.n_ev * kNumSlots * kLayerRow);
+}
+__global__ void k_layer_runs(BatchDev b) {
+    if (halted(b)) return;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < b.n_ev * kNumSlots; t += gridDim.x * blockDim.x) {
+        const int64_t base = (int64_t)(t / kNumSlots) * b.geo.n_mod;
+        int* row = b.layer_runs + t * kLayerRow;
+        int n = 0, sum = 0;
         for (int k = 0; k < 3; ++k) {
-            const int so = sg_layer_outer(si, k);
+            const int so = sg_layer_outer(t % kNumSlots, k);
             if (so < 0) break;
-            const int64_t n = layer_count(b, kMD, ev, so);
-            if (q < n) {
-                bmd = layer_object(b, kMD, ev, so, q);
-                break;
+            for (int r = SR(b, so); r < SR(b, so + 1) && n < kLayerRuns; ++r, ++n) {
+                const int o0 = (int)OFF(b, kMD, base + SR(b, kNumSlots + 1 + 2 * r));
+                row[n] = o0;
+                sum += (int)OFF(b, kMD, base + SR(b, kNumSlots + 2 + 2 * r)) - o0;
+                row[kLayerRuns + n] = sum;
             }
-            q -= n;
         }
-        oi = a; oj = bmd;
-        if (bmd < 0) {
-#ifdef SDL_DEVICE_CHECKS
-            (void)IX(-4, 0);
-#endif
-            return false;
+        for (; n < kLayerRuns; ++n) {
+            row[n] = 0;
+            row[kLayerRuns + n] = sum;
         }
-        const int m2 = OG(b, kMD, bmd) - ev * n_mod;
-        bool connected = false;
-        if (MOD(b, m2).subdet == kEndcap) {
-            const int k0 = AT(b.geo.conn_off, m1, NM(b) + 1), k1 = AT(b.geo.conn_off, m1 + 1, NM(b) + 1);
-            for (int k = k0; k < k1 && !connected; ++k) connected = AT(b.geo.conn_idx, k, NC(b)) == m2;
-        }
-        return sg_pair(b, a, bmd, connected, fv);
     }
-    __device__ static int group_of(const BatchDev& b, int a) { return OG(b, kMD, a); }
-};
+}
+__device__ __forceinline__ int layer_md(const int* row, int q) {
+    int r = 0, before = 0;
+    for (; r < kLayerRuns - 1; ++r) {
+        const int end = row[kLayerRuns + r];
+        if (q < end) break;
+        before = end;
+    }
+    return row[r] + q - before;
+}
+// the endcap algorithm's first requirement for a layer pair: the outer MD's
+// module is in the inner one's connection list (Segment.cc:613-633)
+__device__ __forceinline__ bool sg_connected(const BatchDev& b, int a, int bmd) {
+    const int g1 = OG(b, kMD, a);
+    const int ev = ev_of(b, g1), m1 = g1 - ev * b.geo.n_mod, m2 = OG(b, kMD, bmd) - ev * b.geo.n_mod;
+    for (int k = AT(b.geo.conn_off, m1, NM(b) + 1); k < AT(b.geo.conn_off, m1 + 1, NM(b) + 1); ++k)
+        if (AT(b.geo.conn_idx, k, NC(b)) == m2) return true;
+    return false;
+}
 
 // tracklet candidate q of inner segment s -> outer segment (Event.cc:635-663)
 __device__ __forceinline__ int tl_outer(const BatchDev& b, int s, int64_t q) {
@@ -1287,7 +1303,7 @@ __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_
 #endif
 constexpr int kSgbMinBlocks = SDLG_SGB_MIN_BLOCKS;
 
-// Module-map segment candidates in two passes (Event.cc:445-522 with
+// Segment candidates in two passes (Event.cc:445-522 or 793-821 with
 // Segment.cc:337-859): k_sg_enum_a takes tasks of consecutive candidates
 // like k_enum, runs the algorithm's first cuts (sg_pair_rec<true>: the same
 // float code as the whole algorithm up to its phi cut) and lists the
@@ -1323,6 +1339,7 @@ __device__ __forceinline__ void sg_list_flush(const BatchDev& b, int4* buf, int&
     n = 0;
 }
 
+template <bool kLayers>
 __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     __shared__ int4 sbuf[kEnumThreads / kWarp][2][kPbBuf];
     if (halted(b)) return;
@@ -1358,7 +1375,8 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
             bool pass = false, ob = false;
             if (c < end) {
                 a = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
-                bmd = sg_outer_md(b, a, c - AT(off, a, offlim));
+                const int64_t q = c - AT(off, a, offlim);
+                bmd = kLayers ? layer_md(layer_row(b, a), (int)q) : sg_outer_md(b, a, q);
                 (void)IX(bmd, b.obj[kMD].cap);
                 float fv[6];
                 const MDRec orec = md_rec(b, bmd);
@@ -1398,7 +1416,8 @@ __global__ void __launch_bounds__(kEnumThreads, kSgbMinBlocks) k_sg_b(BatchDev b
             const int4 e = AT(b.pb, kOuter == 1 ? i : b.kept_cap - 1 - i, b.kept_cap);
             a = e.x;
             bmd = e.y;
-            pass = sg_pair_rec<false, kOuter>(md_rec(b, a).v, md_rec(b, bmd), true, fv);
+            const bool conn = kOuter == 1 || !(b.flags & kFlagSGLayers) || sg_connected(b, a, bmd);
+            pass = sg_pair_rec<false, kOuter>(md_rec(b, a).v, md_rec(b, bmd), conn, fv);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pass);
         if (!m) continue;
@@ -2124,16 +2143,7 @@ __global__ void k_sg_lists(BatchDev b) {
 // inner-layer MDs x outer-layer MDs); the reference counts none of them
 struct ScanSgLayers : ScanCand<kSG> {
     __device__ static void load(const BatchDev& b, int64_t a, bool in, int64_t* v) {
-        v[0] = 0;
-        if (!in) return;
-        const int g1 = OG(b, kMD, a);
-        const int ev = ev_of(b, g1);
-        const int si = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
-        for (int k = 0; k < 3; ++k) {
-            const int so = sg_layer_outer(si, k);
-            if (so < 0) break;
-            v[0] += layer_count(b, kMD, ev, so);
-        }
+        v[0] = in ? layer_row(b, (int)a)[kLayerRow - 1] : 0;
     }
 };
 
@@ -2764,14 +2774,14 @@ void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
 }
 
 // stage F's candidates (their offsets scanned by Cand) -> objects
-template <class F, class Cand, bool kCounters = true>
+template <class F, class Cand>
 void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
     constexpr int st = F::kSt;
     scan<Cand>(b, kScanCand + st, b.cand_cap[st], s, h);
     mark(h, kStampEnum + st);
     k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
-    scan<ScanObj<st, kCounters>>(b, kScanObj + st, b.n_gm, s, h);
+    scan<ScanObj<st, true>>(b, kScanObj + st, b.n_gm, s, h);
     scatter<st>(b, s, h);
 }
 
@@ -2812,29 +2822,30 @@ void launch_md(const BatchDev& b, cudaStream_t s, Hooks* h) {
 
 void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_md_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    if (b.flags & kFlagSGLayers) {
-        // Event.cc:793-821 increments no per-layer counter
-        enum_and_group<SGLayerStage, ScanSgLayers, false>(b, s, h);
-        return;
-    }
-    const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
-    if (b.n_gm <= kScanSmall) {
+    const bool layers = (b.flags & kFlagSGLayers) != 0;
+    if (layers) {
+        k_layer_runs<<<grid_for((int64_t)b.n_ev * kNumSlots, 64, b.n_sm), 64, 0, s>>>(take(b, h));
+        scan<ScanSgLayers>(b, kScanCand + kSG, b.cand_cap[kSG], s, h);
+    } else if (b.n_gm <= kScanSmall) {
         scan<ScanSgFront<true>>(b, kScanCand + kSG, b.n_gm, s, h);
     } else {
-        k_conn_sum<true><<<gconn, 256, 0, s>>>(take(b, h), kMD, kSG, false);
+        k_conn_sum<true><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kMD, kSG, false);
         scan<ScanSgFront<false>>(b, kScanCand + kSG, b.n_gm, s, h);
     }
-    k_sg_lists<<<grid_for(8 * (int64_t)b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h));
+    if (!layers) k_sg_lists<<<grid_for(8 * (int64_t)b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h));
     // first cuts -> survivor list -> whole algorithm (k_sg_enum_a, k_sg_b)
     mark(h, kStampEnum + kSG);
     BatchDev l = b;  // with this list's own counts
     l.n_kept = b.n_kept_sg;
     l.n_pb = b.n_pb_sg;
-    k_sg_enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
+    auto* enum_a = layers ? k_sg_enum_a<true> : k_sg_enum_a<false>;
+    enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     k_sg_b<1><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     mark(h, kStampEnumEnd + kSG);
-    scan<ScanObj<kSG, true>>(b, kScanObj + kSG, b.n_gm, s, h);
+    // (Event.cc:793-821, the layer pairs, increments no per-layer counter)
+    if (layers) scan<ScanObj<kSG, false>>(b, kScanObj + kSG, b.n_gm, s, h);
+    else scan<ScanObj<kSG, true>>(b, kScanObj + kSG, b.n_gm, s, h);
     scatter<kSG>(b, s, h);
 }
 

@@ -103,6 +103,7 @@ struct BatchDev {
     int64_t* toff;                 // n_gm + 1: tile counts -> offsets
     int32_t* tile_gm;              // tile_cap: the global module of each tile (when the tiles fit)
     int64_t tile_cap;
+    int* layer_runs;               // n_ev x kNumSlots rows of 24: the layer-pair segments' outer runs (k_layer_runs)
     int64_t* coff;                 // n_gm + 1: offsets of the modules' segment candidates
     int32_t* olist;                // olist_cap: the segment candidates' outer lists (k_sg_lists; offsets in toff)
     int64_t olist_cap;
