@@ -1398,9 +1398,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
 }
 
 template <int kOuter>
-__global__ void __launch_bounds__(kEnumThreads, kSgbMinBlocks) k_sg_b(BatchDev b) {
-    __shared__ int rbuf[kEnumThreads / kWarp][3 + 6][kRecBuf];
-    if (halted(b)) return;
+__device__ __forceinline__ void sg_b(const BatchDev& b, int (*rbuf)[3 + 6][kRecBuf]) {
     // kOuter 1: the barrel part of the first pass's list (front), 2: the endcap part (back)
     const int64_t nfront = min((int64_t)b.n_pb[0], b.kept_cap);
     const int64_t n = kOuter == 1 ? nfront : min((int64_t)b.n_pb[1], b.kept_cap - nfront);
@@ -1433,6 +1431,15 @@ __global__ void __launch_bounds__(kEnumThreads, kSgbMinBlocks) k_sg_b(BatchDev b
         rb.n += __popc(m);
     }
     rec_flush<6>(b, kSG, rb);
+}
+// kOuter 1: the barrel part of the list, 2: the endcap part, 0: both, by
+// blockIdx.y (launch_pair)
+template <int kOuter>
+__global__ void __launch_bounds__(kEnumThreads, kSgbMinBlocks) k_sg_b(BatchDev b) {
+    __shared__ int rbuf[kEnumThreads / kWarp][3 + 6][kRecBuf];
+    if (halted(b)) return;
+    if (kOuter == 1 || (kOuter == 0 && blockIdx.y == 0)) sg_b<1>(b, rbuf);
+    else sg_b<2>(b, rbuf);
 }
 
 // Learned pre-filter of the tracklet candidates (no counterpart in the
@@ -1636,13 +1643,9 @@ __device__ __forceinline__ void pb_flush(const BatchDev& b, int4* buf, int& n, b
 // phase B1 the enumeration decided already (passed), is a tracklet: it is
 // appended here as k_tl_b2 would, and the exact phases skip it.
 template <int kPass>
-__global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4* __restrict__ in,
-                                                        const unsigned long long* n_in) {
+__device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict__ in, const unsigned long long* n_in,
+                                       int4 (*fbuf)[kPassBuf], int4 (*dbuf)[2][kPbBuf], int (*tbuf)[3][kRecBuf]) {
     constexpr bool kDefer = kPass == 0;
-    __shared__ int4 fbuf[kEnumThreads / kWarp][kPassBuf];
-    __shared__ int4 dbuf[kDefer ? kEnumThreads / kWarp : 1][2][kPbBuf];
-    __shared__ int tbuf[kEnumThreads / kWarp][3][kRecBuf];
-    if (halted(b)) return;
     int64_t n;
     if (kPass == 0) {
         n = min((int64_t)*n_in, b.kept_cap);
@@ -1652,8 +1655,8 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4*
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int4* buf = fbuf[w];
-    int4* dfront = dbuf[kDefer ? w : 0][0];
-    int4* dback = dbuf[kDefer ? w : 0][1];
+    int4* dfront = kDefer ? dbuf[w][0] : nullptr;
+    int4* dback = kDefer ? dbuf[w][1] : nullptr;
     RecBuf<0> tl{tbuf[w]};
     int nb = 0, nf = 0, nk = 0;
     // p0 + nb <= the input length <= kept_cap: the filtered list cannot overflow
@@ -1715,6 +1718,24 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4*
     }
 }
 
+// pass 0
+__global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4* __restrict__ in, const unsigned long long* n_in) {
+    __shared__ int4 fbuf[kEnumThreads / kWarp][kPassBuf];
+    __shared__ int4 dbuf[kEnumThreads / kWarp][2][kPbBuf];
+    __shared__ int tbuf[kEnumThreads / kWarp][3][kRecBuf];
+    if (halted(b)) return;
+    tl_b2f<0>(b, in, n_in, fbuf, dbuf, tbuf);
+}
+// passes 1 and 2; 0: both, by blockIdx.y (launch_pair)
+template <int kPass>
+__global__ void __launch_bounds__(kEnumThreads) k_tl_b2f_rest(BatchDev b) {
+    __shared__ int4 fbuf[kEnumThreads / kWarp][kPassBuf];
+    __shared__ int tbuf[kEnumThreads / kWarp][3][kRecBuf];
+    if (halted(b)) return;
+    if (kPass == 1 || (kPass == 0 && blockIdx.y == 0)) tl_b2f<1>(b, nullptr, nullptr, fbuf, nullptr, tbuf);
+    else tl_b2f<2>(b, nullptr, nullptr, fbuf, nullptr, tbuf);
+}
+
 __global__ void __launch_bounds__(kEnumThreads) k_tl_b1(BatchDev b, const int4* __restrict__ list,
                                                          const unsigned long long* count) {
     __shared__ int4 fbuf[kEnumThreads / kWarp][kPbBuf], bbuf[kEnumThreads / kWarp][kPbBuf];
@@ -1769,9 +1790,7 @@ constexpr int kB2MinBlocks = SDLG_B2_MIN_BLOCKS;
 // Phase B2 on one part of the phase-B2 list (kSet kB2BBBB: the front, BBBB
 // entries; kB2Others: the back, BBEE and EEEE entries); appends the tracklets.
 template <int kSet>
-__global__ void __launch_bounds__(kEnumThreads, kB2MinBlocks) k_tl_b2(BatchDev b) {
-    __shared__ int rbuf[kEnumThreads / kWarp][3][kRecBuf];
-    if (halted(b)) return;
+__device__ __forceinline__ void tl_b2(const BatchDev& b, int (*rbuf)[3][kRecBuf]) {
     const int64_t nf = min((int64_t)b.n_pb[0], b.kept_cap);
     const int64_t n = kSet == kB2BBBB ? nf : min((int64_t)b.n_pb[1], b.kept_cap - nf);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1801,6 +1820,15 @@ __global__ void __launch_bounds__(kEnumThreads, kB2MinBlocks) k_tl_b2(BatchDev b
         rb.n += __popc(m);
     }
     rec_flush<0>(b, kTL, rb);
+}
+// blockIdx.y 0: the list's front, 1: its back; an entry takes some 25 us from
+// end to end, so the parts run side by side (phases B1 and B2 of one PU 200
+// event: 55 -> 36 us)
+__global__ void __launch_bounds__(kEnumThreads, kB2MinBlocks) k_tl_b2(BatchDev b) {
+    __shared__ int rbuf[kEnumThreads / kWarp][3][kRecBuf];
+    if (halted(b)) return;
+    if (blockIdx.y == 0) tl_b2<kB2BBBB>(b, rbuf);
+    else tl_b2<kB2Others>(b, rbuf);
 }
 
 __device__ __forceinline__ float hash_unit(unsigned long long c, unsigned long long seed) {
@@ -2741,7 +2769,7 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
     for (int64_t i = t; i < (int64_t)b.n_ev * 110; i += stride) c[i] = b.counters[i];
 }
 
-// cap: an upper bound of the number of elements.  A round of tiles (about 300
+// n: about the number of elements (the grid loops over the tiles).  A round of tiles (about 300
 // CTAs in flight) takes around ten microseconds whatever its size, so the
 // tiles are large where there would be several rounds of small ones (objects
 // per module of 64 events, 2.2M modules: 46 us at 4 per thread, 35 at 8; of
@@ -2749,14 +2777,31 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
 // modules are a kernel of their own for the same reason (64 events: 62 + 43 us
 // against 300 us within the scan; one event: 15 us within it).
 constexpr int64_t kScanSmall = (int64_t)1 << 18;
+// an object array's capacity is about three times what a run puts there
+inline int64_t objects_about(int64_t cap) { return cap / 3; }
 template <class Op>
-void scan(const BatchDev& b, int slot, int64_t cap, cudaStream_t s, Hooks* h) {
-    const int items = cap <= kScanSmall ? Op::kSmall : Op::kBig;
-    auto* k = cap <= kScanSmall ? k_scan<Op, Op::kSmall> : k_scan<Op, Op::kBig>;
-    k<<<grid_for(cap, kScanThreads * items, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
+void scan(const BatchDev& b, int slot, int64_t n, cudaStream_t s, Hooks* h) {
+    const int items = n <= kScanSmall ? Op::kSmall : Op::kBig;
+    auto* k = n <= kScanSmall ? k_scan<Op, Op::kSmall> : k_scan<Op, Op::kBig>;
+    k<<<grid_for(n, kScanThreads * items, b.n_sm * 4), kScanThreads, 0, s>>>(take(b, h), slot);
 }
 
 int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_grid[st] : kGridDefault; }
+
+// The two parts of a list: one kernel for both where neither fills the GPU
+// (one PU 200 event: segments 106 -> 100 us, phase-B2 filter 66 -> 60), one
+// after the other where each does and the other part's code would only take
+// room in the instruction caches (128 dense events: segments 7.15 ms apart,
+// 7.30 together).
+void launch_pair(const BatchDev& b, void (*both)(BatchDev), void (*one)(BatchDev), void (*two)(BatchDev), int grid,
+                 cudaStream_t s, Hooks* h) {
+    if (b.n_hit_cap <= (int64_t)1 << 18) {
+        both<<<dim3((unsigned)grid, 2), kEnumThreads, 0, s>>>(take(b, h));
+    } else {
+        one<<<grid, kEnumThreads, 0, s>>>(take(b, h));
+        two<<<grid, kEnumThreads, 0, s>>>(take(b, h));
+    }
+}
 
 template <int st>
 void scatter(const BatchDev& b, cudaStream_t s, Hooks* h) {
@@ -2767,7 +2812,7 @@ void scatter(const BatchDev& b, cudaStream_t s, Hooks* h) {
 // triplets or track candidates: counts scanned by Count -> objects
 template <int st, class Count, bool kFromTp = false>
 void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    scan<Count>(b, kScanCand + st, b.cand_cap[st], s, h);
+    scan<Count>(b, kScanCand + st, objects_about(b.cand_cap[st]), s, h);
     if (!kFromTp) mark(h, kStampEnum + st);
     k_expand<st, kFromTp><<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
@@ -2777,7 +2822,7 @@ void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
 template <class F, class Cand>
 void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
     constexpr int st = F::kSt;
-    scan<Cand>(b, kScanCand + st, b.cand_cap[st], s, h);
+    scan<Cand>(b, kScanCand + st, st == kMD ? b.n_gm : objects_about(b.cand_cap[st]), s, h);
     mark(h, kStampEnum + st);
     k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
@@ -2825,7 +2870,7 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     const bool layers = (b.flags & kFlagSGLayers) != 0;
     if (layers) {
         k_layer_runs<<<grid_for((int64_t)b.n_ev * kNumSlots, 64, b.n_sm), 64, 0, s>>>(take(b, h));
-        scan<ScanSgLayers>(b, kScanCand + kSG, b.cand_cap[kSG], s, h);
+        scan<ScanSgLayers>(b, kScanCand + kSG, objects_about(b.cand_cap[kSG]), s, h);
     } else if (b.n_gm <= kScanSmall) {
         scan<ScanSgFront<true>>(b, kScanCand + kSG, b.n_gm, s, h);
     } else {
@@ -2840,8 +2885,7 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     l.n_pb = b.n_pb_sg;
     auto* enum_a = layers ? k_sg_enum_a<true> : k_sg_enum_a<false>;
     enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
-    k_sg_b<1><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
-    k_sg_b<2><<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
+    launch_pair(l, k_sg_b<0>, k_sg_b<1>, k_sg_b<2>, b.n_sm * enum_grid(b, kSG), s, h);
     mark(h, kStampEnumEnd + kSG);
     // (Event.cc:793-821, the layer pairs, increments no per-layer counter)
     if (layers) scan<ScanObj<kSG, false>>(b, kScanObj + kSG, b.n_gm, s, h);
@@ -2865,10 +2909,10 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
         scan<ScanTlFront<false>>(b, kScanTlFront, b.n_gm, s, h);
     }
     // the segments by inner mini-doublet, for navigation and the triplets
-    scan<ScanJoin<0>>(b, kScanJoinSg, b.obj[kMD].cap, s, h);
+    scan<ScanJoin<0>>(b, kScanJoinSg, objects_about(b.obj[kMD].cap), s, h);
     k_sg_index<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     if (b.geo.conn_dup) k_sg_keys<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    if (!tiles) scan<ScanTlCand<true>>(b, kScanCand + kTL, b.cand_cap[kTL], s, h);
+    if (!tiles) scan<ScanTlCand<true>>(b, kScanCand + kTL, objects_about(b.cand_cap[kTL]), s, h);
     mark(h, kStampEnum + kTL);
     // enumeration + phase A -> survivor list (-> the pre-filter -> kept list)
     // -> phase B1 -> phase B2
@@ -2891,16 +2935,14 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
     if (filt) {
         BatchDev l = b;  // with the deferred entries' own counts
         l.n_pb = b.n_pb_f;
-        k_tl_b2f<0><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), list, count);
-        k_tl_b2f<1><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), nullptr, nullptr);
-        k_tl_b2f<2><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), nullptr, nullptr);
+        k_tl_b2f<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(l, h), list, count);
+        launch_pair(l, k_tl_b2f_rest<0>, k_tl_b2f_rest<1>, k_tl_b2f_rest<2>, b.n_sm * enum_grid(b, kTL), s, h);
         list = b.passf;
         count = b.n_keptf;
     }
     mark(h, kStampTlMid + 2);
     k_tl_b1<<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h), list, count);
-    k_tl_b2<kB2BBBB><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
-    k_tl_b2<kB2Others><<<b.n_sm * enum_grid(b, kTL), kEnumThreads, 0, s>>>(take(b, h));
+    k_tl_b2<<<dim3((unsigned)(b.n_sm * enum_grid(b, kTL)), 2), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + kTL);
     scan<ScanObj<kTL, true>>(b, kScanObj + kTL, b.n_gm, s, h);
     scatter<kTL>(b, s, h);
@@ -2925,9 +2967,9 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         launch_clear(b, j, s, h);
         const unsigned g = b.n_sm * 8, ge = b.n_sm * enum_grid(b, kTL);
         k_join2_count<<<g, 256, 0, s>>>(take(b, h));
-        scan<ScanJoin<1>>(b, kScanJoinTc, b.obj[kMD].cap, s, h);
+        scan<ScanJoin<1>>(b, kScanJoinTc, objects_about(b.obj[kMD].cap), s, h);
         k_join2_scatter<<<g, 256, 0, s>>>(take(b, h));
-        scan<ScanTctp>(b, kScanTctp, b.cand_cap[kTL], s, h);
+        scan<ScanTctp>(b, kScanTctp, objects_about(b.cand_cap[kTL]), s, h);
         mark(h, kStampEnum + kTC);
         BatchDev l = b;  // the pairs' list is the tracklets' spare one, with a count of its own
         l.passa = b.pb;
@@ -2935,14 +2977,14 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         k_tctp_a<<<ge, kEnumThreads, 0, s>>>(take(l, h));
         k_tctp_b<<<ge, kEnumThreads, 0, s>>>(take(b, h));
         k_tctp_c<<<ge, kEnumThreads, 0, s>>>(take(b, h));
-        scan<ScanJoin<3>>(b, kScanTctpJoin, b.obj[kMD].cap, s, h);
+        scan<ScanJoin<3>>(b, kScanTctpJoin, objects_about(b.obj[kMD].cap), s, h);
         k_tctp_place<<<g, 256, 0, s>>>(take(b, h));
         expand<kTC, ScanTcFromTp, true>(b, s, h);
         return;
     }
     // the tracklets by inner segment
     if (b.first > kTL) k_tl_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));  // (else in k_scatter)
-    scan<ScanJoin<2>>(b, kScanJoinTc, b.obj[kSG].cap, s, h);
+    scan<ScanJoin<2>>(b, kScanJoinTc, objects_about(b.obj[kSG].cap), s, h);
     if (b.flags & kFlagTCFromTL) {
         k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTL, -1, false);
         expand<kTC, ScanTcFromTl>(b, s, h);
@@ -3085,7 +3127,7 @@ static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
     ClearJobs j{};
     j.add(b.scan_state + (int64_t)(kScanCand + kTL) * b.scan_cap, 2 * b.scan_cap);
     launch_clear(b, j, s, nullptr);
-    scan<ScanTlCand<false>>(b, kScanCand + kTL, b.cand_cap[kTL], s, nullptr);
+    scan<ScanTlCand<false>>(b, kScanCand + kTL, objects_about(b.cand_cap[kTL]), s, nullptr);
 }
 
 void launch_tl_collect(const BatchDev& b, const MlpCollect& c, cudaStream_t s) {
