@@ -1088,41 +1088,112 @@ __device__ __forceinline__ void tl_cut_values(int algo, const SGV& S, const TSeg
     sdlCut = add_dsqrt(T.la1, sdlMuls * sdlMuls + sdlPVoff * sdlPVoff);
 }
 
-// ---- phase A's decision alone, from single-precision approximations of the
-// multiple-scattering factor and of the quantities built on it (the phi-cut
-// width, the pointed z window of BBBB, the pointed rt window of EEEE with PS
-// inner modules).  Everything else is the exact float arithmetic of
-// tl_phaseA.  The approximation of the factor, 0.015 sqrt(0.1 + 0.004 d) [x
-// sqrt(q)] with sqrt(u) = u * rsqrtf(u) (rsqrtf: at most 2 ulp), is within
-// 11 * 2^-24 of the exact float, and every quantity compared is then within
-// 2^-24 * 53 * (the sum of the magnitudes of its terms) of its exact value
-// (3 of the 53 from the pointed windows' square roots as u * rsqrtf(u)).
-// A comparison is decided here only when it holds by kQuickMargin times that
-// sum (2^-16: over 4.8 times the bound); otherwise, and for NaNs or the
-// exact functions' fallback ranges, the result is kAlgoUnsure and the caller
-// runs tl_phaseA.  Returns the algorithm, kAlgoNone or kAlgoUnsure.
+// ---- phases A and B1 of the enumeration, from single-precision approximations
+// of every compared quantity.  The candidates of one inner segment share its
+// part of each formula (TLRow, made once per segment and tile), so a candidate
+// costs a few multiply-adds per cut: no division, no arc functions.
+//
+// Phase A.  Each quantity is within 2^-24 * 60 * (the sum of the magnitudes of
+// its terms) of the exact code's float: the terms' own roundings in both (at
+// most a dozen), the multiple-scattering factor (0.015 sqrt(0.1 + 0.004 d)
+// [x sqrt(q)] with sqrt(u) = u * rsqrtf(u), 11), the pointed windows' square
+// root and quotients (under 30).  A comparison is decided only when it holds
+// by kQuickMargin times that sum (2^-16: over four times the bound), or, for
+// the z window of BBBB and the rt windows of BBEE and EEEE, whose terms are
+// within 2^-24 * 14 times the sum, by kWindowMargin (2^-18: over four times).
+// Otherwise, and for NaNs or the exact functions' fallback ranges, the result
+// is kAlgoUnsure and the caller runs tl_phaseA.
 constexpr int kAlgoUnsure = -1;
 constexpr float kQuickMargin = 0x1p-16f;
+constexpr float kWindowMargin = 0x1p-18f;
+// Phase B1.  Its two angles are compared through their sines: with M the
+// mid-point direction, D = OutLo - InLo, c and d the cross and dot product of
+// M and D, |angle(M, D)| <= cut (below 2) is |c| cos(cut) <= d sin(cut), and the
+// two sides differ by |M| |D| sin(|angle| - cut).  So a difference above
+// kB1Margin (|c| + |d|) puts the angle kB1Margin away from the cut; __sinf and
+// __cosf (2^-21.1 absolute), the products' roundings and the approximate cut
+// (3e-6) move it by under 5e-6.  betaIn is dPhiChange less the angle from InLo
+// to the axis; |betaIn| < th = asin(arg) + 0.02 / sdIn_d is decided from
+// sin and cos of the angle less dPhiChange against sin(th) =
+// arg cos(e) + sqrt(1 - arg^2) sin(e), e = 0.02 / sdIn_d, with the same margin
+// (|e| <= 0.25 and |dPhiChange| < 1.6 keep th below pi / 2 and the angle's
+// wrap out of reach).  Every comparison decided holds by over 9e-5 for the
+// exact code's angles, which are within 2e-6 of the true ones.
+constexpr float kB1Margin = 1e-4f;
+
+enum : uint32_t {  // TLRow.fl
+    R_BBBB = 1u, R_BBEE = 2u, R_EEEE = 4u,  // the algorithms the inner segment can take
+    R_IN_PS = 8u, R_UP_PS = 16u, R_DZ_POS = 32u, R_DZ_NEG = 64u,
+};
+struct __align__(16) TLRow {
+    float rt, z, inv_rt, uphi;        // inner anchor, 1 / rt; outer anchor's phi
+    float zp, sq, c3, inv_seg;        // z pitch; 0.18 sqrt(lr3z / lrt); cosh^2 / 3; 1 / (urt - lrt)
+    float dzdr, lx, ly, rtk;          // -rtseg k / ptCut
+    float cosd, sind, cose, sine;     // of dPhiChange and of 0.02 / sdIn_d (NaN: phase B1 undecided)
+    float inv_a, inv_b, drt, dz;      // 1 / (z + dLum), 1 / (z - dLum); urt - lrt, uz - lz
+    float cosh;
+    uint32_t fl;
+    float pad[2];
+};
+__device__ __forceinline__ TLRow tl_row(const SGV& S) {
+    TLRow R;
+    R.rt = S.lrt; R.z = S.lz; R.inv_rt = __fdividef(1.f, S.lrt); R.uphi = S.uphi;
+    R.zp = (S.flags & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch;
+    R.sq = (0.015f * 3.f / kPtCut * 4.f) * S.sqq_hi;
+    R.c3 = S.cosh * S.cosh * (1.f / 3.f);
+    R.drt = S.urt - S.lrt;
+    R.dz = S.uz - S.lz;
+    R.inv_seg = __fdividef(1.f, R.drt);
+    R.dzdr = S.dzdr; R.lx = S.lx; R.ly = S.ly;
+    R.rtk = -S.rtseg * (k2Rinv1GeVf / kPtCut);
+    const float e = __fdividef(0.02f, R.drt);
+    const bool ok = fabsf(S.dpc) < 1.6f && fabsf(e) <= 0.25f;
+    R.cosd = __cosf(S.dpc); R.sind = __sinf(S.dpc);
+    R.cose = __cosf(e);
+    R.sine = ok ? __sinf(e) : __int_as_float(0x7fc00000);
+    const float dLum = f_copysign(kDeltaZLum, S.lz);
+    R.inv_a = __fdividef(1.f, S.lz + dLum);
+    R.inv_b = __fdividef(1.f, S.lz - dLum);
+    R.cosh = S.cosh;
+    const bool b1 = S.flags & F_LO_B, b2 = S.flags & F_UP_B, e1 = S.flags & F_LO_E, e2 = S.flags & F_UP_E;
+    R.fl = (b1 && b2 ? R_BBBB : 0u) | (b1 && (b2 || e2) ? R_BBEE : 0u) | (e1 && e2 ? R_EEEE : 0u) |
+           ((S.flags & F_LO_PS) ? R_IN_PS : 0u) | ((S.flags & F_UP_PS) ? R_UP_PS : 0u) | (R.dz > 0.f ? R_DZ_POS : 0u) |
+           (R.dz < 0.f ? R_DZ_NEG : 0u);
+    R.pad[0] = R.pad[1] = 0.f;
+    return R;
+}
+// the outer segment's part
+struct TLOut {
+    float rt, z, ltd, la1, uphi, pv2, zp;  // pv2: the PV-offset term squared; zp: z pitch
+    uint32_t fl;                           // R_BBBB, or R_BBEE | R_EEEE
+};
+__device__ __forceinline__ TLOut tl_out(const SGOuter& T) {
+    TLOut O;
+    O.rt = T.lrt; O.z = T.lz; O.ltd = T.ltd; O.la1 = T.la1; O.uphi = T.uphi;
+    O.pv2 = T.pvoff * T.pvoff;
+    O.zp = (T.flags & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch;
+    const bool b3 = T.flags & F_LO_B, b4 = T.flags & F_UP_B, e3 = T.flags & F_LO_E, e4 = T.flags & F_UP_E;
+    O.fl = (b3 && (b4 || e4) ? R_BBBB : 0u) | (e3 && e4 ? R_BBEE | R_EEEE : 0u);
+    return O;
+}
 
 // sdlMuls = mulsF * 3 / ptCut * 4 from the approximate factor (NaN when d is
-// outside the exact function's fast range or sq is NaN)
+// outside the exact function's fast range)
 __device__ __forceinline__ float sdl_muls_quick(float d, float sq) {
-    if (!(d >= 0.f && d < 1e4f)) return __int_as_float(0x7fc00000);
-    const float u = __fadd_rn(0.1f, __fmul_rn(d, 0.004f));
-    const float m = __fmul_rn(__fmul_rn(0.015f, __fmul_rn(u, rsqrtf(u))), sq);
-    return m * 3.f / kPtCut * 4.f;
+    const float u = __fmaf_rn(d, 0.004f, 0.1f);
+    return d >= 0.f && d < 1e4f ? __fmul_rn(__fmul_rn(u, rsqrtf(u)), sq) : __int_as_float(0x7fc00000);
 }
 // |dphi| <= la1 + sqrt(sdlMuls^2 + pvoff^2): 1 holds, 0 fails, -1 not
 // decided.  cut: the approximate width (within 25 * 2^-24 * (|la1| + r) of
 // the exact one, below 3e-6 where it is set), NaN where |la1| + r >= 2.
-__device__ __forceinline__ int phi_cut_quick(float adphi, float la1, float sdlMuls, float pvoff, float& cut) {
-    cut = __int_as_float(0x7fc00000);
-    const float y = sdlMuls * sdlMuls + pvoff * pvoff;
-    if (!(y > 0x1p-100f && y < 0x1p100f)) return -1;
+// |dphi| past the wrap is 2 pi - |difference|, within 5e-7.
+__device__ __forceinline__ int phi_cut_quick(float d, float la1, float sdlMuls, float pv2, float& cut) {
+    const float adphi = fminf(fabsf(d), 6.28318531f - fabsf(d));
+    const float y = __fmaf_rn(sdlMuls, sdlMuls, pv2);
     const float r = __fmul_rn(y, rsqrtf(y));
-    const float c = la1 + r;
-    const float m = kQuickMargin * (fabsf(la1) + r);
-    if (fabsf(la1) + r < 2.f) cut = c;
+    const float c = la1 + r, a = fabsf(la1) + r;
+    const float m = __fmaf_rn(kQuickMargin, a, 1e-6f);
+    cut = a < 2.f ? c : __int_as_float(0x7fc00000);
     if (adphi > c + m) return 0;
     if (adphi < c - m) return 1;
     return -1;
@@ -1134,98 +1205,117 @@ __device__ __forceinline__ int window_quick(float v, float lo, float hi, float m
     return -1;
 }
 
-template <class TSeg>
-__device__ __forceinline__ int tl_phaseA_quick(const SGV& S, const TSeg& T, float& cut) {
+__device__ __forceinline__ int tl_phaseA_quick(const TLRow& R, const TLOut& T, float& cut) {
     cut = __int_as_float(0x7fc00000);
-    const uint32_t fs = S.flags, ft = T.flags;
-    const bool b1 = fs & F_LO_B, b2 = fs & F_UP_B, b3 = ft & F_LO_B, b4 = ft & F_UP_B;
-    const bool e1 = fs & F_LO_E, e2 = fs & F_UP_E, e3 = ft & F_LO_E, e4 = ft & F_UP_E;
-    const float rtIn = S.lrt, rtOut = T.lrt, zIn = S.lz, zOut = T.lz;
-    if (b1 && b2 && b3 && (b4 || e4)) {
-        const float zpitch_InLo = (fs & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch;
-        const float zpitch_OutLo = (ft & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch;
-        const float rtRatio = rtOut / rtIn;
-        const float dzDrtScale = T.ltd;
-        const float zHi = zIn + (zIn + kDeltaZLum) * (rtRatio - 1.f) * (zIn < 0.f ? 1.f : dzDrtScale) + (zpitch_InLo + zpitch_OutLo);
-        const float zLo = zIn + (zIn - kDeltaZLum) * (rtRatio - 1.f) * (zIn > 0.f ? 1.f : dzDrtScale) - (zpitch_InLo + zpitch_OutLo);
-        if (!(zOut >= zLo && zOut <= zHi)) return kAlgoNone;
-        const float sdlMuls = sdl_muls_quick(rtOut - rtIn, S.sqq_hi);
-        const int c3 = phi_cut_quick(fabsf(phi_mpi_pi(T.uphi - S.uphi)), T.la1, sdlMuls, pv_off(T), cut);
-        if (c3 <= 0) return c3 == 0 ? kAlgoNone : kAlgoUnsure;
-        const float drt_OutLo_InLo = rtOut - rtIn;
-        const float drt_InSeg = S.urt - S.lrt;
-        const float coshEta = S.cosh;
-        const float zp = zpitch_InLo + zpitch_OutLo;
-        // (the two quotients by __fdividef: 2 ulp instead of 0.5, inside the bound)
-        float dzErr = zp * zp * 2.f;
-        dzErr += __fdividef(sdlMuls * sdlMuls * drt_OutLo_InLo * drt_OutLo_InLo, 3.f) * coshEta * coshEta;
-        dzErr = dzErr * rsqrtf(dzErr);  // (>= 2 zp^2 > 0; 3 ulp, inside the margin)
-        const float dzMean = S.dzdr * drt_OutLo_InLo;
-        const float pw = __fdividef(dzErr, drt_InSeg) * drt_OutLo_InLo;
-        const float zWindow = pw + zp;
-        const float mLo = dzMean * (zIn > 0.f ? 1.f : dzDrtScale), mHi = dzMean * (zIn < 0.f ? 1.f : dzDrtScale);
-        const float zLoPointed = zIn + mLo - zWindow;
-        const float zHiPointed = zIn + mHi + zWindow;
-        const float m = kQuickMargin * (fabsf(zIn) + fabsf(mLo) + fabsf(mHi) + 2.f * (fabsf(pw) + zp));
-        const int c2 = window_quick(zOut, zLoPointed, zHiPointed, m);
-        return c2 > 0 ? kAlgoBBBB : (c2 == 0 ? kAlgoNone : kAlgoUnsure);
+    const uint32_t al = R.fl & T.fl;
+    const float d = T.rt - R.rt, zp = R.zp + T.zp;
+    if (al & R_BBBB) {
+        // cut 1: zIn + (zIn +- 15)(rtOut / rtIn - 1)(1 or dzDrtScale) +- the pitches
+        const float t = __fmaf_rn(T.rt, R.inv_rt, -1.f);
+        const float sHi = R.z < 0.f ? 1.f : T.ltd, sLo = R.z > 0.f ? 1.f : T.ltd;
+        const float hi = __fmaf_rn((R.z + kDeltaZLum) * sHi, t, R.z + zp);
+        const float lo = __fmaf_rn((R.z - kDeltaZLum) * sLo, t, R.z - zp);
+        const float sMax = fmaxf(fabsf(sHi), fabsf(sLo));
+        const float mw = kWindowMargin * __fmaf_rn((fabsf(R.z) + kDeltaZLum) * sMax, fabsf(t) + 2.f, fabsf(R.z) + zp);
+        const int c1 = window_quick(T.z, lo, hi, mw);
+        if (c1 == 0) return kAlgoNone;
+        const float sm = sdl_muls_quick(d, R.sq);
+        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
+        if (c3 == 0) return kAlgoNone;
+        // the pointed window
+        const float smd = sm * d;
+        const float e2 = __fmaf_rn(smd * smd, R.c3, 2.f * zp * zp);
+        const float dzErr = e2 * rsqrtf(e2);
+        const float pw = dzErr * (R.inv_seg * d), zw = pw + zp;
+        const float dzMean = R.dzdr * d;
+        const float plo = __fmaf_rn(dzMean, sLo, R.z - zw), phi = __fmaf_rn(dzMean, sHi, R.z + zw);
+        const float m = kQuickMargin * __fmaf_rn(fabsf(dzMean), fabsf(sLo) + fabsf(sHi), fabsf(R.z) + 2.f * (fabsf(pw) + zp));
+        const int c2 = window_quick(T.z, plo, phi, m);
+        if (c2 == 0) return kAlgoNone;
+        return min(min(c1, c2), c3) > 0 ? kAlgoBBBB : kAlgoUnsure;
     }
-    if (b1 && e3 && e4 && (b2 || e2)) {
-        const float zGeom = ((fs & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch) + ((ft & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch);
-        const float dzDrtScale = T.ltd;
-        if (!(zIn * zOut > 0)) return kAlgoNone;
-        const float dLum = f_copysign(kDeltaZLum, zIn);
-        const float rtGeom1 = (ft & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch;
-        const float zGeom1 = f_copysign(zGeom, zIn);
-        const float rtLo = rtIn * (1.f + (zOut - zIn - zGeom1) / (zIn + zGeom1 + dLum) / dzDrtScale) - rtGeom1;
-        if (!(rtOut >= rtLo)) return kAlgoNone;
-        float zInForHi = zIn - zGeom1 - dLum;
-        if (zInForHi * zIn < 0) zInForHi = f_copysign(0.1f, zIn);
-        const float rtHi = rtIn * (1.f + (zOut - zIn + zGeom1) / zInForHi) + rtGeom1;
-        if (!(rtOut >= rtLo && rtOut <= rtHi)) return kAlgoNone;
-        const float kZ = (zOut - zIn) / (S.uz - S.lz);
-        if (!(kZ >= 0)) return kAlgoNone;
-        const float sdlMuls = sdl_muls_quick(rtOut - rtIn, S.sqq_hi);
-        const int c3 = phi_cut_quick(fabsf(phi_mpi_pi(T.uphi - S.uphi)), T.la1, sdlMuls, pv_off(T), cut);
-        return c3 > 0 ? kAlgoBBEE : (c3 == 0 ? kAlgoNone : kAlgoUnsure);
+    if (al & R_BBEE) {
+        if (!(R.z * T.z > 0)) return kAlgoNone;
+        const float dLum = f_copysign(kDeltaZLum, R.z), rtG = T.zp;
+        const float zG = f_copysign(zp, R.z);
+        const float dz = T.z - R.z;
+        const float q1 = __fdividef(dz - zG, (R.z + zG + dLum) * T.ltd);
+        float zh = R.z - zG - dLum;  // (the exact code's float: its sign decides)
+        if (zh * R.z < 0) zh = f_copysign(0.1f, R.z);
+        const float q2 = __fdividef(dz + zG, zh);
+        const float lo = __fmaf_rn(R.rt, q1, R.rt) - rtG, hi = __fmaf_rn(R.rt, q2, R.rt) + rtG;
+        const float za = fabsf(T.z) + fabsf(R.z) + zp;  // (the numerators' magnitudes)
+        const float mw = 4.f * kWindowMargin *
+                         __fmaf_rn(fabsf(R.rt), 1.f + __fdividef(za, fabsf(zh)) +
+                                                    fabsf(__fdividef(za, (R.z + zG + dLum) * T.ltd)), fabsf(T.rt) + rtG);
+        const int c1 = window_quick(T.rt, lo, hi, mw);
+        if (c1 == 0) return kAlgoNone;
+        // kZ = dz / (uz - lz) >= 0
+        const uint32_t dzs = R.fl & (R_DZ_POS | R_DZ_NEG);
+        if ((dz > 0.f && dzs == R_DZ_NEG) || (dz < 0.f && dzs == R_DZ_POS)) return kAlgoNone;
+        const float sm = sdl_muls_quick(d, R.sq);
+        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
+        if (c3 == 0) return kAlgoNone;
+        return min(c1, c3) > 0 && dzs ? kAlgoBBEE : kAlgoUnsure;
     }
-    if (e1 && e2 && e3 && e4) {
-        const float dzDrtScale = T.ltd;
-        if (!(zIn * zOut > 0)) return kAlgoNone;
-        const float dLum = f_copysign(kDeltaZLum, zIn);
-        const bool inPS = fs & F_LO_PS, outPS = ft & F_LO_PS;
-        const float rtGeom = (inPS && outPS) ? 2.f * kPixelPSZpitch : (inPS || outPS) ? (kPixelPSZpitch + kStrip2SZpitch) : 2.f * kStrip2SZpitch;
-        const float dz = zOut - zIn;
-        const float rtLo = rtIn * (1.f + dz / (zIn + dLum) / dzDrtScale) - rtGeom;
-        if (!(rtOut >= rtLo)) return kAlgoNone;
-        const float rtHi = rtIn * (1.f + dz / (zIn - dLum)) + rtGeom;
-        if (!(rtOut >= rtLo && rtOut <= rtHi)) return kAlgoNone;
-        const float sdlMuls = sdl_muls_quick(rtOut - rtIn, 1.f);
-        const int c3 = phi_cut_quick(fabsf(phi_mpi_pi(T.uphi - S.uphi)), T.la1, sdlMuls, pv_off(T), cut);
-        if (c3 <= 0) return c3 == 0 ? kAlgoNone : kAlgoUnsure;
-        if (inPS && (fs & F_UP_PS)) {
-            const float drtSDIn = S.urt - S.lrt;
-            const float dzSDIn = S.uz - S.lz;
-            const float coshEta = S.cosh;
-            const float dzOutInAbs = fabsf(zOut - zIn);
-            const float multDzDr = dzOutInAbs * coshEta / (coshEta * coshEta - 1.f);
-            const float kZ = (zOut - zIn) / dzSDIn;
-            if (!(kZ >= 0)) return kAlgoNone;
-            float drtErr = kPixelPSZpitch * kPixelPSZpitch * 2.f / dzSDIn / dzSDIn * dzOutInAbs * dzOutInAbs;
-            drtErr += sdlMuls * sdlMuls * multDzDr * multDzDr / 3.f * coshEta * coshEta;
-            drtErr = drtErr * rsqrtf(drtErr);  // (3 ulp, inside the margin; NaN for 0: undecided)
-            const float drtMean = drtSDIn * dzOutInAbs / fabsf(dzSDIn);
-            const float rtWindow = drtErr + rtGeom;
-            const float mLo = drtMean / dzDrtScale;
-            const float rtLo_point = rtIn + mLo - rtWindow;
-            const float rtHi_point = rtIn + drtMean + rtWindow;
-            const float m = kQuickMargin * (fabsf(rtIn) + fabsf(mLo) + fabsf(drtMean) + 2.f * fabsf(rtWindow));
-            const int c2 = window_quick(rtOut, rtLo_point, rtHi_point, m);
-            return c2 > 0 ? kAlgoEEEE : (c2 == 0 ? kAlgoNone : kAlgoUnsure);
+    if (al & R_EEEE) {
+        if (!(R.z * T.z > 0)) return kAlgoNone;
+        const bool inPS = R.fl & R_IN_PS, outPS = T.zp == kPixelPSZpitch;
+        const float rtG = (inPS && outPS) ? 2.f * kPixelPSZpitch : (inPS || outPS) ? (kPixelPSZpitch + kStrip2SZpitch) : 2.f * kStrip2SZpitch;
+        const float dz = T.z - R.z;
+        const float inv_ltd = __fdividef(1.f, T.ltd);
+        const float q1 = dz * R.inv_a * inv_ltd, q2 = dz * R.inv_b;
+        const float lo = __fmaf_rn(R.rt, q1, R.rt) - rtG, hi = __fmaf_rn(R.rt, q2, R.rt) + rtG;
+        const float mw = 4.f * kWindowMargin * __fmaf_rn(fabsf(R.rt), 1.f + fabsf(q1) + fabsf(q2), fabsf(T.rt) + rtG);
+        const int c1 = window_quick(T.rt, lo, hi, mw);
+        if (c1 == 0) return kAlgoNone;
+        const float sm = sdl_muls_quick(d, 0.015f * 3.f / kPtCut * 4.f);
+        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
+        if (c3 == 0) return kAlgoNone;
+        int c2 = 1;
+        if (inPS && (R.fl & R_UP_PS)) {
+            const float adz = fabsf(dz);
+            const uint32_t dzs = R.fl & (R_DZ_POS | R_DZ_NEG);
+            if ((dz > 0.f && dzs == R_DZ_NEG) || (dz < 0.f && dzs == R_DZ_POS)) return kAlgoNone;
+            const float mult = __fdividef(adz * R.cosh, R.cosh * R.cosh - 1.f);
+            const float q = __fdividef(adz, R.dz), smm = sm * mult;
+            const float e2 = __fmaf_rn(smm * smm, R.c3, kPixelPSZpitch * kPixelPSZpitch * 2.f * q * q);
+            const float drtErr = e2 * rsqrtf(e2);
+            const float drtMean = R.drt * fabsf(q), w = drtErr + rtG;
+            const float mLo = drtMean * inv_ltd;
+            const float m = kQuickMargin * (fabsf(R.rt) + fabsf(mLo) + fabsf(drtMean) + 2.f * fabsf(w));
+            c2 = window_quick(T.rt, R.rt + mLo - w, R.rt + drtMean + w, m);
+            if (c2 == 0) return kAlgoNone;
+            if (!dzs) c2 = -1;
         }
-        return kAlgoEEEE;
+        return min(min(c1, c2), c3) > 0 ? kAlgoEEEE : kAlgoUnsure;
     }
     return kAlgoNone;
+}
+
+// Phase B1 with the approximate (or exact) phi-cut width: 1 passes, 0 fails,
+// -1 left to tl_phaseB1_sgv.  txy: the outer segment's (lx, ly, ux, uy).
+__device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4 txy, float cut) {
+    const float mx = R.lx + txy.x, my = R.ly + txy.y, dx = txy.x - R.lx, dy = txy.y - R.ly;
+    const float c = __fmaf_rn(mx, dy, -(my * dx)), dt = __fmaf_rn(mx, dx, my * dy);
+    const float f = __fmaf_rn(fabsf(c), __cosf(cut), -(dt * __sinf(cut)));
+    const float mg = kB1Margin * (fabsf(c) + fabsf(dt));
+    if (f > mg) return 0;
+    const int c5 = f < -mg ? 1 : -1;
+    if (c5 < 0 || algo == kAlgoEEEE) return c5;
+    const float ax = txy.z - R.lx, ay = txy.w - R.ly;
+    const float cx = __fmaf_rn(R.lx, ay, -(R.ly * ax)), dp = __fmaf_rn(R.lx, ax, R.ly * ay);
+    const float q = __fmaf_rn(cx, R.cosd, -(dp * R.sind)), p = __fmaf_rn(dp, R.cosd, cx * R.sind);
+    const float dr2 = __fmaf_rn(ax, ax, ay * ay);
+    const float dr = dr2 * rsqrtf(dr2);
+    const float ar = __fmaf_rn(dr, k2Rinv1GeVf / kPtCut, R.rtk);
+    const float arg = ar > kSinAlphaMax ? kSinAlphaMax : ar;
+    const float u = __fmaf_rn(-arg, arg, 1.f);
+    const float st = __fmaf_rn(u * rsqrtf(u), R.sine, arg * R.cose);
+    const float L = R.rt * dr;
+    if (!(arg >= -kSinAlphaMax)) return -1;
+    if (fabsf(q) > L * (st + kB1Margin) || p < -(kB1Margin * L)) return 0;
+    return fabsf(q) < L * (st - kB1Margin) && p > 0.f ? 1 : -1;
 }
 
 // Phase B1 decides most candidates from single-precision approximations of
@@ -1239,7 +1329,6 @@ __device__ __forceinline__ int tl_phaseA_quick(const SGV& S, const TSeg& T, floa
 // only away from the wrap at +-pi; otherwise the exact evaluation decides.
 // The self-check (functions 16 and 17 of k_math_check) bounds both
 // approximation errors by 2e-6 on the GPU itself.
-constexpr float kB1Margin = 1e-4f;
 
 // approximate direction of (x, y) (Hit.cc:68-83's phi), or false when the
 // point is at the origin, tiny, huge or not finite
@@ -1335,41 +1424,11 @@ __device__ __forceinline__ bool tl_phaseB1_sgv(int algo, const SGV& S, const SGV
 static __device__ __noinline__ bool tl_phaseB1(int algo, const float* __restrict__ pack, int s, int t, float sdlCut) {
     return tl_phaseB1_sgv(algo, load_sgv(pack, s), load_sgv(pack, t), sdlCut);
 }
-// Phase B1 from the approximations alone, with an approximate phi-cut width
-// (tl_phaseA_quick's, within 3e-6 of the exact one, or the exact one): the
-// directions (phi_fast) are within 2.5e-6 of the exact angles and asinf
-// within 2e-6 (functions 20 and 17 of the math self-check), so with the
-// width's error every comparison clear_within decides holds by over 9e-5 in
-// exact arithmetic as well, and the result is tl_phaseB1_sgv's.  txy: the outer segment's (lx, ly, ux, uy).
-// 1: passes, 0: fails, -1: left to tl_phaseB1_sgv (NaN width included).
-__device__ __forceinline__ int tl_phaseB1_quick(int algo, const SGV& S, float4 txy, float cut) {
-    float mx = 0.f, my = 0.f;
-    mx += S.lx; my += S.ly;
-    mx += txy.x; my += txy.y;
-    mx /= 2.f; my /= 2.f;
-    const float dx = txy.x - S.lx, dy = txy.y - S.ly;
-    // the angle from the mid-point direction M to D = OutLo - InLo as one
-    // atan2 of (M x D, M . D): the rounding of the cross and dot products
-    // (below 2^-23 |M| |D| each) moves it by under 2^-22 whatever the lengths,
-    // so it is within 4e-6 of the reference's difference of the two
-    // directions wrapped into [-pi, pi] away from the wrap
-    if (!(fabsf(mx) + fabsf(my) > 0x1p-40f && fabsf(mx) + fabsf(my) < 0x1p40f && fabsf(dx) + fabsf(dy) > 0x1p-40f &&
-          fabsf(dx) + fabsf(dy) < 0x1p40f))
-        return -1;
-    float v;
-    if (!phi_fast(mx * dx + my * dy, mx * dy - my * dx, v)) return -1;
-    const int c5 = clear_within(v, cut);
-    if (c5 <= 0 || algo == kAlgoEEEE) return c5;
-    const float ax = txy.z - S.lx, ay = txy.w - S.ly;
-    const float dr2 = __fadd_rn(__fmul_rn(ax, ax), __fmul_rn(ay, ay));
-    const float dr = dr2 * rsqrtf(dr2);  // (3 ulp: a few 1e-7 on the angle, far inside kB1Margin; NaN for 0: undecided)
-    const float sdIn_d = S.urt - S.lrt;
-    const float arg = fmin_ref((-S.rtseg * 1.f + dr) * k2Rinv1GeVf / kPtCut, kSinAlphaMax);
-    float pa;
-    if (!(phi_fast(ax, ay, pa) && fabsf(arg) <= kSinAlphaMax)) return -1;
-    const float w = wrap_approx(pa - S.lphi);
-    if (!(fabsf(w) < 3.f) || !(fabsf(sdIn_d) > 1e-3f)) return -1;
-    return clear_within(S.dpc - w, asinf(arg) + __fdividef(0.02f, sdIn_d));  // 2 ulp of at most 20
+// Phase A of a candidate the approximations leave open, on the packed records
+// (kAlgoNone or the algorithm, and the exact phi-cut width)
+static __device__ __noinline__ int tl_phaseA_entry(const float* __restrict__ pack, int s, int t, float& cut) {
+    float muls;
+    return tl_phaseA(load_sgv(pack, s), load_sgv(pack, t), cut, muls);
 }
 
 // the multiple-scattering factor of a candidate whose phase B1 passed already

@@ -978,23 +978,21 @@ __device__ __forceinline__ int tl_outer_of(const BatchDev& b, int var, int s, in
     return var == 1 ? tl_outer_layer(b, s, q) : (var == 2 ? tl_outer_nav(b, s, q) : tl_outer(b, s, q));
 }
 
-// Phases A and B1 of a candidate from the single-precision decisions, with
-// tl_phaseA where the first cannot decide: returns the algorithm (kAlgoNone:
-// rejected by phase A or B1) and sets b1 when phase B1 passed already (0:
-// phase B1 is left to k_tl_b1); exact tells whether an exact evaluation was
-// needed.  txy: the outer segment's anchors (load_sgo_xy).  The exact cut
-// values are computed again in phase B1.
-__device__ __forceinline__ int tl_ab1_decide(const SGV& S, const SGOuter& T, float4 txy, int& b1, bool& exact) {
+// Phases A and B1 of a candidate (inner segment s, outer segment t) from the
+// single-precision decisions, with tl_phaseA where the first cannot decide:
+// returns the algorithm (kAlgoNone: rejected by phase A or B1) and sets b1
+// when phase B1 passed already (0: phase B1 is left to k_tl_b1); exact tells
+// whether an exact evaluation was needed.  txy: the outer segment's anchors
+// (load_sgo_xy).  The exact cut values are computed again in phase B1.
+__device__ __forceinline__ int tl_ab1_decide(const TLRow& R, const TLOut& T, float4 txy, const float* __restrict__ pack, int s,
+                                             int t, int& b1, bool& exact) {
     float cut;
-    int algo = tl_phaseA_quick(S, T, cut);
+    int algo = tl_phaseA_quick(R, T, cut);
     exact = algo == kAlgoUnsure;
-    if (exact) {
-        float muls;
-        algo = tl_phaseA(S, T, cut, muls);
-    }
+    if (exact) algo = tl_phaseA_entry(pack, s, t, cut);
     b1 = 0;
     if (algo == kAlgoNone) return algo;
-    const int q = tl_phaseB1_quick(algo, S, txy, cut);
+    const int q = tl_phaseB1_quick(algo, R, txy, cut);
     if (q == 0) return kAlgoNone;
     b1 = q > 0;
     exact = exact || q < 0;
@@ -1088,7 +1086,8 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
                 (void)IX(tt, b.obj[kSG].cap);
                 const int64_t C = b.obj[kSG].cap;
                 bool exact;
-                algo = tl_ab1_decide(load_sgv(b.sgpack, s), load_sgo(b.sgouter, C, tt), load_sgo_xy(b.sgouter, C, tt), b1, exact);
+                algo = tl_ab1_decide(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
+                                     b.sgpack, s, tt, b1, exact);
             }
             passbuf_add(b, pb, algo, s, tt, b1);
         }
@@ -1106,17 +1105,15 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
 // outer segment once per tile, and the inner segments' records are
 // warp-uniform loads.  The candidates, and so the survivor list as a set, are
 // those k_tl_enum_a enumerates.
-#ifndef SDLG_TILE_A
-#define SDLG_TILE_A 24
-#endif
-// inner segments per module-pair tile (a multiple of 4, at most 32); 24
-// measured fastest on the 128-event PU 150-300 batch (enumeration 14.47 ms,
-// against 14.82 at 16 and 14.60 at 32)
-constexpr int kTileA = SDLG_TILE_A;
-static_assert(kTileA % 4 == 0 && kTileA <= 32, "tile rows");
+// Inner segments per module-pair tile: 32, or 16 for small batches, which have
+// few tiles (enumeration of 128 dense events: 10.4 ms at 32, 10.6 at 24, 11.1 at
+// 16; of one PU 200 event: 80 us at 32, 75 at 24, 72 at 16).
+constexpr int kTileA = 32;
+__device__ __forceinline__ int tile_shift(const BatchDev& b) { return b.n_hit_cap <= (int64_t)1 << 18 ? 4 : 5; }
 
-__device__ __forceinline__ int64_t tile_count(int64_t na, int64_t nb) {
-    return (na > 0 && nb > 0) ? ((na + kTileA - 1) / kTileA) * ((nb + kWarp - 1) / kWarp) : 0;
+__device__ __forceinline__ int64_t tile_count(const BatchDev& b, int64_t na, int64_t nb) {
+    const int sh = tile_shift(b);
+    return (na > 0 && nb > 0) ? ((na + (1 << sh) - 1) >> sh) * ((nb + kWarp - 1) / kWarp) : 0;
 }
 
 // the segments by their inner mini-doublet (joff scanned) and, for the
@@ -1220,15 +1217,18 @@ __device__ __forceinline__ int tile_outer(const BatchDev& b, int ev, int m, int 
 // rounds: the module (tile map), its offsets and connection-list range, the
 // inner segments' indices with the connection entries' prefix sums and first
 // segments (one entry per lane while the module has at most 32 connections),
-// then the inner segments' records (staged in shared memory, read there as
-// warp-uniform values) with the lanes' outer-segment fields.
-// CTAs per SM the module-pair enumeration is compiled for (register budget;
-// 3, with 78 registers and no spill, measured 15.7 against 14.5 ms)
+// then the inner segments' records, a lane each, which it turns into the rows
+// of the single-precision decisions (in shared memory, read there as
+// warp-uniform values), with the lanes' outer-segment fields.  Bound by
+// instruction issue: with the decisions on divisions, atan2 polynomials and
+// asinf over the plain records the 128 dense events took 14.9 ms.
+// CTAs per SM it is compiled for (register budget): 10.6 ms at 4 and 5, 11.2
+// at 3.
 #ifndef SDLG_ENUM_MIN_BLOCKS
 #define SDLG_ENUM_MIN_BLOCKS 4
 #endif
 __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_tiles(BatchDev b) {
-    __shared__ __align__(16) float4 srec[kEnumThreads / kWarp][kTileA * (PK_N / 4)];
+    __shared__ TLRow srow[kEnumThreads / kWarp][kTileA];
     __shared__ int sidx[kEnumThreads / kWarp][kTileA];
     __shared__ int4 pbuf[kEnumThreads / kWarp][kPassBuf];
     __shared__ float4 sxy[kEnumThreads / kWarp][kWarp];  // the lanes' outer anchors (phase B1)
@@ -1254,30 +1254,25 @@ __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_
         const int64_t nbb = (nb + kWarp - 1) / kWarp;
         const int64_t local = t - AT(b.toff, g, NG1(b));
         const int64_t ab = local / nbb, bb = local - ab * nbb;
-        const int64_t abase = ab * kTileA;
-        const int nat = (int)min((int64_t)kTileA, na - abase);
+        const int sh = tile_shift(b);
+        const int64_t abase = ab << sh;
+        const int nat = (int)min((int64_t)1 << sh, na - abase);
         // this lane's outer segment: entry q of g's outer list
         const int64_t q0 = bb * kWarp;
         const bool has = q0 + lane < nb;
-        __syncwarp();  // the previous tile's records have been read
-        if (lane < nat) sidx[w][lane] = AT(b.eidx, a0 + abase + lane, sgcap);
+        __syncwarp();  // the previous tile's rows have been read
+        if (lane < nat) {
+            const int sr = AT(b.eidx, a0 + abase + lane, sgcap);
+            (void)IX(sr, sgcap);
+            sidx[w][lane] = sr;
+            srow[w][lane] = tl_row(load_sgv(b.sgpack, sr));
+        }
         const int tt = tile_outer(b, ev, m2, k0, k1, q0, has);
-        SGOuter T{};
+        TLOut T{};
         if (has) {
             (void)IX(tt, sgcap);
-            T = load_sgo(b.sgouter, sgcap, tt);
+            T = tl_out(load_sgo(b.sgouter, sgcap, tt));
             sxy[w][lane] = load_sgo_xy(b.sgouter, sgcap, tt);
-        }
-        __syncwarp();
-        // stage the tile's inner-segment records (nat x 8 float4)
-#pragma unroll
-        for (int r = 0; r < kTileA * (PK_N / 4) / kWarp; ++r) {
-            const int e = lane + r * kWarp;
-            if (e < nat * (PK_N / 4)) {
-                const int sr = sidx[w][e / (PK_N / 4)];
-                (void)IX(sr, sgcap);
-                srec[w][e] = __ldg(reinterpret_cast<const float4*>(b.sgpack + (int64_t)sr * PK_N) + e % (PK_N / 4));
-            }
         }
         __syncwarp();
         for (int r = 0; r < nat; ++r) {
@@ -1285,8 +1280,7 @@ __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_
             int algo = kAlgoNone, b1 = 0;
             if (has) {
                 bool exact;
-                algo = tl_ab1_decide(sgv_from(reinterpret_cast<const float*>(&srec[w][r * (PK_N / 4)])), T, sxy[w][lane], b1,
-                                     exact);
+                algo = tl_ab1_decide(srow[w][r], T, sxy[w][lane], b.sgpack, sr, tt, b1, exact);
             }
             passbuf_add(b, pb, algo, sr, tt, b1);
         }
@@ -1915,7 +1909,8 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
         const int64_t C = b.obj[kSG].cap;
         int b1;
         bool exact;
-        const int q = tl_ab1_decide(S, load_sgo(b.sgouter, C, tt), load_sgo_xy(b.sgouter, C, tt), b1, exact);
+        const int q = tl_ab1_decide(tl_row(S), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt, b1,
+                                    exact);
         float cut, muls;
         const int e = tl_phaseA(S, Tv, cut, muls);
         const bool eb1 = e != kAlgoNone && tl_phaseB1_sgv(e, S, Tv, cut);
@@ -2189,7 +2184,7 @@ struct ScanTlFront : ScanOp {
         int64_t sum = 0;
         if (kFused) sum = conn_sum_of(b, g, in, conn_needed<true>(b, g, in, kSG, true), kSG, kTP);
         else if (v[0] > 0) sum = AT(b.conn_sum, g, b.n_gm);
-        v[1] = tile_count(v[0], sum);
+        v[1] = tile_count(b, v[0], sum);
         v[2] = v[0] * sum;
     }
     __device__ static void store(const BatchDev& b, int64_t g, const int64_t* e, const int64_t* v) {
@@ -2444,7 +2439,8 @@ __global__ void __launch_bounds__(kEnumThreads) k_tctp_a(BatchDev b) {
                 p2 = join2_obj(b, OJ(b, kSG, s), c - AT(off, s, offlim));
                 tt = OJ(b, kTP, p2);
                 bool exact;
-                algo = tl_ab1_decide(load_sgv(b.sgpack, s), load_sgo(b.sgouter, C, tt), load_sgo_xy(b.sgouter, C, tt), b1, exact);
+                algo = tl_ab1_decide(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
+                                     b.sgpack, s, tt, b1, exact);
             }
             passbuf_put(b, pb, algo != kAlgoNone, make_int4(s, tt, algo | (b1 << 8), p2));
         }
