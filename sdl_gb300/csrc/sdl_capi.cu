@@ -488,7 +488,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.pb, b.kept_cap);
     b.jidx3 = reinterpret_cast<int32_t*>(b.pb);  // (k_tctp_b has read its list when k_tctp_place writes)
     AL(b.sgpack, ctx->cap_obj[kSG] * PK_N);
-    AL(b.sgouter, ctx->cap_obj[kSG] * 11);
+    AL(b.sgouter, ctx->cap_obj[kSG] * kSgOuter);
     AL(b.sgfeat, ctx->cap_obj[kSG] * kFeatN);
     AL(b.mdpack, ctx->cap_obj[kMD] * kMdPack);
     AL(b.counters, ctx->n_ev * 110);

@@ -969,6 +969,19 @@ __device__ __forceinline__ SGOuter load_sgo(const float* __restrict__ a, int64_t
 __device__ __forceinline__ float4 load_sgo_xy(const float* __restrict__ a, int64_t cap, int64_t t) {
     return make_float4(__ldg(a + 7 * cap + t), __ldg(a + 8 * cap + t), __ldg(a + 9 * cap + t), __ldg(a + 10 * cap + t));
 }
+// arrays of the outer segment's fields: those, the four below, then what
+// b2_reject_early reads besides
+constexpr int kSgOuter = 14;
+struct SGBeta {
+    float lrt, uphi, ux, uy, alphaup, rtseg, sd;  // sd: urt - lrt
+};
+__device__ __forceinline__ SGBeta load_sgo_beta(const float* __restrict__ a, int64_t cap, int64_t t) {
+    return SGBeta{__ldg(a + t), __ldg(a + 4 * cap + t), __ldg(a + 9 * cap + t), __ldg(a + 10 * cap + t),
+                  __ldg(a + 11 * cap + t), __ldg(a + 12 * cap + t), __ldg(a + 13 * cap + t)};
+}
+__device__ __forceinline__ uint32_t sgo_flags(const float* __restrict__ a, int64_t cap, int64_t t) {
+    return __float_as_uint(__ldg(a + 5 * cap + t));
+}
 // the PV-offset term 0.1f / rtOut of the tracklet cuts (Tracklet.cc:1056 and
 // the like), precomputed for an SGOuter
 __device__ __forceinline__ float pv_off(const SGOuter& T) { return T.pvoff; }
@@ -1889,6 +1902,44 @@ __device__ __forceinline__ int tl_b2_quick(int algo, const SGV& S, const SGV& T,
         hiD * hiD * (1.f + 0x1p-21f) < cut2 - K * eCut2 - ulp_of(cut2))
         return 3;
     return 1;
+}
+
+// A cheap test ahead of tl_b2_quick for BBBB without a 2S endcap outer anchor:
+// true when the deltaBeta cut certainly fails.  With r = rtseg / dr of the two
+// segments and b = max(|betaIn|, |betaOut|) before the iterations, every branch
+// of those adds to betaIn and betaOut angles of the same sign,
+// asin(min(rIn v, 0.95)) and asin(min(rOut v, 0.95)), v = |sin| of a betaAv of at
+// most b + 1.32 min(rMax min(1, b), 0.95) (1.32 is above asin(x) / x up to 0.95).  So
+// deltaBeta moves by at most asin' |rIn - rOut| v, and the final |pt| is at
+// least D / min(1, b + 1.32 min(rMax v, 0.95)), which bounds dBetaMuls from above;
+// the cut's other terms are zero here but dBetaRes.  The directions are
+// phi_fast's (within 2.5e-6); the slack of 5e-5 and 1e-3 of the cut covers them
+// and the roundings.
+__device__ __forceinline__ bool b2_early(int algo, uint32_t outer_flags) {
+    return algo == kAlgoBBBB && !((outer_flags & F_UP_E) && (outer_flags & F_UP_2S));
+}
+__device__ __forceinline__ bool b2_reject_early(const SGV& S, const SGBeta& T) {
+    const float ax = T.ux - S.lx, ay = T.uy - S.ly;
+    const float dr2 = __fmaf_rn(ax, ax, ay * ay);
+    float pa;
+    if (!(dr2 > 1e-6f && dr2 < 1e10f) || !phi_fast(ax, ay, pa)) return false;
+    const float inv = rsqrtf(dr2);
+    const float w1 = wrap_approx(pa - S.lphi), w2 = wrap_approx(pa - T.uphi);
+    if (!(fabsf(w1) < 3.14f && fabsf(w2) < 3.14f)) return false;  // away from the wrap
+    const float bi = S.dpc - w1, bo = w2 - T.alphaup;
+    const float b = fmaxf(fabsf(bi), fabsf(bo));
+    const float ri = S.rtseg * inv, ro = T.rtseg * inv, rm = fmaxf(ri, ro);
+    const float v = fminf(1.f, __fmaf_rn(1.32f, fminf(rm * fminf(1.f, b), 0.95f), b));
+    const float y = fminf(rm * v, 0.95f);
+    const float move = rsqrtf(__fmaf_rn(-y, y, 1.f)) * fabsf(ri - ro) * v;
+    const float v2 = fminf(1.f, __fmaf_rn(1.32f, y, b));
+    const float d = T.lrt - S.lrt;
+    if (!(d >= 0.f && d < 1e4f)) return false;
+    const float u = __fmaf_rn(d, 0.004f, 0.1f);
+    const float muls = 0.06f * (u * rsqrtf(u)) * S.sqq_hi * fmaxf(v2 * inv * (1.f / k2Rinv1GeVf), 1.f / 7.f);
+    const float res = __fdividef(0.02f, fminf(T.sd, S.urt - S.lrt));
+    const float g = fabsf(bi - bo) - move * 1.001f - 5e-5f;
+    return g > 0.f && g * g > __fmaf_rn(__fmaf_rn(2.f * res, res, muls * muls), 1.001f, 1e-9f);
 }
 
 // phase B in one call (phase B1, then phase B2 on its survivors)

@@ -43,9 +43,10 @@ struct BatchDev {
     int32_t* conn_first;           // n_ev * n_conn: offset of the entry's module's first object
     int64_t* conn_sum;             // n_gm
     float* sgpack;                 // segment cap * PK_N packed records for the tracklet stage
-    float* sgouter;                // segment cap * 11, one array per field: what the enumeration reads of an
-                                   //   outer segment (lrt, lz, ltd, la1, uphi, flags, 0.1/lrt: SGOuter;
-                                   //   lx, ly, ux, uy: load_sgo_xy)
+    float* sgouter;                // segment cap * kSgOuter, one array per field: what the enumeration and the
+                                   //   B2 filter read of an outer segment (lrt, lz, ltd, la1, uphi, flags,
+                                   //   0.1/lrt: SGOuter; lx, ly, ux, uy: load_sgo_xy; alphaup, rtseg,
+                                   //   urt - lrt: load_sgo_beta)
     float* sgfeat;                 // segment cap * kFeatN: the pre-filter's per-segment feature records
     float* mdpack;                 // mini-doublet cap * kMdPack: packed records for the segment stage
     uint32_t* counters;            // n_ev * 110
