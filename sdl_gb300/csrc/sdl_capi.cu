@@ -639,6 +639,7 @@ int launch_checked(sdlg_ctx* ctx, int first, int last) {
 
 int launch(sdlg_ctx* ctx, int stop_after, int flags) {
     ctx->b.flags = flags;
+    if (stop_after >= kSG) ctx->b.seg_layers = (flags & SDLG_FLAG_SG_LAYERS) != 0;
     ctx->ran = true;
     wait_readback(ctx);
 #ifdef SDL_DEVICE_CHECKS
@@ -1348,6 +1349,7 @@ int sdlg_run_stages(sdlg_ctx* ctx, int first, int last, int flags) {
     if ((flags & SDLG_FLAG_MLP) && !ctx->mlp.have) return fail(ctx, SDLG_ERR_ARG, "SDLG_FLAG_MLP without pre-filter parameters");
     cudaSetDevice(ctx->device);
     ctx->b.flags = flags;
+    if (first <= kSG && last >= kSG) ctx->b.seg_layers = (flags & SDLG_FLAG_SG_LAYERS) != 0;
     ctx->last_stop = last;
     ctx->last_flags = flags;
     wait_readback(ctx);

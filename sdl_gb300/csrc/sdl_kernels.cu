@@ -1643,9 +1643,8 @@ __device__ __forceinline__ void pb_flush(const BatchDev& b, int4* buf, int& n, b
 // kEarly (pass 0 on the enumeration's list): b2_reject_early drops most of the
 // entries that fail, and the others wait in shared memory for a full warp of
 // tl_b2_quick.  (PU 100-300: 85 % of the entries are dropped; 64 events, 52
-// million entries: the filter 1.64
-// -> 1.10 ms.  The pre-filter's kept list has two passing entries in three and
-// goes straight to tl_b2_quick.)
+// million entries: the filter 1.64 -> 1.10 ms.  The pre-filter's kept list has
+// two passing entries in three and goes straight to tl_b2_quick.)
 template <int kPass, bool kEarly>
 __device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict__ in, const unsigned long long* n_in,
                                        int4 (*fbuf)[kPassBuf], int4 (*dbuf)[2][kPbBuf], int (*tbuf)[3][kRecBuf],
@@ -2003,15 +2002,24 @@ struct ScanObj : ScanOp {
     __device__ static void total(const BatchDev& b, int64_t n, const int64_t* t) { AT(b.obj[st].mod_cnt, n, NG1(b)) = t[0]; }
 };
 
-// a tracklet's place among those of its inner segment s
-__device__ __forceinline__ int tl_join_add(const BatchDev& b, int s) {
-    return (int)atomicAdd((unsigned long long*)&AT(b.joft, sg_key(b, s), b.obj[kSG].cap + 1), 1ull);
+// The tracklets that can be the outer one of a track candidate (g: the inner
+// module): those starting in barrel layer 3 (Event.cc:835), or all for
+// createTrackCandidatesFromTracklets.  Only these are indexed (128 dense events:
+// the track-candidate stage took 0.80 ms with all of them, 0.59 now).
+__device__ __forceinline__ bool tl_joins(const BatchDev& b, int g) {
+    if (b.flags & kFlagTCFromTL) return true;
+    const ModDev& m = MOD(b, mod_of(b, g));
+    return m.subdet == kBarrel && m.layer == 3;
+}
+// a tracklet's place among those of its inner segment s (0 when not indexed)
+__device__ __forceinline__ int tl_join_add(const BatchDev& b, int g, int s) {
+    return tl_joins(b, g) ? (int)atomicAdd((unsigned long long*)&AT(b.joft, sg_key(b, s), b.obj[kSG].cap + 1), 1ull) : 0;
 }
 __global__ void k_tl_join_count(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = n_objects(b, kTL);
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-        AT(b.trank, t, b.obj[kTL].cap) = tl_join_add(b, OI(b, kTL, t));
+        AT(b.trank, t, b.obj[kTL].cap) = tl_join_add(b, OG(b, kTL, t), OI(b, kTL, t));
 }
 
 // The stage's records into the dense arrays grouped by inner module.  kJoin
@@ -2041,7 +2049,7 @@ __global__ void __launch_bounds__(256) k_scatter(BatchDev b) {
 #pragma unroll
         for (int k = 0; k < kNF; ++k)
             AT(O.f, (int64_t)k * O.cap + pos, O.cap * kNF) = AT(R.f, (int64_t)k * O.cap + r, O.cap * kNF);
-        if (kJoin) AT(b.trank, pos, O.cap) = tl_join_add(b, i);
+        if (kJoin) AT(b.trank, pos, O.cap) = tl_join_add(b, g, i);
     }
     if (st == kMD && b.joff)
         for (int64_t k = tid; k <= n; k += stride) AT(b.joff, k, O.cap + 1) = 0;
@@ -2356,6 +2364,10 @@ struct ScanTp : ScanJoined<kTP> {
         const int md = OJ(b, kSG, s);
         const int64_t n = join_n(b, md);
         if (n == 0) return;
+        v[0] = n;
+        // (a module-map segment's outer module is in the list, once unless the
+        // list repeats modules)
+        if (!b.seg_layers && !b.geo.conn_dup) return;
         const int g1 = OG(b, kSG, s);
         const int ev = ev_of(b, g1);
         v[0] = (int64_t)conn_mult(b, g1 - ev * b.geo.n_mod, OG(b, kMD, md) - ev * b.geo.n_mod) * n;
@@ -2386,9 +2398,10 @@ struct ScanTc : ScanJoined<kTC> {
     __device__ static void load(const BatchDev& b, int64_t t, bool in, int64_t* v) {
         v[0] = 0;
         if (!in) return;
-        tl_join_place(b, t);
         const ModDev& m1 = MOD(b, mod_of(b, OG(b, kTL, t)));
-        if (m1.subdet != kBarrel || m1.layer != 1) return;
+        if (m1.subdet != kBarrel) return;
+        if (m1.layer == 3) tl_join_place(b, t);
+        if (m1.layer != 1) return;
         const int sB = OJ(b, kTL, t);
         const ModDev& m3 = MOD(b, mod_of(b, OG(b, kSG, sB)));
         if (m3.subdet == kBarrel && m3.layer == 3) v[0] = tl_join_n(b, sB);

@@ -58,6 +58,7 @@ struct BatchDev {
     int64_t bucket_cap;
     int flags;                     // kFlag* bits
     int first, last;               // the stages being enqueued
+    bool seg_layers;               // the segments are (or will be) those of the layer pairs
     // launch shape of each stage's candidate-evaluation kernel (autotuned):
     // candidates per warp task (a multiple of 32) and CTAs per SM
     int enum_task[kNumStages];
