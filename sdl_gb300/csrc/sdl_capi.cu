@@ -491,6 +491,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.sgouter, ctx->cap_obj[kSG] * kSgOuter);
     AL(b.sgfeat, ctx->cap_obj[kSG] * kFeatN);
     AL(b.mdpack, ctx->cap_obj[kMD] * kMdPack);
+    AL(b.mdlite, ctx->cap_obj[kMD] * kMdLite);
     AL(b.counters, ctx->n_ev * 110);
     int64_t mx = n_gm;
     for (int s = 0; s < kNumStages; ++s) mx = std::max(mx, ctx->cap_obj[s]);

@@ -715,9 +715,6 @@ __device__ __forceinline__ float sg_barrel_cut(int lIn, float rtOut, float outAs
 // Segment.cc:364-599.  outAsin / outTanf: asin(min(rtOut*k,.95)) of the
 // outer anchor and its float tan; cutPrev: sg_barrel_cut for the barrel
 // layer below the outer one (k_md_pack).
-// kPre: only the first cuts (the z window and the phi cut), for the segment
-// stage's first pass; a candidate they reject fails the whole algorithm
-template <bool kPre = false>
 __device__ __forceinline__ bool sg_barrel(const MDView& im, const MDView& om, float outAsin, float outTanf, float cutPrev,
                                           SGVals& v) {
     const float rtIn = im.a.rt, rtOut = om.a.rt, zIn = im.a.z, zOut = om.a.z;
@@ -731,7 +728,6 @@ __device__ __forceinline__ bool sg_barrel(const MDView& im, const MDView& om, fl
     const float sdCut = prev ? cutPrev : sg_barrel_cut(im.m->layer, rtOut, outAsin);
     const float deltaPhi = dphi(im.a, om.a);
     if (!(fabsf(deltaPhi) <= sdCut)) return false;
-    if (kPre) return true;
     v.dphichange = dphichange(im.a, om.a);
     if (!(fabsf(v.dphichange) <= sdCut)) return false;
     return dalpha_cuts(im, om, v.dphichange);
@@ -740,8 +736,6 @@ __device__ __forceinline__ bool sg_barrel(const MDView& im, const MDView& om, fl
 // Segment.cc:601-859.  connected: outer module is in the inner module's
 // connection list (cut #0); phiHi / phiLo: the phi of the outer anchor's
 // strip-edge points (the anchor itself for PS modules; k_md_pack).
-// kPre: only the first cuts (connection, rt window and phi cut), as sg_barrel
-template <bool kPre = false>
 __device__ __forceinline__ bool sg_endcap(const MDView& im, const MDView& om, float outAsin, float outTanf,
                                           bool connected, float phiHi, float phiLo, SGVals& v) {
     const ModDev& I = *im.m;
@@ -763,7 +757,6 @@ __device__ __forceinline__ bool sg_endcap(const MDView& im, const MDView& om, fl
     const float dPhiPos = dphi(im.a, om.a);
     const float sdCut = sdSlope;
     if (!(fabsf(dPhiPos) <= sdCut)) return false;
-    if (kPre) return true;
     const float hiP = phi_mpi_pi(phiHi - im.a.phi);  // dphi(im.a, oHi)
     const float loP = phi_mpi_pi(phiLo - im.a.phi);
     const bool hiBigger = iabs(trunc_i32(hiP)) > iabs(trunc_i32(loP));
@@ -776,6 +769,53 @@ __device__ __forceinline__ bool sg_endcap(const MDView& im, const MDView& om, fl
     v.dphiminchange = v.dphimin / dzFrac * (1.f + dzFrac);
     v.dphimaxchange = v.dphimax / dzFrac * (1.f + dzFrac);
     return dalpha_cuts(im, om, v.dphichange);
+}
+
+// The first pass over the segment candidates: false only when the z or rt
+// window or the phi cut of sg_barrel / sg_endcap certainly fails; the second
+// pass runs the whole algorithm on what is left.  Both mini-doublets come as
+// 32-byte records (k_md_pack): rt, z, phi, the phi cut (barrel: sdCut for the
+// layer below, endcap: asin), dzDrtScale (barrel) or its inverse (endcap), and
+// the layer with the kind.  The windows are within 2^-24 * 14 times the sum of
+// their terms' magnitudes of the exact code's (its roundings and these, one
+// quotient by __fdividef), and are widened by 2^-18 of that sum; the phi
+// difference past the wrap is within 5e-7, and its cut is widened by 1e-6.
+struct MDLite {
+    float rt, z, phi, cut, scale;
+    uint32_t fl;  // layer, kMdBarrel or kMdEndcap
+};
+enum : uint32_t { kMdLayer = 15u, kMdBarrel = 16u, kMdEndcap = 32u };
+constexpr int kMdLite = 8;  // floats per record
+__device__ __forceinline__ bool sg_first_cuts(const MDLite& I, const MDLite& O) {
+    constexpr float kM = 0x1p-18f;
+    const float d = O.phi - I.phi;
+    const float adphi = fminf(fabsf(d), 6.28318531f - fabsf(d));
+    if (O.fl & kMdBarrel) {
+        const uint32_t layer = I.fl & kMdLayer;
+        const float zGeom = layer <= 2 ? 2.f * kPixelPSZpitch : 2.f * kStrip2SZpitch;
+        const float t = __fdividef(O.rt, I.rt) - 1.f;
+        const float sLo = I.z > 0.f ? 1.f : O.scale, sHi = I.z < 0.f ? 1.f : O.scale;
+        const float lo = __fmaf_rn((I.z - kDeltaZLum) * sLo, t, I.z - zGeom);
+        const float hi = __fmaf_rn((I.z + kDeltaZLum) * sHi, t, I.z + zGeom);
+        const float m = kM * __fmaf_rn((fabsf(I.z) + kDeltaZLum) * fmaxf(fabsf(sLo), fabsf(sHi)), fabsf(t) + 2.f,
+                                       fabsf(I.z) + zGeom);
+        if (O.z < lo - m || O.z > hi + m) return false;
+        // (the cut of another layer pair is left to the second pass)
+        const bool prev = (I.fl & kMdBarrel) && layer + 1u == (O.fl & kMdLayer);
+        return !(prev && adphi > __fmaf_rn(O.cut, 1.f + 1e-6f, 1e-6f));
+    }
+    const float kR = 60.f;
+    const float rtGeom = (I.rt < kR && O.rt < kR) ? 2.f * kPixelPSZpitch
+                       : ((I.rt < kR || O.rt < kR) ? kPixelPSZpitch + kStrip2SZpitch : 2.f * kStrip2SZpitch);
+    if (I.z * O.z < 0) return false;
+    const float dLum = f_copysign(kDeltaZLum, I.z);
+    const float q1 = __fdividef((O.z - I.z) * O.scale, I.z + dLum), q2 = __fdividef(O.z - dLum, I.z - dLum);
+    const float lo = fmaxf(__fmaf_rn(I.rt, q1, I.rt) - rtGeom, __fmaf_rn(-0.5f, rtGeom, I.rt));
+    const float hi = __fmaf_rn(I.rt, q2, rtGeom);
+    // (the first quotient's numerator is a difference: its terms' magnitudes)
+    const float m = 4.f * kM * (fabsf(I.rt) * (1.f + fabsf(__fdividef((fabsf(O.z) + fabsf(I.z)) * O.scale, I.z + dLum)) + fabsf(q2)) + rtGeom);
+    if (O.rt < lo - m || O.rt > hi + m) return false;
+    return !(adphi > __fmaf_rn(O.cut, 1.f + 1e-6f, 1e-6f));
 }
 
 // ------------------------------------------------------------------ tracklets

@@ -473,6 +473,12 @@ __device__ __forceinline__ MDRec md_rec(const BatchDev& b, int64_t a) {
     return r;
 }
 
+__device__ __forceinline__ MDLite md_lite(const BatchDev& b, int64_t a) {
+    const float4* q = reinterpret_cast<const float4*>(&AT(b.mdlite, a * kMdLite, b.obj[kMD].cap * kMdLite));
+    const float4 r0 = __ldg(q);
+    const float2 r1 = __ldg(reinterpret_cast<const float2*>(q + 1));
+    return MDLite{r0.x, r0.y, r0.z, r0.w, r1.x, __float_as_uint(r1.y)};
+}
 __global__ void k_md_pack(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = n_objects(b, kMD);
@@ -500,6 +506,13 @@ __global__ void k_md_pack(BatchDev b) {
             c0 = c1 = p.phi;
         }
         q[3] = make_float4(__int_as_float(lm), __int_as_float(am), c0, c1);
+        // the first pass's record (sg_first_cuts)
+        const bool barrel = M.subdet == kBarrel;
+        const float tf = AT(b.htf, anc, H(b));
+        float4* l = reinterpret_cast<float4*>(&AT(b.mdlite, a * kMdLite, b.obj[kMD].cap * kMdLite));
+        l[0] = make_float4(p.rt, p.z, p.phi, barrel ? c0 : a1);
+        l[1] = make_float4(barrel ? tf / a1 : a1 / tf, __uint_as_float((uint32_t)(M.layer & 15) | (barrel ? kMdBarrel : kMdEndcap)),
+                           0.f, 0.f);
     }
 }
 
@@ -509,15 +522,15 @@ __global__ void k_md_pack(BatchDev b) {
 // kOuter: 0 either algorithm, 1 only the barrel one (outer MD in the barrel),
 // 2 only the endcap one (a kernel compiled for one keeps the other's code out
 // of its instruction caches); a candidate of the other kind fails
-template <bool kPre = false, int kOuter = 0>
+template <int kOuter = 0>
 __device__ __forceinline__ bool sg_pair_rec(const MDView& im, const MDRec& orec, bool connected, float* fv) {
     const MDView& om = orec.v;
     SGVals v;
     v.dphi = v.dphimin = v.dphimax = v.dphichange = v.dphiminchange = v.dphimaxchange = 0.f;
     bool pass = false;
     const bool ob = om.m->subdet == kBarrel;
-    if (kOuter != 2 && ob) pass = sg_barrel<kPre>(im, om, orec.a1, orec.tf, orec.c0, v);
-    else if (kOuter != 1 && !ob) pass = sg_endcap<kPre>(im, om, orec.a1, orec.tf, connected, orec.c0, orec.c1, v);
+    if (kOuter != 2 && ob) pass = sg_barrel(im, om, orec.a1, orec.tf, orec.c0, v);
+    else if (kOuter != 1 && !ob) pass = sg_endcap(im, om, orec.a1, orec.tf, connected, orec.c0, orec.c1, v);
     fv[0] = v.dphi; fv[1] = v.dphimin; fv[2] = v.dphimax;
     fv[3] = v.dphichange; fv[4] = v.dphiminchange; fv[5] = v.dphimaxchange;
     return pass;
@@ -1302,10 +1315,10 @@ constexpr int kSgbMinBlocks = SDLG_SGB_MIN_BLOCKS;
 
 // Segment candidates in two passes (Event.cc:445-522 or 793-821 with
 // Segment.cc:337-859): k_sg_enum_a takes tasks of consecutive candidates
-// like k_enum, runs the algorithm's first cuts (sg_pair_rec<true>: the same
-// float code as the whole algorithm up to its phi cut) and lists the
-// survivors in the passa list; k_sg_b runs the whole algorithm on the list on
-// full warps and appends the segments.  The first cuts reject most
+// like k_enum and lists those the algorithm's first cuts do not certainly
+// reject (sg_first_cuts, on 32-byte records: with the exact first cuts on the
+// 64-byte records it took 547 us for 64 events, 412 now); k_sg_b runs the whole algorithm on the list
+// on full warps and appends the segments.  The first cuts reject most
 // candidates, so the expensive rest (the direction-change and dAlpha cuts)
 // no longer runs beside idle lanes.
 // A warp's segment first-pass survivors appended to the spare list pb:
@@ -1375,10 +1388,9 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
                 const int64_t q = c - AT(off, a, offlim);
                 bmd = kLayers ? layer_md(layer_row(b, a), (int)q) : sg_outer_md(b, a, q);
                 (void)IX(bmd, b.obj[kMD].cap);
-                float fv[6];
-                const MDRec orec = md_rec(b, bmd);
-                ob = orec.v.m->subdet == kBarrel;
-                pass = sg_pair_rec<true>(md_rec(b, a).v, orec, true, fv);
+                const MDLite O = md_lite(b, bmd);
+                ob = (O.fl & kMdBarrel) != 0;
+                pass = sg_first_cuts(md_lite(b, a), O);
             }
             const unsigned lt = (1u << lane) - 1u;
             const unsigned mf = __ballot_sync(0xffffffffu, pass && ob), mb = __ballot_sync(0xffffffffu, pass && !ob);
@@ -1412,7 +1424,7 @@ __device__ __forceinline__ void sg_b(const BatchDev& b, int (*rbuf)[3 + 6][kRecB
             a = e.x;
             bmd = e.y;
             const bool conn = kOuter == 1 || !(b.flags & kFlagSGLayers) || sg_connected(b, a, bmd);
-            pass = sg_pair_rec<false, kOuter>(md_rec(b, a).v, md_rec(b, bmd), conn, fv);
+            pass = sg_pair_rec<kOuter>(md_rec(b, a).v, md_rec(b, bmd), conn, fv);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pass);
         if (!m) continue;

@@ -49,6 +49,7 @@ struct BatchDev {
                                    //   urt - lrt: load_sgo_beta)
     float* sgfeat;                 // segment cap * kFeatN: the pre-filter's per-segment feature records
     float* mdpack;                 // mini-doublet cap * kMdPack: packed records for the segment stage
+    float* mdlite;                 // mini-doublet cap * kMdLite: what its first pass reads
     uint32_t* counters;            // n_ev * 110
     uint32_t* status;
     unsigned long long* task;      // per stage (kLine apart): work counter
