@@ -771,20 +771,24 @@ __device__ __forceinline__ bool sg_endcap(const MDView& im, const MDView& om, fl
     return dalpha_cuts(im, om, v.dphichange);
 }
 
-// The first pass over the segment candidates: false only when the z or rt
-// window or the phi cut of sg_barrel / sg_endcap certainly fails; the second
-// pass runs the whole algorithm on what is left.  Both mini-doublets come as
-// 32-byte records (k_md_pack): rt, z, phi, the phi cut (barrel: sdCut for the
-// layer below, endcap: asin), dzDrtScale (barrel) or its inverse (endcap), and
-// the layer with the kind.  The windows are within 2^-24 * 14 times the sum of
-// their terms' magnitudes of the exact code's (its roundings and these, one
-// quotient by __fdividef), and are widened by 2^-18 of that sum; the phi
-// difference past the wrap is within 5e-7, and its cut is widened by 1e-6.
+// The first pass over the segment candidates, in two steps that reject only
+// what sg_barrel / sg_endcap certainly reject; the second pass runs the whole
+// algorithm on what is left.  Both mini-doublets come as 32-byte records
+// (k_md_pack): rt, z, phi of the anchor, the phi cut (barrel: sdCut for the
+// layer below, endcap: asin), dzDrtScale (barrel) or its inverse (endcap), the
+// luminosity term's factor (tilted barrel: tilt, other barrel: 0, endcap: the
+// term itself), dphichange, and 0.02 / gap with the layer and kind in its last
+// six bits.
+// sg_first_cuts: the z or rt window and the phi cut.  The windows are within
+// 2^-24 * 14 times the sum of their terms' magnitudes of the exact code's (its
+// roundings and these, one quotient by __fdividef), and are widened by 2^-18
+// of that sum; the phi difference past the wrap is within 5e-7, and its cut is
+// widened by 1e-6.
 struct MDLite {
-    float rt, z, phi, cut, scale;
+    float rt, z, phi, cut, scale, lum, dpc, res;
     uint32_t fl;  // layer, kMdBarrel or kMdEndcap
 };
-enum : uint32_t { kMdLayer = 15u, kMdBarrel = 16u, kMdEndcap = 32u };
+enum : uint32_t { kMdLayer = 15u, kMdBarrel = 16u, kMdEndcap = 32u, kMdFlags = 63u };
 constexpr int kMdLite = 8;  // floats per record
 __device__ __forceinline__ bool sg_first_cuts(const MDLite& I, const MDLite& O) {
     constexpr float kM = 0x1p-18f;
@@ -816,6 +820,49 @@ __device__ __forceinline__ bool sg_first_cuts(const MDLite& I, const MDLite& O) 
     const float m = 4.f * kM * (fabsf(I.rt) * (1.f + fabsf(__fdividef((fabsf(O.z) + fabsf(I.z)) * O.scale, I.z + dLum)) + fabsf(q2)) + rtGeom);
     if (O.rt < lo - m || O.rt > hi + m) return false;
     return !(adphi > __fmaf_rn(O.cut, 1.f + 1e-6f, 1e-6f));
+}
+// sg_later_cuts: the direction-change and dAlpha cuts, with the outer anchor
+// in the frame of the inner one's phi.  sin and cos of the phi difference are
+// within 5e-7 (its own rounding included) and 4e-7 (__sinf, __cosf), so with
+// R = rtIn + rtOut the two coordinates and dr are within 1.2e-6 R of the exact
+// code's, the barrel's direction change within 1.2e-6 R / dr + 1e-6, and the
+// endcap's within 5e-7 of its factor plus 5e-7 of itself: four times that is
+// allowed.  The bend asin(min(dr * k, .95)) is within 3.2 (the slope at .95) *
+// k * 1.2e-6 R = 2.2e-8 R, and 0.02 / gap within 2^-17 of itself (the flag
+// bits), so each dAlpha threshold is widened by 1e-7 R + 1e-5 + 1e-4 of itself.
+// Values that are not finite fail no cut here.
+__device__ __forceinline__ bool sg_later_cuts(const MDLite& I, const MDLite& O) {
+    const bool ib = (I.fl & kMdBarrel) != 0, ob = (O.fl & kMdBarrel) != 0;
+    float d = O.phi - I.phi;
+    if (d > kPiF) d -= 2.f * kPiF;
+    else if (d < -kPiF) d += 2.f * kPiF;
+    const float x = __fmaf_rn(O.rt, __cosf(d), -I.rt), y = O.rt * __sinf(d);
+    const float dr2 = __fmaf_rn(x, x, y * y), rdr = rsqrtf(dr2), dr = dr2 * rdr, R = I.rt + O.rt;
+    float q, eq;
+    bool cut = true;
+    const uint32_t layer = I.fl & kMdLayer;
+    if (ob) {
+        q = atan2f(y, x);
+        eq = __fmaf_rn(5e-6f * R, rdr, 4e-6f);
+        cut = ib && layer + 1u == (O.fl & kMdLayer);  // (another layer pair's cut is left to the second pass)
+    } else {
+        const float f = __fdividef(O.z - I.z, I.z), g = __fdividef(1.f + f, f);
+        q = d * g;
+        eq = 2e-6f * (fabsf(g) + fabsf(q));
+    }
+    if (cut && fabsf(q) > __fmaf_rn(O.cut, 1.f + 1e-6f, 1e-6f) + eq) return false;
+    const float al = asinf(fminf(dr * (k2Rinv1GeVf / kPtCut), kSinAlphaMax));
+    float muls = 0.006f * 3.f / kPtCut;
+    if (ib) muls = (layer == 1u ? 0.0052f : layer == 2u ? 0.0038f : layer == 5u ? 0.0032f : 0.0034f) * 3.f / kPtCut;
+    const float res = I.res * ((ib ? 1.f : fabsf(__fdividef(I.z, I.rt))) + (ob ? 1.f : fabsf(__fdividef(O.z, O.rt))));
+    const float v = __fmaf_rn(res, res, muls * muls);
+    auto outside = [&](float u, float lum, float e) {
+        const float t = al + __fsqrt_rn(__fmaf_rn(lum, lum, v));
+        return fabsf(u) > __fmaf_rn(t, 1.f + 1e-4f, __fmaf_rn(1e-7f, R, 1e-5f)) + e;
+    };
+    if (outside(O.dpc - I.dpc, 0.f, 0.f)) return false;
+    if (outside(I.dpc - q, ib ? I.lum * al : I.lum, eq)) return false;
+    return !outside(O.dpc - q, ob ? O.lum * al : O.lum, eq);
 }
 
 // ------------------------------------------------------------------ tracklets

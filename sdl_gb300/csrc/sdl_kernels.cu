@@ -475,9 +475,8 @@ __device__ __forceinline__ MDRec md_rec(const BatchDev& b, int64_t a) {
 
 __device__ __forceinline__ MDLite md_lite(const BatchDev& b, int64_t a) {
     const float4* q = reinterpret_cast<const float4*>(&AT(b.mdlite, a * kMdLite, b.obj[kMD].cap * kMdLite));
-    const float4 r0 = __ldg(q);
-    const float2 r1 = __ldg(reinterpret_cast<const float2*>(q + 1));
-    return MDLite{r0.x, r0.y, r0.z, r0.w, r1.x, __float_as_uint(r1.y)};
+    const float4 r0 = __ldg(q), r1 = __ldg(q + 1);
+    return MDLite{r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, __float_as_uint(r1.w) & kMdFlags};
 }
 __global__ void k_md_pack(BatchDev b) {
     if (halted(b)) return;
@@ -506,13 +505,16 @@ __global__ void k_md_pack(BatchDev b) {
             c0 = c1 = p.phi;
         }
         q[3] = make_float4(__int_as_float(lm), __int_as_float(am), c0, c1);
-        // the first pass's record (sg_first_cuts)
+        // the first pass's record (sg_first_cuts, sg_later_cuts)
         const bool barrel = M.subdet == kBarrel;
         const float tf = AT(b.htf, anc, H(b));
         float4* l = reinterpret_cast<float4*>(&AT(b.mdlite, a * kMdLite, b.obj[kMD].cap * kMdLite));
         l[0] = make_float4(p.rt, p.z, p.phi, barrel ? c0 : a1);
-        l[1] = make_float4(barrel ? tf / a1 : a1 / tf, __uint_as_float((uint32_t)(M.layer & 15) | (barrel ? kMdBarrel : kMdEndcap)),
-                           0.f, 0.f);
+        const float lum = barrel ? (M.side != kCenter ? M.tilt : 0.f)
+                                 : 15.f * OF(b, kMD, 2, a) / OF(b, kMD, M.type == kPS ? 1 : 0, a);
+        const uint32_t fl = (uint32_t)(M.layer & 15) | (barrel ? kMdBarrel : kMdEndcap);
+        l[1] = make_float4(barrel ? tf / a1 : a1 / tf, lum, OF(b, kMD, 3, a),
+                           __uint_as_float((__float_as_uint(0.02f / M.gap) & ~kMdFlags) | fl));
     }
 }
 
@@ -1315,12 +1317,13 @@ constexpr int kSgbMinBlocks = SDLG_SGB_MIN_BLOCKS;
 
 // Segment candidates in two passes (Event.cc:445-522 or 793-821 with
 // Segment.cc:337-859): k_sg_enum_a takes tasks of consecutive candidates
-// like k_enum and lists those the algorithm's first cuts do not certainly
-// reject (sg_first_cuts, on 32-byte records: with the exact first cuts on the
-// 64-byte records it took 547 us for 64 events, 412 now); k_sg_b runs the whole algorithm on the list
-// on full warps and appends the segments.  The first cuts reject most
-// candidates, so the expensive rest (the direction-change and dAlpha cuts)
-// no longer runs beside idle lanes.
+// like k_enum, gathers those the algorithm's first cuts do not certainly
+// reject (40 % of them) to full warps, and lists those that the later cuts do
+// not certainly reject either (7.7 %; 7.6 % are segments); k_sg_b runs the
+// whole algorithm on the list and appends the segments.  Both are bound by
+// instruction issue.  64 events: with the exact first cuts on 64-byte records
+// the first pass took 547 us and the second, on the 40 %, 870; with
+// sg_first_cuts alone 412 and 870; with the later cuts 437 and 257.
 // A warp's segment first-pass survivors appended to the spare list pb:
 // candidates with a barrel outer MD at its front (count n_pb[0]), the others
 // at its back (n_pb[1]), so that the second pass runs each algorithm in its
@@ -1352,6 +1355,7 @@ __device__ __forceinline__ void sg_list_flush(const BatchDev& b, int4* buf, int&
 template <bool kLayers>
 __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     __shared__ int4 sbuf[kEnumThreads / kWarp][2][kPbBuf];
+    __shared__ int2 mbuf[kEnumThreads / kWarp][2 * kWarp];
     if (halted(b)) return;
     const int64_t nobj = n_inner(b, kSG);
     if (nobj <= 0) return;
@@ -1363,7 +1367,30 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     const int lane = threadIdx.x & 31;
     int4* fb = sbuf[threadIdx.x >> 5][0];
     int4* bb = sbuf[threadIdx.x >> 5][1];
-    int nf = 0, nb = 0;
+    int2* mb = mbuf[threadIdx.x >> 5];
+    int nf = 0, nb = 0, nm = 0;
+    const unsigned lt = (1u << lane) - 1u;
+    // the later cuts on the last n of mb's pairs, one a lane
+    auto later = [&](int n) {
+        __syncwarp();
+        int2 e = make_int2(0, 0);
+        bool pass = false, ob = false;
+        if (lane < n) {
+            e = mb[nm - n + lane];
+            const MDLite O = md_lite(b, e.y);
+            ob = (O.fl & kMdBarrel) != 0;
+            pass = sg_later_cuts(md_lite(b, e.x), O);
+        }
+        __syncwarp();
+        nm -= n;
+        const unsigned mf = __ballot_sync(0xffffffffu, pass && ob), mo = __ballot_sync(0xffffffffu, pass && !ob);
+        if (nf + __popc(mf) > kPbBuf) sg_list_flush(b, fb, nf, true);
+        if (nb + __popc(mo) > kPbBuf) sg_list_flush(b, bb, nb, false);
+        if (pass && ob) fb[nf + __popc(mf & lt)] = make_int4(e.x, e.y, 1, 0);
+        if (pass && !ob) bb[nb + __popc(mo & lt)] = make_int4(e.x, e.y, 2, 0);
+        nf += __popc(mf);
+        nb += __popc(mo);
+    };
     for (;;) {
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(b.task + kSG * kLine, 1ull);
@@ -1382,26 +1409,21 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
         for (int64_t cb = base; cb < end; cb += kWarp) {
             const int64_t c = cb + lane;
             int a = 0, bmd = 0;
-            bool pass = false, ob = false;
+            bool pass = false;
             if (c < end) {
                 a = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
                 const int64_t q = c - AT(off, a, offlim);
                 bmd = kLayers ? layer_md(layer_row(b, a), (int)q) : sg_outer_md(b, a, q);
                 (void)IX(bmd, b.obj[kMD].cap);
-                const MDLite O = md_lite(b, bmd);
-                ob = (O.fl & kMdBarrel) != 0;
-                pass = sg_first_cuts(md_lite(b, a), O);
+                pass = sg_first_cuts(md_lite(b, a), md_lite(b, bmd));
             }
-            const unsigned lt = (1u << lane) - 1u;
-            const unsigned mf = __ballot_sync(0xffffffffu, pass && ob), mb = __ballot_sync(0xffffffffu, pass && !ob);
-            if (nf + __popc(mf) > kPbBuf) sg_list_flush(b, fb, nf, true);
-            if (nb + __popc(mb) > kPbBuf) sg_list_flush(b, bb, nb, false);
-            if (pass && ob) fb[nf + __popc(mf & lt)] = make_int4(a, bmd, 1, 0);
-            if (pass && !ob) bb[nb + __popc(mb & lt)] = make_int4(a, bmd, 2, 0);
-            nf += __popc(mf);
-            nb += __popc(mb);
+            const unsigned m = __ballot_sync(0xffffffffu, pass);
+            if (pass) mb[nm + __popc(m & lt)] = make_int2(a, bmd);
+            nm += __popc(m);
+            if (nm >= kWarp) later(kWarp);
         }
     }
+    later(nm);
     sg_list_flush(b, fb, nf, true);
     sg_list_flush(b, bb, nb, false);
 }
