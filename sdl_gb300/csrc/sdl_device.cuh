@@ -473,11 +473,10 @@ __device__ constexpr float kDeltaZLum = 15.f;
 
 // ------------------------------------------------------------------ mini-doublets
 // MiniDoublet.cc:741-810
-__device__ __forceinline__ float dphi_threshold(float rt, float asin_rt1, const ModDev& m, float dPhi, float dz) {
+// the multiple-scattering and vertex terms of module m's layer
+__device__ __forceinline__ void dphi_layer_terms(const ModDev& m, float& miniMuls, float& miniPVoff) {
     const float mulsB[6] = {0.0052f, 0.0038f, 0.0034f, 0.0034f, 0.0032f, 0.0034f};
     const unsigned iL = m.layer - 1;
-    const float miniSlope = asin_rt1;  // asin(min(rt * k2Rinv1GeVf / 1, 0.95))
-    (void)rt;
     const bool barrel = m.subdet == kBarrel;
     // (float)(0.1 / (double)rLay) for the layer radii 21.8 ... 106.8 (barrel) and
     // 131.4 ... 261.5 (endcap) of MiniDoublet.cc:763-767: constant per layer
@@ -485,8 +484,14 @@ __device__ __forceinline__ float dphi_threshold(float rt, float asin_rt1, const 
                               (float)(0.1 / (double)67.4f), (float)(0.1 / (double)87.6f), (float)(0.1 / (double)106.8f)};
     constexpr float pvE[5] = {(float)(0.1 / (double)131.4f), (float)(0.1 / (double)156.2f), (float)(0.1 / (double)185.6f),
                               (float)(0.1 / (double)220.3f), (float)(0.1 / (double)261.5f)};
-    const float miniPVoff = barrel ? pvB[iL] : pvE[iL];
-    const float miniMuls = barrel ? mulsB[iL] * 3.f / kPtCut : 0.006f * 3.f / kPtCut;
+    miniPVoff = barrel ? pvB[iL] : pvE[iL];
+    miniMuls = barrel ? mulsB[iL] * 3.f / kPtCut : 0.006f * 3.f / kPtCut;
+}
+// miniSlope: asin(min(rt * k2Rinv1GeVf / 1, 0.95))
+__device__ __forceinline__ float dphi_threshold(float miniSlope, const ModDev& m, float dPhi, float dz) {
+    float miniMuls, miniPVoff;
+    dphi_layer_terms(m, miniMuls, miniPVoff);
+    const bool barrel = m.subdet == kBarrel;
     if (barrel && m.side == kCenter) return add_dsqrt3(miniSlope, miniMuls, miniPVoff, 0.f);
     if (barrel) return add_dsqrt3(miniSlope, miniMuls, miniPVoff, m.tilt * miniSlope);
     const float miniLum = (float)iabs(trunc_i32(dPhi * kDeltaZLum / dz));
@@ -574,7 +579,7 @@ __device__ __forceinline__ bool md_barrel(const P3& lo, const P3& up, float pixA
     const float sign = (float)(((dz > 0) - (dz < 0)) * ((lo.z > 0) - (lo.z < 0)));
     const float inverted = (float)(iabs(trunc_i32(dz)) > 2) * sign;
     if (!(fabsf(dz) < dzCut && inverted <= 0)) return false;
-    const float miniCut = dphi_threshold(0.f, pixAsin, lm, 0.f, 1.f);
+    const float miniCut = dphi_threshold(pixAsin, lm, 0.f, 1.f);
     P3 shifted;
     if (lm.side != kCenter) {
         float xn, yn;
@@ -593,10 +598,6 @@ __device__ __forceinline__ bool md_barrel(const P3& lo, const P3& up, float pixA
         if (lm.ltype == kPixel) { a = lo.rt < shifted.rt ? &lo : &shifted; b = lo.rt < shifted.rt ? &shifted : &lo; }
         else { a = shifted.rt < up.rt ? &shifted : &up; b = shifted.rt < up.rt ? &up : &shifted; }
     }
-    // most candidates fail this cut: the direction of b - a from atan2f (a's
-    // direction is exact) rejects those clearly outside it before the exact one
-    float q;
-    if (dphi_q(a->phi, atan2f(b->y - a->y, b->x - a->x), q) && fabsf(q) >= miniCut + kB2qSafety * kB2qDir) return false;
     v.dphichange = dphichange(*a, *b);
     return fabsf(v.dphichange) < miniCut;
 }
@@ -619,11 +620,64 @@ __device__ __forceinline__ bool md_endcap(const P3& lo, const P3& up, float pixA
         v.shiftedDz = lm.ltype == kPixel ? lo.z - zn : up.z - zn;
         dz = v.shiftedDz;
     }
-    const float miniCut = dphi_threshold(0.f, pixAsin, lm, v.dphi, dz);
+    const float miniCut = dphi_threshold(pixAsin, lm, v.dphi, dz);
     if (!(fabsf(v.dphi) < miniCut)) return false;
     const float dzFrac = fabsf(dz) / fabsf(lo.z);  // a double division of two floats rounded to float
     v.dphichange = v.dphi / dzFrac * (1.f + dzFrac);
     return fabsf(v.dphichange) < miniCut;
+}
+
+// The first pass over the mini-doublet candidates: false only when md_barrel /
+// md_endcap certainly reject; the second pass runs the whole algorithm on what
+// is left.  The cuts that need no direction are taken as they are; a direction
+// difference is judged by its sine, the cross product of the two points over
+// their lengths (never larger than the angle), which single precision gives
+// within 4e-7 with the coordinates' difference as one factor.  The thresholds
+// are widened by 1e-5 and 1e-5 of themselves, for this and for the exact
+// code's roundings (its angle is within 6e-7).  Values that are not finite
+// fail only the cuts taken as they are.
+__device__ __forceinline__ bool md_first_cuts(const P3& lo, const P3& up, float pixAsin, const ModDev& lm, const float* sh) {
+    const bool barrel = lm.subdet == kBarrel, ps = lm.type == kPS, pixLower = lm.ltype == kPixel;
+    float dz = lo.z - up.z;
+    if (barrel) {
+        const float sign = (float)(((dz > 0) - (dz < 0)) * ((lo.z > 0) - (lo.z < 0)));
+        const float inverted = (float)(iabs(trunc_i32(dz)) > 2) * sign;
+        if (!(fabsf(dz) < (ps ? 2.f : 10.f) && inverted <= 0)) return false;
+    } else if (!(fabsf(dz) < 10.f && fabsf(lo.rt - up.rt) < (ps ? 2.f : 10.f))) {
+        return false;
+    }
+    // the two points whose directions are compared: the hits, one of them shifted
+    float ax = lo.x, ay = lo.y, ar = lo.rt, bx = up.x, by = up.y, br = up.rt;
+    const bool shift = !barrel || lm.side != kCenter;
+    if (shift) {
+        float xn, yn;
+        shift_finish(sh[0], sh[1], md_upper_anchors(lm) ? lo : up, lm, xn, yn);
+        const float rn = __fsqrt_rn(__fmaf_rn(xn, xn, yn * yn));
+        if (barrel ? pixLower : !(ps && !pixLower)) { bx = xn; by = yn; br = rn; }
+        else { ax = xn; ay = yn; ar = rn; }
+    }
+    const float dx = bx - ax, dy = by - ay;
+    const float num = fabsf(__fmaf_rn(ax, dy, -(ay * dx)));
+    float muls, pv;
+    dphi_layer_terms(lm, muls, pv);
+    const float v = __fmaf_rn(muls, muls, pv * pv);
+    if (barrel) {
+        const float t = shift ? lm.tilt * pixAsin : 0.f;
+        const float cut = __fmaf_rn(pixAsin + __fsqrt_rn(__fmaf_rn(t, t, v)), 1.f + 1e-5f, 1e-5f);
+        if (num > cut * ar * br) return false;
+        // the direction from the point at smaller rt to the other against its own
+        const float n = cut * (shift ? fminf(ar, br) : ar);
+        return !(num * num > n * n * __fmaf_rn(dx, dx, dy * dy));
+    }
+    const float s = __fdividef(num, ar * br);
+    if (!(s <= 0.5f) || __fmaf_rn(ax, bx, ay * by) < 0.f) return true;  // (an angle above 30 degrees: asin(s) <= 1.05 s below)
+    if (ps) dz = (pixLower ? lo.z : up.z) - sh[2];
+    const float adz = fabsf(dz);
+    const float lum = floorf(__fdividef(__fmaf_rn(1.05f, s, 1e-6f) * kDeltaZLum, adz) * (1.f + 1e-5f));
+    const float cut = __fmaf_rn(pixAsin + __fsqrt_rn(__fmaf_rn(lum, lum, v)), 1.f + 1e-5f, 1e-5f);
+    if (s > cut) return false;
+    const float f = __fdividef(adz, fabsf(lo.z)), g = __fdividef(1.f + f, f);
+    return !(s * g > __fmaf_rn(2e-6f, g, cut));
 }
 
 // ------------------------------------------------------------------ segments
