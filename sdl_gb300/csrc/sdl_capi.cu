@@ -458,7 +458,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.in_x = fx; b.in_y = fy; b.in_z = fz; b.in_idx = fi; b.in_det = fd; b.ev_off = eo;
     AL(b.hit_gm, H); AL(b.hit_rank, H); AL(b.hit_perm, H); AL(b.mod_hit, n_gm + 1);
     AL(b.hx, H); AL(b.hy, H); AL(b.hz, H); AL(b.hrt, H); AL(b.hphi, H); AL(b.hr3, H);
-    AL(b.ha1, H); AL(b.htf, H); AL(b.htd, H); AL(b.ha3, H); AL(b.hidx, H); AL(b.hgm, H);
+    AL(b.ha1, H); AL(b.hidx, H); AL(b.hgm, H);
     AL(b.hsx, H); AL(b.hsy, H); AL(b.hsz, H);
     const int nf[kNumStages] = {4, 6, 0, 0, 0};
     for (int s = 0; s < kNumStages; ++s) {
@@ -491,6 +491,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.sgouter, ctx->cap_obj[kSG] * kSgOuter);
     AL(b.sgfeat, ctx->cap_obj[kSG] * kFeatN);
     AL(b.mdpack, ctx->cap_obj[kMD] * kMdPack);
+    AL(b.mdbend, ctx->cap_obj[kMD] * 2);
     AL(b.mdlite, ctx->cap_obj[kMD] * kMdLite);
     AL(b.counters, ctx->n_ev * 110);
     int64_t mx = n_gm;

@@ -111,26 +111,23 @@ __device__ __forceinline__ bool f_sincos_fast(float x, int shift, float& r) {
     ffm::ff v;
     return ffm::sincos_ff(x, shift, v) && ffm::round_unique_rel(v, r);
 }
-// (float)tan((double)x) and (float)(tan((double)x) / (double)x), the hits'
+// (float)tan((double)x) and (float)(tan((double)x) / (double)x), the anchors'
 // tan of their asin angle (0 < x <= asin(0.95)): sine over cosine in
 // float-float (relative error below 2^-41), answered when the rounding is
 // unique; the double evaluation otherwise
 static __device__ __noinline__ float f_tan_over_d(float x) { return (float)(tan((double)x) / (double)x); }
-__device__ __forceinline__ bool f_tan_fast(float x, bool over_x, float& r) {
+__device__ __forceinline__ bool tan_ff(float x, ffm::ff& t) {
     if (!(x > 0x1p-30f && x < 1.5f)) return false;
     ffm::ff s, c;
-    if (!ffm::sincos_ff(x, 0, s) || !ffm::sincos_ff(x, 1, c)) return false;
-    ffm::ff t = ffm::div(s, c);
+    if (!ffm::sincos2_ff(x, s, c)) return false;
+    t = ffm::div(s, c);
+    return true;
+}
+__device__ __forceinline__ bool f_tan_fast(float x, bool over_x, float& r) {
+    ffm::ff t;
+    if (!tan_ff(x, t)) return false;
     if (over_x) t = ffm::div(t, ffm::ff{x, 0.f});
     return ffm::round_unique_rel(t, r);
-}
-static __device__ __noinline__ float f_tan_ff(float x) {
-    float r;
-    return f_tan_fast(x, false, r) ? r : f_tan(x);
-}
-static __device__ __noinline__ float f_tan_over(float x) {
-    float r;
-    return f_tan_fast(x, true, r) ? r : f_tan_over_d(x);
 }
 static __device__ __noinline__ float f_sin(float x) {
     float r;
@@ -230,6 +227,19 @@ static __device__ __noinline__ float g_cos(float x) {
     if (!f_sincos_fast(ax, 1, r)) r = f_cos_d(ax);
     return libm_pick(kLmCos, lw, ax, r);
 }
+// the sine and the cosine of one argument
+static __device__ __noinline__ void g_sincos(float x, float& sn, float& cs) {
+    const float ax = fabsf(x);
+    const LibmWord ls = libm_word(kLmSin, ax), lc = libm_word(kLmCos, ax);
+    ffm::ff s, c;
+    const bool ok = ax > 0x1p-60f && ffm::sincos2_ff(ax, s, c);
+    float r = ax;  // (sin 0 = 0)
+    if (ax != 0.f && !(ok && ffm::round_unique_rel(s, r))) r = f_sin_d(ax);
+    r = libm_pick(kLmSin, ls, ax, r);
+    sn = x < 0.f ? -r : r;
+    if (!(ok && ffm::round_unique_rel(c, r))) r = f_cos_d(ax);
+    cs = libm_pick(kLmCos, lc, ax, r);
+}
 static __device__ __noinline__ float g_tan(float x) {
     const float ax = fabsf(x);
     const LibmWord lw = libm_word(kLmTan, ax);
@@ -238,7 +248,16 @@ static __device__ __noinline__ float g_tan(float x) {
     r = libm_pick(kLmTan, lw, ax, r);
     return x < 0.f ? -r : r;
 }
-
+// g_tan(x) and (float)(tan((double)x) / (double)x) of x >= 0
+static __device__ __noinline__ void g_tan_both(float x, float& t, float& over) {
+    const LibmWord lw = libm_word(kLmTan, x);
+    ffm::ff q;
+    const bool ok = tan_ff(x, q);
+    float r;
+    if (!(ok && ffm::round_unique_rel(q, r))) r = f_tan(x);
+    t = libm_pick(kLmTan, lw, x, r);
+    if (!(ok && ffm::round_unique_rel(ffm::div(q, ffm::ff{x, 0.f}), over))) over = f_tan_over_d(x);
+}
 
 // (float)sqrt((double)a*a + (double)b*b)
 static __device__ __noinline__ float hypot_d(float a, float b) {
@@ -512,7 +531,9 @@ __device__ __forceinline__ void shift_anchor(const P3& pix, const ModDev& lm, fl
     float sep = lm.gap;
     if (ps && !pixLower) sep *= -1;
     const float sAB = g_sin(angleA + angleB);
-    const float drprime = (sep / sAB) * g_sin(angleA);
+    float sA, cA;
+    g_sincos(angleA, sA, cA);
+    const float drprime = (sep / sAB) * sA;
     // angleM: |atan(slope)| (pi / 2 for the "infinite" slope), pi - it, pi +
     // it, 2 pi - it by quadrant; its sine and cosine come with the module
     const float xp = pix.x, yp = pix.y;
@@ -521,7 +542,7 @@ __device__ __forceinline__ void shift_anchor(const P3& pix, const ModDev& lm, fl
     const float dy = drprime * lm.sh_cos[q];
     xa = xp + dx;
     ya = yp + dy;
-    const float absdzprime = fabsf(sep / sAB * g_cos(angleA));
+    const float absdzprime = fabsf(sep / sAB * cA);
     float abszn;
     // one double operation on two floats rounded to float: the float operation
     if (pixLower) abszn = fabsf(pix.z) + absdzprime;

@@ -199,20 +199,15 @@ __device__ __forceinline__ ff cos_small_ff(float x) {
     return add(mul(x2, h), 1.f);
 }
 
-// sin(x) (cosine: shift = 1) for |x| <= 8: x = r + k pi/2 with pi/2 split in
-// three parts (the first two with at most 20 significant bits, so k times
-// them is exact; the split is 2e-21 off), then the series on |r| <= pi/4.
-// Relative error below 2^-42; false when |r| < 2^-16 after a reduction
-// (a result near a zero of the function).
-static __device__ __noinline__ bool sincos_ff(float x, int shift, ff& out) {
+// sin(r) and cos(r) of x = r + k pi/2 for |x| <= 8, pi/2 split in three parts
+// (the first two with at most 20 significant bits, so k times them is exact;
+// the split is 2e-21 off), by the series on |r| <= pi/4.  Relative error below
+// 2^-42; false when |r| < 2^-16 after a reduction (a result near a zero of
+// the function).
+__device__ __forceinline__ bool sincos_reduced(float x, ff& s, ff& c, int& k) {
     if (!(fabsf(x) <= 8.f)) return false;
-    const int k = __float2int_rn(__fmul_rn(x, 0x1.45f306p-1f));
-    ff s, c;
+    k = __float2int_rn(__fmul_rn(x, 0x1.45f306p-1f));
     if (k == 0) {
-        if (shift == 0) {
-            out = sin_small_ff(x);
-            return true;
-        }
         s = sin_small_ff(x);
         c = cos_small_ff(x);
     } else {
@@ -225,12 +220,35 @@ static __device__ __noinline__ bool sincos_ff(float x, int shift, ff& out) {
         s = add(s0, __fmul_rn(c0.hi, r.lo));  // sin(hi + lo) = sin hi + lo cos hi + O(lo^2)
         c = add(c0, -__fmul_rn(s0.hi, r.lo));
     }
-    switch ((k + shift) & 3) {
-        case 0: out = s; break;
-        case 1: out = c; break;
-        case 2: out = neg(s); break;
-        default: out = neg(c);
+    return true;
+}
+__device__ __forceinline__ ff quadrant(ff s, ff c, int k) {
+    switch (k & 3) {
+        case 0: return s;
+        case 1: return c;
+        case 2: return neg(s);
+        default: return neg(c);
     }
+}
+// sin(x) (cosine: shift = 1), with sincos_reduced's range and error
+static __device__ __noinline__ bool sincos_ff(float x, int shift, ff& out) {
+    if (shift == 0 && fabsf(x) <= 0.78f) {  // no reduction: the sine's series alone
+        out = sin_small_ff(x);
+        return true;
+    }
+    ff s, c;
+    int k;
+    if (!sincos_reduced(x, s, c, k)) return false;
+    out = quadrant(s, c, k + shift);
+    return true;
+}
+// both at once
+static __device__ __noinline__ bool sincos2_ff(float x, ff& sn, ff& cs) {
+    ff s, c;
+    int k;
+    if (!sincos_reduced(x, s, c, k)) return false;
+    sn = quadrant(s, c, k);
+    cs = quadrant(s, c, k + 1);
     return true;
 }
 

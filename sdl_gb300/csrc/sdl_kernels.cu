@@ -345,8 +345,17 @@ __global__ void k_hit_perm(BatchDev b) {
     }
 }
 
-// the sorted hit arrays, one thread per sorted position (coalesced writes;
-// the input hit is gathered through hit_perm)
+// asin(min(rt * k, .95)) of a hit
+__device__ __forceinline__ float rt_asin(float rt) { return g_asin(fmin_ref(rt * k2Rinv1GeVf / kPtCut, kSinAlphaMax)); }
+
+// The sorted hit arrays, one thread per sorted position (coalesced writes;
+// the input hit is gathered through hit_perm) and part (blockIdx.y): the hit,
+// its direction and, where its pair's dPhiThreshold reads it, its asin term;
+// and the strip shift of the hits that anchor their pair.  Bound by the
+// instructions of the float-float functions (64 events: 588 us with every
+// function for every hit in one thread, a third of it stalled on instruction
+// fetches; 339 in two parts, with the segments' terms left to k_md_pack;
+// 391 with the asin in a part of its own, which gathers each hit once more).
 __global__ void k_hit_scatter(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = min(AT(b.mod_hit, b.n_gm, NG1(b)), *b.n_hit);  // hits in known modules
@@ -354,26 +363,27 @@ __global__ void k_hit_scatter(BatchDev b) {
         const int64_t h = AT(b.hit_perm, pos, H(b));
         const int gm = AT(b.hit_gm, h, H(b));
         const float x = AT(b.in_x, h, H(b)), y = AT(b.in_y, h, H(b)), z = AT(b.in_z, h, H(b));
-        const P3 p = mk(x, y, z);
-        AT(b.hx, pos, H(b)) = x; AT(b.hy, pos, H(b)) = y; AT(b.hz, pos, H(b)) = z;
-        AT(b.hrt, pos, H(b)) = p.rt; AT(b.hphi, pos, H(b)) = p.phi; AT(b.hr3, pos, H(b)) = p.r3;
-        const float a1 = g_asin(fmin_ref(p.rt * k2Rinv1GeVf / kPtCut, kSinAlphaMax));
-        AT(b.ha1, pos, H(b)) = a1;
-        AT(b.htf, pos, H(b)) = g_tan(a1);
-        AT(b.htd, pos, H(b)) = f_tan_over(a1);
-        AT(b.ha3, pos, H(b)) = g_asin(fmin_ref(p.rt * k2Rinv1GeVf / 3.0f, kSinAlphaMax));
-        AT(b.hidx, pos, H(b)) = AT(b.in_idx, h, H(b));
-        AT(b.hgm, pos, H(b)) = gm;
-        // the strip shift of the mini-doublets this hit anchors
         const int m = mod_of(b, gm);
         const ModDev& M = MOD(b, m);
         const int lmi = M.lower ? m : M.partner;
-        float xa = 0.f, ya = 0.f, zn = 0.f;
-        if (lmi >= 0) {
-            const ModDev& lm = MOD(b, lmi);
-            if (md_shifts(lm) && (md_upper_anchors(lm) != (bool)M.lower)) shift_anchor(p, lm, xa, ya, zn);
+        const bool pair = lmi >= 0;
+        const ModDev& lm = MOD(b, pair ? lmi : m);
+        const bool lower = (bool)M.lower;
+        if (blockIdx.y == 0) {
+            const P3 p = mk(x, y, z);
+            AT(b.hx, pos, H(b)) = x; AT(b.hy, pos, H(b)) = y; AT(b.hz, pos, H(b)) = z;
+            AT(b.hrt, pos, H(b)) = p.rt; AT(b.hphi, pos, H(b)) = p.phi; AT(b.hr3, pos, H(b)) = p.r3;
+            AT(b.hidx, pos, H(b)) = AT(b.in_idx, h, H(b));
+            AT(b.hgm, pos, H(b)) = gm;
+            AT(b.ha1, pos, H(b)) = pair && (lm.ltype == kPixel) == lower ? rt_asin(p.rt) : 0.f;
+        } else {
+            P3 p;
+            p.x = x; p.y = y; p.z = z;
+            p.rt = __fsqrt_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)));
+            float xa = 0.f, ya = 0.f, zn = 0.f;
+            if (pair && md_shifts(lm) && md_upper_anchors(lm) != lower) shift_anchor(p, lm, xa, ya, zn);
+            AT(b.hsx, pos, H(b)) = xa; AT(b.hsy, pos, H(b)) = ya; AT(b.hsz, pos, H(b)) = zn;
         }
-        AT(b.hsx, pos, H(b)) = xa; AT(b.hsy, pos, H(b)) = ya; AT(b.hsz, pos, H(b)) = zn;
     }
 }
 
@@ -479,36 +489,49 @@ __device__ __forceinline__ MDLite md_lite(const BatchDev& b, int64_t a) {
     const float4 r0 = __ldg(q), r1 = __ldg(q + 1);
     return MDLite{r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, __float_as_uint(r1.w) & kMdFlags};
 }
-__global__ void k_md_pack(BatchDev b) {
+// One thread per mini-doublet and part (blockIdx.y): the records with the
+// anchor's bend terms; the endcap strip edges' phi and the third-layer asin.
+__global__ void __launch_bounds__(256, 4) k_md_pack(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = n_objects(b, kMD);
+    const int part = blockIdx.y;
     for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += (int64_t)gridDim.x * blockDim.x) {
         const int lm = mod_of(b, OG(b, kMD, a));
         const ModDev& M = MOD(b, lm);
         const int anc = md_anchor(M, OI(b, kMD, a), OJ(b, kMD, a));
-        const P3 p = hit(b, anc);
-        const float a1 = AT(b.ha1, anc, H(b));
-        float4* q = reinterpret_cast<float4*>(&AT(b.mdpack, a * kMdPack, b.obj[kMD].cap * kMdPack));
-        q[0] = make_float4(p.x, p.y, p.z, p.rt);
-        q[1] = make_float4(p.phi, p.r3, a1, AT(b.htf, anc, H(b)));
-        q[2] = make_float4(OF(b, kMD, 0, a), OF(b, kMD, 1, a), OF(b, kMD, 2, a), OF(b, kMD, 3, a));
-        // what the segment algorithms compute from this mini-doublet alone as
-        // the outer one: the barrel cut for the layer below, the endcap strip
-        // edges' phi
-        const int am = mod_of(b, AT(b.hgm, anc, H(b)));
-        float c0 = 0.f, c1 = 0.f;
-        if (M.subdet == kBarrel) {
-            if (M.layer >= 2) c0 = sg_barrel_cut(M.layer - 1, p.rt, a1);
-        } else if (M.type == kTwoS) {
-            c0 = strip_edge(p, MOD(b, am), true).phi;
-            c1 = strip_edge(p, MOD(b, am), false).phi;
-        } else {
-            c0 = c1 = p.phi;
-        }
-        q[3] = make_float4(__int_as_float(lm), __int_as_float(am), c0, c1);
-        // the first pass's record (sg_first_cuts, sg_later_cuts)
         const bool barrel = M.subdet == kBarrel;
-        const float tf = AT(b.htf, anc, H(b));
+        float4* q = reinterpret_cast<float4*>(&AT(b.mdpack, a * kMdPack, b.obj[kMD].cap * kMdPack));
+        float* bend = &AT(b.mdbend, 2 * a, 2 * b.obj[kMD].cap);
+        const P3 p = hit(b, anc);
+        if (part == 1) {
+            bend[1] = g_asin(fmin_ref(p.rt * k2Rinv1GeVf / 3.0f, kSinAlphaMax));
+            // what the segment algorithms compute from this mini-doublet alone
+            // as the outer one: the endcap strip edges' phi
+            if (barrel) continue;
+            float c0 = p.phi, c1 = p.phi;
+            if (M.type == kTwoS) {
+                const ModDev& A = MOD(b, mod_of(b, AT(b.hgm, anc, H(b))));
+                c0 = strip_edge(p, A, true).phi;
+                c1 = strip_edge(p, A, false).phi;
+            }
+            reinterpret_cast<float2*>(q + 3)[1] = make_float2(c0, c1);
+            continue;
+        }
+        // (the anchor that is not the pair's pixel side has no asin term yet)
+        const float a1 = md_upper_anchors(M) || M.ltype == kPixel ? AT(b.ha1, anc, H(b)) : rt_asin(p.rt);
+        float tf;
+        g_tan_both(a1, tf, bend[0]);
+        q[0] = make_float4(p.x, p.y, p.z, p.rt);
+        q[1] = make_float4(p.phi, p.r3, a1, tf);
+        q[2] = make_float4(OF(b, kMD, 0, a), OF(b, kMD, 1, a), OF(b, kMD, 2, a), OF(b, kMD, 3, a));
+        reinterpret_cast<float2*>(q + 3)[0] = make_float2(__int_as_float(lm), __int_as_float(mod_of(b, AT(b.hgm, anc, H(b)))));
+        // and the barrel cut for the layer below
+        float c0 = 0.f;
+        if (barrel) {
+            if (M.layer >= 2) c0 = sg_barrel_cut(M.layer - 1, p.rt, a1);
+            reinterpret_cast<float2*>(q + 3)[1] = make_float2(c0, 0.f);
+        }
+        // the first pass's record (sg_first_cuts, sg_later_cuts)
         float4* l = reinterpret_cast<float4*>(&AT(b.mdlite, a * kMdLite, b.obj[kMD].cap * kMdLite));
         l[0] = make_float4(p.rt, p.z, p.phi, barrel ? c0 : a1);
         const float lum = barrel ? (M.side != kCenter ? M.tilt : 0.f)
@@ -954,13 +977,11 @@ __global__ void __launch_bounds__(kEnumThreads) k_enum(BatchDev b) {
 // with the segment algorithm's six values f6 (dPhi, dPhiMin, dPhiMax,
 // dPhiChange, dPhiMinChange, dPhiMaxChange)
 __device__ __forceinline__ void sg_pack_record(const BatchDev& b, int im, int om, const float* f6, float* v) {
-    const ModDev& ilm = MOD(b, mod_of(b, OG(b, kMD, im)));
-    const ModDev& olm = MOD(b, mod_of(b, OG(b, kMD, om)));
-    const int la = md_anchor(ilm, OI(b, kMD, im), OJ(b, kMD, im));
-    const int ua = md_anchor(olm, OI(b, kMD, om), OJ(b, kMD, om));
-    const P3 lo = hit(b, la), up = hit(b, ua);
-    const ModDev& lam = MOD(b, mod_of(b, AT(b.hgm, la, H(b))));
-    const ModDev& uam = MOD(b, mod_of(b, AT(b.hgm, ua, H(b))));
+    const MDRec I = md_rec(b, im), O = md_rec(b, om);
+    const float2 bend = __ldg(reinterpret_cast<const float2*>(&AT(b.mdbend, 2 * (int64_t)im, 2 * b.obj[kMD].cap)));
+    const P3 lo = I.v.a, up = O.v.a;
+    const ModDev& lam = MOD(b, I.anc_mod);
+    const ModDev& uam = MOD(b, O.anc_mod);
     uint32_t fl = 0;
     fl |= lam.subdet == kBarrel ? F_LO_B : 0u;
     fl |= lam.subdet == kEndcap ? F_LO_E : 0u;
@@ -970,8 +991,8 @@ __device__ __forceinline__ void sg_pack_record(const BatchDev& b, int im, int om
     fl |= uam.type == kPS ? F_UP_PS : 0u;
     fl |= uam.type == kTwoS ? F_UP_2S : 0u;
     v[PK_LX] = lo.x; v[PK_LY] = lo.y; v[PK_LZ] = lo.z; v[PK_LRT] = lo.rt;
-    v[PK_LPHI] = lo.phi; v[PK_LR3] = lo.r3; v[PK_LA1] = AT(b.ha1, la, H(b)); v[PK_LTD] = AT(b.htd, la, H(b));
-    v[PK_LA3] = AT(b.ha3, la, H(b));
+    v[PK_LPHI] = lo.phi; v[PK_LR3] = lo.r3; v[PK_LA1] = I.a1; v[PK_LTD] = bend.x;
+    v[PK_LA3] = bend.y;
     v[PK_LR3Z] = __fsqrt_rn(lo.z * lo.z + lo.rt * lo.rt);
     v[PK_UX] = up.x; v[PK_UY] = up.y; v[PK_UZ] = up.z; v[PK_URT] = up.rt; v[PK_UPHI] = up.phi; v[PK_UR3] = up.r3;
     v[PK_DPC] = f6[3]; v[PK_DPMIN] = f6[1]; v[PK_DPMAX] = f6[2];
@@ -1031,7 +1052,7 @@ __device__ __forceinline__ void sg_pack_write(const BatchDev& b, int64_t s, int 
     fd[2] = make_float4(v[PK_UX], v[PK_UY], uz, urt);
     fd[3] = make_float4(v[PK_UPHI], v[PK_ALPHAUP], tcode, 0.f);
 }
-__global__ void k_sg_pack(BatchDev b) {
+__global__ void __launch_bounds__(256, 4) k_sg_pack(BatchDev b) {
     if (halted(b)) return;
     const int64_t n = n_objects(b, kSG);
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
@@ -3063,7 +3084,7 @@ void launch_ingest(const BatchDev& b, cudaStream_t s, Hooks* h) {
     k_hit_map<<<g, 256, 0, s>>>(take(b, h));
     scan<ScanHits>(b, kScanHit, b.n_gm, s, h);
     k_hit_perm<<<g, 256, 0, s>>>(take(b, h));
-    k_hit_scatter<<<g, 256, 0, s>>>(take(b, h));
+    k_hit_scatter<<<dim3(g, 2), 256, 0, s>>>(take(b, h));
 }
 
 void launch_md(const BatchDev& b, cudaStream_t s, Hooks* h) {
@@ -3076,7 +3097,7 @@ void launch_md(const BatchDev& b, cudaStream_t s, Hooks* h) {
 }
 
 void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    k_md_pack<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
+    k_md_pack<<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
     const bool layers = (b.flags & kFlagSGLayers) != 0;
     if (layers) {
         k_layer_runs<<<grid_for((int64_t)b.n_ev * kNumSlots, 64, b.n_sm), 64, 0, s>>>(take(b, h));

@@ -29,7 +29,7 @@ struct BatchDev {
     int32_t* hit_perm;       // sorted position -> input hit
     int64_t* mod_hit;        // n_gm + 1: counts -> offsets
     // sorted hits (SoA)
-    float *hx, *hy, *hz, *hrt, *hphi, *hr3, *ha1, *htf, *htd, *ha3;
+    float *hx, *hy, *hz, *hrt, *hphi, *hr3, *ha1;
     float *hsx, *hsy, *hsz;  // the strip-shift anchor point of an anchoring hit (shift_anchor)
     int32_t *hidx, *hgm;
     // stages
@@ -49,6 +49,7 @@ struct BatchDev {
                                    //   urt - lrt: load_sgo_beta)
     float* sgfeat;                 // segment cap * kFeatN: the pre-filter's per-segment feature records
     float* mdpack;                 // mini-doublet cap * kMdPack: packed records for the segment stage
+    float* mdbend;                 // mini-doublet cap * 2: tan over the asin angle, and the third-layer asin, of the anchor
     float* mdlite;                 // mini-doublet cap * kMdLite: what its first pass reads
     uint32_t* counters;            // n_ev * 110
     uint32_t* status;

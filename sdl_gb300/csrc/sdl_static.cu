@@ -43,7 +43,7 @@ constexpr int64_t kModCnt = kCandMD + kMaxModules + 1;          // kMaxModules +
 constexpr int64_t kSpare = kModCnt + kMaxModules + 1;           // 32 (free)
 constexpr int64_t kWords64 = (kSpare + 32 + 31) / 32 * 32;  // 256-byte multiple: the 4-byte regions start aligned
 // 4-byte regions follow the 8-byte ones
-constexpr int64_t kHitArrays = 18;                              // hit_gm, hit_rank, hit_perm and 15 sorted arrays
+constexpr int64_t kHitArrays = 18;                              // hit_gm, hit_rank, hit_perm, 12 sorted arrays, 3 (free)
 constexpr int64_t kObjWords = 3 + 4;                            // i, j, g, f[4]
 constexpr int64_t kRecWords = 4 + 4;                            // i, j, g, rank, f[4]
 constexpr int64_t kWords32Raw = kHitArrays * kMaxHits + (kObjWords + kRecWords) * kMaxMD + 110 + 1;
@@ -159,7 +159,7 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.hit_gm = w32 + o; o += H;
     b.hit_rank = w32 + o; o += H;
     b.hit_perm = w32 + o; o += H;
-    float** hf[13] = {&b.hx, &b.hy, &b.hz, &b.hrt, &b.hphi, &b.hr3, &b.ha1, &b.htf, &b.htd, &b.ha3, &b.hsx, &b.hsy, &b.hsz};
+    float** hf[10] = {&b.hx, &b.hy, &b.hz, &b.hrt, &b.hphi, &b.hr3, &b.ha1, &b.hsx, &b.hsy, &b.hsz};
     for (float** f : hf) { *f = f32 + o; o += H; }
     b.hidx = w32 + o; o += H;
     b.hgm = w32 + o; o += H;
