@@ -1298,17 +1298,18 @@ constexpr float kB1Margin = 1e-4f;
 
 enum : uint32_t {  // TLRow.fl
     R_BBBB = 1u, R_BBEE = 2u, R_EEEE = 4u,  // the algorithms the inner segment can take
-    R_IN_PS = 8u, R_UP_PS = 16u, R_DZ_POS = 32u, R_DZ_NEG = 64u,
+    R_IN_PS = 8u, R_UP_PS = 16u,
 };
 struct __align__(16) TLRow {
     float rt, z, inv_rt, uphi;        // inner anchor, 1 / rt; outer anchor's phi
     float zp, sq, c3, inv_seg;        // z pitch; 0.18 sqrt(lr3z / lrt); cosh^2 / 3; 1 / (urt - lrt)
-    float dzdr, lx, ly, rtk;          // -rtseg k / ptCut
-    float cosd, sind, cose, sine;     // of dPhiChange and of 0.02 / sdIn_d (NaN: phase B1 undecided)
-    float inv_a, inv_b, drt, dz;      // 1 / (z + dLum), 1 / (z - dLum); urt - lrt, uz - lz
-    float cosh;
+    float dzdr, hi, lo, zhi;          // dz / drt; 1 where BBBB's upper (lower) window scales with dzDrtScale; z + 15
+    float zlo, mz, mw, mq;            // z - 15; the BBBB windows' margins: kWindowMargin (|z| + 15), their constant parts
+    float lx, ly, rtk, cosd;          // -rtseg k / ptCut; cos and sin of dPhiChange
+    float sind, cose, sine;           //   and of 0.02 / sdIn_d (NaN: phase B1 undecided)
     uint32_t fl;
-    float pad[2];
+    float inv_a, inv_b, drt, dz;      // 1 / (z + dLum), 1 / (z - dLum); urt - lrt, uz - lz
+    float cosh, pad[3];
 };
 __device__ __forceinline__ TLRow tl_row(const SGV& S) {
     TLRow R;
@@ -1332,9 +1333,16 @@ __device__ __forceinline__ TLRow tl_row(const SGV& S) {
     R.cosh = S.cosh;
     const bool b1 = S.flags & F_LO_B, b2 = S.flags & F_UP_B, e1 = S.flags & F_LO_E, e2 = S.flags & F_UP_E;
     R.fl = (b1 && b2 ? R_BBBB : 0u) | (b1 && (b2 || e2) ? R_BBEE : 0u) | (e1 && e2 ? R_EEEE : 0u) |
-           ((S.flags & F_LO_PS) ? R_IN_PS : 0u) | ((S.flags & F_UP_PS) ? R_UP_PS : 0u) | (R.dz > 0.f ? R_DZ_POS : 0u) |
-           (R.dz < 0.f ? R_DZ_NEG : 0u);
-    R.pad[0] = R.pad[1] = 0.f;
+           ((S.flags & F_LO_PS) ? R_IN_PS : 0u) | ((S.flags & F_UP_PS) ? R_UP_PS : 0u);
+    R.hi = S.lz < 0.f ? 0.f : 1.f;
+    R.lo = S.lz > 0.f ? 0.f : 1.f;
+    R.zhi = S.lz + kDeltaZLum;
+    R.zlo = S.lz - kDeltaZLum;
+    // (the outer segment's z pitch is at most the strips')
+    const float zp = R.zp + kStrip2SZpitch;
+    R.mz = kWindowMargin * (fabsf(S.lz) + kDeltaZLum);
+    R.mw = kWindowMargin * (fabsf(S.lz) + zp);
+    R.mq = kQuickMargin * (fabsf(S.lz) + 2.f * zp);
     return R;
 }
 // the outer segment's part
@@ -1356,114 +1364,112 @@ __device__ __forceinline__ TLOut tl_out(const SGOuter& T) {
 // outside the exact function's fast range)
 __device__ __forceinline__ float sdl_muls_quick(float d, float sq) {
     const float u = __fmaf_rn(d, 0.004f, 0.1f);
-    return d >= 0.f && d < 1e4f ? __fmul_rn(__fmul_rn(u, rsqrtf(u)), sq) : __int_as_float(0x7fc00000);
+    // 0 <= d < 1e4 in one comparison (a sign bit or a NaN is above)
+    return __float_as_uint(d) < 0x461c4000u ? __fmul_rn(__fmul_rn(u, rsqrtf(u)), sq) : __int_as_float(0x7fc00000);
 }
-// |dphi| <= la1 + sqrt(sdlMuls^2 + pvoff^2): 1 holds, 0 fails, -1 not
-// decided.  cut: the approximate width (within 25 * 2^-24 * (|la1| + r) of
-// the exact one, below 3e-6 where it is set), NaN where |la1| + r >= 2.
-// |dphi| past the wrap is 2 pi - |difference|, within 5e-7.
-__device__ __forceinline__ int phi_cut_quick(float d, float la1, float sdlMuls, float pv2, float& cut) {
+// The verdict of several cuts, each a distance d by which a quantity is inside
+// its cut (a bound within m of the exact one): rejected when one fails by more
+// than m, sure when all hold by m.  A NaN is neither.
+struct CutsQuick {
+    bool rej = false, sure = true;
+    __device__ __forceinline__ void within(float d, float m) {
+        rej = rej || d < -m;
+        sure = sure && d >= m;
+    }
+    __device__ __forceinline__ int algo(int a) const { return rej ? kAlgoNone : sure ? a : kAlgoUnsure; }
+};
+__device__ __forceinline__ float min_nan(float a, float b) {  // NaN when either is
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// how far v lies inside [lo, hi]
+__device__ __forceinline__ float inside(float v, float lo, float hi) { return min_nan(v - lo, hi - v); }
+// |dphi| <= la1 + sqrt(sdlMuls^2 + pvoff^2).  cut: the approximate width
+// (within 25 * 2^-24 * (la1 + r) of the exact one, below 3e-6 where it is set;
+// la1, an arcsine, is not negative), NaN where it is 2 or more.  |dphi| past
+// the wrap is 2 pi - |difference|, within 5e-7.
+__device__ __forceinline__ void phi_cut_quick(CutsQuick& q, float d, float la1, float sdlMuls, float pv2, float& cut) {
     const float adphi = fminf(fabsf(d), 6.28318531f - fabsf(d));
     const float y = __fmaf_rn(sdlMuls, sdlMuls, pv2);
-    const float r = __fmul_rn(y, rsqrtf(y));
-    const float c = la1 + r, a = fabsf(la1) + r;
-    const float m = __fmaf_rn(kQuickMargin, a, 1e-6f);
-    cut = a < 2.f ? c : __int_as_float(0x7fc00000);
-    if (adphi > c + m) return 0;
-    if (adphi < c - m) return 1;
-    return -1;
-}
-// lo <= v <= hi with both bounds within m of their exact values
-__device__ __forceinline__ int window_quick(float v, float lo, float hi, float m) {
-    if (v < lo - m || v > hi + m) return 0;
-    if (v >= lo + m && v <= hi - m) return 1;
-    return -1;
+    const float c = __fmaf_rn(y, rsqrtf(y), la1);
+    cut = c < 2.f ? c : __int_as_float(0x7fc00000);
+    q.within(c - adphi, __fmaf_rn(kQuickMargin, c, 1e-6f));
 }
 
+// kEarly: return at the first window's rejection (layer pairs, where it is the
+// common case for a whole warp; in the module-pair tiles nine of ten
+// candidates pass it and the branches cost more: 10.3 -> 9.5 ms for 128 dense
+// events without them)
+template <bool kEarly>
 __device__ __forceinline__ int tl_phaseA_quick(const TLRow& R, const TLOut& T, float& cut) {
     cut = __int_as_float(0x7fc00000);
     const uint32_t al = R.fl & T.fl;
     const float d = T.rt - R.rt, zp = R.zp + T.zp;
+    CutsQuick q;
     if (al & R_BBBB) {
         // cut 1: zIn + (zIn +- 15)(rtOut / rtIn - 1)(1 or dzDrtScale) +- the pitches
+        const float lt1 = T.ltd - 1.f, sMax = fmaxf(1.f, fabsf(T.ltd));
+        const float sHi = __fmaf_rn(R.hi, lt1, 1.f), sLo = __fmaf_rn(R.lo, lt1, 1.f);
         const float t = __fmaf_rn(T.rt, R.inv_rt, -1.f);
-        const float sHi = R.z < 0.f ? 1.f : T.ltd, sLo = R.z > 0.f ? 1.f : T.ltd;
-        const float hi = __fmaf_rn((R.z + kDeltaZLum) * sHi, t, R.z + zp);
-        const float lo = __fmaf_rn((R.z - kDeltaZLum) * sLo, t, R.z - zp);
-        const float sMax = fmaxf(fabsf(sHi), fabsf(sLo));
-        const float mw = kWindowMargin * __fmaf_rn((fabsf(R.z) + kDeltaZLum) * sMax, fabsf(t) + 2.f, fabsf(R.z) + zp);
-        const int c1 = window_quick(T.z, lo, hi, mw);
-        if (c1 == 0) return kAlgoNone;
+        q.within(inside(T.z, __fmaf_rn(R.zlo * sLo, t, R.z - zp), __fmaf_rn(R.zhi * sHi, t, R.z + zp)),
+                 __fmaf_rn(R.mz * sMax, fabsf(t) + 2.f, R.mw));
+        if (kEarly && q.rej) return kAlgoNone;
         const float sm = sdl_muls_quick(d, R.sq);
-        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
-        if (c3 == 0) return kAlgoNone;
+        phi_cut_quick(q, T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
         // the pointed window
         const float smd = sm * d;
         const float e2 = __fmaf_rn(smd * smd, R.c3, 2.f * zp * zp);
-        const float dzErr = e2 * rsqrtf(e2);
-        const float pw = dzErr * (R.inv_seg * d), zw = pw + zp;
+        const float pw = e2 * rsqrtf(e2) * (R.inv_seg * d), zw = pw + zp;
         const float dzMean = R.dzdr * d;
-        const float plo = __fmaf_rn(dzMean, sLo, R.z - zw), phi = __fmaf_rn(dzMean, sHi, R.z + zw);
-        const float m = kQuickMargin * __fmaf_rn(fabsf(dzMean), fabsf(sLo) + fabsf(sHi), fabsf(R.z) + 2.f * (fabsf(pw) + zp));
-        const int c2 = window_quick(T.z, plo, phi, m);
-        if (c2 == 0) return kAlgoNone;
-        return min(min(c1, c2), c3) > 0 ? kAlgoBBBB : kAlgoUnsure;
+        q.within(inside(T.z, __fmaf_rn(dzMean, sLo, R.z - zw), __fmaf_rn(dzMean, sHi, R.z + zw)),
+                 __fmaf_rn(2.f * kQuickMargin * sMax, fabsf(dzMean), __fmaf_rn(2.f * kQuickMargin, fabsf(pw), R.mq)));
+        return q.algo(kAlgoBBBB);
     }
+    const float dz = T.z - R.z, rdz = R.dz;  // (kZ = dz / rdz is not negative)
     if (al & R_BBEE) {
-        if (!(R.z * T.z > 0)) return kAlgoNone;
         const float dLum = f_copysign(kDeltaZLum, R.z), rtG = T.zp;
         const float zG = f_copysign(zp, R.z);
-        const float dz = T.z - R.z;
         const float q1 = __fdividef(dz - zG, (R.z + zG + dLum) * T.ltd);
         float zh = R.z - zG - dLum;  // (the exact code's float: its sign decides)
         if (zh * R.z < 0) zh = f_copysign(0.1f, R.z);
         const float q2 = __fdividef(dz + zG, zh);
-        const float lo = __fmaf_rn(R.rt, q1, R.rt) - rtG, hi = __fmaf_rn(R.rt, q2, R.rt) + rtG;
         const float za = fabsf(T.z) + fabsf(R.z) + zp;  // (the numerators' magnitudes)
         const float mw = 4.f * kWindowMargin *
                          __fmaf_rn(fabsf(R.rt), 1.f + __fdividef(za, fabsf(zh)) +
                                                     fabsf(__fdividef(za, (R.z + zG + dLum) * T.ltd)), fabsf(T.rt) + rtG);
-        const int c1 = window_quick(T.rt, lo, hi, mw);
-        if (c1 == 0) return kAlgoNone;
-        // kZ = dz / (uz - lz) >= 0
-        const uint32_t dzs = R.fl & (R_DZ_POS | R_DZ_NEG);
-        if ((dz > 0.f && dzs == R_DZ_NEG) || (dz < 0.f && dzs == R_DZ_POS)) return kAlgoNone;
-        const float sm = sdl_muls_quick(d, R.sq);
-        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
-        if (c3 == 0) return kAlgoNone;
-        return min(c1, c3) > 0 && dzs ? kAlgoBBEE : kAlgoUnsure;
+        q.within(inside(T.rt, __fmaf_rn(R.rt, q1, R.rt) - rtG, __fmaf_rn(R.rt, q2, R.rt) + rtG), mw);
+        if (kEarly && q.rej) return kAlgoNone;
+        phi_cut_quick(q, T.uphi - R.uphi, T.la1, sdl_muls_quick(d, R.sq), T.pv2, cut);
+        q.rej = q.rej || !(R.z * T.z > 0) || dz * rdz < 0.f;
+        q.sure = q.sure && dz * rdz > 0.f;
+        return q.algo(kAlgoBBEE);
     }
     if (al & R_EEEE) {
-        if (!(R.z * T.z > 0)) return kAlgoNone;
         const bool inPS = R.fl & R_IN_PS, outPS = T.zp == kPixelPSZpitch;
         const float rtG = (inPS && outPS) ? 2.f * kPixelPSZpitch : (inPS || outPS) ? (kPixelPSZpitch + kStrip2SZpitch) : 2.f * kStrip2SZpitch;
-        const float dz = T.z - R.z;
         const float inv_ltd = __fdividef(1.f, T.ltd);
         const float q1 = dz * R.inv_a * inv_ltd, q2 = dz * R.inv_b;
-        const float lo = __fmaf_rn(R.rt, q1, R.rt) - rtG, hi = __fmaf_rn(R.rt, q2, R.rt) + rtG;
         const float mw = 4.f * kWindowMargin * __fmaf_rn(fabsf(R.rt), 1.f + fabsf(q1) + fabsf(q2), fabsf(T.rt) + rtG);
-        const int c1 = window_quick(T.rt, lo, hi, mw);
-        if (c1 == 0) return kAlgoNone;
+        q.within(inside(T.rt, __fmaf_rn(R.rt, q1, R.rt) - rtG, __fmaf_rn(R.rt, q2, R.rt) + rtG), mw);
+        if (kEarly && q.rej) return kAlgoNone;
         const float sm = sdl_muls_quick(d, 0.015f * 3.f / kPtCut * 4.f);
-        const int c3 = phi_cut_quick(T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
-        if (c3 == 0) return kAlgoNone;
-        int c2 = 1;
+        phi_cut_quick(q, T.uphi - R.uphi, T.la1, sm, T.pv2, cut);
+        q.rej = q.rej || !(R.z * T.z > 0);
         if (inPS && (R.fl & R_UP_PS)) {
             const float adz = fabsf(dz);
-            const uint32_t dzs = R.fl & (R_DZ_POS | R_DZ_NEG);
-            if ((dz > 0.f && dzs == R_DZ_NEG) || (dz < 0.f && dzs == R_DZ_POS)) return kAlgoNone;
             const float mult = __fdividef(adz * R.cosh, R.cosh * R.cosh - 1.f);
-            const float q = __fdividef(adz, R.dz), smm = sm * mult;
-            const float e2 = __fmaf_rn(smm * smm, R.c3, kPixelPSZpitch * kPixelPSZpitch * 2.f * q * q);
+            const float p = __fdividef(adz, rdz), smm = sm * mult;
+            const float e2 = __fmaf_rn(smm * smm, R.c3, kPixelPSZpitch * kPixelPSZpitch * 2.f * p * p);
             const float drtErr = e2 * rsqrtf(e2);
-            const float drtMean = R.drt * fabsf(q), w = drtErr + rtG;
+            const float drtMean = R.drt * fabsf(p), w = drtErr + rtG;
             const float mLo = drtMean * inv_ltd;
             const float m = kQuickMargin * (fabsf(R.rt) + fabsf(mLo) + fabsf(drtMean) + 2.f * fabsf(w));
-            c2 = window_quick(T.rt, R.rt + mLo - w, R.rt + drtMean + w, m);
-            if (c2 == 0) return kAlgoNone;
-            if (!dzs) c2 = -1;
+            q.within(inside(T.rt, R.rt + mLo - w, R.rt + drtMean + w), m);
+            q.rej = q.rej || dz * rdz < 0.f;
+            q.sure = q.sure && dz * rdz > 0.f;
         }
-        return min(min(c1, c2), c3) > 0 ? kAlgoEEEE : kAlgoUnsure;
+        return q.algo(kAlgoEEEE);
     }
     return kAlgoNone;
 }
@@ -1475,12 +1481,10 @@ __device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4
     const float c = __fmaf_rn(mx, dy, -(my * dx)), dt = __fmaf_rn(mx, dx, my * dy);
     const float f = __fmaf_rn(fabsf(c), __cosf(cut), -(dt * __sinf(cut)));
     const float mg = kB1Margin * (fabsf(c) + fabsf(dt));
-    if (f > mg) return 0;
-    const int c5 = f < -mg ? 1 : -1;
-    if (c5 < 0 || algo == kAlgoEEEE) return c5;
+    // the betaIn cut decides only where the first does (EEEE has none)
     const float ax = txy.z - R.lx, ay = txy.w - R.ly;
     const float cx = __fmaf_rn(R.lx, ay, -(R.ly * ax)), dp = __fmaf_rn(R.lx, ax, R.ly * ay);
-    const float q = __fmaf_rn(cx, R.cosd, -(dp * R.sind)), p = __fmaf_rn(dp, R.cosd, cx * R.sind);
+    const float q = fabsf(__fmaf_rn(cx, R.cosd, -(dp * R.sind))), p = __fmaf_rn(dp, R.cosd, cx * R.sind);
     const float dr2 = __fmaf_rn(ax, ax, ay * ay);
     const float dr = dr2 * rsqrtf(dr2);
     const float ar = __fmaf_rn(dr, k2Rinv1GeVf / kPtCut, R.rtk);
@@ -1488,9 +1492,10 @@ __device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4
     const float u = __fmaf_rn(-arg, arg, 1.f);
     const float st = __fmaf_rn(u * rsqrtf(u), R.sine, arg * R.cose);
     const float L = R.rt * dr;
-    if (!(arg >= -kSinAlphaMax)) return -1;
-    if (fabsf(q) > L * (st + kB1Margin) || p < -(kB1Margin * L)) return 0;
-    return fabsf(q) < L * (st - kB1Margin) && p > 0.f ? 1 : -1;
+    const bool c5 = f < -mg, e4 = algo == kAlgoEEEE, fast = arg >= -kSinAlphaMax;
+    const bool in = e4 || (fast && q < L * (st - kB1Margin) && p > 0.f);
+    const bool out = !e4 && fast && (q > L * (st + kB1Margin) || p < -(kB1Margin * L));
+    return f > mg || (c5 && out) ? 0 : c5 && in ? 1 : -1;
 }
 
 // Phase B1 decides most candidates from single-precision approximations of

@@ -1132,10 +1132,11 @@ __device__ __forceinline__ int tl_outer_of(const BatchDev& b, int var, int s, in
 // when phase B1 passed already (0: phase B1 is left to k_tl_b1); exact tells
 // whether an exact evaluation was needed.  txy: the outer segment's anchors
 // (load_sgo_xy).  The exact cut values are computed again in phase B1.
+template <bool kEarly>
 __device__ __forceinline__ int tl_ab1_decide(const TLRow& R, const TLOut& T, float4 txy, const float* __restrict__ pack, int s,
                                              int t, int& b1, bool& exact) {
     float cut;
-    int algo = tl_phaseA_quick(R, T, cut);
+    int algo = tl_phaseA_quick<kEarly>(R, T, cut);
     exact = algo == kAlgoUnsure;
     if (exact) algo = tl_phaseA_entry(pack, s, t, cut);
     b1 = 0;
@@ -1234,7 +1235,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
                 (void)IX(tt, b.obj[kSG].cap);
                 const int64_t C = b.obj[kSG].cap;
                 bool exact;
-                algo = tl_ab1_decide(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
+                algo = tl_ab1_decide<true>(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
                                      b.sgpack, s, tt, b1, exact);
             }
             passbuf_add(b, pb, algo, s, tt, b1);
@@ -1369,9 +1370,9 @@ __device__ __forceinline__ int tile_outer(const BatchDev& b, int ev, int m, int 
 // of the single-precision decisions (in shared memory, read there as
 // warp-uniform values), with the lanes' outer-segment fields.  Bound by
 // instruction issue: with the decisions on divisions, atan2 polynomials and
-// asinf over the plain records the 128 dense events took 14.9 ms.
-// CTAs per SM it is compiled for (register budget): 10.6 ms at 4 and 5, 11.2
-// at 3.
+// asinf over the plain records the 128 dense events took 14.9 ms, 9.5 now.
+// CTAs per SM it is compiled for (register budget): 9.5 ms at 4, 10.2 at 3,
+// 10.3 at 5.
 #ifndef SDLG_ENUM_MIN_BLOCKS
 #define SDLG_ENUM_MIN_BLOCKS 4
 #endif
@@ -1425,11 +1426,9 @@ __global__ void __launch_bounds__(kEnumThreads, SDLG_ENUM_MIN_BLOCKS) k_tl_enum_
         __syncwarp();
         for (int r = 0; r < nat; ++r) {
             const int sr = sidx[w][r];
-            int algo = kAlgoNone, b1 = 0;
-            if (has) {
-                bool exact;
-                algo = tl_ab1_decide(srow[w][r], T, sxy[w][lane], b.sgpack, sr, tt, b1, exact);
-            }
+            int b1;
+            bool exact;  // (a lane without an outer segment has no algorithm)
+            const int algo = tl_ab1_decide<false>(srow[w][r], T, sxy[w][lane], b.sgpack, sr, tt, b1, exact);
             passbuf_add(b, pb, algo, sr, tt, b1);
         }
     }
@@ -2125,7 +2124,7 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
         const int64_t C = b.obj[kSG].cap;
         int b1;
         bool exact;
-        const int q = tl_ab1_decide(tl_row(S), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt, b1,
+        const int q = tl_ab1_decide<false>(tl_row(S), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt, b1,
                                     exact);
         float cut, muls;
         const int e = tl_phaseA(S, Tv, cut, muls);
@@ -2669,7 +2668,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tctp_a(BatchDev b) {
                 p2 = join2_obj(b, OJ(b, kSG, s), c - AT(off, s, offlim));
                 tt = OJ(b, kTP, p2);
                 bool exact;
-                algo = tl_ab1_decide(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
+                algo = tl_ab1_decide<true>(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
                                      b.sgpack, s, tt, b1, exact);
             }
             passbuf_put(b, pb, algo != kAlgoNone, make_int4(s, tt, algo | (b1 << 8), p2));
