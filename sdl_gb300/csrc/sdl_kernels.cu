@@ -1837,6 +1837,9 @@ __device__ __forceinline__ void pb_flush(const BatchDev& b, int4* buf, int& n, b
 // tl_b2_quick.  (PU 100-300: 85 % of the entries are dropped; 64 events, 52
 // million entries: the filter 1.64 -> 1.10 ms.  The pre-filter's kept list has
 // two passing entries in three and goes straight to tl_b2_quick.)
+// The first pass is bound by the latency of its loads at 32 warps an SM: the
+// next entry is loaded ahead and the fields of both segments together (64
+// events: 936 -> 842 us).
 template <int kPass, bool kEarly>
 __device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict__ in, const unsigned long long* n_in,
                                        int4 (*fbuf)[kPassBuf], int4 (*dbuf)[2][kPbBuf], int (*tbuf)[3][kRecBuf],
@@ -1905,13 +1908,20 @@ __device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict
         }
     };
     const int64_t warps = (int64_t)gridDim.x * (kEnumThreads / kWarp);
-    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * kWarp; base < n; base += warps * kWarp) {
+    auto entry = [&](int64_t i) {
+        return i >= n ? make_int4(0, 0, 0, 0)
+                      : kPass == 0 ? AT(in, i, b.kept_cap) : AT(b.pb, kPass == 1 ? i : b.kept_cap - 1 - i, b.kept_cap);
+    };
+    const int64_t first = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * kWarp;
+    // (the next entry is on its way while one is judged)
+    int4 next = entry(first + lane);
+    for (int64_t base = first; base < n; base += warps * kWarp) {
         const int64_t i = base + lane;
         int r = 0;
         bool queue = false;
-        int4 e = make_int4(0, 0, 0, 0);
+        const int4 e = next;
+        next = entry(i + warps * kWarp);
         if (i < n) {
-            e = kPass == 0 ? AT(in, i, b.kept_cap) : AT(b.pb, kPass == 1 ? i : b.kept_cap - 1 - i, b.kept_cap);
             (void)IX(e.x, b.obj[kSG].cap);
             (void)IX(e.y, b.obj[kSG].cap);
             if (kEarly) {
@@ -1919,8 +1929,16 @@ __device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict
                 // entries are neighbours there, while the 128-byte records
                 // cost a cache line per lane and load)
                 const int64_t C = b.obj[kSG].cap;
-                if (!b2_early(e.z, sgo_flags(b.sgouter, C, e.y))) r = 2;
-                else queue = !b2_reject_early(load_sgv(b.sgpack, e.x), load_sgo_beta(b.sgouter, C, e.y));
+                r = 2;
+                if (e.z == kAlgoBBBB) {
+                    // (all loads together: the flags decide afterwards)
+                    const uint32_t flags = sgo_flags(b.sgouter, C, e.y);
+                    const bool out = b2_reject_early(load_sgv(b.sgpack, e.x), load_sgo_beta(b.sgouter, C, e.y));
+                    if (b2_early(e.z, flags)) {
+                        r = 0;
+                        queue = !out;
+                    }
+                }
             } else {
                 r = judge(e);
             }
@@ -1956,7 +1974,7 @@ __device__ __forceinline__ void tl_b2f(const BatchDev& b, const int4* __restrict
 }
 // pass 0
 template <bool kEarly>
-__global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4* __restrict__ in, const unsigned long long* n_in) {
+__global__ void __launch_bounds__(kEnumThreads, 4) k_tl_b2f(BatchDev b, const int4* __restrict__ in, const unsigned long long* n_in) {
     __shared__ int4 fbuf[kEnumThreads / kWarp][kPassBuf];
     __shared__ int4 dbuf[kEnumThreads / kWarp][2][kPbBuf];
     __shared__ int tbuf[kEnumThreads / kWarp][3][kRecBuf];
@@ -1966,7 +1984,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_b2f(BatchDev b, const int4*
 }
 // passes 1 and 2; 0: both, by blockIdx.y (launch_pair)
 template <int kPass>
-__global__ void __launch_bounds__(kEnumThreads) k_tl_b2f_rest(BatchDev b) {
+__global__ void __launch_bounds__(kEnumThreads, 4) k_tl_b2f_rest(BatchDev b) {
     __shared__ int4 fbuf[kEnumThreads / kWarp][kPassBuf];
     __shared__ int tbuf[kEnumThreads / kWarp][3][kRecBuf];
     if (halted(b)) return;
