@@ -333,9 +333,10 @@ def run_reference_arm(a, rank, world, pg):
 
 
 def timed_runs(ch, flags, steps, flush):
-    """device ms per run (CUDA events around the chain on its stream), per
-    stage, of the tracklet kernels, and of the tracklet passes (enumeration +
-    float cuts, pre-filter, double-precision cuts)"""
+    """device ms per run (CUDA events around the chain on its stream), and,
+    between the device clock stamps of their kernels, per stage, of the
+    tracklet kernels, and of the tracklet passes (enumeration + float cuts,
+    pre-filter, single-precision filter, exact cuts)"""
     out, stage, tl, pf = [], [], [], []
     for _ in range(steps):
         flush()
@@ -625,7 +626,7 @@ def main():
     # Algorithmic bytes = the tracklet stage's input, 28 B per segment read
     # once (the tracklets, 8 B each, are written by k_tl_b2).  layout_bytes =
     # what this kernel's own data layout reads and writes once: each
-    # segment's record as inner segment (112 B), its eleven outer-role fields
+    # segment's record as inner segment (96 B of it), its eleven outer-role fields
     # (44 B) and its entry in the index of segments by outer module (4 B),
     # each global module's tile offset, segment offset and connection sum
     # (24 B), each surviving candidate's list entry (16 B).  traffic = DRAM
@@ -637,7 +638,7 @@ def main():
     n_sg = int(n_pruned[1])
     n_gm = len(batch) * ch.num_modules
     en_alg = 28 * n_sg
-    en_layout = (112 + 44 + 4) * n_sg + 24 * n_gm + 16 * lists["listed"]
+    en_layout = (96 + 44 + 4) * n_sg + 24 * n_gm + 16 * lists["listed"]
     # k_tl_b2f (phase B2's single-precision filter over the pre-filter's kept
     # list): each entry read once (16 B), each segment's 128-byte record read
     # once, each entry it leaves written once (16 B)

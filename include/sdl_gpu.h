@@ -281,7 +281,9 @@ int sdlg_get_tracklet_vars(sdlg_ctx* ctx, int64_t event, float* out, int64_t cap
  * 5 stages x {candidates, objects} x {barrel layers 1-6, endcap layers 1-5}. */
 int sdlg_get_counters(sdlg_ctx* ctx, int64_t event, uint32_t* out110);
 
-/* Device time of the last run: [0] ingest, [1..5] MD..TC stages, [6] total (ms). */
+/* Device time of the last run: [0] ingest, [1..5] MD..TC stages, [6] total (ms).
+ * The stages lie between device clock stamps that their kernels write at their
+ * start, the total between CUDA events. */
 int sdlg_last_times(sdlg_ctx* ctx, float* out7);
 
 /* Device time of each stage's candidate-evaluation kernel in the last run (ms). */
