@@ -1144,7 +1144,7 @@ __device__ __forceinline__ int tl_outer_nav(const BatchDev& b, int s, int64_t q)
 #ifdef SDL_DEVICE_CHECKS
     IX(-3, 0);
 #endif
-    return 0;  // q is below the candidate count (k_tl_count_nav)
+    return 0;  // q is below the candidate count (ScanTlCand)
 }
 
 // the tracklet variant of a run: 0 module map, 1 layer pairs, 2 navigation
@@ -1992,6 +1992,14 @@ __global__ void __launch_bounds__(kEnumThreads, 4) k_tl_b2f_rest(BatchDev b) {
     else tl_b2f<2, false>(b, nullptr, nullptr, fbuf, nullptr, tbuf, nullptr);
 }
 
+// Entries a warp takes at a time of a list of n: 32, or one where there are four
+// warps for each.  The lanes of a warp part ways in the exact phases, so a short
+// list (what the phase-B2 filter leaves of one event) takes as long as all their
+// ways one after the other: phases B1 and B2 of one PU 200 event 36 us with 32
+// entries a warp, 30 with one.  A longer list spread over all warps only fetches
+// more instructions (64 events: 42 us with 32 entries a warp, 88 spread out).
+__device__ __forceinline__ int entries_per_warp(int64_t n, int64_t nwarp) { return 4 * n <= nwarp ? 1 : kWarp; }
+
 __global__ void __launch_bounds__(kEnumThreads) k_tl_b1(BatchDev b, const int4* __restrict__ list,
                                                          const unsigned long long* count) {
     __shared__ int4 fbuf[kEnumThreads / kWarp][kPbBuf], bbuf[kEnumThreads / kWarp][kPbBuf];
@@ -2000,12 +2008,13 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_b1(BatchDev b, const int4* 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int nfb = 0, nbb = 0;  // entries held in this warp's buffers
     const int64_t nwarp = (int64_t)gridDim.x * (kEnumThreads / 32);
-    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / 32) + w) * kWarp; base < n; base += nwarp * kWarp) {
+    const int per = entries_per_warp(n, nwarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / 32) + w) * per; base < n; base += nwarp * per) {
         const int64_t i = base + lane;
         bool pass = false;
         int4 p = make_int4(0, 0, kAlgoNone, 0);
         float muls = 0.f;
-        if (i < n) {
+        if (lane < per && i < n) {
             p = AT(list, i, b.kept_cap);
             if (p.w) {  // phase B1 passed in the enumeration
                 pass = true;
@@ -2053,11 +2062,12 @@ __device__ __forceinline__ void tl_b2(const BatchDev& b, int (*rbuf)[3][kRecBuf]
     const bool nm1 = (b.flags & kFlagTLNm1) != 0;
     const int64_t nwarp = (int64_t)gridDim.x * (kEnumThreads / 32);
     RecBuf<0> rb{rbuf[w]};
-    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / 32) + w) * kWarp; base < n; base += nwarp * kWarp) {
+    const int per = entries_per_warp(n, nwarp);
+    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / 32) + w) * per; base < n; base += nwarp * per) {
         const int64_t i = base + lane;
         bool pass = false;
         int s = 0, tt = 0;
-        if (i < n) {
+        if (lane < per && i < n) {
             const int64_t k = kSet == kB2BBBB ? i : b.kept_cap - 1 - i;
             const int4 p = AT(b.pb, k, b.kept_cap);
             s = p.x;
