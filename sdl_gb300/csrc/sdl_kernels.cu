@@ -2777,10 +2777,11 @@ __global__ void __launch_bounds__(kEnumThreads) k_tctp_c(BatchDev b) {
     const int64_t n = min((int64_t)*b.n_tc_open, b.kept_cap);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t warps = (int64_t)gridDim.x * (kEnumThreads / kWarp);
-    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * kWarp; base < n; base += warps * kWarp) {
+    const int per = entries_per_warp(n, warps);  // (3 events: 57 -> 25 us)
+    for (int64_t base = ((int64_t)blockIdx.x * (kEnumThreads / kWarp) + w) * per; base < n; base += warps * per) {
         bool pass = false;
         int4 e = make_int4(0, 0, 0, 0);
-        if (base + lane < n) {
+        if (lane < per && base + lane < n) {
             e = AT(b.passf, base + lane, b.kept_cap);
             float cut, muls;
             const int algo = tl_phaseA(load_sgv(b.sgpack, e.x), load_sgv(b.sgpack, e.y), cut, muls);
