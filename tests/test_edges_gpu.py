@@ -82,3 +82,20 @@ def test_around_two_to_the_eighteenth_hits(above, flags, gpu, oracle_lib):
     assert (n * len(ev.x) > 1 << 18) == above
     for e in (0, n // 2, n - 1):
         assert digests(gpu, oracle_lib, e) == want
+
+
+@pytest.mark.parametrize("n", [1, 2, 25, 120, 240])
+def test_copies_of_an_event(n, gpu, oracle_lib):
+    """From a few thousand candidates a stage to millions: candidates judged in place or gathered, exact phases on
+    one entry a warp or 32"""
+    from sdl_gb300 import synth
+    det = synth.detector("full")
+    ev = synth.make_event(det, 982, "full", n_pu=700)
+    gpu.upload_detector(det)
+    ref, cnt, _ = oracle_lib.Oracle(det).run(ev)
+    want = [oracle_lib.digest(ref[s]) for s in range(5)]
+    gpu.set_events([ev] * n)
+    gpu.run(4)
+    for e in {0, n // 2, n - 1}:
+        assert digests(gpu, oracle_lib, e) == want
+        assert np.array_equal(gpu.counters(e), cnt)
