@@ -1012,25 +1012,28 @@ __device__ __forceinline__ SGV sgv_from(const float* p) {
 // betaOut angles the exact cuts test (Tracklet.cc:1205-1260), the rz
 // pointing residual of the outer anchor against the inner segment, a signed
 // 1/pT estimate from the mean beta, and a code of the anchor module types.
-// Every feature is scaled to O(1) and clamped to [-16, 16].  They read one
-// 32-byte record of each segment (k_sg_pack): the inner segment's in its
-// inner role, the outer segment's in its outer role.
+// Every feature is scaled to O(1) and clamped to [-16, 16].  They read two
+// 16-byte words of each segment (k_sg_pack): two of the inner segment's for its
+// inner role, two of the outer segment's for its outer role, each word in an
+// array of its own (cap entries): a tile row's outer segments are neighbours
+// (the pre-filter on 274 million entries of 128 dense events, bound by its passes
+// through L1: 7.5 ms with 64-byte records, 7.2 so).
 __device__ __forceinline__ float wrap_pi_f(float x) { return x - 6.28318531f * rintf(x * 0.159154943f); }
-constexpr int kFeatN = 16;  // floats per segment: inner-role record, outer-role record
+constexpr int kFeatN = 16;  // floats per segment: two words of the inner role, two of the outer role
 struct FeatS {               // a segment as the inner one
     float lx, ly, lz, lrt, lphi, dpc, slope, code;  // lower anchor; dPhiChange; rz slope; module code
 };
 struct FeatT {               // a segment as the outer one
     float ux, uy, uz, urt, uphi, alphaup, code, pad;  // upper anchor; direction angle; module code
 };
-__device__ __forceinline__ FeatS feat_s(const float* __restrict__ f, int64_t s) {
-    const float4* q = reinterpret_cast<const float4*>(f + s * kFeatN);
-    const float4 a = __ldg(q), b = __ldg(q + 1);
+__device__ __forceinline__ FeatS feat_s(const float* __restrict__ f, int64_t cap, int64_t s) {
+    const float4* q = reinterpret_cast<const float4*>(f) + s;
+    const float4 a = __ldg(q), b = __ldg(q + cap);
     return FeatS{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
-__device__ __forceinline__ FeatT feat_t(const float* __restrict__ f, int64_t t) {
-    const float4* q = reinterpret_cast<const float4*>(f + t * kFeatN + 8);
-    const float4 a = __ldg(q), b = __ldg(q + 1);
+__device__ __forceinline__ FeatT feat_t(const float* __restrict__ f, int64_t cap, int64_t t) {
+    const float4* q = reinterpret_cast<const float4*>(f) + 2 * cap + t;
+    const float4 a = __ldg(q), b = __ldg(q + cap);
     return FeatT{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 __device__ __forceinline__ void tl_features(const FeatS& S, const FeatT& T, float* f) {

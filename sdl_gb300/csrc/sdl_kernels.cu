@@ -1088,7 +1088,10 @@ __global__ void __launch_bounds__(256, 4) k_sg_pack(BatchDev b) {
             for (int k = 0; k < PK_N / 4; ++k) rec[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         }
         store_records<PK_N / 4>(reinterpret_cast<float4*>(&AT(b.sgpack, s0 * PK_N, C * PK_N)), tmp[w], rec, m);
-        store_records<kFeatN / 4>(reinterpret_cast<float4*>(&AT(b.sgfeat, s0 * kFeatN, C * kFeatN)), tmp[w], fd, m);
+        if (lane < m) {
+#pragma unroll
+            for (int k = 0; k < kFeatN / 4; ++k) *reinterpret_cast<float4*>(&AT(b.sgfeat, 4 * (k * C + s), C * kFeatN)) = fd[k];
+        }
     }
 }
 
@@ -1697,8 +1700,8 @@ __global__ void __launch_bounds__(kMlpTile, kPfCtasPerSm) k_tl_prefilter(BatchDe
     FeatS rs{};
     FeatT rt{};
     if (valid) {
-        rs = feat_s(b.sgfeat, cur.e.x);
-        rt = feat_t(b.sgfeat, cur.e.y);
+        rs = feat_s(b.sgfeat, b.obj[kSG].cap, cur.e.x);
+        rt = feat_t(b.sgfeat, b.obj[kSG].cap, cur.e.y);
     }
     while (t < ntile) {
         float f[kMlpIn];
@@ -1711,8 +1714,8 @@ __global__ void __launch_bounds__(kMlpTile, kPfCtasPerSm) k_tl_prefilter(BatchDe
         mlp_tile_begin(sm, f, st);
         const bool v2 = entry(t + 2 * G, e2);
         if (v1) {
-            rs = feat_s(b.sgfeat, e1.x);
-            rt = feat_t(b.sgfeat, e1.y);
+            rs = feat_s(b.sgfeat, b.obj[kSG].cap, e1.x);
+            rt = feat_t(b.sgfeat, b.obj[kSG].cap, e1.y);
         }
         pf_flush(b, pend);
         const float z = mlp_tile_end(sm, st);
@@ -2137,7 +2140,7 @@ __global__ void k_tl_collect(BatchDev b, MlpCollect col) {
                 const bool pass = tl_phaseB(algo, b.sgpack, s, tt, cut, muls, false);
                 label = pass ? 1.f : 0.f;
                 keep = pass || hash_unit((unsigned long long)c, col.seed) < col.neg_keep;
-                if (keep) tl_features(feat_s(b.sgfeat, s), feat_t(b.sgfeat, tt), f);
+                if (keep) tl_features(feat_s(b.sgfeat, b.obj[kSG].cap, s), feat_t(b.sgfeat, b.obj[kSG].cap, tt), f);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);

@@ -47,7 +47,7 @@ struct BatchDev {
                                    //   B2 filter read of an outer segment (lrt, lz, ltd, la1, uphi, flags,
                                    //   0.1/lrt: SGOuter; lx, ly, ux, uy: load_sgo_xy; alphaup, rtseg,
                                    //   urt - lrt: load_sgo_beta)
-    float* sgfeat;                 // segment cap * kFeatN: the pre-filter's per-segment feature records
+    float* sgfeat;                 // [kFeatN / 4][segment cap] 16-byte words: what the pre-filter reads of a segment
     float* mdpack;                 // mini-doublet cap * kMdPack: packed records for the segment stage
     float* mdbend;                 // mini-doublet cap * 2: tan over the asin angle, and the third-layer asin, of the anchor
     float* mdlite;                 // mini-doublet cap * kMdLite: what its first pass reads
