@@ -1295,7 +1295,7 @@ constexpr float kWindowMargin = 0x1p-18f;
 // sin and cos of the angle less dPhiChange against sin(th) =
 // arg cos(e) + sqrt(1 - arg^2) sin(e), e = 0.02 / sdIn_d, with the same margin
 // (|e| <= 0.25 and |dPhiChange| < 1.6 keep th below pi / 2 and the angle's
-// wrap out of reach).  Every comparison decided holds by over 9e-5 for the
+// wrap out of reach; without them betaIn is left to the exact code).  Every comparison decided holds by over 9e-5 for the
 // exact code's angles, which are within 2e-6 of the true ones.
 constexpr float kB1Margin = 1e-4f;
 
@@ -1497,7 +1497,8 @@ __device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4
     const float L = R.rt * dr;
     const bool c5 = f < -mg, e4 = algo == kAlgoEEEE, fast = arg >= -kSinAlphaMax;
     const bool in = e4 || (fast && q < L * (st - kB1Margin) && p > 0.f);
-    const bool out = !e4 && fast && (q > L * (st + kB1Margin) || p < -(kB1Margin * L));
+    // (past a right angle fails too, where the threshold is below one: not without e)
+    const bool out = !e4 && fast && (q > L * (st + kB1Margin) || (R.sine == R.sine && p < -(kB1Margin * L)));
     return f > mg || (c5 && out) ? 0 : c5 && in ? 1 : -1;
 }
 
