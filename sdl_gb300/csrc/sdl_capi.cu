@@ -515,7 +515,14 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.eidx, ctx->cap_obj[kSG]);
     AL(b.toff, n_gm + 1);
     AL(b.coff, n_gm + 1);
-    AL(b.layer_runs, ctx->n_ev * kNumSlots * 24);
+    // the runs of an inner slot's outer layers (sg_layer_outer)
+    b.layer_width = kLayerRuns;
+    for (int si = 0; si < kNumSlots; ++si) {
+        int n = 0;
+        for (int k = 0, so; k < 3 && (so = sg_layer_outer(si, k)) >= 0; ++k) n += ctx->slot_run[so + 1] - ctx->slot_run[so];
+        b.layer_width = std::max(b.layer_width, n);
+    }
+    AL(b.layer_runs, ctx->n_ev * kNumSlots * 2 * b.layer_width);
     b.tile_cap = 2 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);
     AL(b.tile_gm, b.tile_cap);
     b.olist_cap = 4 * std::max<int64_t>(ctx->cap_obj[kSG], n_gm);

@@ -579,17 +579,6 @@ __device__ __forceinline__ int sg_outer_md(const BatchDev& b, int a, int64_t q) 
 }
 
 // ------------------------------------------------------------------ layer pairs
-// Layer.cc:32-50: the outer layer slots paired with inner slot si (barrel
-// layers 1-5 -> the next barrel layer and endcap layer 1; endcap 1 -> 2;
-// endcap 2 -> 3, 4, 5; endcap 3 -> 4; endcap 4 -> 5); -1 past the last
-__device__ __forceinline__ int sg_layer_outer(int si, int k) {
-    if (si <= 4) return k == 0 ? si + 1 : (k == 1 ? 6 : -1);
-    if (si == 6) return k == 0 ? 7 : -1;
-    if (si == 7) return k < 3 ? 8 + k : -1;
-    if (si == 8 || si == 9) return k == 0 ? si + 1 : -1;
-    return -1;
-}
-
 // Layer.cc:19-24: tracklet layer pairs are barrel (1,3), (2,4), (3,5)
 __device__ __forceinline__ int tl_layer_outer(int si) { return si <= 2 ? si + 2 : -1; }
 
@@ -621,43 +610,55 @@ __device__ __forceinline__ int layer_object(const BatchDev& b, int st, int ev, i
 
 // Segment candidates by layer pairs (Event.cc:432-443, 793-821): candidate q
 // of an inner MD runs over the MDs of the paired outer layers, in table order.
-// Those are up to kLayerRuns runs of consecutive MDs, the same for all MDs of
-// an event's layer slot: one table row per event and slot (k_layer_runs) holds
-// the runs' first MDs, then their cumulative counts.
-constexpr int kLayerRuns = 12;  // three endcap layers of four sides (the detId's two bits)
-constexpr int kLayerRow = 2 * kLayerRuns;
+// Those are runs of consecutive MDs, the same for all MDs of an event's layer
+// slot: one table row per event and slot (k_layer_runs) holds the runs' first
+// MDs, then their cumulative counts.  A row has room for b.layer_width runs,
+// kLayerRuns where those are enough (three endcap layers of four sides, the
+// detId's two bits), else as many as the module table makes (detIds that
+// differ in bits the decoding ignores).  kWide: rows of any width; the usual
+// one is a constant of the kernel (48 registers and 111 to 120 us for the
+// segment stage's candidates of 5 events with a variable width, 40 and 103 with
+// the constant).
+template <bool kWide>
+__device__ __forceinline__ int layer_width(const BatchDev& b) { return kWide ? b.layer_width : kLayerRuns; }
+template <bool kWide>
 __device__ __forceinline__ const int* layer_row(const BatchDev& b, int a) {
     const int g1 = OG(b, kMD, a);
     const int ev = ev_of(b, g1);
     const int slot = MOD(b, g1 - ev * b.geo.n_mod).layer_slot;
-    return &AT(b.layer_runs, (ev * kNumSlots + slot) * kLayerRow, (int64_t)b.n_ev * kNumSlots * kLayerRow);
+    const int w = 2 * layer_width<kWide>(b);
+    if (kWide) return &AT(b.layer_runs, (int64_t)(ev * kNumSlots + slot) * w, (int64_t)b.n_ev * kNumSlots * w);
+    return &AT(b.layer_runs, (ev * kNumSlots + slot) * w, (int64_t)b.n_ev * kNumSlots * w);
 }
 __global__ void k_layer_runs(BatchDev b) {
     if (halted(b)) return;
+    const int w = b.layer_width;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < b.n_ev * kNumSlots; t += gridDim.x * blockDim.x) {
         const int64_t base = (int64_t)(t / kNumSlots) * b.geo.n_mod;
-        int* row = b.layer_runs + t * kLayerRow;
+        int* row = b.layer_runs + (int64_t)t * 2 * w;
         int n = 0, sum = 0;
         for (int k = 0; k < 3; ++k) {
             const int so = sg_layer_outer(t % kNumSlots, k);
             if (so < 0) break;
-            for (int r = SR(b, so); r < SR(b, so + 1) && n < kLayerRuns; ++r, ++n) {
+            for (int r = SR(b, so); r < SR(b, so + 1); ++r, ++n) {
                 const int o0 = (int)OFF(b, kMD, base + SR(b, kNumSlots + 1 + 2 * r));
                 row[n] = o0;
                 sum += (int)OFF(b, kMD, base + SR(b, kNumSlots + 2 + 2 * r)) - o0;
-                row[kLayerRuns + n] = sum;
+                row[w + n] = sum;
             }
         }
-        for (; n < kLayerRuns; ++n) {
+        for (; n < w; ++n) {
             row[n] = 0;
-            row[kLayerRuns + n] = sum;
+            row[w + n] = sum;
         }
     }
 }
-__device__ __forceinline__ int layer_md(const int* row, int q) {
+template <bool kWide>
+__device__ __forceinline__ int layer_md(const BatchDev& b, const int* row, int q) {
+    const int w = layer_width<kWide>(b);
     int r = 0, before = 0;
-    for (; r < kLayerRuns - 1; ++r) {
-        const int end = row[kLayerRuns + r];
+    for (; r < w - 1; ++r) {
+        const int end = row[w + r];
         if (q < end) break;
         before = end;
     }
@@ -1513,7 +1514,8 @@ __device__ __forceinline__ void sg_list_flush(const BatchDev& b, int4* buf, int&
     n = 0;
 }
 
-template <bool kLayers>
+// kVar: 0 the module map, 1 the layer pairs, 2 the layer pairs with rows of any width
+template <int kVar>
 __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
     __shared__ int4 sbuf[kEnumThreads / kWarp][2][kPbBuf];
     __shared__ int2 mbuf[kEnumThreads / kWarp][2 * kWarp];
@@ -1574,7 +1576,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_sg_enum_a(BatchDev b) {
             if (c < end) {
                 a = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
                 const int64_t q = c - AT(off, a, offlim);
-                bmd = kLayers ? layer_md(layer_row(b, a), (int)q) : sg_outer_md(b, a, q);
+                bmd = kVar ? layer_md<kVar == 2>(b, layer_row<kVar == 2>(b, a), (int)q) : sg_outer_md(b, a, q);
                 (void)IX(bmd, b.obj[kMD].cap);
                 pass = sg_first_cuts(md_lite(b, a), md_lite(b, bmd));
             }
@@ -2450,7 +2452,7 @@ __global__ void k_sg_lists(BatchDev b) {
 // inner-layer MDs x outer-layer MDs); the reference counts none of them
 struct ScanSgLayers : ScanCand<kSG> {
     __device__ static void load(const BatchDev& b, int64_t a, bool in, int64_t* v) {
-        v[0] = in ? layer_row(b, (int)a)[kLayerRow - 1] : 0;
+        v[0] = in ? layer_row<true>(b, (int)a)[2 * b.layer_width - 1] : 0;
     }
 };
 
@@ -3174,7 +3176,7 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     BatchDev l = b;  // with this list's own counts
     l.n_kept = b.n_kept_sg;
     l.n_pb = b.n_pb_sg;
-    auto* enum_a = layers ? k_sg_enum_a<true> : k_sg_enum_a<false>;
+    auto* enum_a = !layers ? k_sg_enum_a<0> : b.layer_width == kLayerRuns ? k_sg_enum_a<1> : k_sg_enum_a<2>;
     enum_a<<<b.n_sm * enum_grid(b, kSG), kEnumThreads, 0, s>>>(take(l, h));
     launch_pair(l, k_sg_b<0>, k_sg_b<1>, k_sg_b<2>, b.n_sm * enum_grid(b, kSG), s, h);
     mark(h, kStampEnumEnd + kSG);

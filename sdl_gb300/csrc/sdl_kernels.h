@@ -8,6 +8,19 @@
 
 namespace sdlg {
 
+// Layer.cc:32-50: the outer layer slots paired with inner slot si (barrel
+// layers 1-5 -> the next barrel layer and endcap layer 1; endcap 1 -> 2;
+// endcap 2 -> 3, 4, 5; endcap 3 -> 4; endcap 4 -> 5); -1 past the last
+__host__ __device__ inline int sg_layer_outer(int si, int k) {
+    if (si <= 4) return k == 0 ? si + 1 : (k == 1 ? 6 : -1);
+    if (si == 6) return k == 0 ? 7 : -1;
+    if (si == 7) return k < 3 ? 8 + k : -1;
+    if (si == 8 || si == 9) return k == 0 ? si + 1 : -1;
+    return -1;
+}
+
+constexpr int kLayerRuns = 12;
+
 // Counters that kernels update atomically at the same time lie 256 bytes
 // apart (8-byte words): atomics on one line take turns at its L2 slice.
 constexpr int64_t kLine = 32;
@@ -107,7 +120,8 @@ struct BatchDev {
     int64_t* toff;                 // n_gm + 1: tile counts -> offsets
     int32_t* tile_gm;              // tile_cap: the global module of each tile (when the tiles fit)
     int64_t tile_cap;
-    int* layer_runs;               // n_ev x kNumSlots rows of 24: the layer-pair segments' outer runs (k_layer_runs)
+    int* layer_runs;               // n_ev x kNumSlots rows of 2 * layer_width: the layer-pair segments' outer runs (k_layer_runs)
+    int layer_width;               // the most outer runs of one inner layer slot, at least kLayerRuns
     int64_t* coff;                 // n_gm + 1: offsets of the modules' segment candidates
     int32_t* olist;                // olist_cap: the segment candidates' outer lists (k_sg_lists; offsets in toff)
     int64_t olist_cap;
