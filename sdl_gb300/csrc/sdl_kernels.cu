@@ -3416,8 +3416,12 @@ void launch_math_check(int fn, int exhaustive, unsigned long long start, long lo
 }
 
 // the tracklet candidates as a flat space, after a run: the module map's
-// enumeration needs none, and the bucket table holds the last stage's
+// enumeration needs none, the bucket table holds the last stage's, and the
+// connection sums may be those over tracklets or triplets
+// (createTrackCandidatesFromTracklets / FromTriplets)
 static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
+    if (!(b.flags & (kFlagTLLayers | kFlagTLNav)))
+        k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(b, kSG, -1, false);
     ClearJobs j{};
     j.add(b.scan_state + (int64_t)(kScanCand + kTL) * b.scan_cap, 2 * b.scan_cap);
     launch_clear(b, j, s, nullptr);
