@@ -1071,7 +1071,7 @@ int set_events_impl(sdlg_ctx* ctx, int64_t n_events, const int64_t* ev_off, cons
     void* dstp[5] = {(void*)b.in_x, (void*)b.in_y, (void*)b.in_z, (void*)b.in_idx, (void*)b.in_det};
     const size_t bytes = (size_t)n * 4;
     // pinned callers are copied directly; others through the pinned staging buffer
-    bool all_pinned = true, aligned = true;
+    bool all_pinned = true, aligned = true, words = true;
     const void* dev[5] = {};  // the device's addresses of the sources
     for (int k = 0; k < 5 && n > 0; ++k) {
         cudaPointerAttributes a;
@@ -1081,6 +1081,7 @@ int set_events_impl(sdlg_ctx* ctx, int64_t n_events, const int64_t* ev_off, cons
         } else {
             dev[k] = a.devicePointer;
             aligned = aligned && (reinterpret_cast<uintptr_t>(a.devicePointer) & 15u) == 0;
+            words = words && (reinterpret_cast<uintptr_t>(a.devicePointer) & 3u) == 0;
         }
     }
     if (n > 0 && !all_pinned) {
@@ -1097,7 +1098,7 @@ int set_events_impl(sdlg_ctx* ctx, int64_t n_events, const int64_t* ev_off, cons
             std::memcpy(p + k * stride, src[k], bytes);
             src[k] = dev[k] = p + k * stride;
         }
-        aligned = true;
+        aligned = words = true;
     }
     if (ctx->h_ev_cap < n_events + 2) {
         if (ctx->h_ev) cudaFreeHost(ctx->h_ev);
@@ -1112,9 +1113,10 @@ int set_events_impl(sdlg_ctx* ctx, int64_t n_events, const int64_t* ev_off, cons
     // takes 10 us less at any size (10.4 against 21.1 us at 2,304 hits, 20.2
     // against 30.5 at 97k, 465 against 477 at 4.8M).  Arrays that are not
     // 16-byte aligned go a word at a time, so large ones are left to the copy
-    // engines.
+    // engines, and so are arrays off a word's boundary (views into packed
+    // records), which a kernel cannot load.
     CopyJobs j{};
-    const bool kernel = aligned || n <= (int64_t)1 << 18;
+    const bool kernel = aligned || (words && n <= (int64_t)1 << 18);
     for (int k = 0; k < 5 && n > 0; ++k) {
         if (kernel) j.add(dev[k], dstp[k], n);
         else CK(cudaMemcpyAsync(dstp[k], src[k], bytes, cudaMemcpyHostToDevice, s));
