@@ -180,9 +180,12 @@ struct sdlg_ctx {
         cudaStream_t stream = nullptr;
         cudaEvent_t ev_in = nullptr, ev_used = nullptr;
     } stage;
-    // graph
-    cudaGraphExec_t graph = nullptr;
-    int graph_stop = -1, graph_flags = -1;
+    // graphs: of a batch that the buffers were made for, of a small one in larger buffers (batch_hits)
+    struct {
+        cudaGraphExec_t exec = nullptr;
+        int stop = -1, flags = -1;
+        int launches = 0;
+    } graph[2];
     // timing
     cudaEvent_t ev[2];  // around a run
     Hooks hooks;
@@ -225,10 +228,11 @@ void free_batch(sdlg_ctx* ctx) {
         cudaStreamSynchronize(ctx->gather_stream);
         ctx->read_pending = false;
     }
-    if (ctx->graph) {
-        cudaGraphExecDestroy(ctx->graph);
-        ctx->graph = nullptr;
-    }
+    for (auto& g : ctx->graph)
+        if (g.exec) {
+            cudaGraphExecDestroy(g.exec);
+            g.exec = nullptr;
+        }
     for (void* p : ctx->allocs) cudaFree(p);
     ctx->allocs.clear();
     ctx->buffers_ok = false;
@@ -419,7 +423,7 @@ int ensure_buffers(sdlg_ctx* ctx) {
     b.geo.n_slot_run = (int)ctx->slot_run.size();
     b.n_ev = (int)ctx->n_ev;
     b.n_gm = (int)n_gm;
-    b.n_hit_cap = H;
+    b.n_hit_cap = b.hits_about = H;
     b.n_sm = ctx->n_sm;
     b.mlp_pack = ctx->mlp.pack;
     b.mlp_stats = ctx->mlp.stats;
@@ -648,6 +652,7 @@ int launch_checked(sdlg_ctx* ctx, int first, int last) {
 
 int launch(sdlg_ctx* ctx, int stop_after, int flags) {
     ctx->b.flags = flags;
+    ctx->b.hits_about = batch_hits(ctx->n_hit, ctx->b.n_hit_cap);
     if (stop_after >= kSG) ctx->b.seg_layers = (flags & SDLG_FLAG_SG_LAYERS) != 0;
     ctx->ran = true;
     wait_readback(ctx);
@@ -662,23 +667,26 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
         CK(cudaGetLastError());
         return SDLG_OK;
     }
-    if (!ctx->graph || ctx->graph_stop != stop_after || ctx->graph_flags != flags) {
-        if (ctx->graph) {
-            cudaGraphExecDestroy(ctx->graph);
-            ctx->graph = nullptr;
+    auto& G = ctx->graph[ctx->b.hits_about == ctx->b.n_hit_cap ? 0 : 1];
+    if (!G.exec || G.stop != stop_after || G.flags != flags) {
+        if (G.exec) {
+            cudaGraphExecDestroy(G.exec);
+            G.exec = nullptr;
         }
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         enqueue_chain(ctx, 0, stop_after);
         CK(cudaStreamEndCapture(ctx->stream, &g));
-        cudaError_t e = cudaGraphInstantiate(&ctx->graph, g, 0);
+        cudaError_t e = cudaGraphInstantiate(&G.exec, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
-        ctx->graph_stop = stop_after;
-        ctx->graph_flags = flags;
+        G.stop = stop_after;
+        G.flags = flags;
+        G.launches = ctx->launches_per_run;
     }
+    ctx->launches_per_run = G.launches;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CK(cudaGraphLaunch(ctx->graph, ctx->stream));
+    CK(cudaGraphLaunch(G.exec, ctx->stream));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     return SDLG_OK;
 }
@@ -1714,7 +1722,7 @@ int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10) {
             out10[kNumStages + st] = bg[st];
         }
     }
-    ctx->graph_stop = -1;  // the launch graph holds the old shapes
+    for (auto& g : ctx->graph) g.stop = -1;  // the launch graphs hold the old shapes
     return SDLG_OK;
 }
 

@@ -1293,7 +1293,7 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
 // few tiles (enumeration of 128 dense events: 10.4 ms at 32, 10.6 at 24, 11.1 at
 // 16; of one PU 200 event: 80 us at 32, 75 at 24, 72 at 16).
 constexpr int kTileA = 32;
-__device__ __forceinline__ int tile_shift(const BatchDev& b) { return b.n_hit_cap <= (int64_t)1 << 18 ? 4 : 5; }
+__device__ __forceinline__ int tile_shift(const BatchDev& b) { return b.hits_about <= kSmallBatch ? 4 : 5; }
 
 __device__ __forceinline__ int64_t tile_count(const BatchDev& b, int64_t na, int64_t nb) {
     const int sh = tile_shift(b);
@@ -3067,8 +3067,11 @@ __global__ void __launch_bounds__(256) k_finish(BatchDev b, int64_t* host) {
 // modules are a kernel of their own for the same reason (64 events: 62 + 43 us
 // against 300 us within the scan; one event: 15 us within it).
 constexpr int64_t kScanSmall = (int64_t)1 << 18;
-// an object array's capacity is about three times what a run puts there
-inline int64_t objects_about(int64_t cap) { return cap / 3; }
+// an object array's capacity is about three times what a batch that fills the
+// hits' capacity puts there
+inline int64_t objects_about(const BatchDev& b, int64_t cap) {
+    return b.hits_about == b.n_hit_cap ? cap / 3 : (int64_t)((double)cap / 3 * (double)b.hits_about / (double)b.n_hit_cap);
+}
 template <class Op>
 void scan(const BatchDev& b, int slot, int64_t n, cudaStream_t s, Hooks* h) {
     const int items = n <= kScanSmall ? Op::kSmall : Op::kBig;
@@ -3085,7 +3088,7 @@ int enum_grid(const BatchDev& b, int st) { return b.enum_grid[st] > 0 ? b.enum_g
 // 7.30 together).
 void launch_pair(const BatchDev& b, void (*both)(BatchDev), void (*one)(BatchDev), void (*two)(BatchDev), int grid,
                  cudaStream_t s, Hooks* h) {
-    if (b.n_hit_cap <= (int64_t)1 << 18) {
+    if (b.hits_about <= kSmallBatch) {
         both<<<dim3((unsigned)grid, 2), kEnumThreads, 0, s>>>(take(b, h));
     } else {
         one<<<grid, kEnumThreads, 0, s>>>(take(b, h));
@@ -3102,7 +3105,7 @@ void scatter(const BatchDev& b, cudaStream_t s, Hooks* h) {
 // triplets or track candidates: counts scanned by Count -> objects
 template <int st, class Count, bool kFromTp = false>
 void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    scan<Count>(b, kScanCand + st, objects_about(b.cand_cap[st]), s, h);
+    scan<Count>(b, kScanCand + st, objects_about(b, b.cand_cap[st]), s, h);
     if (!kFromTp) mark(h, kStampEnum + st);
     k_expand<st, kFromTp><<<dim3((unsigned)b.n_sm * 8, 2), 256, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
@@ -3112,7 +3115,7 @@ void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
 template <class F, class Cand>
 void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
     constexpr int st = F::kSt;
-    scan<Cand>(b, kScanCand + st, st == kMD ? b.n_gm : objects_about(b.cand_cap[st]), s, h);
+    scan<Cand>(b, kScanCand + st, st == kMD ? b.n_gm : objects_about(b, b.cand_cap[st]), s, h);
     mark(h, kStampEnum + st);
     k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
     mark(h, kStampEnumEnd + st);
@@ -3144,7 +3147,7 @@ __global__ void __launch_bounds__(256) k_copy_words(CopyJobs j) {
 }  // namespace
 
 void launch_ingest(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    const unsigned g = grid_for(b.n_hit_cap, 256, b.n_sm * 16);
+    const unsigned g = grid_for(b.hits_about, 256, b.n_sm * 16);
     k_hit_map<<<g, 256, 0, s>>>(take(b, h));
     scan<ScanHits>(b, kScanHit, b.n_gm, s, h);
     k_hit_perm<<<g, 256, 0, s>>>(take(b, h));
@@ -3165,7 +3168,7 @@ void launch_sg(const BatchDev& b, cudaStream_t s, Hooks* h) {
     const bool layers = (b.flags & kFlagSGLayers) != 0;
     if (layers) {
         k_layer_runs<<<grid_for((int64_t)b.n_ev * kNumSlots, 64, b.n_sm), 64, 0, s>>>(take(b, h));
-        scan<ScanSgLayers>(b, kScanCand + kSG, objects_about(b.cand_cap[kSG]), s, h);
+        scan<ScanSgLayers>(b, kScanCand + kSG, objects_about(b, b.cand_cap[kSG]), s, h);
     } else if (b.n_gm <= kScanSmall) {
         scan<ScanSgFront<true>>(b, kScanCand + kSG, b.n_gm, s, h);
     } else {
@@ -3204,10 +3207,10 @@ void launch_tl(const BatchDev& b, cudaStream_t s, Hooks* h) {
         scan<ScanTlFront<false>>(b, kScanTlFront, b.n_gm, s, h);
     }
     // the segments by inner mini-doublet, for navigation and the triplets
-    scan<ScanJoin<0>>(b, kScanJoinSg, objects_about(b.obj[kMD].cap), s, h);
+    scan<ScanJoin<0>>(b, kScanJoinSg, objects_about(b, b.obj[kMD].cap), s, h);
     k_sg_index<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
     if (b.geo.conn_dup) k_sg_keys<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));
-    if (!tiles) scan<ScanTlCand<true>>(b, kScanCand + kTL, objects_about(b.cand_cap[kTL]), s, h);
+    if (!tiles) scan<ScanTlCand<true>>(b, kScanCand + kTL, objects_about(b, b.cand_cap[kTL]), s, h);
     mark(h, kStampEnum + kTL);
     // enumeration + phase A -> survivor list (-> the pre-filter -> kept list)
     // -> phase B1 -> phase B2
@@ -3263,9 +3266,9 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         launch_clear(b, j, s, h);
         const unsigned g = b.n_sm * 8, ge = b.n_sm * enum_grid(b, kTL);
         k_join2_count<<<g, 256, 0, s>>>(take(b, h));
-        scan<ScanJoin<1>>(b, kScanJoinTc, objects_about(b.obj[kMD].cap), s, h);
+        scan<ScanJoin<1>>(b, kScanJoinTc, objects_about(b, b.obj[kMD].cap), s, h);
         k_join2_scatter<<<g, 256, 0, s>>>(take(b, h));
-        scan<ScanTctp>(b, kScanTctp, objects_about(b.cand_cap[kTL]), s, h);
+        scan<ScanTctp>(b, kScanTctp, objects_about(b, b.cand_cap[kTL]), s, h);
         mark(h, kStampEnum + kTC);
         BatchDev l = b;  // the pairs' list is the tracklets' spare one, with a count of its own
         l.passa = b.pb;
@@ -3273,14 +3276,14 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         k_tctp_a<<<ge, kEnumThreads, 0, s>>>(take(l, h));
         k_tctp_b<<<ge, kEnumThreads, 0, s>>>(take(b, h));
         k_tctp_c<<<ge, kEnumThreads, 0, s>>>(take(b, h));
-        scan<ScanJoin<3>>(b, kScanTctpJoin, objects_about(b.obj[kMD].cap), s, h);
+        scan<ScanJoin<3>>(b, kScanTctpJoin, objects_about(b, b.obj[kMD].cap), s, h);
         k_tctp_place<<<g, 256, 0, s>>>(take(b, h));
         expand<kTC, ScanTcFromTp, true>(b, s, h);
         return;
     }
     // the tracklets by inner segment
     if (b.first > kTL) k_tl_join_count<<<b.n_sm * 8, 256, 0, s>>>(take(b, h));  // (else in k_scatter)
-    scan<ScanJoin<2>>(b, kScanJoinTc, objects_about(b.obj[kSG].cap), s, h);
+    scan<ScanJoin<2>>(b, kScanJoinTc, objects_about(b, b.obj[kSG].cap), s, h);
     if (b.flags & kFlagTCFromTL) {
         k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(take(b, h), kTL, -1, false);
         expand<kTC, ScanTcFromTl>(b, s, h);
@@ -3427,7 +3430,7 @@ static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
     ClearJobs j{};
     j.add(b.scan_state + (int64_t)(kScanCand + kTL) * b.scan_cap, 2 * b.scan_cap);
     launch_clear(b, j, s, nullptr);
-    scan<ScanTlCand<false>>(b, kScanCand + kTL, objects_about(b.cand_cap[kTL]), s, nullptr);
+    scan<ScanTlCand<false>>(b, kScanCand + kTL, objects_about(b, b.cand_cap[kTL]), s, nullptr);
 }
 
 void launch_tl_collect(const BatchDev& b, const MlpCollect& c, cudaStream_t s) {

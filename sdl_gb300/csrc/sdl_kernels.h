@@ -21,6 +21,18 @@ __host__ __device__ inline int sg_layer_outer(int si, int k) {
 
 constexpr int kLayerRuns = 12;
 
+// Batches of up to so many hits take the launch shapes of small ones: tiles of
+// 16 rows, both parts of a list in one launch, small scan tiles (each measured
+// where it is chosen).
+constexpr int64_t kSmallBatch = (int64_t)1 << 18;
+// The hits that a batch's launch shapes are made for: the buffers' capacity,
+// or, for a small batch in larger buffers (a context that once held a large
+// batch), half the limit.  So two figures per set of buffers, and two graphs,
+// serve any order of batches.
+constexpr int64_t batch_hits(int64_t n_hit, int64_t cap) {
+    return n_hit <= kSmallBatch && cap > kSmallBatch ? kSmallBatch / 2 : cap;
+}
+
 // Counters that kernels update atomically at the same time lie 256 bytes
 // apart (8-byte words): atomics on one line take turns at its L2 slice.
 constexpr int64_t kLine = 32;
@@ -30,6 +42,7 @@ struct BatchDev {
     int n_ev;
     int n_gm;          // n_ev * n_mod
     int64_t n_hit_cap;
+    int64_t hits_about;     // the hits that the launch shapes are made for (batch_hits)
     const int64_t* n_hit;   // device scalar
     // inputs (concatenated events)
     const float *in_x, *in_y, *in_z;

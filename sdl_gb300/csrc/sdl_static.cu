@@ -146,7 +146,7 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     b.geo = geo;
     b.n_ev = 1;
     b.n_gm = geo.n_mod;
-    b.n_hit_cap = H;
+    b.n_hit_cap = b.hits_about = H;
     b.n_hit = w64 + kSmall;
     b.task_size = reinterpret_cast<int*>(w64 + kSmall + 8);
     b.n_rec = w64 + kSmall + 2;
