@@ -1494,11 +1494,11 @@ __device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4
     const float arg = ar > kSinAlphaMax ? kSinAlphaMax : ar;
     const float u = __fmaf_rn(-arg, arg, 1.f);
     const float st = __fmaf_rn(u * rsqrtf(u), R.sine, arg * R.cose);
-    const float L = R.rt * dr;
+    const float L = R.rt * dr, hi = L * (st + kB1Margin);
     const bool c5 = f < -mg, e4 = algo == kAlgoEEEE, fast = arg >= -kSinAlphaMax;
     const bool in = e4 || (fast && q < L * (st - kB1Margin) && p > 0.f);
-    // (past a right angle fails too, where the threshold is below one: not without e)
-    const bool out = !e4 && fast && (q > L * (st + kB1Margin) || (R.sine == R.sine && p < -(kB1Margin * L)));
+    // (an angle past pi / 2 + th, by its cosine, fails too; a NaN threshold rejects nothing)
+    const bool out = !e4 && fast && (q > hi || p < -hi);
     return f > mg || (c5 && out) ? 0 : c5 && in ? 1 : -1;
 }
 
