@@ -215,9 +215,9 @@ template <class Op, int kI>
 __global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
     constexpr int kK = Op::kVals, kWarps = kScanThreads / kWarp;
     constexpr int kTile = kScanThreads * kI;
-    // (a scan can halt the run itself while its last CTAs start, so one thread
-    // decides for its CTA)
-    const bool stop = threadIdx.x == 0 && halted(b);
+    // (a scan can halt the run itself while its last CTAs start, so the CTA
+    // decides as one)
+    if (__syncthreads_or(halted(b))) return;
     Op::begin(b);
     const int64_t n = Op::size(b);
     const int64_t ntile = n > 0 ? (n + kTile - 1) / kTile : 1;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(BatchDev b, int slot) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
-            s_tile = stop ? INT64_MAX : (int64_t)atomicAdd(ticket, 1ull);
+            s_tile = (int64_t)atomicAdd(ticket, 1ull);
             s_back.ok = 1;
         }
         __syncthreads();
