@@ -533,10 +533,13 @@ int ensure_buffers(sdlg_ctx* ctx) {
     AL(b.olist, b.olist_cap);
 #undef AL
     if (ctx->h_run_words < run_words(ctx->n_ev)) {
+        int64_t* p = nullptr;
+        CK(cudaMallocHost((void**)&p, run_words(ctx->n_ev) * sizeof(int64_t)));
+        // (the last run's stamps stay readable: sdlg_last_times)
+        if (ctx->h_run) std::memcpy(p, ctx->h_run, kRunOffsets * sizeof(int64_t));
+        else std::memset(p, 0, kRunOffsets * sizeof(int64_t));
         if (ctx->h_run) cudaFreeHost(ctx->h_run);
-        ctx->h_run = nullptr;
-        ctx->h_run_words = 0;
-        CK(cudaMallocHost((void**)&ctx->h_run, run_words(ctx->n_ev) * sizeof(int64_t)));
+        ctx->h_run = p;
         ctx->h_run_words = run_words(ctx->n_ev);
     }
     ctx->buffers_ok = true;
