@@ -440,7 +440,10 @@ int sdlg_mlp_clear_samples(sdlg_ctx* ctx);
  * epoch_loss[e] (optional) receives each epoch's mean loss. */
 int sdlg_mlp_train(sdlg_ctx* ctx, int epochs, int batch, float lr, float pos_weight, uint64_t seed, float* epoch_loss);
 /* Gradient of mean_i w_i * (softplus(z_i) - y_i z_i) at the current
- * parameters over n samples (the training kernels), and the loss. */
+ * parameters over n samples (the training kernels), and the loss.  The
+ * samples (56 bytes each; 52 for sdlg_mlp_score) pass through device scratch of
+ * the context, of which a call leaves at most 64 MiB behind unless the object
+ * readbacks had grown it further. */
 int sdlg_mlp_gradient(sdlg_ctx* ctx, int64_t n, const float* x, const float* y, const float* w, float* grad, double* loss);
 /* logits of n feature rows (n x 12) through the tensor-core kernel */
 int sdlg_mlp_score(sdlg_ctx* ctx, int64_t n, const float* x, float* logits);
