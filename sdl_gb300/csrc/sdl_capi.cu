@@ -568,7 +568,7 @@ void (*const kLaunch[kNumStages])(const BatchDev&, cudaStream_t, Hooks*) = {laun
                                                                             launch_tc};
 
 // what stages first..last accumulate into, set to zero
-void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
+cudaError_t enqueue_clear(sdlg_ctx* ctx, int first, int last) {
     BatchDev& b = ctx->b;
     ClearJobs j{};
     const int64_t n_gm = b.n_gm;
@@ -607,13 +607,13 @@ void enqueue_clear(sdlg_ctx* ctx, int first, int last) {
     }
     j.add(b.scan_state, 2 * kScanSlots * b.scan_cap);
     if (last >= kTL && first <= kTL) j.add(b.eoff, 2 * (n_gm + 1));
-    launch_clear(b, j, ctx->stream, &ctx->hooks);
+    return launch_clear(b, j, ctx->stream, &ctx->hooks);
 }
 
 // stages first..last (from the hits when first is 0, else on the objects the
 // previous run left for the stages below first), enqueued on the context
 // stream; for first 0 also the body of the CUDA graph
-void enqueue_chain(sdlg_ctx* ctx, int first, int last) {
+cudaError_t enqueue_chain(sdlg_ctx* ctx, int first, int last) {
     BatchDev& b = ctx->b;
     cudaStream_t s = ctx->stream;
     Hooks* h = &ctx->hooks;
@@ -621,7 +621,8 @@ void enqueue_chain(sdlg_ctx* ctx, int first, int last) {
     h->ts = stamp_bit(kStampStart);
     b.first = first;
     b.last = last;
-    enqueue_clear(ctx, first, last);
+    const cudaError_t cleared = enqueue_clear(ctx, first, last);
+    if (cleared != cudaSuccess) return cleared;
     if (first == 0) launch_ingest(b, s, h);
     for (int st = first; st <= last; ++st) {
         h->ts |= stamp_bit(kStampStage + st);
@@ -631,6 +632,7 @@ void enqueue_chain(sdlg_ctx* ctx, int first, int last) {
     h->ts |= stamp_bit(kStampEnd);
     launch_finish(b, ctx->h_run, s, h);
     ctx->launches_per_run = h->launches;
+    return cudaSuccess;
 }
 
 #ifdef SDL_DEVICE_CHECKS
@@ -655,7 +657,7 @@ int launch_checked(sdlg_ctx* ctx, int first, int last) {
     h->ts = stamp_bit(kStampStart);
     b.first = first;
     b.last = last;
-    enqueue_clear(ctx, first, last);
+    CK(enqueue_clear(ctx, first, last));
     if (first == 0) launch_ingest(b, s, h);
     if ((rc = check_stage(ctx, "ingest"))) return rc;
     static const char* names[5] = {"MD", "SG", "TL", "TP", "TC"};
@@ -683,7 +685,7 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
     const bool use_graph = !(flags & SDLG_FLAG_NO_GRAPH);
     if (!use_graph) {
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        enqueue_chain(ctx, 0, stop_after);
+        CK(enqueue_chain(ctx, 0, stop_after));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         CK(cudaGetLastError());
         return SDLG_OK;
@@ -696,11 +698,11 @@ int launch(sdlg_ctx* ctx, int stop_after, int flags) {
         }
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_chain(ctx, 0, stop_after);
+        cudaError_t e = enqueue_chain(ctx, 0, stop_after);
         CK(cudaStreamEndCapture(ctx->stream, &g));
-        cudaError_t e = cudaGraphInstantiate(&G.exec, g, 0);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, g, 0);
         cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "launch graph: %s", cudaGetErrorString(e));
         G.stop = stop_after;
         G.flags = flags;
         G.launches = ctx->launches_per_run;
@@ -1152,7 +1154,7 @@ int set_events_impl(sdlg_ctx* ctx, int64_t n_events, const int64_t* ev_off, cons
     }
     j.add(ctx->h_ev, const_cast<int64_t*>(b.n_hit), 2);
     j.add(ctx->h_ev + 1, const_cast<int64_t*>(b.ev_off), 2 * (n_events + 1));
-    launch_copy_words(j, ctx->n_sm, s);
+    CK(launch_copy_words(j, ctx->n_sm, s));
     CK(cudaGetLastError());
     // the caller's buffers are read when this returns
     CK(cudaStreamSynchronize(s));
@@ -1309,7 +1311,7 @@ int install_staged(sdlg_ctx* ctx) {
     for (int k = 0; k < 5; ++k) j.add(S.dev + k * stage_stride(S.hits), dstp[k], S.n_hit);
     j.add(offs, const_cast<int64_t*>(b.ev_off), (S.n_ev + 1) * 2);
     j.add(offs + (S.n_ev + 1) * sizeof(int64_t), const_cast<int64_t*>(b.n_hit), 2);
-    launch_copy_words(j, ctx->n_sm, s);
+    CK(launch_copy_words(j, ctx->n_sm, s));
     CK(cudaGetLastError());
     CK(cudaEventRecord(S.ev_used, s));
     S.used_pending = true;
@@ -1398,7 +1400,7 @@ int sdlg_run_stages(sdlg_ctx* ctx, int first, int last, int flags) {
     if (rc) return rc;
 #else
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    enqueue_chain(ctx, first, last);
+    CK(enqueue_chain(ctx, first, last));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     CK(cudaGetLastError());
 #endif

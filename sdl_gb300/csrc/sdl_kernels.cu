@@ -3263,7 +3263,8 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         j.add(b.jcur2, b.obj[kMD].cap);
         j.add(b.tpend, b.obj[kMD].cap);
         j.add(b.joff3, 2 * (b.obj[kMD].cap + 1));
-        launch_clear(b, j, s, h);
+        static_assert(kClearJobs >= 4, "the jobs fit");
+        (void)launch_clear(b, j, s, h);
         const unsigned g = b.n_sm * 8, ge = b.n_sm * enum_grid(b, kTL);
         k_join2_count<<<g, 256, 0, s>>>(take(b, h));
         scan<ScanJoin<1>>(b, kScanJoinTc, objects_about(b, b.obj[kMD].cap), s, h);
@@ -3429,7 +3430,7 @@ static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
         k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(b, kSG, -1, false);
     ClearJobs j{};
     j.add(b.scan_state + (int64_t)(kScanCand + kTL) * b.scan_cap, 2 * b.scan_cap);
-    launch_clear(b, j, s, nullptr);
+    (void)launch_clear(b, j, s, nullptr);
     scan<ScanTlCand<false>>(b, kScanCand + kTL, objects_about(b, b.cand_cap[kTL]), s, nullptr);
 }
 
@@ -3491,19 +3492,23 @@ void launch_libm_eval(int fn, uint32_t start, int64_t n, float* out, int n_sm, c
     k_libm_eval<<<grid_for(n, 256, n_sm * 16), 256, 0, s>>>(fn, start, n, out);
 }
 
-void launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h) {
+cudaError_t launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h) {
+    if (j.full) return cudaErrorInvalidValue;
     int64_t most = 1;
     for (int k = 0; k < j.count; ++k) most = most > j.words[k] * j.rows[k] ? most : j.words[k] * j.rows[k];
     k_clear<<<dim3(grid_for((most + 3) / 4, 256, b.n_sm * 4), (unsigned)j.count), 256, 0, s>>>(take(b, h), j);
+    return cudaSuccess;
 }
 
 void launch_finish(const BatchDev& b, int64_t* host, cudaStream_t s, Hooks* h) {
     k_finish<<<grid_for((int64_t)b.n_ev * 110, 256, b.n_sm), 256, 0, s>>>(take(b, h), host);
 }
 
-void launch_copy_words(const CopyJobs& j, int n_sm, cudaStream_t s) {
-    if (j.count <= 0) return;
+cudaError_t launch_copy_words(const CopyJobs& j, int n_sm, cudaStream_t s) {
+    if (j.full) return cudaErrorInvalidValue;
+    if (j.count <= 0) return cudaSuccess;
     k_copy_words<<<dim3((unsigned)(n_sm * 2), (unsigned)j.count), 256, 0, s>>>(j);
+    return cudaSuccess;
 }
 
 void launch_materialize(const BatchDev& b, int st, int64_t first, int64_t n, int32_t* out, cudaStream_t s) {

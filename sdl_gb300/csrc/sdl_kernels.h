@@ -205,15 +205,19 @@ struct ClearJobs {
     int64_t pitch[kClearJobs];
     int count;
     int stamps;  // the first so many stamps too
+    bool full;   // a job did not fit: the launch is refused
     void add(void* q, int64_t n_words, int64_t n_rows = 1, int64_t n_pitch = 0) {
-        if (count == kClearJobs) return;
+        if (count == kClearJobs) {
+            full = true;
+            return;
+        }
         p[count] = static_cast<uint32_t*>(q);
         words[count] = n_words;
         rows[count] = n_rows;
         pitch[count++] = n_pitch;
     }
 };
-void launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h);
+cudaError_t launch_clear(const BatchDev& b, const ClearJobs& j, cudaStream_t s, Hooks* h);
 
 // What the host reads after a run, written by the run's last kernel to
 // pinned memory (8-byte words): the appends attempted per stage, the status
@@ -278,13 +282,17 @@ struct CopyJobs {
     uint32_t* dst[kCopyJobs];
     int64_t n[kCopyJobs];  // words
     int count;
+    bool full;  // a job did not fit: the launch is refused
     void add(const void* from, void* to, int64_t words) {
-        if (count == kCopyJobs) return;
+        if (count == kCopyJobs) {
+            full = true;
+            return;
+        }
         src[count] = static_cast<const uint32_t*>(from);
         dst[count] = static_cast<uint32_t*>(to);
         n[count++] = words;
     }
 };
-void launch_copy_words(const CopyJobs& j, int n_sm, cudaStream_t s);
+cudaError_t launch_copy_words(const CopyJobs& j, int n_sm, cudaStream_t s);
 
 }  // namespace sdlg

@@ -200,12 +200,16 @@ extern "C" int sdlg_mini_doublets_static(sdlg_ctx* ctx, int64_t n_hits, const fl
     j.add(b.mod_hit, 2 * (geo.n_mod + 1));
     j.add(O.mod_cnt, 2 * (geo.n_mod + 1));
     j.add(b.scan_state, 2 * kScanSlots * b.scan_cap);
-    launch_clear(b, j, s, nullptr);
+    cudaError_t e = launch_clear(b, j, s, nullptr);
+    if (e != cudaSuccess) {
+        ctx_set_error(ctx, "too many buffers to clear");
+        return SDLG_ERR_CUDA;
+    }
     k_static_init<<<1, 32, 0, s>>>(b, n_hits);
     launch_ingest(b, s, nullptr);
     launch_md(b, s, nullptr);
     k_static_out<<<n_sm * 4, 256, 0, s>>>(b, d_pairs, pair_cap, d_count, d_status);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) {
         snprintf(msg, sizeof(msg), "launch failed: %s", cudaGetErrorString(e));
         ctx_set_error(ctx, msg);
