@@ -293,7 +293,10 @@ int sdlg_last_kernel_times(sdlg_ctx* ctx, float* out5);
  * batch with each of a grid of launch shapes for the stages' candidate
  * evaluation kernels (candidates per warp task 128-1024, 4-16 CTAs per SM),
  * keeps the fastest shape per stage for later runs of this context, and
- * returns it in out10 (tasks[5], CTAs per SM[5]; may be NULL).  Results do
+ * returns it in out10 (tasks[5], CTAs per SM[5]; may be NULL).  Triplets and
+ * track candidates evaluate no candidates (but the track candidates from
+ * triplets after layer-pair segments): their shape stays as it was (256 and 8),
+ * as does that of a stage past stop_after (0 until it is tuned).  Results do
  * not depend on the shapes.  Takes about 24 runs of the chain. */
 int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10);
 

@@ -1705,6 +1705,11 @@ int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10) {
     if (!ctx->have_geo) return fail(ctx, SDLG_ERR_NO_GEOMETRY, "no geometry loaded");
     if (!ctx->buffers_ok || ctx->n_ev <= 0) return fail(ctx, SDLG_ERR_NO_EVENTS, "no events set");
     if (stop_after < 0 || stop_after > 4) return fail(ctx, SDLG_ERR_ARG, "stop_after out of range");
+    // the stages that evaluate candidates: the triplets and the track
+    // candidates are written from counts, except those from triplets after
+    // layer-pair segments
+    const bool tc_enum = (flags & SDLG_FLAG_TC_FROM_TP) && (flags & SDLG_FLAG_SG_LAYERS);
+    auto tunable = [&](int st) { return st <= kTL || (st == kTC && tc_enum); };
     static const int kTasks[] = {128, 256, 512, 1024};
     static const int kGrids[] = {4, 8, 16};
     float best[kNumStages];
@@ -1717,6 +1722,7 @@ int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10) {
     for (int task : kTasks) {
         for (int grid : kGrids) {
             for (int st = 0; st < kNumStages; ++st) {  // (a capacity regrow re-reads the context's values)
+                if (!tunable(st)) continue;
                 ctx->tune_task[st] = ctx->b.enum_task[st] = task;
                 ctx->tune_grid[st] = ctx->b.enum_grid[st] = grid;
             }
@@ -1728,7 +1734,7 @@ int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10) {
                 if (rc) return rc;
             }
             for (int st = 0; st <= stop_after; ++st)
-                if (t[st] < best[st]) {
+                if (tunable(st) && t[st] < best[st]) {
                     best[st] = t[st];
                     bt[st] = task;
                     bg[st] = grid;
@@ -1741,8 +1747,9 @@ int sdlg_autotune(sdlg_ctx* ctx, int stop_after, int flags, int32_t* out10) {
         ctx->b.enum_task[st] = bt[st];
         ctx->b.enum_grid[st] = bg[st];
         if (out10) {
-            out10[st] = bt[st];
-            out10[kNumStages + st] = bg[st];
+            const bool shape = bt[st] > 0 || st > stop_after;  // (a stage past stop_after: 0 until it is tuned)
+            out10[st] = shape ? bt[st] : kTaskDefault;
+            out10[kNumStages + st] = shape ? bg[st] : kGridDefault;
         }
     }
     for (auto& g : ctx->graph) g.stop = -1;  // the launch graphs hold the old shapes

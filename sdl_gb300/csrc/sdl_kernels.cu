@@ -43,8 +43,6 @@ __device__ __forceinline__ int64_t checked_idx(int64_t i, int64_t lim, int line,
 
 constexpr int kWarp = 32;
 constexpr int kEnumThreads = 256;
-constexpr int kTaskDefault = 256;  // candidates per warp task unless tuned
-constexpr int kGridDefault = 8;    // CTAs per SM of an enumeration unless tuned
 
 // the launch's device time stamps (none for most launches)
 __device__ __forceinline__ void stamp(const BatchDev& b) {

@@ -21,6 +21,9 @@ __host__ __device__ inline int sg_layer_outer(int si, int k) {
 
 constexpr int kLayerRuns = 12;
 
+constexpr int kTaskDefault = 256;  // candidates per warp task unless tuned
+constexpr int kGridDefault = 8;    // CTAs per SM of an enumeration unless tuned
+
 // Batches of up to so many hits take the launch shapes of small ones: tiles of
 // 16 rows, both parts of a list in one launch, small scan tiles (each measured
 // where it is chosen).
