@@ -910,67 +910,6 @@ __global__ void __launch_bounds__(kEnumThreads) k_md_enum(BatchDev b) {
     rec_flush<4>(b, kMD, rb);
 }
 
-template <class F>
-__global__ void __launch_bounds__(kEnumThreads) k_enum(BatchDev b) {
-    constexpr int st = F::kSt;
-    constexpr int kNF = st == kMD ? 4 : (st == kSG ? 6 : 0);  // the stage's float values per object
-    __shared__ int rbuf[kEnumThreads / kWarp][3 + kNF][kRecBuf];
-    if (halted(b)) return;
-    const int64_t nobj = n_inner(b, st);
-    if (nobj <= 0) return;
-    const int64_t* off = b.cand[st];
-    const int64_t offlim = b.cand_cap[st] + 1;
-    const int64_t total = AT(off, nobj, offlim);
-    const int task = b.task_size[st];
-    const int64_t ntask = (total + task - 1) / task;
-    const int lane = threadIdx.x & 31;
-    RecBuf<kNF> rb{rbuf[threadIdx.x >> 5]};
-    for (;;) {
-        unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(b.task + st * kLine, 1ull);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if ((int64_t)t >= ntask) break;
-        const int64_t base = (int64_t)t * task;
-        const int64_t end = min(base + task, total);
-        int ilo = 0;
-        if (lane < 2) {
-            int lo, hi;
-            obj_bounds(b, nobj, total, base, end - 1, lo, hi);
-            ilo = find_obj(b, off, offlim, lo, hi, lane == 0 ? base : end - 1);
-        }
-        const int i0 = __shfl_sync(0xffffffffu, ilo, 0);
-        const int i1 = __shfl_sync(0xffffffffu, ilo, 1);
-        for (int64_t cb = base; cb < end; cb += kWarp) {
-            const int64_t c = cb + lane;
-            const bool valid = c < end;
-            int oi = 0, oj = 0, g = 0;
-            float fv[6];
-            bool pass = false;
-            if (valid) {
-                const int i = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
-                pass = F::eval(b, i, c - AT(off, i, offlim), oi, oj, fv);
-                if (pass) g = F::group_of(b, i);
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, pass);
-            if (m) {
-                const int c = __popc(m);
-                if (rb.n + c > kRecBuf) rec_flush<kNF>(b, st, rb);
-                if (pass) {
-                    const int k = rb.n + __popc(m & ((1u << lane) - 1u));
-                    rb.e[0][k] = oi;
-                    rb.e[1][k] = oj;
-                    rb.e[2][k] = g;
-#pragma unroll
-                    for (int q = 0; q < kNF; ++q) rb.e[3 + q][k] = __float_as_int(fv[q]);
-                }
-                rb.n += c;
-            }
-        }
-    }
-    rec_flush<kNF>(b, st, rb);
-}
-
-
 // One packed record per segment for the tracklet stage (the anchors of both
 // mini-doublets, the segment's angles and the per-segment sub-expressions of
 // Tracklet.cc that depend on one segment only).
@@ -1102,37 +1041,79 @@ __global__ void __launch_bounds__(256, 4) k_sg_pack(BatchDev b) {
 // when the trial segment from that MD to p2's innermost MD passes the segment
 // algorithm and the tracklet (trial segment, p2's outer segment) passes the
 // default tracklet algorithm.  The trial segment is not kept.
-struct TCTPStage {
-    static constexpr int kSt = kTC;
-    __device__ static bool eval(const BatchDev& b, int p1, int64_t q, int& oi, int& oj, float* fv) {
-        const int n_mod = b.geo.n_mod;
-        const int mdA = OJ(b, kSG, OJ(b, kTP, p1));
-        const int gA = OG(b, kMD, mdA);
-        const int ev = ev_of(b, gA), mA = gA - ev * n_mod;
-        int pref;
-        const int k = conn_entry(b, ev, mA, q, pref);
-        const int g3 = ev * n_mod + AT(b.geo.conn_idx, k, NC(b));
-        const int p2 = (int)(OFF(b, kTP, g3) + (q - pref));
-        oi = p1;
-        oj = p2;
-        (void)fv;
-        const int mdB = OI(b, kSG, OI(b, kTP, p2));
-        float f6[6];
-        if (!sg_pair(b, mdA, mdB, true, f6)) return false;
-        float v[PK_N];
-        sg_pack_record(b, mdA, mdB, f6, v);
-        const SGV S = sgv_from(v);
-        const int so = OJ(b, kTP, p2);
-        const SGV T = load_sgv(b.sgpack, so);
-        float cut, muls;
-        const int algo = tl_phaseA(S, T, cut, muls);
-        if (algo == kAlgoNone || !tl_phaseB1_sgv(algo, S, T, cut)) return false;
-        return tl_phaseB2_sgv<kB2All>(algo, S, T, muls, false);
+// (After layer-pair segments; after those of the module map see ScanTctp.)
+__device__ __forceinline__ bool tctp_trial(const BatchDev& b, int p1, int64_t q, int& p2) {
+    const int n_mod = b.geo.n_mod;
+    const int mdA = OJ(b, kSG, OJ(b, kTP, p1));
+    const int gA = OG(b, kMD, mdA);
+    const int ev = ev_of(b, gA), mA = gA - ev * n_mod;
+    int pref;
+    const int k = conn_entry(b, ev, mA, q, pref);
+    const int g3 = ev * n_mod + AT(b.geo.conn_idx, k, NC(b));
+    p2 = (int)(OFF(b, kTP, g3) + (q - pref));
+    const int mdB = OI(b, kSG, OI(b, kTP, p2));
+    float f6[6];
+    if (!sg_pair(b, mdA, mdB, true, f6)) return false;
+    float v[PK_N];
+    sg_pack_record(b, mdA, mdB, f6, v);
+    const SGV S = sgv_from(v);
+    const int so = OJ(b, kTP, p2);
+    const SGV T = load_sgv(b.sgpack, so);
+    float cut, muls;
+    const int algo = tl_phaseA(S, T, cut, muls);
+    if (algo == kAlgoNone || !tl_phaseB1_sgv(algo, S, T, cut)) return false;
+    return tl_phaseB2_sgv<kB2All>(algo, S, T, muls, false);
+}
+__global__ void __launch_bounds__(kEnumThreads) k_tctp_trial(BatchDev b) {
+    __shared__ int rbuf[kEnumThreads / kWarp][3][kRecBuf];
+    if (halted(b)) return;
+    const int64_t nobj = n_inner(b, kTC);
+    if (nobj <= 0) return;
+    const int64_t* off = b.cand[kTC];
+    const int64_t offlim = b.cand_cap[kTC] + 1;
+    const int64_t total = AT(off, nobj, offlim);
+    const int task = b.task_size[kTC];
+    const int64_t ntask = (total + task - 1) / task;
+    const int lane = threadIdx.x & 31;
+    RecBuf<0> rb{rbuf[threadIdx.x >> 5]};
+    for (;;) {
+        unsigned long long t = 0;
+        if (lane == 0) t = atomicAdd(b.task + kTC * kLine, 1ull);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if ((int64_t)t >= ntask) break;
+        const int64_t base = (int64_t)t * task;
+        const int64_t end = min(base + task, total);
+        int ilo = 0;
+        if (lane < 2) {
+            int lo, hi;
+            obj_bounds(b, nobj, total, base, end - 1, lo, hi);
+            ilo = find_obj(b, off, offlim, lo, hi, lane == 0 ? base : end - 1);
+        }
+        const int i0 = __shfl_sync(0xffffffffu, ilo, 0);
+        const int i1 = __shfl_sync(0xffffffffu, ilo, 1);
+        for (int64_t cb = base; cb < end; cb += kWarp) {
+            const int64_t c = cb + lane;
+            int p1 = 0, p2 = 0;
+            bool pass = false;
+            if (c < end) {
+                p1 = (i0 == i1) ? i0 : find_obj(b, off, offlim, i0, i1, c);
+                pass = tctp_trial(b, p1, c - AT(off, p1, offlim), p2);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, pass);
+            if (!m) continue;
+            if (rb.n + __popc(m) > kRecBuf) rec_flush<0>(b, kTC, rb);
+            if (pass) {
+                const int k = rb.n + __popc(m & ((1u << lane) - 1u));
+                rb.e[0][k] = p1;
+                rb.e[1][k] = p2;
+                rb.e[2][k] = OG(b, kTP, p1);
+            }
+            rb.n += __popc(m);
+        }
     }
-    __device__ static int group_of(const BatchDev& b, int p) { return OG(b, kTP, p); }
-};
+    rec_flush<0>(b, kTC, rb);
+}
 
-// outer segment of flat tracklet candidate c of inner segment s
 // tracklet candidate q of inner segment s by navigation (Event.cc:694-751):
 // over the segments leaving s's outer MD, the segments leaving their outer MD
 // (both lists from the join index of segments by inner MD)
@@ -1479,7 +1460,7 @@ constexpr int kSgbMinBlocks = SDLG_SGB_MIN_BLOCKS;
 
 // Segment candidates in two passes (Event.cc:445-522 or 793-821 with
 // Segment.cc:337-859): k_sg_enum_a takes tasks of consecutive candidates
-// like k_enum, gathers those the algorithm's first cuts do not certainly
+// like k_tl_enum_a, gathers those the algorithm's first cuts do not certainly
 // reject (40 % of them) to full warps, and lists those that the later cuts do
 // not certainly reject either (7.7 %; 7.6 % are segments); k_sg_b runs the
 // whole algorithm on the list and appends the segments.  Both are bound by
@@ -2670,7 +2651,7 @@ __device__ __forceinline__ int64_t tctp_cand(const BatchDev& b, int64_t p, bool 
     count_cand(b, kTC, c ? OG(b, kTP, p) : 0, c);
     return c;
 }
-// each evaluated with its trial segment (TCTPStage, after layer-pair segments)
+// each evaluated with its trial segment (k_tctp_trial, after layer-pair segments)
 struct ScanTcTrial : ScanCand<kTC> {
     __device__ static void load(const BatchDev& b, int64_t p, bool in, int64_t* v) { v[0] = tctp_cand(b, p, in); }
 };
@@ -3109,18 +3090,6 @@ void expand(const BatchDev& b, cudaStream_t s, Hooks* h) {
     mark(h, kStampEnumEnd + st);
 }
 
-// stage F's candidates (their offsets scanned by Cand) -> objects
-template <class F, class Cand>
-void enum_and_group(const BatchDev& b, cudaStream_t s, Hooks* h) {
-    constexpr int st = F::kSt;
-    scan<Cand>(b, kScanCand + st, st == kMD ? b.n_gm : objects_about(b, b.cand_cap[st]), s, h);
-    mark(h, kStampEnum + st);
-    k_enum<F><<<b.n_sm * enum_grid(b, st), kEnumThreads, 0, s>>>(take(b, h));
-    mark(h, kStampEnumEnd + st);
-    scan<ScanObj<st, true>>(b, kScanObj + st, b.n_gm, s, h);
-    scatter<st>(b, s, h);
-}
-
 // device-to-device copies of 4-byte words (job blockIdx.y), 16 bytes at a
 // time where both buffers are 16-byte aligned
 __global__ void __launch_bounds__(256) k_copy_words(CopyJobs j) {
@@ -3253,7 +3222,12 @@ void launch_tc(const BatchDev& b, cudaStream_t s, Hooks* h) {
         const unsigned gconn = grid_for(b.n_gm, 256, b.n_sm * 32);
         k_conn_sum<false><<<gconn, 256, 0, s>>>(take(b, h), kTP, -1, false);
         if (b.flags & kFlagSGLayers) {
-            enum_and_group<TCTPStage, ScanTcTrial>(b, s, h);
+            scan<ScanTcTrial>(b, kScanCand + kTC, objects_about(b, b.cand_cap[kTC]), s, h);
+            mark(h, kStampEnum + kTC);
+            k_tctp_trial<<<b.n_sm * enum_grid(b, kTC), kEnumThreads, 0, s>>>(take(b, h));
+            mark(h, kStampEnumEnd + kTC);
+            scan<ScanObj<kTC, true>>(b, kScanObj + kTC, b.n_gm, s, h);
+            scatter<kTC>(b, s, h);
             return;
         }
         ClearJobs j{};
