@@ -384,14 +384,15 @@ int64_t sdlg_last_launches(const sdlg_ctx* ctx);
  * and forbid allocation afterwards, and plugins whose host owns the
  * allocator.  Inputs (n_hits hits: x, y, z, idx, detid) and outputs are the
  * caller's DEVICE buffers; the stage's working memory is a fixed array inside
- * the library (18,875,496 bytes, about 18 MiB, held on every GPU that loads
+ * the library (17,302,376 bytes, about 16.5 MiB, held on every GPU that loads
  * the library until the process exits).  Results: d_pairs receives up to
  * pair_cap (lower idx, upper idx) pairs (the first pair_cap when there are
  * more), *d_count the number of mini-doublets (or, if the array's capacity
  * overflowed, the number needed)
  * and *d_status the device status word (0 = clean; bit 0 = more than
  * SDLG_STATIC_MAX_MINI_DOUBLETS mini-doublets, nothing written; bit 8 = hits
- * in modules the geometry does not list, which are skipped).  Asynchronous on
+ * in modules the geometry does not list, which are skipped; bit 12 = a wait
+ * inside a prefix sum gave up, nothing written).  Asynchronous on
  * `stream` (NULL: the context's stream); the geometry must be loaded.
  * Limits: n_hits <= SDLG_STATIC_MAX_HITS and at most SDLG_STATIC_MAX_MODULES
  * modules, else SDLG_ERR_CAPACITY.  The first call on a device looks up the

@@ -27,29 +27,28 @@ using namespace sdlg;
 
 namespace {
 
-// Limits of one call; the array size follows from them (kBytes = 18,875,496
-// bytes, about 18 MiB, held on every GPU that loads this library until the
+// Limits of one call; the array size follows from them (kBytes = 17,302,376
+// bytes, about 16.5 MiB, held on every GPU that loads this library until the
 // process exits).
 constexpr int64_t kMaxHits = SDLG_STATIC_MAX_HITS;
 constexpr int64_t kMaxModules = SDLG_STATIC_MAX_MODULES;
 constexpr int64_t kMaxMD = SDLG_STATIC_MAX_MINI_DOUBLETS;
 
 // Layout of the array, in 8-byte words.
-constexpr int64_t kSmall = 0;                                   // n_hit, (free), n_rec[5], (free), task_size
+constexpr int64_t kSmall = 0;                                   // n_hit, 1 unused, n_rec[5], 1 unused, task_size
 constexpr int64_t kEvOff = 16;                                  // ev_off[2]
 constexpr int64_t kModHit = kEvOff + 2;                         // kMaxModules + 1
 constexpr int64_t kCandMD = kModHit + kMaxModules + 1;          // kMaxModules + 1
 constexpr int64_t kModCnt = kCandMD + kMaxModules + 1;          // kMaxModules + 1
-constexpr int64_t kSpare = kModCnt + kMaxModules + 1;           // 32 (free)
-constexpr int64_t kWords64 = (kSpare + 32 + 31) / 32 * 32;  // 256-byte multiple: the 4-byte regions start aligned
+constexpr int64_t kWords64 = (kModCnt + kMaxModules + 1 + 31) / 32 * 32;  // 256-byte multiple: the 4-byte regions start aligned
 // 4-byte regions follow the 8-byte ones
-constexpr int64_t kHitArrays = 18;                              // hit_gm, hit_rank, hit_perm, 12 sorted arrays, 3 (free)
+constexpr int64_t kHitArrays = 15;                              // hit_gm, hit_rank, hit_perm, 12 sorted arrays
 constexpr int64_t kObjWords = 3 + 4;                            // i, j, g, f[4]
 constexpr int64_t kRecWords = 4 + 4;                            // i, j, g, rank, f[4]
 constexpr int64_t kWords32Raw = kHitArrays * kMaxHits + (kObjWords + kRecWords) * kMaxMD + 110 + 1;
 constexpr int64_t kWords32 = (kWords32Raw + 63) / 64 * 64;  // 256-byte multiple: the 8-byte tail starts aligned
 constexpr int64_t kBytes = kWords64 * 8 + kWords32 * 4 + 8 * (5 + 8);
-static_assert(kBytes == 18875496, "the documented size of the fixed array (include/sdl_gpu.h)");
+static_assert(kBytes == 17302376, "the documented size of the fixed array (include/sdl_gpu.h)");
 
 static __device__ __align__(256) unsigned char g_scratch[kBytes];
 
