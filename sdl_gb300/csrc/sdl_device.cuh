@@ -652,11 +652,14 @@ __device__ __forceinline__ bool md_endcap(const P3& lo, const P3& up, float pixA
 // md_endcap certainly reject; the second pass runs the whole algorithm on what
 // is left.  The cuts that need no direction are taken as they are; a direction
 // difference is judged by its sine, the cross product of the two points over
-// their lengths (never larger than the angle), which single precision gives
-// within 4e-7 with the coordinates' difference as one factor.  The thresholds
-// are widened by 1e-5 and 1e-5 of themselves, for this and for the exact
-// code's roundings (its angle is within 6e-7).  Values that are not finite
-// fail only the cuts taken as they are.
+// their lengths (never larger than the angle).  With one point's coordinates
+// and their difference to the other's as factors the product is within
+// 3 * 2^-24 |a| |b - a| of the exact one, so over |a| |b| within 1.8e-7 (1 +
+// |a| / |b|).  The thresholds are widened by 1e-5 and 1e-5 of themselves, for
+// this and for the exact code's roundings (its angle is within 6e-7), and |b|
+// is taken as 0.03 |a| where it is less, which makes up for the ratio: its
+// widening is then 3e-7 |a|^2 or more, the error at most 1.9e-7 |a|^2.  Values
+// that are not finite fail only the cuts taken as they are.
 __device__ __forceinline__ bool md_first_cuts(const P3& lo, const P3& up, float pixAsin, const ModDev& lm, const float* sh) {
     const bool barrel = lm.subdet == kBarrel, ps = lm.type == kPS, pixLower = lm.ltype == kPixel;
     float dz = lo.z - up.z;
@@ -685,16 +688,18 @@ __device__ __forceinline__ bool md_first_cuts(const P3& lo, const P3& up, float 
     if (barrel) {
         const float t = shift ? lm.tilt * pixAsin : 0.f;
         const float cut = __fmaf_rn(pixAsin + __fsqrt_rn(__fmaf_rn(t, t, v)), 1.f + 1e-5f, 1e-5f);
-        if (num > cut * ar * br) return false;
+        const float bw = fmaxf(br, 0.03f * ar);
+        if (num > cut * ar * bw) return false;
         // the direction from the point at smaller rt to the other against its own
-        const float n = cut * (shift ? fminf(ar, br) : ar);
+        const float n = cut * (shift ? fminf(ar, bw) : ar);
         return !(num * num > n * n * __fmaf_rn(dx, dx, dy * dy));
     }
     const float s = __fdividef(num, ar * br);
-    if (!(s <= 0.5f) || __fmaf_rn(ax, bx, ay * by) < 0.f) return true;  // (an angle above 30 degrees: asin(s) <= 1.05 s below)
+    // (up to 30 degrees asin(s) <= 1.05 s; up to a ratio of 4 the sine is within 9e-7)
+    if (!(s <= 0.5f) || __fmaf_rn(ax, bx, ay * by) < 0.f || 4.f * br < ar) return true;
     if (ps) dz = (pixLower ? lo.z : up.z) - sh[2];
     const float adz = fabsf(dz);
-    const float lum = floorf(__fdividef(__fmaf_rn(1.05f, s, 1e-6f) * kDeltaZLum, adz) * (1.f + 1e-5f));
+    const float lum = floorf(__fdividef(__fmaf_rn(1.05f, s, 2e-6f) * kDeltaZLum, adz) * (1.f + 1e-5f));
     const float cut = __fmaf_rn(pixAsin + __fsqrt_rn(__fmaf_rn(lum, lum, v)), 1.f + 1e-5f, 1e-5f);
     if (s > cut) return false;
     const float f = __fdividef(adz, fabsf(lo.z)), g = __fdividef(1.f + f, f);
