@@ -925,6 +925,7 @@ __device__ __forceinline__ bool sg_later_cuts(const MDLite& I, const MDLite& O) 
         q = atan2f(y, x);
         eq = __fmaf_rn(5e-6f * R, rdr, 4e-6f);
         cut = ib && layer + 1u == (O.fl & kMdLayer);  // (another layer pair's cut is left to the second pass)
+        if (!cut && fabsf(q) + eq > 3.14f) return true;  // (the exact code's angle may have the other sign)
     } else {
         const float f = __fdividef(O.z - I.z, I.z), g = __fdividef(1.f + f, f);
         q = d * g;
