@@ -352,6 +352,15 @@ int sdlg_math_check(sdlg_ctx* ctx, int fn, int exhaustive, uint64_t start, int64
 int sdlg_libm_eval(sdlg_ctx* ctx, int fn, uint32_t start_bits, int64_t n, float* out);
 int sdlg_libm_stats(int fn, uint64_t* out3);
 
+/* Self-check of the first passes over the mini-doublet and segment candidates
+ * (no counterpart in the reference): after a run through the segment stage,
+ * every candidate of both stages is judged by the single-precision cuts that
+ * the stage applies first and by the whole algorithm.  out8: for the
+ * mini-doublets, then for the segments, the candidates, those the first pass
+ * rejects, those among them that the algorithm accepts (must be 0), and those
+ * that the algorithm accepts. */
+int sdlg_first_cuts_check(sdlg_ctx* ctx, uint64_t* out8);
+
 /* Self-check of the tracklet enumeration's single-precision decisions (no
  * counterpart in the reference): after a run through the tracklet stage,
  * every tracklet candidate of the batch is judged both by the fast decisions

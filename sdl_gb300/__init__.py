@@ -88,6 +88,7 @@ def lib():
         L.sdlg_last_tl_list_counts.argtypes = [vp, vp]
         L.sdlg_math_check.argtypes = [vp, i32, i32, ctypes.c_uint64, i64, ctypes.c_uint64, vp]
         L.sdlg_tl_phase_a_check.argtypes = [vp, vp]
+        L.sdlg_first_cuts_check.argtypes = [vp, vp]
         L.sdlg_autotune.argtypes = [vp, i32, i32, vp]
         L.sdlg_last_launches.argtypes = [vp]
         L.sdlg_last_launches.restype = i64
@@ -587,6 +588,15 @@ class Chain:
                                        out.ctypes.data))
         return {"answered": int(out[0]), "mismatches": int(out[1]),
                 "first": [int(v) for v in out[3:8]] if out[2] else None}
+
+    def first_cuts_check(self) -> dict:
+        """Self-check of the first passes over the last run's mini-doublet and
+        segment candidates: how many they rejected, how many of those the
+        whole algorithm accepts (0), and how many it accepts."""
+        out = np.zeros(8, dtype=np.uint64)
+        self._ck(lib().sdlg_first_cuts_check(self.h, out.ctypes.data))
+        keys = ("candidates", "rejected", "violations", "accepted")
+        return {s: dict(zip(keys, (int(v) for v in out[4 * k:4 * k + 4]))) for k, s in enumerate(("MD", "SG"))}
 
     def tl_phase_a_check(self) -> dict:
         """Self-check of the tracklet enumeration's single-precision decisions

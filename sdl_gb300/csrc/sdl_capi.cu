@@ -1638,6 +1638,25 @@ int sdlg_get_tracklet_vars(sdlg_ctx* ctx, int64_t event, float* out, int64_t cap
     return SDLG_OK;
 }
 
+int sdlg_first_cuts_check(sdlg_ctx* ctx, uint64_t* out8) {
+    if (!ctx || !out8) return SDLG_ERR_ARG;
+    if (!ctx->ran || !ctx->buffers_ok || ctx->last_stop < kSG)
+        return fail(ctx, SDLG_ERR_ARG, "run the chain through the segment stage first");
+    cudaSetDevice(ctx->device);
+    unsigned long long* d = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&d, 8 * sizeof(unsigned long long), ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, SDLG_ERR_CUDA, "cudaMallocAsync: %s", cudaGetErrorString(e));
+    CK(cudaMemsetAsync(d, 0, 8 * sizeof(unsigned long long), ctx->stream));
+    launch_first_cuts_check(ctx->b, d, ctx->stream);
+    CK(cudaGetLastError());
+    unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    CK(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaFreeAsync(d, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    for (int k = 0; k < 8; ++k) out8[k] = h[k];
+    return SDLG_OK;
+}
+
 int sdlg_tl_phase_a_check(sdlg_ctx* ctx, uint64_t* out4) {
     if (!ctx || !out4) return SDLG_ERR_ARG;
     if (!ctx->ran || ctx->last_stop < kTL) return fail(ctx, SDLG_ERR_ARG, "run the chain through the tracklet stage first");

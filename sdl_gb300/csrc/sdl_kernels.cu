@@ -567,15 +567,19 @@ __device__ __forceinline__ bool sg_pair(const BatchDev& b, int a, int bmd, bool 
 
 // segment candidates along the module map (Event.cc:445-522): candidate q of
 // inner MD a is an MD of a connected module, in connection-list order
-__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int a, int64_t q) {
-    const int g1 = OG(b, kMD, a);
-    if (AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap) return AT(b.olist, AT(b.toff, g1, NG1(b)) + q, b.olist_cap);  // k_sg_lists
+__device__ __forceinline__ int sg_outer_conn(const BatchDev& b, int a, int64_t q) {
     const int n_mod = b.geo.n_mod;
+    const int g1 = OG(b, kMD, a);
     const int ev = ev_of(b, g1), m1 = g1 - ev * n_mod;
     int pref;
     const int k = conn_entry(b, ev, m1, q, pref);
     const int g2 = ev * n_mod + AT(b.geo.conn_idx, k, NC(b));
     return (int)(OFF(b, kMD, g2) + (q - pref));
+}
+__device__ __forceinline__ int sg_outer_md(const BatchDev& b, int a, int64_t q) {
+    const int g1 = OG(b, kMD, a);
+    if (AT(b.toff, b.n_gm, NG1(b)) <= b.olist_cap) return AT(b.olist, AT(b.toff, g1, NG1(b)) + q, b.olist_cap);  // k_sg_lists
+    return sg_outer_conn(b, a, q);
 }
 
 // ------------------------------------------------------------------ layer pairs
@@ -2186,6 +2190,61 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
     }
 }
 
+// Self-check of the first passes over the mini-doublet and segment candidates
+// (md_first_cuts; sg_first_cuts and sg_later_cuts): every candidate of the last
+// run judged by them and by the whole algorithm.  out[0..3] mini-doublets,
+// out[4..7] segments: candidates, rejected by the first pass, of those accepted
+// by the algorithm (must be 0), accepted by the algorithm.
+__device__ __forceinline__ void first_cuts_count(unsigned long long* out, unsigned long long (&n)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        for (int o = 16; o; o >>= 1) n[k] += __shfl_down_sync(0xffffffffu, n[k], o);
+        if ((threadIdx.x & 31) == 0 && n[k]) atomicAdd(out + k, n[k]);
+    }
+}
+__global__ void k_md_first_check(BatchDev b, unsigned long long* out) {
+    const int64_t* off = b.cand[kMD];
+    const int64_t offlim = b.cand_cap[kMD] + 1;
+    const int64_t total = b.n_gm > 0 ? AT(off, b.n_gm, offlim) : 0;
+    unsigned long long n[4] = {0ull, 0ull, 0ull, 0ull};
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (int64_t)gridDim.x * blockDim.x) {
+        const int g = find_obj(b, off, offlim, 0, b.n_gm - 1, c);
+        int2 e;
+        if (!md_candidate(b, g, c - AT(off, g, offlim), e)) continue;
+        const ModDev& lm = MOD(b, mod_of(b, g));
+        const MDCand d = md_cand(b, lm, e);
+        const bool first = md_first_cuts(d.L, d.U, d.pixAsin, lm, d.sh);
+        MDVals v;
+        const bool pass = lm.subdet == kBarrel ? md_barrel(d.L, d.U, d.pixAsin, lm, d.sh, v) : md_endcap(d.L, d.U, d.pixAsin, lm, d.sh, v);
+        n[0] += 1;
+        n[1] += !first;
+        n[2] += !first && pass;
+        n[3] += pass;
+    }
+    first_cuts_count(out, n);
+}
+__global__ void k_sg_first_check(BatchDev b, unsigned long long* out) {
+    const int64_t nobj = n_objects(b, kMD);
+    const int64_t* off = b.cand[kSG];
+    const int64_t offlim = b.cand_cap[kSG] + 1;
+    const int64_t total = nobj > 0 ? AT(off, nobj, offlim) : 0;
+    unsigned long long n[4] = {0ull, 0ull, 0ull, 0ull};
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += (int64_t)gridDim.x * blockDim.x) {
+        const int a = find_obj(b, off, offlim, 0, (int)nobj - 1, c);
+        const int64_t q = c - AT(off, a, offlim);
+        const int bmd = b.seg_layers ? layer_md<true>(b, layer_row<true>(b, a), (int)q) : sg_outer_conn(b, a, q);
+        const MDLite I = md_lite(b, a), O = md_lite(b, bmd);
+        const bool first = sg_first_cuts(I, O) && sg_later_cuts(I, O);
+        float f6[6];
+        const bool pass = sg_pair(b, a, bmd, !b.seg_layers || sg_connected(b, a, bmd), f6);
+        n[0] += 1;
+        n[1] += !first;
+        n[2] += !first && pass;
+        n[3] += pass;
+    }
+    first_cuts_count(out, n);
+}
+
 // per-module object counts of a stage -> offsets, and the layer counters
 template <int st, bool kCounters>
 struct ScanObj : ScanOp {
@@ -3409,6 +3468,13 @@ static void tl_cand_space(const BatchDev& b, cudaStream_t s) {
 void launch_tl_collect(const BatchDev& b, const MlpCollect& c, cudaStream_t s) {
     tl_cand_space(b, s);
     k_tl_collect<<<b.n_sm * 8, 256, 0, s>>>(b, c);
+}
+
+void launch_first_cuts_check(const BatchDev& b, unsigned long long* out, cudaStream_t s) {
+    // (the connection sums are those of a later stage)
+    if (!b.seg_layers) k_conn_sum<false><<<grid_for(b.n_gm, 256, b.n_sm * 32), 256, 0, s>>>(b, kMD, -1, false);
+    k_md_first_check<<<b.n_sm * 8, 256, 0, s>>>(b, out);
+    k_sg_first_check<<<b.n_sm * 8, 256, 0, s>>>(b, out + 4);
 }
 
 void launch_tl_b2q_check(const BatchDev& b, unsigned long long* out, cudaStream_t s) {

@@ -256,6 +256,8 @@ void launch_tl_collect(const BatchDev& b, const MlpCollect& c, cudaStream_t s);
 // self-check of the float-float fast paths (out[8]: see k_math_check)
 void launch_math_check(int fn, int exhaustive, unsigned long long start, long long n, unsigned long long seed,
                        unsigned long long* out, int n_sm, cudaStream_t s);
+// self-check of the mini-doublets' and segments' first passes (out[8]: see k_md_first_check)
+void launch_first_cuts_check(const BatchDev& b, unsigned long long* out, cudaStream_t s);
 // self-check of phase A's single-precision decision (out[4]: see k_tl_quick_check)
 void launch_tl_b2q_check(const BatchDev& b, unsigned long long* out, cudaStream_t s);
 void launch_tl_quick_check(const BatchDev& b, unsigned long long* out, cudaStream_t s);
