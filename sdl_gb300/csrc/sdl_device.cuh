@@ -1483,6 +1483,28 @@ __device__ __forceinline__ int tl_phaseA_quick(const TLRow& R, const TLOut& T, f
     return kAlgoNone;
 }
 
+// The layer pairs' candidates ahead of their rows: true when BBBB's first
+// window or the phi cut certainly fails, by the values and margins of
+// tl_phaseA_quick, from the few fields these need.
+__device__ __forceinline__ bool tl_layer_out(const float* __restrict__ pack, int64_t s, const SGOuter& T) {
+    const float4* q = reinterpret_cast<const float4*>(pack + s * PK_N);
+    const float4 w0 = __ldg(q);  // lx, ly, lz, lrt
+    const uint32_t fl = __float_as_uint(__ldg(pack + s * PK_N + PK_FLAGS));
+    if ((fl & (F_LO_B | F_UP_B)) != (F_LO_B | F_UP_B) || !(T.flags & F_LO_B) || !(T.flags & (F_UP_B | F_UP_E))) return false;
+    const float rt = w0.w, z = w0.z;
+    const float zp = ((fl & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch) + ((T.flags & F_LO_PS) ? kPixelPSZpitch : kStrip2SZpitch);
+    const float t = __fmaf_rn(T.lrt, __fdividef(1.f, rt), -1.f);
+    const float sHi = z < 0.f ? 1.f : T.ltd, sLo = z > 0.f ? 1.f : T.ltd;
+    CutsQuick c;
+    c.within(inside(T.lz, __fmaf_rn((z - kDeltaZLum) * sLo, t, z - zp), __fmaf_rn((z + kDeltaZLum) * sHi, t, z + zp)),
+             kWindowMargin * __fmaf_rn((fabsf(z) + kDeltaZLum) * fmaxf(1.f, fabsf(T.ltd)), fabsf(t) + 2.f, fabsf(z) + zp));
+    if (c.rej) return true;
+    const float sq = (0.015f * 3.f / kPtCut * 4.f) * __ldg(pack + s * PK_N + PK_S2);
+    float cut;
+    phi_cut_quick(c, T.uphi - __ldg(pack + s * PK_N + PK_UPHI), T.la1, sdl_muls_quick(T.lrt - rt, sq), T.pvoff * T.pvoff, cut);
+    return c.rej;
+}
+
 // Phase B1 with the approximate (or exact) phi-cut width: 1 passes, 0 fails,
 // -1 left to tl_phaseB1_sgv.  txy: the outer segment's (lx, ly, ux, uy).
 __device__ __forceinline__ int tl_phaseB1_quick(int algo, const TLRow& R, float4 txy, float cut) {

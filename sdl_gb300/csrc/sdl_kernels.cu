@@ -1214,7 +1214,10 @@ __device__ __forceinline__ void passbuf_add(const BatchDev& b, PassBuf& pb, int 
 // survivors, marking those through phase B1 already; k_tl_b1 and k_tl_b2 run
 // the two parts of phase B on compacted lists and append the tracklets.  The
 // survivor list shares the pre-filter's capacity and overflow handling (its
-// count is n_kept).
+// count is n_kept).  A layer pair's candidates mostly fail the first window or
+// the phi cut, so these are judged ahead of the row (tl_layer_out; one PU 200
+// event, module-map segments: 3,425 us with the row of every candidate, 2,719
+// so).
 __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
     __shared__ int4 pbuf[kEnumThreads / kWarp][kPassBuf];
     if (halted(b)) return;
@@ -1252,9 +1255,11 @@ __global__ void __launch_bounds__(kEnumThreads) k_tl_enum_a(BatchDev b) {
                 (void)IX(s, b.obj[kSG].cap);
                 (void)IX(tt, b.obj[kSG].cap);
                 const int64_t C = b.obj[kSG].cap;
+                const SGOuter T = load_sgo(b.sgouter, C, tt);
                 bool exact;
-                algo = tl_ab1_decide<true>(tl_row(load_sgv(b.sgpack, s)), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt),
-                                     b.sgpack, s, tt, b1, exact);
+                if (lay != 1 || !tl_layer_out(b.sgpack, s, T))
+                    algo = tl_ab1_decide<true>(tl_row(load_sgv(b.sgpack, s)), tl_out(T), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt,
+                                               b1, exact);
             }
             passbuf_add(b, pb, algo, s, tt, b1);
         }
@@ -2146,7 +2151,7 @@ __global__ void k_tl_collect(BatchDev b, MlpCollect col) {
 }
 
 // Self-check of the enumeration's single-precision decisions (tl_ab1_decide:
-// phase A, then phase B1 for its survivors) over the tracklet candidates of
+// phase A, then phase B1 for its survivors; tl_layer_out ahead of it) over the tracklet candidates of
 // the last run, against the exact phase A and B1 on the packed records:
 // out[0] candidates, out[1] settled by the approximations alone, out[2] that
 // needed an exact evaluation, out[3] settled wrongly (0 when the margins
@@ -2169,10 +2174,11 @@ __global__ void k_tl_quick_check(BatchDev b, unsigned long long* out) {
         const int tt = tl_outer_of(b, lay, s, c - AT(off, s, offlim));
         const SGV S = load_sgv(b.sgpack, s), Tv = load_sgv(b.sgpack, tt);
         const int64_t C = b.obj[kSG].cap;
-        int b1;
-        bool exact;
-        const int q = tl_ab1_decide<false>(tl_row(S), tl_out(load_sgo(b.sgouter, C, tt)), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt, b1,
-                                    exact);
+        const SGOuter T = load_sgo(b.sgouter, C, tt);
+        int b1 = 0, q = kAlgoNone;
+        bool exact = false;
+        if (lay != 1 || !tl_layer_out(b.sgpack, s, T))
+            q = tl_ab1_decide<false>(tl_row(S), tl_out(T), load_sgo_xy(b.sgouter, C, tt), b.sgpack, s, tt, b1, exact);
         float cut, muls;
         const int e = tl_phaseA(S, Tv, cut, muls);
         const bool eb1 = e != kAlgoNone && tl_phaseB1_sgv(e, S, Tv, cut);
