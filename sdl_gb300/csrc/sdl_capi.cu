@@ -270,7 +270,7 @@ int scratch_for(sdlg_ctx* ctx, size_t bytes, void** p) {
 }
 
 // The first scratch buffer for the samples of one call.  What the call makes it
-// grow to is kept up to kSampleScratch (1.1 million samples; three allocations
+// grow to is kept up to kSampleScratch (950,000 samples; three allocations
 // and their frees took 0.2 ms a call) and given back otherwise, at the end of
 // the call whatever its outcome.
 constexpr int64_t kSampleScratch = (int64_t)64 << 20;
